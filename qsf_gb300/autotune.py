@@ -1,13 +1,11 @@
-"""Autotuner of the pass kernels: the shape of the row / axis passes per line length
-(points per block and threads per block), and the radix plan (points per thread) of the
-one-CTA 1D line kernel per length.
+"""Autotuner of the pass kernels: the points per thread of the row passes per line length,
+and the radix plan (points per thread) of the one-CTA 1D line kernel per length.
 
-A row / axis shape is a tile of whole lines (1024, 2048 or 4096 points per block, or
-one line when lines are longer) and a thread count; their ratio, the points each thread
-carries per pass, sets the radix plan (16: radix 16, 128 registers; 8: radix 8).
-Smaller tiles give small grids more blocks (a 256^2 grid is 16 blocks of 4096 points
-on 152 SMs).  For each candidate shape the library is built with every line length
-forced to it (`QSF_TILE`, `QSF_ROW_THREADS`, in qsf_gb300/_build/tune_<tile>_<threads>/);
+A row shape is written as points x threads (4096 x 256: 16 points per thread, radix-16
+plans, 128 registers; 4096 x 512: 8 points per thread, radix-8 plans, 80 registers and
+half the code per pass, twice the warps); the ratio selects the line plan
+(qsf_lines.cuh).  For each candidate the library is built with every line length forced
+to it (`QSF_TILE`, `QSF_ROW_THREADS`, in qsf_gb300/_build/tune_<points>_<threads>/);
 each tuning workload's fused step is timed as a user runs it (`profile_step --timed`:
 one call of K graph-replayed steps after a warm-up call) in a subprocess that loads that
 build; per line length the shape with the least summed step time over the workloads of
@@ -32,18 +30,16 @@ import sys
 from . import build as B
 from .profile_step import WORKLOADS
 
-# (points per block, threads per block) of the row / axis passes.  The committed table
-# comes from the 4096-point tiles: smaller tiles (--shapes all) make small grids faster
-# alone (2D 512^2 0.0725 -> 0.0499 ms per step with 1024 x 128) but the 256-solve batch
-# slower (1.25e10 -> 1.19e10 grid-pt-steps/s), where the solves already fill the GPU.
+# points x threads of the row passes (their ratio is the points per thread)
 CANDIDATES = ((4096, 256), (4096, 512))
-ALL_CANDIDATES = ((4096, 256), (4096, 512), (2048, 128), (2048, 256), (1024, 128))
+ALL_CANDIDATES = CANDIDATES
 DEFAULT_SHAPE = (4096, 256)
 LINE_CANDIDATES = (4, 8, 16)
 LINE_WORKLOADS = [("1d1024", 400), ("1d1536", 400), ("1d2048", 400), ("1d3072", 400), ("1d4096", 400)]
 # (workload of profile_step, steps per timed call)
-TUNE_WORKLOADS = [("2d256", 400), ("2d320", 400), ("2d384", 400), ("2d512", 400), ("2d640", 300), ("2d768", 300),
-                  ("2d1024", 300), ("2d2048", 100), ("2d4096", 30), ("3d128", 100), ("3d256", 30)]
+TUNE_WORKLOADS = [("2d64", 400), ("2d128", 400), ("2d192", 400), ("2d256", 400), ("2d320", 400), ("2d384", 400), ("2d512", 400), ("2d640", 300), ("2d768", 300),
+                  ("2d1024", 300), ("2d1280", 200),
+                  ("2d1536", 100), ("2d2048", 100), ("2d4096", 30), ("3d128", 100), ("3d256", 30)]
 HEADER = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc", "qsf_tuning.h")
 
 
@@ -117,15 +113,14 @@ def header_text(choice: dict, times: dict, lchoice: dict = None, ltimes: dict = 
         cells = "  ".join(f"{p}: {ltimes[(w, p)]:.4f}" for p in LINE_CANDIDATES if ltimes and (w, p) in ltimes)
         if cells:
             lrows.append(f"//   {w:7s} ms/step  {cells}")
-    return f"""// qsf_tuning.h -- pass kernel shapes per line length: points and threads per block of
-// the row / axis passes, and the radix plan of the one-CTA 1D line kernel.
+    return f"""// qsf_tuning.h -- pass kernel shapes per line length: the points per thread of the row
+// passes, and the radix plan of the one-CTA 1D line kernel.
 //
 // Written by the autotuner (qsf_gb300/autotune.py) from step times measured on a GB300:
 //   python -m qsf_gb300.autotune --write
-// Row / axis shapes: points per block x threads per block (16 points per thread:
-// radix-16 plans, 128 registers; 8: radix-8 plans); lengths not listed take
-// {DEFAULT_SHAPE[0]}x{DEFAULT_SHAPE[1]}.  Chosen among {", ".join(f"{c[0]}x{c[1]}" for c in CANDIDATES)}; smaller tiles, timed
-// beside them, speed up small grids run alone but slow the batched form down.
+// Row passes: points x threads, whose ratio is the points per thread and selects the
+// line plan (16: radix-16 plans, 128 registers; 8: radix-8 plans); lengths not listed
+// take {DEFAULT_SHAPE[0]}x{DEFAULT_SHAPE[1]}.
 // Measured (one call of graph-replayed steps per workload, ms per step):
 {chr(10).join(rows)}
 #pragma once
@@ -181,13 +176,10 @@ def main():
     ap.add_argument("--repeat", type=int, default=2)
     ap.add_argument("--write", action="store_true", help="rewrite qsf_gb300/csrc/qsf_tuning.h")
     ap.add_argument("--only", choices=["rows", "lines"], default=None)
-    ap.add_argument("--shapes", choices=["tiles4096", "all"], default="tiles4096",
-                    help="row / axis candidates: 4096-point tiles (the committed table) or all shapes")
     args = ap.parse_args()
-    cands = CANDIDATES if args.shapes == "tiles4096" else ALL_CANDIDATES
     times, ltimes = {}, {}
     if args.only != "lines":
-        for c in cands:
+        for c in CANDIDATES:
             lib_path = B.build(defines=[f"QSF_TILE={c[0]}", f"QSF_ROW_THREADS={c[1]}"], tag=f"tune_{c[0]}_{c[1]}")
             for w, steps in TUNE_WORKLOADS:
                 times[(w, c)] = time_workload(lib_path, w, steps, args.repeat)
@@ -203,7 +195,7 @@ def main():
                 print(json.dumps({"workload": w, "points_per_thread": p, "ms_per_step": ltimes[(w, p)]}), flush=True)
     if not times:
         times = committed_row_times()
-    choice = choose({k: v for k, v in times.items() if k[1] in cands})
+    choice = choose({k: v for k, v in times.items() if k[1] in CANDIDATES})
     if not ltimes:
         ltimes = committed_line_times()
     lchoice = choose_lines(ltimes) if ltimes else None

@@ -60,7 +60,7 @@ std::vector<KernelSet>& kernel_table();
 // kernel launch geometry
 constexpr int kMaxLine1D = 16384;       // 1D line in shared memory (one CTA up to 8192, a cluster pair above)
 constexpr int kMaxFluxBlocks = 512;  // blocks of the flux-term sums (256 terms each)
-constexpr int kMaxTile = 4096;          // points per block in row / axis passes
+constexpr int kMaxAxis = 4096;          // points per axis in 2D and 3D
 
 }  // namespace
 
@@ -105,17 +105,12 @@ int init_kernel_table() {
     QSF_CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     return QSF_OK;
   };
-  // dynamic shared memory actually requested: tiles of kMaxTile points (row / axis
-  // passes), lines of up to 16 * kLineThreads points (line kernel, plain row FFT)
-  const int tile = kMaxTile * (int)sizeof(double2);
-  const int line = 16 * kLineThreads * (int)sizeof(double2);
   for (const KernelSet& k : t) {
     int rc;
-    if ((rc = lim((const void*)k.row_open, tile)) || (rc = lim((const void*)k.row_close, tile)) ||
-        (rc = lim((const void*)k.axis_fwd, tile)) || (rc = lim((const void*)k.axis_inv, tile)) ||
-        (rc = lim((const void*)k.axis_fpi, tile)) || (rc = lim((const void*)k.axis_ekin, tile)) ||
-        (rc = lim((const void*)k.axis_fft_f, tile)) || (rc = lim((const void*)k.axis_fft_b, tile)) ||
-        (rc = lim((const void*)k.row_fft_f, line)) || (rc = lim((const void*)k.row_fft_b, line)) ||
+    if ((rc = lim((const void*)k.row_open, k.row_smem)) || (rc = lim((const void*)k.row_close, k.row_smem)) ||
+        (rc = lim((const void*)k.row_ekin, k.row_smem)) || (rc = lim((const void*)k.axis_one, k.col_smem)) ||
+        (rc = lim((const void*)k.axis_fpi, k.col_smem)) || (rc = lim((const void*)k.axis_ekin, k.col_smem)) ||
+        (rc = lim((const void*)k.axis_fft, k.col_smem)) || (rc = lim((const void*)k.row_fft, k.fft_smem)) ||
         (rc = lim((const void*)k.line_step, k.n / k.line_ctas * (int)sizeof(double2))))
       return rc;
   }
@@ -175,8 +170,9 @@ EncodeTiledFn encode_tiled() {
 }
 
 // Tensor maps of psi for the strided-axis passes of axes 0 .. dim-2: psi as 64-bit
-// words, dims {2 * stride, n, outer}, box {2 * tile columns, tma_box_rows(n), 1} (the
-// boxes the pass's load_aligned issues); left null (cp.async loads) without an encoder.
+// words, dims {2 * stride, n, outer}, box {2 * block columns, tma_box_rows(n), 1}, each
+// box row swizzled over its own length (column_swz); left null (plain copies) without an
+// encoder.
 int make_tensor_maps(qsf_grid* g) {
   GridDev& G = g->G;
   for (int ax = 0; ax < kMaxDim; ++ax) G.tmap[ax] = nullptr;
@@ -188,13 +184,18 @@ int make_tensor_maps(qsf_grid* g) {
     const long long inner = a.stride, outer = G.m / ((long long)a.n * inner);
     const cuuint64_t dims[3] = {(cuuint64_t)(2 * inner), (cuuint64_t)a.n, (cuuint64_t)outer};
     const cuuint64_t strides[2] = {(cuuint64_t)(16 * inner), (cuuint64_t)(16 * inner * a.n)};
-    const cuuint32_t box[3] = {(cuuint32_t)(2 * g->ax_C[ax]), (cuuint32_t)tma_box_rows(a.n), 1};
+    const int C = g->ks->col_lines;
+    const CUtensorMapSwizzle swz = C == 8   ? CU_TENSOR_MAP_SWIZZLE_128B
+                                   : C == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                   : C == 2 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                            : CU_TENSOR_MAP_SWIZZLE_NONE;
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * C), (cuuint32_t)tma_box_rows(a.n), 1};
     const cuuint32_t elem[3] = {1, 1, 1};
     alignas(64) CUtensorMap map;
     if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, G.psi, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
+           swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
         CUDA_SUCCESS)
-      continue;  // this axis keeps cp.async loads
+      continue;  // this axis keeps plain copies
     // on the grid's stream and waited for: a pageable copy on another stream may still
     // be in flight when it returns, unordered with the grid's later work
     QSF_CU(cudaMemcpyAsync(g->tmaps + 128 * ax, &map, sizeof(map), cudaMemcpyHostToDevice, g->stream));
@@ -205,6 +206,21 @@ int make_tensor_maps(qsf_grid* g) {
 }
 
 }  // namespace
+
+// One transform of axis ax of the array G.psi with the kernels K of that axis' length.
+void qsf::launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd, double sc, cudaStream_t st) {
+  GridDev V = G;
+  for (int k = 0; k < kMaxDim; ++k) V.tmap[k] = nullptr;  // G.psi need not be the mapped array
+  const long long n = G.ax[ax].n, lines = G.m / n;
+  if (ax == G.dim - 1) {
+    const int blocks = K.fft_ctas > 1 ? K.fft_ctas : (int)((lines + K.fft_lines - 1) / K.fft_lines);
+    K.row_fft<<<blocks, K.fft_threads, K.fft_smem, st>>>(V, fwd, sc);
+  } else {
+    const long long inner = G.ax[ax].stride, outer = lines / inner;
+    K.axis_fft<<<(unsigned)(outer * ((inner + K.col_lines - 1) / K.col_lines)), K.col_threads, K.col_smem, st>>>(V, ax, fwd,
+                                                                                                                sc);
+  }
+}
 
 bool qsf::fused_length(int n) { return init_kernel_table() == QSF_OK && kernels_for(n) != nullptr; }
 
@@ -258,6 +274,54 @@ int qsf::shared_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf) 
   *tw = (double2*)it->second[0];
   *twx = (longlong2*)it->second[1];
   *twf = (longlong2*)it->second[2];
+  return QSF_OK;
+}
+
+// Per-pass twiddles of a length's line plans (qsf_lines.cuh): kTwVar copies each, copy r
+// scaled by 2^-r; pass p's entry [(q - 1) ns + jm] = exp(-2 pi i jm q / (ns R)) in split
+// form.  Made once per length, process and device and shared by every grid.
+int qsf::shared_line_twiddles(const KernelSet& K, const int4* out[2]) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, std::array<int4*, 2>> cache;
+  out[0] = out[1] = nullptr;
+  if (!K.plan[0]) return QSF_OK;
+  int dev = 0;
+  QSF_CU(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = cache.find({dev, K.n});
+  if (it == cache.end()) {
+    const long double twopi = 6.283185307179586476925286766559005768L;
+    std::vector<longlong2> h;
+    size_t second = 0;
+    for (int plan = 0; plan < 2; ++plan) {
+      for (int r = 0; r < kTwVar; ++r) {
+        const long double one = ldexpl(1.0L, 62 - r);
+        long long ns = K.plan[plan][0];
+        for (int p = 1; K.plan[plan][p]; ++p) {
+          const int R = K.plan[plan][p];
+          for (int q = 1; q < R; ++q)
+            for (long long jm = 0; jm < ns; ++jm) {
+              const long double ang = twopi * (long double)((jm * q) % (ns * R)) / (long double)(ns * R);
+              h.push_back(split_twiddle(make_longlong2(llroundl(cosl(ang) * one), llroundl(-sinl(ang) * one))));
+            }
+          ns *= R;
+        }
+      }
+      if (plan == 0) second = h.size();
+    }
+    int4* d = nullptr;
+    if (int rc = dev_alloc(d, h.size() + 1)) return rc;
+    cudaError_t ce = cudaMemcpy(d, h.data(), h.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    // a pageable copy may return before its transfer lands; every stream shares the table
+    if (ce == cudaSuccess) ce = cudaDeviceSynchronize();
+    if (ce != cudaSuccess) {
+      cudaFree(d);
+      return fail(QSF_ECUDA, std::string("line twiddles: ") + cudaGetErrorString(ce));
+    }
+    it = cache.emplace(std::make_pair(dev, K.n), std::array<int4*, 2>{d, d + second}).first;
+  }
+  out[0] = it->second[0];
+  out[1] = it->second[1];
   return QSF_OK;
 }
 
@@ -491,10 +555,8 @@ struct Prof {
 // Launch geometry shared by every solve of one (dim, line length) group.
 struct Geom {
   int dim = 1, n = 0, nmax = 0, gauge = 0;
-  int nrowblk = 1, row_L = 1;
-  size_t row_smem = 0;
-  int ax_blocks[3] = {0, 0, 0}, ax_C[3] = {1, 1, 1};
-  size_t ax_smem[3] = {0, 0, 0};
+  int nrowblk = 1;
+  int ax_blocks[3] = {0, 0, 0};
 };
 
 Geom geom_of(const qsf_grid* g) {
@@ -504,13 +566,7 @@ Geom geom_of(const qsf_grid* g) {
   q.nmax = g->nmax;
   q.gauge = g->G.gauge;
   q.nrowblk = g->nrowblk;
-  q.row_L = g->row_L;
-  q.row_smem = g->row_smem;
-  for (int k = 0; k < 3; ++k) {
-    q.ax_blocks[k] = g->ax_blocks[k];
-    q.ax_C[k] = g->ax_C[k];
-    q.ax_smem[k] = g->ax_smem[k];
-  }
+  for (int k = 0; k < 3; ++k) q.ax_blocks[k] = g->ax_blocks[k];
   return q;
 }
 
@@ -553,21 +609,20 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
                                                (size_t)(q.n / K.line_ctas) * sizeof(double2), st>>>(dG, dS)));
   } else {
     const dim3 gr(q.nrowblk, count);
-    if (with_open) QSF_TIMED(QSF_K_ROW_OPEN, (K.row_open<<<gr, K.row_threads, q.row_smem, st>>>(dG, dS, q.row_L)));
+    if (with_open) QSF_TIMED(QSF_K_ROW_OPEN, (K.row_open<<<gr, K.row_threads, K.row_smem, st>>>(dG, dS)));
     if (D == 3)
-      QSF_TIMED(QSF_K_AXIS_FWD,
-                (K.axis_fwd<<<dim3(q.ax_blocks[1], count), K.row_threads, q.ax_smem[1], st>>>(dG, dS, 1, q.ax_C[1])));
-    QSF_TIMED(QSF_K_AXIS_FPI,
-              (K.axis_fpi<<<dim3(q.ax_blocks[0], count), K.row_threads, q.ax_smem[0], st>>>(dG, dS, 0, q.ax_C[0])));
+      QSF_TIMED(QSF_K_AXIS_FWD, (K.axis_one<<<dim3(q.ax_blocks[1], count), K.col_threads, K.col_smem, st>>>(dG, dS, 1, 0)));
+    QSF_TIMED(QSF_K_AXIS_FPI, (K.axis_fpi<<<dim3(q.ax_blocks[0], count), K.col_threads, K.col_smem, st>>>(dG, dS, 0, 0)));
     if (D == 3)
-      QSF_TIMED(QSF_K_AXIS_INV,
-                (K.axis_inv<<<dim3(q.ax_blocks[1], count), K.row_threads, q.ax_smem[1], st>>>(dG, dS, 1, q.ax_C[1])));
+      QSF_TIMED(QSF_K_AXIS_INV, (K.axis_one<<<dim3(q.ax_blocks[1], count), K.col_threads, K.col_smem, st>>>(dG, dS, 1, 1)));
     if (wait_fin) QSF_CU(cudaStreamWaitEvent(st, ov->done, 0));
-    QSF_TIMED(QSF_K_ROW_CLOSE, (K.row_close<<<gr, K.row_threads, q.row_smem, st>>>(dG, dS, q.row_L)));
-    if (ekin)
+    QSF_TIMED(QSF_K_ROW_CLOSE, (K.row_close<<<gr, K.row_threads, K.row_smem, st>>>(dG, dS)));
+    if (ekin) {
+      QSF_TIMED(QSF_K_AXIS_EKIN, (K.row_ekin<<<gr, K.row_threads, K.row_smem, st>>>(dG, dS)));
       for (int ax = 0; ax < D - 1; ++ax)
         QSF_TIMED(QSF_K_AXIS_EKIN,
-                  (K.axis_ekin<<<dim3(q.ax_blocks[ax], count), K.row_threads, q.ax_smem[ax], st>>>(dG, dS, ax, q.ax_C[ax])));
+                  (K.axis_ekin<<<dim3(q.ax_blocks[ax], count), K.col_threads, K.col_smem, st>>>(dG, dS, ax, 0)));
+    }
   }
   if (ov) ov->pending = false;
   if (!full && ov) {
@@ -668,7 +723,10 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   if (nb == 0) S.obs &= ~QSF_OBS_FLUX;
   // steps of a call stay in fixed point between steps, except after the steps whose
   // E_kin needs psi_n in memory (every ekin_interval-th step and the last one)
-  S.fused = G.dim >= 2 ? 1 : 0;
+  // (an imaginary-time run with a length-gauge field changes |psi| by its x.E factors, so
+  // its steps end and open one by one)
+  S.lg = G.dim >= 2 && G.gauge == QSF_GAUGE_LENGTH && G.n_fields && coup ? 1 : 0;
+  S.fused = G.dim >= 2 && !(S.lg && d->mode == QSF_MODE_IM) ? 1 : 0;
   S.ekin_every = d->ekin_interval > 1 ? d->ekin_interval : 1;
   S.normalize = d->normalize;
   S.energy_after_normalize = d->energy_after_normalize;
@@ -881,7 +939,7 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
         return fail(QSF_EINVAL, "dim >= 2 needs the same n and dx on every axis (the reference's P layout)");
   if (d->dim == 1 && d->n[0] > kMaxLine1D)
     return fail(QSF_EINVAL, "1D lines longer than " + std::to_string(kMaxLine1D) + " points are not supported");
-  if (d->dim >= 2 && d->n[0] > kMaxTile) return fail(QSF_EINVAL, "axes longer than 4096 points are not supported");
+  if (d->dim >= 2 && d->n[0] > kMaxAxis) return fail(QSF_EINVAL, "axes longer than 4096 points are not supported");
   if (d->potential < 0 || d->potential > 3) return fail(QSF_EINVAL, "unknown potential");
   if (d->gauge != QSF_GAUGE_VELOCITY && d->gauge != QSF_GAUGE_LENGTH) return fail(QSF_EINVAL, "unknown gauge");
   if (d->multi_region != 0 && d->multi_region != 1) return fail(QSF_EINVAL, "multi_region must be 0 or 1");
@@ -966,6 +1024,14 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
       a.twf = reinterpret_cast<decltype(a.twf)>(twfs[a.n]);
     }
   }
+  if (ks) {
+    const int4* twl[2];
+    if (int rc = shared_line_twiddles(*ks, twl)) {
+      qsf_grid_destroy(g);
+      return rc;
+    }
+    for (int k = 0; k < d->dim; ++k) std::copy(twl, twl + 2, G.ax[k].twl);
+  }
   G.inv_m = 1.0 / (double)G.m;
   G.dVm = G.dV * G.inv_m;
   G.nCAP = d->nCAP;
@@ -997,17 +1063,13 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   const int nlast = G.ax[D - 1].n;
   const long long nrows = G.m / nlast;
   if (D >= 2) {
-    g->row_L = (int)std::max<long long>(1, std::min<long long>(nrows, tile_pts(nlast) / nlast));
-    g->nrowblk = (int)((nrows + g->row_L - 1) / g->row_L);
-    g->row_smem = (size_t)g->row_L * nlast * sizeof(double2);
-    for (int ax = 0; ax < D - 1; ++ax) {
-      const AxisDev& a = G.ax[ax];
-      const long long inner = a.stride;
-      int C = (int)std::max<long long>(1, std::min<long long>({64, (long long)tile_pts(a.n) / a.n, inner}));
-      g->ax_C[ax] = C;
-      const long long outer = G.m / ((long long)a.n * inner);
-      g->ax_blocks[ax] = (int)(outer * ((inner + C - 1) / C));
-      g->ax_smem[ax] = (size_t)a.n * C * sizeof(double2);
+    if (ks) {
+      g->nrowblk = (int)((nrows + ks->row_lines - 1) / ks->row_lines);
+      for (int ax = 0; ax < D - 1; ++ax) {
+        const AxisDev& a = G.ax[ax];
+        const long long inner = a.stride, outer = G.m / ((long long)a.n * inner);
+        g->ax_blocks[ax] = (int)(outer * ((inner + ks->col_lines - 1) / ks->col_lines));
+      }
     }
   } else {
     g->nrowblk = ks ? ks->line_ctas : 1;  // partial sums per CTA of the line
@@ -1015,7 +1077,7 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   g->nmax = 0;
   for (int k = 0; k < D; ++k) g->nmax = std::max(g->nmax, G.ax[k].n);
   g->pmax = std::max({g->nrowblk, g->ax_blocks[0], g->ax_blocks[1], g->ax_blocks[2], 256});
-  g->scmax = std::max({g->nrowblk, g->ax_blocks[0], g->ax_blocks[1], g->ax_blocks[2], 1});
+  g->scmax = D >= 2 ? (int)nrows : 1;  // lines of a pass
   // 1/m = m_mant * 2^-l2m with m_mant in (0.5, 1]
   g->l2m = 0;
   while ((1LL << (g->l2m + 1)) <= G.m) ++g->l2m;
@@ -1140,28 +1202,7 @@ static int ensure_mtab(qsf_grid* g) {
 
 // one-axis transform of the array G.psi (grid geometry of g), scaled by sc on the way out
 static void axis_fft(qsf_grid* g, const GridDev& G, int ax, bool fwd, double sc) {
-  const KernelSet& K = *g->ks;
-  const int D = G.dim;
-  cudaStream_t st = g->stream;
-  {
-    if (ax == D - 1) {
-      // rows of the last axis with up to 16 * kLineThreads points per block
-      const int n = G.ax[ax].n;
-      const long long nrows = G.m / n;
-      const int L = (int)std::max<long long>(1, std::min<long long>(nrows, (16LL * kLineThreads) / n));
-      int blocks = (int)((nrows + L - 1) / L);
-      size_t smem = (size_t)L * n * sizeof(double2);
-      if (K.fft_ctas > 1) {  // one 1D line held by a cluster pair
-        blocks = K.fft_ctas;
-        smem = (size_t)(n / K.fft_ctas) * sizeof(double2);
-      }
-      if (fwd) K.row_fft_f<<<blocks, kLineThreads, smem, st>>>(G, L, sc);
-      else K.row_fft_b<<<blocks, kLineThreads, smem, st>>>(G, L, sc);
-    } else {
-      if (fwd) K.axis_fft_f<<<g->ax_blocks[ax], K.row_threads, g->ax_smem[ax], st>>>(G, ax, g->ax_C[ax], sc);
-      else K.axis_fft_b<<<g->ax_blocks[ax], K.row_threads, g->ax_smem[ax], st>>>(G, ax, g->ax_C[ax], sc);
-    }
-  }
+  launch_axis_fft(*g->ks, G, ax, fwd, sc, g->stream);
 }
 
 int qsf_fourier(qsf_grid* g, int to_rep) {

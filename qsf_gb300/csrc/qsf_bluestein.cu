@@ -18,6 +18,7 @@
 // transformed once per grid.  Grids of such lengths step through the member operations
 // (qsf_step's step programs, replayed from graphs); batches take built lengths only,
 // the server runs such solves beside its batch.
+#include <algorithm>
 #include <array>
 #include <cmath>
 #include <map>
@@ -118,34 +119,6 @@ int blocks_for(long long count) {
   return (int)std::min<long long>(std::max<long long>(b, 1), (long long)device_sm_count() * 16);
 }
 
-// one row transform (length n = S.ax[last].n, kernels K) over all rows of S
-void row_pass(const KernelSet& K, const GridDev& S, bool fwd, double post, cudaStream_t st) {
-  const int n = S.ax[S.dim - 1].n;
-  const long long nrows = S.m / n;
-  const int L = (int)std::max<long long>(1, std::min<long long>(nrows, (16LL * kLineThreads) / n));
-  int blocks = (int)((nrows + L - 1) / L);
-  size_t smem = (size_t)L * n * sizeof(double2);
-  if (K.fft_ctas > 1) {
-    blocks = K.fft_ctas;
-    smem = (size_t)(n / K.fft_ctas) * sizeof(double2);
-  }
-  if (fwd) K.row_fft_f<<<blocks, kLineThreads, smem, st>>>(S, L, post);
-  else K.row_fft_b<<<blocks, kLineThreads, smem, st>>>(S, L, post);
-}
-
-// one strided-axis transform (length S.ax[ax].n, kernels K) over all columns of S
-void axis_pass(const KernelSet& K, const GridDev& S, int ax, bool fwd, double post, cudaStream_t st) {
-  const int n = S.ax[ax].n;
-  const long long inner = S.ax[ax].stride;
-  // the tile the kernels are compiled for (tile_pts(n) points: C columns of n)
-  const int C = (int)std::max<long long>(1, std::min<long long>({64, (long long)tile_pts(n) / n, inner}));
-  const long long outer = S.m / ((long long)n * inner);
-  const int blocks = (int)(outer * ((inner + C - 1) / C));
-  const size_t smem = (size_t)n * C * sizeof(double2);
-  if (fwd) K.axis_fft_f<<<blocks, K.row_threads, smem, st>>>(S, ax, C, post);
-  else K.axis_fft_b<<<blocks, K.row_threads, smem, st>>>(S, ax, C, post);
-}
-
 // the M-point transform along axis ax of the array S.psi (geometry of S), on stream st
 int fft_M(const qsf_grid* g, const GridDev& S, int ax, bool fwd, double post, cudaStream_t st) {
   const qsf_grid::Bluestein& b = g->bs;
@@ -164,6 +137,7 @@ int fft_M(const qsf_grid* g, const GridDev& S, int ax, bool fwd, double post, cu
     V.ax[0].tw = b.tw1;
     V.ax[0].twx = b.twx1;
     V.ax[0].twf = reinterpret_cast<decltype(V.ax[0].twf)>(b.twf1);
+    std::copy(b.twl1, b.twl1 + 2, V.ax[0].twl);
     V.ax[1] = S.ax[0];
     V.ax[1].n = b.M2;
     V.ax[1].n2 = b.M2 / 2;
@@ -172,21 +146,20 @@ int fft_M(const qsf_grid* g, const GridDev& S, int ax, bool fwd, double post, cu
     V.ax[1].tw = b.tw;
     V.ax[1].twx = b.twx;
     V.ax[1].twf = reinterpret_cast<decltype(V.ax[1].twf)>(b.twf);
-    for (int k = 0; k < kMaxDim; ++k) V.tmap[k] = nullptr;
+    std::copy(b.twl, b.twl + 2, V.ax[1].twl);
     if (fwd) {
-      axis_pass(*b.ks1, V, 0, true, 1.0, st);
+      launch_axis_fft(*b.ks1, V, 0, true, 1.0, st);
       k_bs_twiddle<<<blocks_for(V.m), 256, 0, st>>>(V.psi, b.tw4, V.m, M, 0);
-      row_pass(K, V, true, post, st);
+      launch_axis_fft(K, V, 1, true, post, st);
     } else {
-      row_pass(K, V, false, 1.0, st);
+      launch_axis_fft(K, V, 1, false, 1.0, st);
       k_bs_twiddle<<<blocks_for(V.m), 256, 0, st>>>(V.psi, b.tw4, V.m, M, 1);
-      axis_pass(*b.ks1, V, 0, false, post, st);
+      launch_axis_fft(*b.ks1, V, 0, false, post, st);
     }
     QSF_CU(cudaGetLastError());
     return QSF_OK;
   }
-  if (ax == S.dim - 1) row_pass(K, S, fwd, post, st);
-  else axis_pass(K, S, ax, fwd, post, st);
+  launch_axis_fft(K, S, ax, fwd, post, st);
   QSF_CU(cudaGetLastError());
   return QSF_OK;
 }
@@ -201,13 +174,13 @@ GridDev scratch_view(const qsf_grid* g, int ax) {
   S.ax[ax].tw = g->bs.tw;
   S.ax[ax].twx = g->bs.twx;
   S.ax[ax].twf = reinterpret_cast<decltype(S.ax[ax].twf)>(g->bs.twf);
+  std::copy(g->bs.twl, g->bs.twl + 2, S.ax[ax].twl);
   long long st = 1;
   for (int k = S.dim - 1; k >= 0; --k) {
     S.ax[k].stride = st;
     st *= S.ax[k].n;
   }
   S.m = st;
-  for (int k = 0; k < kMaxDim; ++k) S.tmap[k] = nullptr;
   return S;
 }
 
@@ -227,8 +200,8 @@ bool bs_plan(int n, int dim, int* M, int* M1, int* M2) {
   std::vector<int> cols, rows;
   for (int a = 8; a <= 8192; ++a) {
     const KernelSet* k = kernels_for(a);
-    if (k && a <= 4096 && k->axis_fft_f) cols.push_back(a);
-    if (k && k->row_fft_f && k->fft_ctas == 1) rows.push_back(a);
+    if (k && a <= 4096 && k->axis_fft) cols.push_back(a);
+    if (k && k->row_fft && k->fft_ctas == 1) rows.push_back(a);
   }
   long long best = 0;
   for (int a : cols) {
@@ -289,8 +262,10 @@ int bs_setup(qsf_grid* g) {
   b.ks = kernels_for(M1 ? M2 : M);
   b.ks1 = M1 ? kernels_for(M1) : nullptr;
   int rc;
-  if ((rc = shared_twiddles(M1 ? M2 : M, &b.tw, &b.twx, &b.twf))) return rc;
-  if (M1 && ((rc = shared_twiddles(M1, &b.tw1, &b.twx1, &b.twf1)) || (rc = shared_w4(M1, M2, &b.tw4)))) return rc;
+  if ((rc = shared_twiddles(M1 ? M2 : M, &b.tw, &b.twx, &b.twf)) || (rc = shared_line_twiddles(*b.ks, b.twl))) return rc;
+  if (M1 && ((rc = shared_twiddles(M1, &b.tw1, &b.twx1, &b.twf1)) || (rc = shared_line_twiddles(*b.ks1, b.twl1)) ||
+             (rc = shared_w4(M1, M2, &b.tw4))))
+    return rc;
   const size_t scr = (size_t)(G.m / n) * (size_t)M;
   if ((rc = dev_alloc(b.chirp, (size_t)n)) || (rc = dev_alloc(b.bhat, (size_t)M)) ||
       (rc = dev_alloc(b.scratch, std::max(scr, (size_t)M))))
@@ -308,8 +283,8 @@ int bs_setup(qsf_grid* g) {
   L.ax[0].tw = b.tw;
   L.ax[0].twx = b.twx;
   L.ax[0].twf = reinterpret_cast<decltype(L.ax[0].twf)>(b.twf);
+  std::copy(b.twl, b.twl + 2, L.ax[0].twl);
   L.m = M;
-  for (int k = 0; k < kMaxDim; ++k) L.tmap[k] = nullptr;
   return fft_M(g, L, 0, true, 1.0, g->stream);
 }
 

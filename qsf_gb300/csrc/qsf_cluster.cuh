@@ -227,9 +227,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLineThreads, 1)
 }
 
 // fourier<R>() of a 1D line held by a CTA pair (qsf_fourier)
-template <int N, bool FWD>
+template <int N>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLineThreads, 1)
-    k_row_fft_cl(GridDev g, int L, double post_scale) {
+    k_row_fft_cl(GridDev g, int fwd, double post_scale) {
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(128) longlong2 smx[];
   __shared__ int red[kRedInts];
@@ -248,14 +248,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLineThreads, 1)
   for (int e = threadIdx.x; e < H; e += blockDim.x) {
     const double2 v = sd[e];
     const longlong2 x = make_longlong2(d2fx(v.x, scale), d2fx(v.y, scale));
-    smx[e] = FWD ? x : fconj(x);
+    smx[e] = fwd ? x : fconj(x);
   }
   cl.sync();
   const SplitLine line = split_line(smx, cl, H);
   int bits = 0;
   fft_fx_split<N>(line, g.ax[0].twx, rank * blockDim.x + threadIdx.x, 2 * blockDim.x, scale, bits, red, cl);
   for (int e = threadIdx.x; e < H; e += blockDim.x) {
-    const longlong2 x = FWD ? smx[e] : fconj(smx[e]);
+    const longlong2 x = fwd ? smx[e] : fconj(smx[e]);
     double2 v = make_double2(fx2d(x.x, scale), fx2d(x.y, scale));
     if (post_scale != 1.0) v = cscale(v, post_scale);
     g.psi[base + e] = v;

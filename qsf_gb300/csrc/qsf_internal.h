@@ -112,12 +112,8 @@ struct qsf_grid {
   FluxTerm* fterms = nullptr;
   int nsnap = 0, nfterms = 0, nfpts = 0, nfblk = 1;
   // launch geometry
-  int row_L = 1;
   int nrowblk = 1;
-  size_t row_smem = 0;
-  int ax_C[3] = {1, 1, 1};
   int ax_blocks[3] = {0, 0, 0};
-  size_t ax_smem[3] = {0, 0, 0};
   // multi-region transfer: slice buffer (m points) and the event that orders streams
   double2* mg_slice = nullptr;
   // member evolve: cached X-phase factors for (mode, delta) and per-axis P factors
@@ -176,6 +172,8 @@ struct qsf_grid {
     longlong2* twx1 = nullptr;
     longlong2* twf1 = nullptr;
     double2* tw4 = nullptr;  // four-step twiddles [k1][n2]
+    const int4* twl[2] = {};   // line-plan twiddles of M (or M2)
+    const int4* twl1[2] = {};  // and of M1
   } bs;
 };
 
@@ -206,6 +204,8 @@ int batch_finish(qsf_batch* b, int64_t* active);
 // be freed by the caller)
 int shared_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf);
 // twiddle tables of an n-point transform (FP64, 2^62 fixed point, split form)
+int shared_line_twiddles(const KernelSet& K, const int4* out[2]);
+void launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd, double sc, cudaStream_t st);
 int make_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf);
 // Bluestein plan of a grid without fused kernels (qsf_bluestein.cu)
 int bs_setup(qsf_grid* g);

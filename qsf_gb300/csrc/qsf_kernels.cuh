@@ -10,8 +10,8 @@
 //   k_axis        forward FFT axis 0 . P phase . inverse FFT axis 0 (1/m folded in)
 //   k_axis  (3D)  inverse FFT axis 1
 //   k_row_close   inverse FFT (last axis) . X half-phase . norm / E_pot partials,
-//                 flux snapshot, E_kin partial of the last axis
-//   k_axis  (E_kin only) forward FFT of the other axes of psi_n, sum k^2 |.|^2
+//                 flux snapshot . [next step's X half-phase . forward FFT (last axis)]
+//   k_row_ekin, k_axis (E_kin only) forward FFT of psi_n along each axis, sum k^2 |.|^2
 //   k_finalize    deterministic reductions, border fluxes, Normalize scale,
 //                 imaginary-time convergence, step counter
 //
@@ -25,38 +25,21 @@
 //
 // Arithmetic: psi is stored as complex128 between steps; inside a step every pass
 // works in block fixed point (int64 components sharing one power-of-two exponent per
-// thread block, qsf_fxfft.cuh), because GB300's integer pipes issue ~64x more
-// instructions per clock than its FP64 pipe.  Intermediate passes write int64 pairs
-// into psi's own buffer together with their block exponents; the next pass aligns every
-// element to the smallest exponent of the producing pass.  Phase tables are stored in
-// 2^62 fixed point with magnitude <= 1.  Norm and E_pot partials are exact 128-bit
-// integer sums per block.
+// line, or per group of lines that one warp or block holds, qsf_lines.cuh), because
+// GB300's integer pipes issue ~64x more instructions per clock than its FP64 pipe.
+// Intermediate passes write int64 pairs into psi's own buffer together with their line
+// exponents; the next pass aligns every element to the smallest exponent of the
+// producing pass.  Phase tables are stored in 2^62 fixed point with magnitude <= 1.
+// Norm and E_pot sums of a thread's points are integers.
 #pragma once
 #include "qsf_fft.cuh"
 #include "qsf_fxfft.cuh"
+#include "qsf_lines.cuh"
 #include "qsf_tuning.h"
 
 namespace qsf {
 
 constexpr int kMaxDim = 3;
-// Shape of the row / axis pass kernels per line length, as the autotuner measured it
-// (qsf_tuning.h): points per block (a tile of whole lines, 1024-4096 points) and
-// threads per block, which together set the points per thread and with them the radix
-// plan (16 points: radix 16, 8: radix 8).  The autotuner's candidate builds define
-// QSF_TILE and QSF_ROW_THREADS to force one shape everywhere.
-#ifdef QSF_ROW_THREADS
-__host__ __device__ constexpr int row_threads(int) { return QSF_ROW_THREADS; }
-#else
-__host__ __device__ constexpr int row_threads(int n) { return tuned_row_threads(n); }
-#endif
-#ifdef QSF_TILE
-__host__ __device__ constexpr int tile_size(int) { return QSF_TILE; }
-#else
-__host__ __device__ constexpr int tile_size(int n) { return tuned_tile(n); }
-#endif
-// points per block: the tile, or one whole line when lines are longer
-__host__ __device__ constexpr int tile_pts(int n) { return n > tile_size(n) ? n : tile_size(n); }
-__host__ __device__ constexpr int row_ppt(int n) { return tile_pts(n) / row_threads(n); }
 constexpr int kLinePptDiv = 512;  // threads of the one-CTA line kernel (kLineThreads)
 // Points per thread of the one-CTA line kernel (512 threads, one line of n points): a
 // line shorter than 8192 points leaves threads idle in radix-16 passes, and with one
@@ -85,12 +68,6 @@ constexpr int kMaxFluxBorders = 16;
 #ifndef QSF_FFT_MIN_BLOCKS
 #define QSF_FFT_MIN_BLOCKS 2
 #endif
-// resident blocks per SM the row / axis pass kernels are compiled for: twice as many
-// for blocks of 128 threads or fewer (the registers per thread stay the same)
-__host__ __device__ constexpr int row_min_blocks(int n) {
-  return row_threads(n) <= 128 ? 2 * QSF_FFT_MIN_BLOCKS : QSF_FFT_MIN_BLOCKS;
-}
-
 struct AxisDev {
   int n, n2;
   int shift;  // log2(n) when n is a power of two, else -1
@@ -103,6 +80,7 @@ struct AxisDev {
 #else
   const longlong2* twf;
 #endif
+  const int4* twl[2];  // per-pass twiddle tables of the 8- and the 16-point line plan (qsf_lines.cuh), kTwVar copies
 };
 
 struct GridDev {
@@ -121,8 +99,8 @@ struct GridDev {
   double2* psi;
   // TMA tensor maps (CUtensorMap, 128 bytes, 64-byte aligned, in device memory) of psi
   // for the strided-axis passes of axis d < dim - 1: psi as 64-bit words, dims
-  // {2 * stride_d, n_d, outer}, box {2 * tile columns, tma_box_rows(n_d), 1}; null when
-  // the driver offers no encoder (the passes then copy with cp.async)
+  // {2 * stride_d, n_d, outer}, box {2 * tile columns, tma_box_rows(n_d), 1}, swizzled
+  // over the row of a box; null when the driver offers no encoder (plain copies then)
   const void* tmap[kMaxDim];
 };
 
@@ -166,14 +144,15 @@ struct StepDev {
   const int4* xs;          // static X half-step factor per point (dt/2, incl. absorber), * 2^-xs_exp
   const long long* Vx;     // potential per point in 2^vshift fixed point
   int4* ptab;              // [dim][nmax] P-phase tables of the current step (|.| <= 1)
-  int4* xdyn;              // [3][dim][nmax] length-gauge factors: open half, close half, next open half
+  int4* xdyn;              // [3][dim][nmax] length-gauge factors: open half, close half, close . next open half
+  int lg;                  // 2D / 3D: the X halves carry length-gauge factors (a field couples x.E)
   int xs_exp;              // exponent taken out of xs (imaginary time: factors above 1)
   int vshift;              // Vx = round(V * 2^vshift)
   int l2m;                 // 1/m = m_mant * 2^-l2m, m_mant in (0.5, 1] (folded into axis 0's P table)
   double m_mant;
   int* texp;               // [3][3] exponents taken out of the per-step tables (set by k_tables)
   int* gmin;               // [kGmin] minimum block exponent of each fixed-point pass (gmin_slot)
-  int* sc;                 // [4][scmax] block exponents of each fixed-point pass
+  int* sc;                 // [4][scmax] line exponents of each fixed-point pass (qsf_passes.cuh)
   int scmax;
   // fused: a sub-step's closing row pass also applies the next sub-step's opening X half
   // and forward transform (ψ stays in fixed point between the steps of a call); the
@@ -361,32 +340,14 @@ __device__ __forceinline__ double2 expop(int mode, double val) {
 }
 
 // ------------------------------------------------------------ fixed-point helpers
-// Rows per block of the last-axis passes and columns per tile of the strided-axis
-// passes are compile-time functions of the line length (<= kMaxTile points per block),
-// so a consumer pass finds the block that produced an element with a few integer ops.
-// 16-byte global -> shared copy that bypasses registers (cp.async, cache-global); the
-// copies of a thread are visible to that thread after cp_async_wait_all.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// Contiguous global -> shared copies on the TMA engine (cp.async.bulk completing on an
-// mbarrier): one thread issues the copy of a whole tile, the others wait on the barrier.
+// Tile copies on the TMA engine complete on an mbarrier: one thread issues the copies of
+// a whole tile, the others wait on the barrier.
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// dst, src 16-byte aligned, bytes a multiple of 16
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned phase) {
   unsigned ok;
@@ -414,23 +375,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned phas
   return false;
 }
 
-// (i, c) = (e / Ch, e % Ch) for e = e0, e0 + step, e0 + 2 step, ... without a division
-// per element (Ch is a runtime tile width in the strided-axis passes)
-struct TileWalk {
-  int i, c, di, dc, Ch;
-  __device__ __forceinline__ TileWalk(int e0, int step, int ch)
-      : i(e0 / ch), c(e0 % ch), di(step / ch), dc(step % ch), Ch(ch) {}
-  __device__ __forceinline__ void next() {
-    i += di;
-    c += dc;
-    if (c >= Ch) {
-      c -= Ch;
-      ++i;
-    }
-  }
-};
-
-__host__ __device__ constexpr int row_lines(int n) { return tile_pts(n) / n; }
 // rows of one TMA box of a strided-axis tile: the largest divisor of n up to 256 (the
 // box limit), so that the boxes cover the n rows exactly and none writes past the tile
 __host__ __device__ constexpr int tma_box_rows(int n) {
@@ -438,27 +382,10 @@ __host__ __device__ constexpr int tma_box_rows(int n) {
   while (n % b) --b;
   return b;
 }
-__host__ __device__ constexpr int tile_cols(int n) { return (tile_pts(n) / n) < 64 ? (tile_pts(n) / n) : 64; }
-
-// Passes that leave the wavefunction in fixed point inside a step; each block of a
-// pass records its exponent in sc[pass][block] and the pass minimum in gmin[pass]:
-// 0 last-axis rows (open), 1 axis-1 tiles forward (3D), 2 axis-0 tiles, 3 axis-1
-// tiles inverse (3D).  The next pass aligns every element to gmin of its producer.
-template <int N>
-__device__ __forceinline__ int producer_block(int pass, int dim, long long p) {
-  if (pass == 0) return (int)((p / N) / row_lines(N));
-  if (pass == 2) {  // axis 0: a single outer index, inner = m / N
-    const long long inner = dim == 2 ? (long long)N : (long long)N * N;
-    const long long C = tile_cols(N) < inner ? tile_cols(N) : inner;
-    return (int)((p % inner) / C);
-  }
-  // axis 1 of a 3D grid: outer index i0, inner = N
-  constexpr long long C = tile_cols(N) < N ? tile_cols(N) : N;
-  constexpr long long tpo = (N + C - 1) / C;
-  const long long o = p / ((long long)N * N);
-  return (int)(o * tpo + (p % N) / C);
-}
-
+// Passes that leave the wavefunction in fixed point inside a step; each line of a pass
+// records its exponent in sc[pass] and the pass minimum in gmin[pass]: 0 last-axis rows
+// (open), 1 axis-1 lines forward (3D), 2 axis-0 lines, 3 axis-1 lines inverse (3D).  The
+// next pass aligns every element to gmin of its producer.
 // Exponent bookkeeping of the step's fixed-point tables: every table is stored with
 // magnitude <= 1 in 2^62 fixed point; a table whose exact values exceed 1 (imaginary
 // time) is stored times 2^-e and e is added back to the block exponent.
@@ -565,8 +492,8 @@ __device__ __forceinline__ int product_headroom(int bits) { return bits ? 61 - b
 
 // value of one per-step table entry: kind 0 P phase (hamiltonian.h:52-58: kinetic and,
 // in the velocity gauge, A.k), kind 1 / 2 length-gauge x.E factor of the open / close
-// X half (hamiltonian.h:60-66 via DipoleCoupling), kind 3 the open half of the next
-// sub-step (coupling row `cn`)
+// X half (hamiltonian.h:60-66 via DipoleCoupling), kind 3 the close half times the open
+// half of the next sub-step (coupling row `cn`)
 __device__ __forceinline__ double2 table_entry(const GridDev& g, const StepDev& S, const double* cp, const double* cn,
                                                int kind, int d, int i) {
   const AxisDev& a = g.ax[d];
@@ -580,8 +507,11 @@ __device__ __forceinline__ double2 table_entry(const GridDev& g, const StepDev& 
     const double k = kpos(a, i);
     return expop(S.mode, S.dt * (0.5 * k * k + k * A));
   }
-  const double* row = kind == 3 ? cn : cp;
-  const double E = (row && g.n_fields) ? row[(kind == 2 ? 3 : 0) + d] : 0.0;
+  double E = 0.0;
+  if (g.n_fields) {
+    if (cp) E = cp[(kind == 1 ? 0 : 3) + d];
+    if (kind == 3 && cn) E += cn[d];
+  }
   return expop(S.mode, (S.dt * 0.5) * (xpos(a, i) * E));
 }
 
@@ -689,16 +619,16 @@ __device__ __forceinline__ void finalize_tail(const GridDev& g, const StepDev& S
   for (int i = threadIdx.x; i < S.nrowblk; i += blockDim.x) {
     acc[0] += S.partials[0 * S.pmax + i];
     acc[1] += S.partials[1 * S.pmax + i];
-    acc[2 + g.dim - 1] += S.partials[(2 + g.dim - 1) * S.pmax + i];
   }
   if (ek) {
-    for (int d = 0; d < g.dim - 1; ++d)
-      for (int i = threadIdx.x; i < S.naxblk[d]; i += blockDim.x) acc[2 + d] += S.partials[(2 + d) * S.pmax + i];
+    for (int d = 0; d < g.dim; ++d)
+      for (int i = threadIdx.x; i < (d == g.dim - 1 ? S.nrowblk : S.naxblk[d]); i += blockDim.x)
+        acc[2 + d] += S.partials[(2 + d) * S.pmax + i];
   }
   __shared__ double fsum[kMaxFluxBorders];
   if (threadIdx.x < nb) {  // per border, the blocks' partials in block order
-    double v = 0.0;
-    for (int k = 0; k < nfb; ++k) v += S.fpartials[k * kMaxFluxBorders + threadIdx.x];
+    double v = 0.0;  // 0 where no point of the grid lies on a border (no block wrote partials)
+    for (int k = 0; k < nfb && S.nfterms > 0; ++k) v += S.fpartials[k * kMaxFluxBorders + threadIdx.x];
     fsum[threadIdx.x] = v;
   }
   block_sum<5>(acc, red);  // its barriers also publish fsum
@@ -966,111 +896,6 @@ __device__ __forceinline__ void close_block(const GridDev& g, const StepDev& S, 
   dacc[4] = (double)(2 * q - 2 * scale + 50 - S.vshift);
 }
 
-// Fused close of one sub-step and open of the next (no E_kin, psi_n not stored): in one
-// sweep over the block (held conjugated in smx after the inverse transform), psi_n =
-// f1 x feeds the norm / E_pot sums and becomes f2 psi_n, the next sub-step's opening X
-// half, left in smx.  The bit length of psi_n is bounded by that of x plus one (|f1| <=
-// 1), which fixes its accumulation shift and product headroom before the sweep.  The
-// flux snapshot of psi_n is taken first, at its listed points only.
-template <int N>
-__device__ __forceinline__ void close_open_block(const GridDev& g, const StepDev& S, longlong2* smx, long long base,
-                                                 int cnt, long long row0, int Lh, int* red, int& scale, int& bits,
-                                                 double* dacc) {
-  const bool real_f = S.mode == 1 && g.gauge != 1;
-  // length gauge in 3D: the x.E factors of the first two axes are constant along a row;
-  // their product per row and half is formed once, so that a half is three products
-  constexpr int kRowPre = 64;
-  __shared__ int4 rowpre[2][kRowPre];
-  const bool hoist = g.gauge == 1 && g.dim == 3 && Lh <= kRowPre;
-  const int4* t1 = S.xdyn + (size_t)1 * 3 * S.nmax;  // close half, axes 0..2
-  const int4* t2 = S.xdyn + (size_t)2 * 3 * S.nmax;  // next open half
-  if (hoist) {
-    for (int t = threadIdx.x; t < 2 * Lh; t += blockDim.x) {
-      const int h = t / Lh, rl = t % Lh;
-      const long long r = row0 + rl;
-      const int4* tab = h ? t2 : t1;
-      rowpre[h][rl] = split_fx(fmul62(tw_join(tab[S.nmax + (int)(r % N)]), tw_join(tab[(int)(r / N)])));
-    }
-    __syncthreads();
-  }
-  // half h (1: close, 2: next open) at block element e
-  auto half = [&](longlong2 x, int e, int h) -> longlong2 {
-    const long long p = base + e;
-    if (hoist) {
-      x = fapply(x, S.xs[p], false);
-      x = fapply(x, rowpre[h - 1][e / N], false);
-      x = fshl2(x);
-      return fapply(x, (h == 1 ? t1 : t2)[2 * S.nmax + e % N], false);
-    }
-    return xhalf<N>(g, S, x, p, row0 + e / N, e % N, h, real_f);
-  };
-  const int kf = hoist ? 3 : xfactors(g);  // products per half
-  const int pre = product_headroom(bits);
-  const int by = min(bits + pre + xbits(kf), 62);
-  const int sy = scale + pre - xfactor_exp(g, S, 1) - xshift(kf) + S.l2m;
-  const int q = by > 56 ? by - 56 : 0;
-  const int pre2 = product_headroom(by);
-  if (S.row_ptr) {
-    const int e0 = S.row_ptr[row0], e1 = S.row_ptr[row0 + Lh];
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      const int k = (int)(S.snap_idx[e] - base);
-      longlong2 x = fconj(smx[k]);
-      if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-      x = half(x, k, 1);
-      S.snap[e] = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
-    }
-    __syncthreads();
-  }
-  Acc128 an{0ull, 0ll}, av{0ull, 0ll};
-  const bool epot = (S.obs & 2u) != 0;
-  u64 mag = 0;
-  if (g.gauge != 1) {
-    // the velocity gauge and imaginary time: the static factor alone, loaded one
-    // element ahead (with the potential) so that the sweep does not wait on memory
-    int4 f_next = make_int4(0, 0, 0, 0);
-    long long v_next = 0;
-    if ((int)threadIdx.x < cnt) {
-      f_next = S.xs[base + threadIdx.x];
-      if (epot) v_next = S.Vx[base + threadIdx.x];
-    }
-#pragma unroll 1  // a large body: unrolling costs more in instruction fetch than it gains
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-      const int4 f = f_next;
-      const long long v = v_next;
-      if (e + (int)blockDim.x < cnt) {
-        f_next = S.xs[base + e + blockDim.x];
-        if (epot) v_next = S.Vx[base + e + blockDim.x];
-      }
-      longlong2 x = fconj(smx[e]);
-      if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-      x = fapply(x, f, real_f);
-      acc_point_v(an, av, x, q, v, epot);
-      if (pre2) x = make_longlong2(fshift(x.x, pre2), fshift(x.y, pre2));
-      x = fapply(x, f, real_f);
-      smx[e] = x;
-      mag |= fmag(x);
-    }
-  } else {
-#pragma unroll 1
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-      longlong2 x = fconj(smx[e]);
-      if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-      x = half(x, e, 1);
-      acc_point(an, av, x, q, S.Vx, base + e, epot);
-      if (pre2) x = make_longlong2(fshift(x.x, pre2), fshift(x.y, pre2));
-      x = half(x, e, 2);
-      smx[e] = x;
-      mag |= fmag(x);
-    }
-  }
-  dacc[0] = acc_value(an);
-  dacc[1] = acc_value(av);
-  dacc[3] = (double)(2 * q - 2 * sy);
-  dacc[4] = (double)(2 * q - 2 * sy + 50 - S.vshift);
-  scale = sy + pre2 - xfactor_exp(g, S, 2) - xshift(kf);
-  bits = block_max_int(bitlen(mag), red);
-}
-
 // E_kin part of the last axis: forward transform of psi_n (in smx) and sum k^2 |.|^2
 template <int N, int PPT>
 __device__ __forceinline__ double ekin_rows(const AxisDev& a, longlong2* smx, const LineSet& ls, int cnt, int scale,
@@ -1088,352 +913,23 @@ __device__ __forceinline__ double ekin_rows(const AxisDev& a, longlong2* smx, co
   return ek;
 }
 
-// ------------------------------------------------------------ row passes
-// Rows of the last axis: L rows of N points per block, contiguous in memory.
-// Open: psi (double) . [Normalize] . X half . forward FFT -> fixed point (pass 0).
-template <int N>
-__global__ void __launch_bounds__(row_threads(N), row_min_blocks(N)) k_row_open(const GridDev* __restrict__ Gs,
-                                                          const StepDev* __restrict__ Ss, int L) {
-  const GridDev& g = Gs[blockIdx.y];
-  const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
-  const long long sub = S.ctl[5];
-  // the previous sub-step's closing pass produced pass 0, unless it ended with psi_n in
-  // memory for E_kin
-  if (S.fused && sub > 0 && !ekin_at(S, sub - 1)) return;
-  extern __shared__ __align__(128) longlong2 smx[];
-  __shared__ int red[kRedInts];
-  const long long row0 = (long long)blockIdx.x * L;
-  const int Lh = (int)min((long long)L, g.m / N - row0);
-  const long long base = row0 * N;
-  const int cnt = Lh * N;
-  int bits = 0;
-  int scale = open_block<N>(g, S, smx, base, cnt, row0, red, bits);
-  const int sh = first_pass_shift<N>(bits);
-  scale += sh;
-  const LineSet ls{Lh, N, 1, false};
-  fft_fx<N, row_ppt(N)>(smx, ls, g.ax[g.dim - 1].twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  longlong2* out = reinterpret_cast<longlong2*>(g.psi);
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) out[base + e] = smx[e];
-  if (threadIdx.x == 0) {
-    S.sc[blockIdx.x] = scale;
-    atomicMin(&S.gmin[gmin_slot(0, sub)], scale);
-  }
-}
-
-// Loads the elements [obase + i * inner + c] (i < rows, c < Ch) of a fixed-point pass
-// output into smx[i * ldc + c] aligned to the pass minimum exponent (conjugated when
-// conj); returns the block's common exponent and the bit length of its largest
-// component.  With dtab, the alignment shift of element (i, c) is dtab[key], key = i
-// (tab_by_row) or (obase + i * inner + c) % N; otherwise it is looked up per element.
-template <int N>
-__device__ __forceinline__ int load_aligned(const GridDev& g, const StepDev& S, int in_pass, longlong2* smx,
-                                            long long obase, long long inner, int rows, int Ch, int ldc, int* red,
-                                            int& bits, bool conj, const int* dtab = nullptr,
-                                            bool tab_by_row = false, const void* tmap = nullptr,
-                                            int tx = 0, int tz = 0) {
-  const int gm = S.gmin[gmin_slot(in_pass, S.ctl[5])];
-  const int* sc = S.sc + (size_t)in_pass * S.scmax;
-  const longlong2* in = reinterpret_cast<const longlong2*>(g.psi);
-  const int cnt = rows * Ch;
-  u64 mag = 0;
-  // on the TMA engine: a contiguous tile (the row passes) as one bulk copy (shared and
-  // global addresses on 16 bytes); a strided tile (rows of ldc columns, the axis passes,
-  // rows == N) as boxes of tma_box_rows(N) rows of the tensor map, whose columns past
-  // the grid's edge arrive as zeros (each box's shared address on 128 bytes).  A tile
-  // whose addresses miss those alignments takes the cp.async loads.
-  const unsigned sa = smem_u32(smx);
-  constexpr int br = tma_box_rows(N);
-  const bool contiguous = Ch == 1 && inner == 1 && ldc == 1 && (sa & 15u) == 0 &&
-                          ((reinterpret_cast<unsigned long long>(in + obase)) & 15ull) == 0;
-  const bool boxes = tmap && rows == N && (sa & 127u) == 0 && ((unsigned)br * (unsigned)ldc * 16u) % 128u == 0;
-  if (contiguous || boxes) {
-    __shared__ __align__(8) unsigned long long bar;
-    if (threadIdx.x == 0) {
-      mbar_init(&bar, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      if (contiguous) {
-        mbar_expect_tx(&bar, (unsigned)cnt * 16u);
-        bulk_g2s(smx, in + obase, (unsigned)cnt * 16u, &bar);
-      } else {
-        mbar_expect_tx(&bar, (unsigned)rows * (unsigned)ldc * 16u);
-        for (int r0 = 0; r0 < rows; r0 += br) tma_load3(smx + (size_t)r0 * ldc, tmap, tx, r0, tz, &bar);
-      }
-    }
-    if (!mbar_wait(&bar, 0)) {
-      S.ctl[4] = 2;  // the copy did not complete in time: the call reports QSF_ETIMEDOUT
-      mbar_wait(&bar, 0);
-    }
-  } else {  // all of this thread's copies in flight at once, then fixed up in place
-    TileWalk w(threadIdx.x, blockDim.x, Ch);
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x, w.next())
-      cp_async16(&smx[w.i * ldc + w.c], in + obase + (long long)w.i * inner + w.c);
-    cp_async_wait_all();
-  }
-  TileWalk w(threadIdx.x, blockDim.x, Ch);
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x, w.next()) {
-    const int i = w.i, c = w.c;
-    const long long p = obase + (long long)i * inner + c;
-    longlong2 x = smx[i * ldc + c];
-    const int d = dtab ? dtab[tab_by_row ? i : (int)(p % N)] : gm - sc[producer_block<N>(in_pass, g.dim, p)];
-    if (d) x = make_longlong2(fshift(x.x, d), fshift(x.y, d));
-    if (conj) x = fconj(x);
-    smx[i * ldc + c] = x;
-    mag |= fmag(x);
-  }
-  bits = block_max_int(bitlen(mag), red);
-  return gm;
-}
-
-// Alignment shifts of a consumer block whose producer depends on one index of N values:
-// dtab[k] = gmin - sc[producer(k)], producer(k) = base_block + (kbase + k) / div.
-template <int N>
-__device__ __forceinline__ void build_dtab(const StepDev& S, int in_pass, int* dtab, long long base_block,
-                                           long long kbase, int div) {
-  const int gm = S.gmin[gmin_slot(in_pass, S.ctl[5])];
-  const int* sc = S.sc + (size_t)in_pass * S.scmax;
-  for (int k = threadIdx.x; k < N; k += blockDim.x) dtab[k] = gm - sc[base_block + (kbase + k) / div];
-  __syncthreads();
-}
-
-// Close: (fixed point, produced by the last strided-axis pass) inverse FFT . X half
-// -> psi_n: norm / E_pot partials, flux snapshot, E_kin part of the last axis.  The
-// inverse transform is the forward one on conjugated data.  psi_n is stored as double
-// at the last sub-step of the call (or always when not fused); otherwise the pass goes
-// on into the next sub-step: its opening X half and the forward transform of the last
-// axis, leaving pass 0 of that sub-step in fixed point.
-template <int N>
-__global__ void __launch_bounds__(row_threads(N), row_min_blocks(N)) k_row_close(const GridDev* __restrict__ Gs,
-                                                           const StepDev* __restrict__ Ss, int L) {
-  const GridDev& g = Gs[blockIdx.y];
-  const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
-  extern __shared__ __align__(128) longlong2 smx[];
-  __shared__ int red[kRedInts];
-  __shared__ double dred[32 * 3];
-  const AxisDev& a = g.ax[g.dim - 1];
-  const long long sub = S.ctl[5];
-  if (blockIdx.x == 0 && threadIdx.x == 0) S.ctl[6] = sub + 1;  // the sub-step's last pass
-  // the step ends here, psi_n stored as complex128: the call's last sub-step, and steps
-  // whose E_kin needs psi_n in memory
-  const bool ek = ekin_at(S, sub);
-  const bool last = !S.fused || sub >= S.ctl[1] || sub + 1 >= S.nsteps || ek;
-  const long long row0 = (long long)blockIdx.x * L;
-  const int Lh = (int)min((long long)L, g.m / N - row0);
-  const long long base = row0 * N;
-  const int cnt = Lh * N;
-  // 3D: the sweep after the inverse transform reads this block's slice of the X table
-  // (16 B per point) and of the potential (8 B per point, E_pot): start moving it into
-  // L2 now, one prefetch per 128-byte line, so that those loads do not wait on DRAM
-  // (256^3 step 2.11 -> 2.08 ms; no gain for the 2D passes, so they skip it)
-  if (g.dim == 3) {
-    for (int e = threadIdx.x * 8; e < cnt; e += blockDim.x * 8) prefetch_l2(S.xs + base + e);
-    if (S.obs & 2u)
-      for (int e = threadIdx.x * 16; e < cnt; e += blockDim.x * 16) prefetch_l2(S.Vx + base + e);
-  }
-  int bits = 0;
-  // producer of element (row, j): axis-0 tile j / C (2D) or axis-1 tile (i0, j / C) (3D,
-  // when the block's rows share i0)
-  __shared__ int dtab[N];
-  const bool use_tab = g.dim == 2 || N % row_lines(N) == 0;
-  if (use_tab) {
-    constexpr int C = tile_cols(N) < N ? tile_cols(N) : N;
-    const long long i0 = g.dim == 3 ? row0 / N : 0;
-    build_dtab<N>(S, g.dim == 3 ? 3 : 2, dtab, g.dim == 3 ? i0 * ((N + C - 1) / C) : 0, 0, C);
-  }
-  // rows are contiguous: treat the block as one "column" of cnt elements
-  int scale = load_aligned<N>(g, S, g.dim == 3 ? 3 : 2, smx, base, 1, cnt, 1, 1, red, bits, true,
-                              use_tab ? dtab : nullptr, false);
-  int sh = first_pass_shift<N>(bits);
-  scale += sh;
-  const LineSet ls{Lh, N, 1, false};
-  fft_fx<N, row_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  double dacc[5];
-  const bool fuse_x = !last;
-  if (fuse_x) {
-    close_open_block<N>(g, S, smx, base, cnt, row0, Lh, red, scale, bits, dacc);
-    dacc[2] = 0.0;
-  } else {
-    close_block<N>(g, S, smx, base, cnt, row0, red, scale, bits, dacc, true, last);
-    if (S.row_ptr) {  // flux snapshot of psi_n (this thread's own elements of smx are not needed)
-      const int e0 = S.row_ptr[row0], e1 = S.row_ptr[row0 + Lh];
-      for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        const longlong2 x = smx[S.snap_idx[e] - base];
-        S.snap[e] = make_double2(fx2d(x.x, scale), fx2d(x.y, scale));
-      }
-    }
-    dacc[2] = ek ? ekin_rows<N, row_ppt(N)>(a, smx, ls, cnt, scale, bits, red) : 0.0;
-  }
-  const double e_n = dacc[3], e_v = dacc[4];
-  block_sum<3>(dacc, dred);  // its barriers also end the snapshot reads of smx
-  if (threadIdx.x == 0) {
-    S.partials[0 * S.pmax + blockIdx.x] = ldexp(dacc[0], (int)e_n);
-    S.partials[1 * S.pmax + blockIdx.x] = ldexp(dacc[1], (int)e_v);
-    S.partials[(2 + g.dim - 1) * S.pmax + blockIdx.x] = dacc[2];
-  }
-  if (last) return;
-  // next sub-step: opening X half (static factor and the length-gauge factors of the
-  // next coupling row; already applied when fused) and the forward transform of the last axis
-  if (!fuse_x) {
-    const bool real_f = S.mode == 1 && g.gauge != 1;
-    const int pre = product_headroom(bits);
-    u64 mag = 0;
-#pragma unroll 4
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-      const long long p = base + e;
-      longlong2 x = smx[e];
-      if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-      x = xhalf<N>(g, S, x, p, row0 + e / N, e % N, 2, real_f);
-      smx[e] = x;
-      mag |= fmag(x);
-    }
-    scale += pre - xhalf_exp(g, S, 2);
-    bits = block_max_int(bitlen(mag), red);
-  }
-  sh = first_pass_shift<N>(bits);
-  scale += sh;
-  fft_fx<N, row_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  longlong2* out = reinterpret_cast<longlong2*>(g.psi);
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) out[base + e] = smx[e];
-  if (threadIdx.x == 0) {
-    S.sc[blockIdx.x] = scale;
-    atomicMin(&S.gmin[gmin_slot(0, sub + 1)], scale);
-  }
-}
-
-// P phase between the forward and the inverse transform of axis `ax` (element (i, c)
-// of the tile at smx[i * ldc + c]), written conjugated so that the inverse transform
-// runs as a forward one; returns the exponent change and the new bit length.
-__device__ __forceinline__ int p_phase(const GridDev& g, const StepDev& S, longlong2* smx, int ax, int rows, int Ch,
-                                       int ldc, const int4* pcol, int* red, int& bits) {
+// P phase of a 1D line between the forward and the inverse transform, written conjugated
+// so that the inverse transform runs as a forward one; returns the exponent change and
+// the new bit length.
+__device__ __forceinline__ int p_phase(const StepDev& S, longlong2* smx, int n, int* red, int& bits) {
   const bool real_f = S.mode == 1;
   const int pre = product_headroom(bits);
-  const int cnt = rows * Ch;
   u64 mag = 0;
-  TileWalk w(threadIdx.x, blockDim.x, Ch);
 #pragma unroll 1
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x, w.next()) {
-    const int i = w.i, c = w.c;
-    longlong2 x = smx[i * ldc + c];
+  for (int e = threadIdx.x; e < n; e += blockDim.x) {
+    longlong2 x = smx[e];
     if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-    x = fapply(x, S.ptab[(size_t)ax * S.nmax + i], real_f);
-    if (pcol) x = fapply(x, pcol[c], real_f);
-    x = fconj(x);
-    smx[i * ldc + c] = x;
+    x = fconj(fapply(x, S.ptab[e], real_f));
+    smx[e] = x;
     mag |= fmag(x);
   }
-  int pe = xshift(pcol ? 2 : 1);
-  for (int d = 0; d < g.dim; ++d) pe += S.texp[d];
   bits = block_max_int(bitlen(mag), red);
-  return pre - pe;
-}
-
-// ------------------------------------------------------------ strided axes
-// Axis `ax` (not the last): tiles of C adjacent columns; element (i, c) of tile
-// (o, c0) is psi[o * N * stride + i * stride + c0 + c].  Modes:
-//   0 forward (3D axis 1: pass 0 -> 1), 1 inverse (3D axis 1: pass 2 -> 3),
-//   2 forward . P phase . inverse (axis 0: pass 0 (2D) or 1 (3D) -> 2),
-//   3 forward of psi_n (double) + E_kin partial
-// Inverse transforms run as forward ones on conjugated data.
-template <int MODE, int N>
-__global__ void __launch_bounds__(row_threads(N), row_min_blocks(N)) k_axis(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss,
-                                                      int ax, int C) {
-  const GridDev& g = Gs[blockIdx.y];
-  const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
-  if (MODE == 3 && !ekin_at(S, S.ctl[5])) return;
-  extern __shared__ __align__(128) longlong2 smx[];
-  __shared__ int red[kRedInts];
-  __shared__ double dred[32];
-  __shared__ int4 pcol[64];
-  const AxisDev& a = g.ax[ax];
-  const long long inner = a.stride;
-  const long long tiles_per_outer = (inner + C - 1) / C;
-  const long long o = blockIdx.x / tiles_per_outer;
-  const long long c0 = (blockIdx.x % tiles_per_outer) * C;
-  const int Ch = (int)min((long long)C, inner - c0);
-  const long long obase = o * (long long)N * inner + c0;
-  const int cnt = N * Ch;
-  const LineSet ls{Ch, 1, C, true};
-  int scale = 0, bits = 0;
-  if (MODE == 3) {
-    double2* sd = reinterpret_cast<double2*>(smx);
-    int em = 0;
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-      const int i = e / Ch, c = e % Ch;
-      const double2 v = g.psi[obase + (long long)i * inner + c];
-      sd[i * C + c] = v;
-      em = max(em, max(dexp(v.x), dexp(v.y)));
-    }
-    em = block_max_int(em, red);
-    scale = (62 - fguard(radix_at(N, 0))) - (em - 1022);
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-      const int i = e / Ch, c = e % Ch;
-      const double2 v = sd[i * C + c];
-      smx[i * C + c] = make_longlong2(d2fx(v.x, scale), d2fx(v.y, scale));
-    }
-    __syncthreads();
-    fft_fx<N, row_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red);
-    double acc = 0.0;
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-      const int i = e / Ch, c = e % Ch;
-      const double k = kpos(a, i);
-      const longlong2 x = smx[i * C + c];
-      const double xr = fx2d(x.x, scale), xi = fx2d(x.y, scale);
-      acc = fma(k * k, fma(xr, xr, xi * xi), acc);
-    }
-    block_sum<1>(&acc, dred);
-    if (threadIdx.x == 0) S.partials[(2 + ax) * S.pmax + blockIdx.x] = acc;
-    return;
-  }
-  const int in_pass = MODE == 0 ? 0 : MODE == 1 ? 2 : (g.dim == 3 ? 1 : 0);
-  const int out_pass = MODE == 0 ? 1 : MODE == 1 ? 3 : 2;
-  // producer row block of element (i, c) when the input is the row pass: (o N + i) / L
-  __shared__ int dtab[N];
-  const bool by_row = in_pass == 0;
-  if (by_row) build_dtab<N>(S, 0, dtab, 0, o * N, row_lines(N));
-  scale = load_aligned<N>(g, S, in_pass, smx, obase, inner, N, Ch, C, red, bits, MODE == 1, by_row ? dtab : nullptr,
-                          true, g.tmap[ax], (int)(2 * c0), (int)o);
-  const bool multi_col = MODE == 2 && ax + 1 < g.dim;
-  if (multi_col && threadIdx.x < Ch) {
-    // per-column factor: product of the P tables of the axes after `ax`
-    long long cc = c0 + threadIdx.x;
-    longlong2 f = make_longlong2(4611686018427387904LL, 0LL);  // 1.0
-    for (int d2 = g.dim - 1; d2 > ax; --d2) {
-      const int i = (int)(cc % g.ax[d2].n);
-      cc /= g.ax[d2].n;
-      f = fmul62(f, tw_join(S.ptab[(size_t)d2 * S.nmax + i]));
-    }
-    pcol[threadIdx.x] = split_fx(f);
-  }
-  int sh = first_pass_shift<N>(bits);
-  scale += sh;
-  fft_fx<N, row_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  if (MODE == 2) {
-    scale += p_phase(g, S, smx, ax, N, Ch, C, multi_col ? pcol : nullptr, red, bits);
-    sh = first_pass_shift<N>(bits);
-    scale += sh;
-    fft_fx<N, row_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  }
-  longlong2* out = reinterpret_cast<longlong2*>(g.psi);
-  const bool conj_out = MODE != 0;
-  TileWalk w(threadIdx.x, blockDim.x, Ch);
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x, w.next()) {
-    const int i = w.i, c = w.c;
-    const longlong2 x = smx[i * C + c];
-    out[obase + (long long)i * inner + c] = conj_out ? fconj(x) : x;
-  }
-  if (threadIdx.x == 0) {
-    S.sc[(size_t)out_pass * S.scmax + blockIdx.x] = scale;
-    atomicMin(&S.gmin[out_pass], scale);
-  }
+  return pre - xshift(1) - S.texp[0];
 }
 
 // ------------------------------------------------------------ 1D whole step
@@ -1455,7 +951,7 @@ __global__ void __launch_bounds__(kLineThreads, (QSF_FFT_MIN_BLOCKS + 1) / 2) k_
   scale += sh;
   const LineSet ls{1, N, 1, false};
   fft_fx<N, line_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  scale += p_phase(g, S, smx, 0, N, 1, 1, nullptr, red, bits);
+  scale += p_phase(S, smx, N, red, bits);
   sh = first_pass_shift<N>(bits);
   scale += sh;
   fft_fx<N, line_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
@@ -1485,88 +981,6 @@ __global__ void __launch_bounds__(kLineThreads, (QSF_FFT_MIN_BLOCKS + 1) / 2) k_
       flux_block(g, S.fpts, S.fterms, 0, S.nfterms, S.snap, A, nb, dred, S.fpartials);
     }
     finalize_tail(g, S, sub, step_end, step, nb, 1, dred);
-  }
-}
-
-// ------------------------------------------------------------ plain FFT passes
-// fourier<R>() without phases (qsf_fourier), in block fixed point: each block takes
-// its exponent from the largest double it loads (one global read, staged in smem),
-// converts with integer operations, runs the fixed-point passes (an inverse is the
-// forward transform between two conjugations) and converts back (times post_scale).
-template <int N, bool FWD>
-__global__ void __launch_bounds__(kLineThreads, (QSF_FFT_MIN_BLOCKS + 1) / 2) k_row_fft(GridDev g, int L, double post_scale) {
-  extern __shared__ __align__(128) longlong2 smx[];
-  __shared__ int red[kRedInts];
-  const AxisDev& a = g.ax[g.dim - 1];
-  const long long row0 = (long long)blockIdx.x * L;
-  const long long nrows = g.m / N;
-  const int Lh = (int)min((long long)L, nrows - row0);
-  const long long base = row0 * N;
-  const int cnt = Lh * N;
-  double2* sd = reinterpret_cast<double2*>(smx);
-  int em = 0;
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const double2 v = g.psi[base + e];
-    sd[e] = v;
-    em = max(em, max(dexp(v.x), dexp(v.y)));
-  }
-  em = block_max_int(em, red);
-  int scale = (62 - fguard(radix_at(N, 0))) - (em - 1022);
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const double2 v = sd[e];
-    const longlong2 x = make_longlong2(d2fx(v.x, scale), d2fx(v.y, scale));
-    smx[e] = FWD ? x : fconj(x);
-  }
-  __syncthreads();
-  const LineSet ls{Lh, N, 1, false};
-  int bits = 0;
-  fft_fx<N>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red);
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const longlong2 x = FWD ? smx[e] : fconj(smx[e]);
-    double2 v = make_double2(fx2d(x.x, scale), fx2d(x.y, scale));
-    if (post_scale != 1.0) v = cscale(v, post_scale);
-    g.psi[base + e] = v;
-  }
-}
-
-template <int N, bool FWD>
-__global__ void __launch_bounds__(row_threads(N), row_min_blocks(N)) k_axis_fft(GridDev g, int ax, int C, double post_scale) {
-  extern __shared__ __align__(128) longlong2 smx[];
-  __shared__ int red[kRedInts];
-  const AxisDev& a = g.ax[ax];
-  const long long inner = a.stride;
-  const long long tiles_per_outer = (inner + C - 1) / C;
-  const long long o = blockIdx.x / tiles_per_outer;
-  const long long c0 = (blockIdx.x % tiles_per_outer) * C;
-  const int Ch = (int)min((long long)C, inner - c0);
-  const long long obase = o * (long long)N * inner + c0;
-  const int cnt = N * Ch;
-  double2* sd = reinterpret_cast<double2*>(smx);
-  int em = 0;
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const int i = e / Ch, c = e % Ch;
-    const double2 v = g.psi[obase + (long long)i * inner + c];
-    sd[i * C + c] = v;
-    em = max(em, max(dexp(v.x), dexp(v.y)));
-  }
-  em = block_max_int(em, red);
-  int scale = (62 - fguard(radix_at(N, 0))) - (em - 1022);
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const int i = e / Ch, c = e % Ch;
-    const double2 v = sd[i * C + c];
-    const longlong2 x = make_longlong2(d2fx(v.x, scale), d2fx(v.y, scale));
-    smx[i * C + c] = FWD ? x : fconj(x);
-  }
-  __syncthreads();
-  const LineSet ls{Ch, 1, C, true};
-  int bits = 0;
-  fft_fx<N, row_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red);
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const int i = e / Ch, c = e % Ch;
-    const longlong2 x = FWD ? smx[i * C + c] : fconj(smx[i * C + c]);
-    double2 v = make_double2(fx2d(x.x, scale), fx2d(x.y, scale));
-    if (post_scale != 1.0) v = cscale(v, post_scale);
-    g.psi[obase + (long long)i * inner + c] = v;
   }
 }
 
@@ -1918,22 +1332,23 @@ __global__ void k_add_gaussian(GridDev g, double at, double delta) {
 // ------------------------------------------------------------ per-size kernel table
 struct KernelSet {
   int n;
-  void (*row_open)(const GridDev*, const StepDev*, int);
-  void (*row_close)(const GridDev*, const StepDev*, int);
-  void (*axis_fwd)(const GridDev*, const StepDev*, int, int);
-  void (*axis_inv)(const GridDev*, const StepDev*, int, int);
+  void (*row_open)(const GridDev*, const StepDev*);
+  void (*row_close)(const GridDev*, const StepDev*);
+  void (*row_ekin)(const GridDev*, const StepDev*);
+  void (*axis_one)(const GridDev*, const StepDev*, int, int);  // one transform: forward or inverse (last argument)
   void (*axis_fpi)(const GridDev*, const StepDev*, int, int);
   void (*axis_ekin)(const GridDev*, const StepDev*, int, int);
   void (*line_step)(const GridDev*, const StepDev*);
-  void (*row_fft_f)(GridDev, int, double);
-  void (*row_fft_b)(GridDev, int, double);
-  void (*axis_fft_f)(GridDev, int, int, double);
-  void (*axis_fft_b)(GridDev, int, int, double);
+  void (*row_fft)(GridDev, int, double);        // forward flag, scale on the way out
+  void (*axis_fft)(GridDev, int, int, double);  // axis, forward flag, scale
   int line_ctas;     // CTAs holding one 1D line in the step kernel (a cluster of 2 .. 8 CTAs for
                      // power-of-two lines of 1024 or more points)
   int line_threads;  // threads per CTA of the 1D line step kernel
   int fft_ctas;      // CTAs of the plain row transform of one line (2: a cluster pair above 8192 points)
-  int row_threads;  // threads per block of the row / axis passes
+  int row_lines, row_threads, row_smem;  // last-axis passes: lines, threads, dynamic shared memory of a block
+  int col_lines, col_threads, col_smem;  // strided-axis passes: columns, threads, dynamic shared memory
+  int fft_lines, fft_threads, fft_smem;  // row_fft
+  const int* plan[2];                    // radices of the 8- and the 16-point line plan, 0-terminated
   bool line_full;   // line_step also ends the step (fluxes, row, counters: no k_finalize)
 };
 
@@ -1941,6 +1356,7 @@ struct KernelSet {
 const KernelSet* kernels_for(int n);
 
 }  // namespace qsf
+#include "qsf_passes.cuh"
 #include "qsf_cluster.cuh"
 namespace qsf {
 
@@ -1955,39 +1371,51 @@ KernelSet make_kernel_set() {
   k.line_ctas = 1;
   k.line_threads = kLineThreads;
   k.fft_ctas = 1;
-  k.row_threads = row_threads(N);
   k.line_full = false;
   if constexpr (N > 8192) {
     k.line_ctas = 2;
     k.fft_ctas = 2;
     k.line_step = k_line_step_cl<N>;
-    k.row_fft_f = k_row_fft_cl<N, true>;
-    k.row_fft_b = k_row_fft_cl<N, false>;
+    k.row_fft = k_row_fft_cl<N>;
+    k.fft_lines = 1;
+    k.fft_threads = kLineThreads;
+    k.fft_smem = N / 2 * (int)sizeof(double2);
     return k;
   } else {
-  if constexpr (N <= 4096) {
-    k.row_open = k_row_open<N>;
-    k.row_close = k_row_close<N>;
-    k.axis_fwd = k_axis<0, N>;
-    k.axis_inv = k_axis<1, N>;
-    k.axis_fpi = k_axis<2, N>;
-    k.axis_ekin = k_axis<3, N>;
-    k.axis_fft_f = k_axis_fft<N, true>;
-    k.axis_fft_b = k_axis_fft<N, false>;
-  }
-  k.line_step = k_line_step<N, true>;
-  k.line_full = true;
+    using G = Ln<N, tuned_ppt(N)>;
+    using A = Ln<N, axis_ppt(N)>;
+    if constexpr (N <= 4096) {
+      k.row_open = k_row_open<G>;
+      k.row_close = k_row_close<G>;
+      k.row_ekin = k_row_ekin<G>;
+      k.axis_one = k_axis<0, A>;
+      k.axis_fpi = k_axis<2, A>;
+      k.axis_ekin = k_axis<3, A>;
+      k.axis_fft = k_axis_fft<A>;
+      k.row_lines = G::L;
+      k.row_threads = G::kRowThreads;
+      k.row_smem = G::kRowSmem;
+      k.col_lines = A::C;
+      k.col_threads = A::kColThreads;
+      k.col_smem = A::kColSmem;
+    }
+    k.line_step = k_line_step<N, true>;
+    k.line_full = true;
 #if QSF_LINE_CLUSTER
-  if constexpr (N >= 1024 && (N & (N - 1)) == 0) {  // the line spread over a cluster
-    constexpr int C = N / 512 < 8 ? N / 512 : 8;
-    k.line_ctas = C;
-    k.line_threads = mc_threads<N, C>();
-    k.line_step = k_line_step_mc<N, C>;
-  }
+    if constexpr (N >= 1024 && (N & (N - 1)) == 0) {  // the line spread over a cluster
+      constexpr int C = N / 512 < 8 ? N / 512 : 8;
+      k.line_ctas = C;
+      k.line_threads = mc_threads<N, C>();
+      k.line_step = k_line_step_mc<N, C>;
+    }
 #endif
-  k.row_fft_f = k_row_fft<N, true>;
-  k.row_fft_b = k_row_fft<N, false>;
-  return k;
+    k.row_fft = k_row_fft<G>;
+    k.fft_lines = G::L;
+    k.fft_threads = G::kRowThreads;
+    k.fft_smem = G::kRowSmem;
+    k.plan[0] = line_radices<N, 8>();
+    k.plan[1] = line_radices<N, 16>();
+    return k;
   }
 }
 

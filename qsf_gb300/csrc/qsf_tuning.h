@@ -1,30 +1,34 @@
-// qsf_tuning.h -- pass kernel shapes per line length: points and threads per block of
-// the row / axis passes, and the radix plan of the one-CTA 1D line kernel.
+// qsf_tuning.h -- pass kernel shapes per line length: the points per thread of the row
+// passes, and the radix plan of the one-CTA 1D line kernel.
 //
 // Written by the autotuner (qsf_gb300/autotune.py) from step times measured on a GB300:
 //   python -m qsf_gb300.autotune --write
-// Row / axis shapes: points per block x threads per block (16 points per thread:
-// radix-16 plans, 128 registers; 8: radix-8 plans); lengths not listed take
-// 4096x256.  Chosen among 4096x256, 4096x512; smaller tiles, timed
-// beside them, speed up small grids run alone but slow the batched form down.
+// Row passes: points x threads, whose ratio is the points per thread and selects the
+// line plan (16: radix-16 plans, 128 registers; 8: radix-8 plans); lengths not listed
+// take 4096x256.
 // Measured (one call of graph-replayed steps per workload, ms per step):
-//   2d256   ms/step  4096x256: 0.0693  4096x512: 0.0691  2048x128: 0.0577  2048x256: 0.0511  1024x128: 0.0449
-//   2d320   ms/step  4096x256: 0.0904  4096x512: 0.0744  2048x128: 0.0823  2048x256: 0.0552  1024x128: 0.0510
-//   2d384   ms/step  4096x256: 0.0860  4096x512: 0.0801  2048x128: 0.0777  2048x256: 0.0608  1024x128: 0.0522
-//   2d512   ms/step  4096x256: 0.0889  4096x512: 0.0725  2048x128: 0.0776  2048x256: 0.0513  1024x128: 0.0499
-//   2d640   ms/step  4096x256: 0.0921  4096x512: 0.0863  2048x128: 0.0869  2048x256: 0.0765  1024x128: 0.1035
-//   2d768   ms/step  4096x256: 0.1050  4096x512: 0.1213  2048x128: 0.0830  2048x256: 0.1095  1024x128: 0.1096
-//   2d1024  ms/step  4096x256: 0.1069  4096x512: 0.1276  2048x128: 0.1098  2048x256: 0.1376  1024x128: 0.1306
-//   2d2048  ms/step  4096x256: 0.4450  4096x512: 0.4330  2048x128: 0.4477  2048x256: 0.5127  1024x128: 0.4559
-//   2d4096  ms/step  4096x256: 1.6895  4096x512: 1.8929  2048x128: 2.6868  2048x256: 1.6912  1024x128: 2.7324
-//   3d128   ms/step  4096x256: 0.2978  4096x512: 0.3166  2048x128: 0.2872  2048x256: 0.3250  1024x128: 0.3178
-//   3d256   ms/step  4096x256: 1.8134  4096x512: 1.9213  2048x128: 1.8110  2048x256: 2.2277  1024x128: 2.2397
+//   2d64    ms/step  4096x256: 0.0356  4096x512: 0.0308
+//   2d128   ms/step  4096x256: 0.0382  4096x512: 0.0343
+//   2d192   ms/step  4096x256: 0.0355  4096x512: 0.0339
+//   2d256   ms/step  4096x256: 0.0397  4096x512: 0.0339
+//   2d320   ms/step  4096x256: 0.0527  4096x512: 0.0403
+//   2d384   ms/step  4096x256: 0.0443  4096x512: 0.0380
+//   2d512   ms/step  4096x256: 0.0400  4096x512: 0.0342
+//   2d640   ms/step  4096x256: 0.0674  4096x512: 0.0603
+//   2d768   ms/step  4096x256: 0.0630  4096x512: 0.0629
+//   2d1024  ms/step  4096x256: 0.0853  4096x512: 0.0793
+//   2d1280  ms/step  4096x256: 0.1569  4096x512: 0.1661
+//   2d1536  ms/step  4096x256: 0.2077  4096x512: 0.2000
+//   2d2048  ms/step  4096x256: 0.2871  4096x512: 0.2873
+//   2d4096  ms/step  4096x256: 1.1613  4096x512: 1.3885
+//   3d128   ms/step  4096x256: 0.1928  4096x512: 0.1854
+//   3d256   ms/step  4096x256: 1.3193  4096x512: 1.2235
 #pragma once
 
 namespace qsf {
 
 __host__ __device__ constexpr int tuned_row_threads(int n) {
-  return n == 320 ? 512 : n == 384 ? 512 : n == 512 ? 512 : n == 640 ? 512 : n == 2048 ? 512 : 256;
+  return n == 64 ? 512 : n == 128 ? 512 : n == 192 ? 512 : n == 256 ? 512 : n == 320 ? 512 : n == 384 ? 512 : n == 512 ? 512 : n == 640 ? 512 : n == 768 ? 512 : n == 1024 ? 512 : n == 1536 ? 512 : 256;
 }
 
 __host__ __device__ constexpr int tuned_tile(int n) {

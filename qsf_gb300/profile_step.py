@@ -24,6 +24,11 @@ WORKLOADS = {
     "3d256": (3, 256, 0.4, 26, 3.0, 1, 1e15, 800.0, 2.0, "ZOA_FLUX_3D", 0),
     # further edges of the batched / served 2D mix and a smaller 3D cube
     "2d256": (2, 256, 0.3, 26, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
+    "2d64": (2, 64, 0.3, 6, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
+    "2d128": (2, 128, 0.3, 13, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
+    "2d192": (2, 192, 0.3, 19, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
+    "2d1280": (2, 1280, 0.3, 128, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
+    "2d1536": (2, 1536, 0.3, 154, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
     "2d320": (2, 320, 0.3, 32, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
     "2d384": (2, 384, 0.3, 38, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
     "2d640": (2, 640, 0.3, 64, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
