@@ -110,10 +110,10 @@ int init_kernel_table() {
     if ((rc = lim((const void*)k.row_open, k.row_smem)) || (rc = lim((const void*)k.row_close, k.row_smem)) ||
         (rc = lim((const void*)k.row_ekin, k.row_smem)) || (rc = lim((const void*)k.axis_one, k.col_smem)) ||
         (rc = lim((const void*)k.axis_fpi, k.col_smem)) || (rc = lim((const void*)k.axis_ekin, k.col_smem)) ||
-        (rc = lim((const void*)k.axis_fft, k.col_smem)) || (rc = lim((const void*)k.row_fft, k.fft_smem)) ||
-        (rc = lim((const void*)k.line_step, k.n / k.line_ctas * (int)sizeof(double2))))
+        (rc = lim((const void*)k.axis_fft, k.col_smem)) || (rc = lim((const void*)k.row_fft, k.fft_smem)))
       return rc;
   }
+  if (int rc = init_line_table()) return rc;
   done = true;
   return QSF_OK;
 }
@@ -121,29 +121,6 @@ int init_kernel_table() {
 int grid_blocks(long long m) {
   long long b = (m + 255) / 256;
   return (int)std::min<long long>(std::max<long long>(b, 1), (long long)device_sm_count() * 16);
-}
-
-// One twiddle as the fixed-point FFT reads it.  With pre-split tables (QSF_TWQ) each
-// component w becomes its signed 32-bit halves {lo = (int)w, hi} (the bytes of an int4
-// {re lo, re hi, im lo, im hi}); a component whose low half would be -2^31 moves one
-// unit (2^-62) so that the kernels can negate the halves.
-longlong2 split_twiddle(longlong2 w) {
-#if QSF_TWQ
-  int q[4];
-  const long long c[2] = {w.x, w.y};
-  for (int k = 0; k < 2; ++k) {
-    long long v = c[k];
-    if ((v & 0xffffffffLL) == 0x80000000LL) v += 1;
-    const int lo = k_lo(v), hi = k_hi(v);
-    q[2 * k] = lo;
-    q[2 * k + 1] = hi;
-  }
-  longlong2 out;
-  std::memcpy(&out, q, sizeof out);
-  return out;
-#else
-  return w;
-#endif
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against the
@@ -213,7 +190,7 @@ void qsf::launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd
   for (int k = 0; k < kMaxDim; ++k) V.tmap[k] = nullptr;  // G.psi need not be the mapped array
   const long long n = G.ax[ax].n, lines = G.m / n;
   if (ax == G.dim - 1) {
-    const int blocks = K.fft_ctas > 1 ? K.fft_ctas : (int)((lines + K.fft_lines - 1) / K.fft_lines);
+    const int blocks = (int)((lines + K.fft_lines - 1) / K.fft_lines);
     K.row_fft<<<blocks, K.fft_threads, K.fft_smem, st>>>(V, fwd, sc);
   } else {
     const long long inner = G.ax[ax].stride, outer = lines / inner;
@@ -224,90 +201,56 @@ void qsf::launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd
 
 bool qsf::fused_length(int n) { return init_kernel_table() == QSF_OK && kernels_for(n) != nullptr; }
 
-// FP64, 2^62 fixed-point and split-form twiddles exp(-2 pi i t / n), t < n
-int qsf::make_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf) {
-  std::vector<double2> h((size_t)n);
-  std::vector<longlong2> hx((size_t)n), hf((size_t)n);
-  const long double twopi = 6.283185307179586476925286766559005768L;
-  const long double q62 = 4611686018427387904.0L;
-  for (int t = 0; t < n; ++t) {
-    const long double ang = twopi * (long double)t / (long double)n;
-    const long double c = cosl(ang), sn = -sinl(ang);
-    h[(size_t)t] = make_double2((double)c, (double)sn);
-    hx[(size_t)t] = make_longlong2(llroundl(c * q62), llroundl(sn * q62));
-    hf[(size_t)t] = split_twiddle(hx[(size_t)t]);
+// exp(-2 pi i t / n) 2^-r in the split form of the kernels (2^62 fixed point, the signed
+// 32-bit halves of each component; a component whose low half would be -2^31 moves one
+// unit, 2^-62, so that the kernels can negate the halves).  The angle is reduced to the
+// first octant.
+int4 qsf::split_root(long long t, long long n, int r) {
+  t %= n;
+  long double c, s;
+  const long long o = 8 * t / n;  // octant
+  const long double a = 6.283185307179586476925286766559005768L;
+  // distance to the octant's axis, as a fraction of n / 8 turns
+  auto base = [&](long long num) { return a * (long double)num / (8.0L * (long double)n); };
+  switch (o) {
+    case 0: c = cosl(base(8 * t)); s = sinl(base(8 * t)); break;
+    case 1: c = sinl(base(2 * n - 8 * t)); s = cosl(base(2 * n - 8 * t)); break;
+    case 2: c = -sinl(base(8 * t - 2 * n)); s = cosl(base(8 * t - 2 * n)); break;
+    case 3: c = -cosl(base(4 * n - 8 * t)); s = sinl(base(4 * n - 8 * t)); break;
+    case 4: c = -cosl(base(8 * t - 4 * n)); s = -sinl(base(8 * t - 4 * n)); break;
+    case 5: c = -sinl(base(6 * n - 8 * t)); s = -cosl(base(6 * n - 8 * t)); break;
+    case 6: c = sinl(base(8 * t - 6 * n)); s = -cosl(base(8 * t - 6 * n)); break;
+    default: c = cosl(base(8 * n - 8 * t)); s = -sinl(base(8 * n - 8 * t)); break;
   }
-  *tw = nullptr;
-  *twx = *twf = nullptr;
-  int rc;
-  if ((rc = dev_alloc(*tw, h.size())) || (rc = dev_alloc(*twx, hx.size())) || (rc = dev_alloc(*twf, hf.size()))) {
-    if (*tw) cudaFree(*tw);
-    if (*twx) cudaFree(*twx);
-    *tw = nullptr;
-    *twx = nullptr;
-    return rc;
-  }
-  QSF_CU(cudaMemcpy(*tw, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
-  QSF_CU(cudaMemcpy(*twx, hx.data(), hx.size() * sizeof(longlong2), cudaMemcpyHostToDevice));
-  QSF_CU(cudaMemcpy(*twf, hf.data(), hf.size() * sizeof(longlong2), cudaMemcpyHostToDevice));
-  // a pageable copy may return before its transfer lands; the tables are shared by
-  // every stream, so wait for the device
-  QSF_CU(cudaDeviceSynchronize());
-  return QSF_OK;
+  const long double one = ldexpl(1.0L, 62 - r);
+  long long q[2] = {llroundl(c * one), llroundl(-s * one)};
+  for (long long& v : q)
+    if ((v & 0xffffffffLL) == 0x80000000LL) v += 1;
+  return make_int4(k_lo(q[0]), k_hi(q[0]), k_lo(q[1]), k_hi(q[1]));
 }
 
-// Twiddle tables of a length, made once per process and device and shared by every
-// grid (never freed: one set per built length, at most a few MB in all).
-int qsf::shared_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf) {
+// Per-pass twiddles of a line plan (qsf_lines.cuh): kTwVar copies, copy r scaled by 2^-r;
+// pass p's entry [(q - 1) ns + jm] = exp(-2 pi i jm q / (ns R)).  Made once per length,
+// plan, process and device and shared by every grid (never freed: a few MB in all).
+int qsf::shared_line_twiddles(int n, int ppt, const int4** out) {
   static std::mutex mu;
-  static std::map<std::pair<int, int>, std::array<void*, 3>> cache;
+  static std::map<std::array<int, 3>, int4*> cache;
+  *out = nullptr;
+  const LinePlan P = line_plan(n, ppt);
   int dev = 0;
   QSF_CU(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
-  auto it = cache.find({dev, n});
+  auto it = cache.find({dev, n, ppt});
   if (it == cache.end()) {
-    double2* a = nullptr;
-    longlong2 *b = nullptr, *c = nullptr;
-    if (int rc = make_twiddles(n, &a, &b, &c)) return rc;
-    it = cache.emplace(std::make_pair(dev, n), std::array<void*, 3>{a, b, c}).first;
-  }
-  *tw = (double2*)it->second[0];
-  *twx = (longlong2*)it->second[1];
-  *twf = (longlong2*)it->second[2];
-  return QSF_OK;
-}
-
-// Per-pass twiddles of a length's line plans (qsf_lines.cuh): kTwVar copies each, copy r
-// scaled by 2^-r; pass p's entry [(q - 1) ns + jm] = exp(-2 pi i jm q / (ns R)) in split
-// form.  Made once per length, process and device and shared by every grid.
-int qsf::shared_line_twiddles(const KernelSet& K, const int4* out[2]) {
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, std::array<int4*, 2>> cache;
-  out[0] = out[1] = nullptr;
-  if (!K.plan[0]) return QSF_OK;
-  int dev = 0;
-  QSF_CU(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = cache.find({dev, K.n});
-  if (it == cache.end()) {
-    const long double twopi = 6.283185307179586476925286766559005768L;
-    std::vector<longlong2> h;
-    size_t second = 0;
-    for (int plan = 0; plan < 2; ++plan) {
-      for (int r = 0; r < kTwVar; ++r) {
-        const long double one = ldexpl(1.0L, 62 - r);
-        long long ns = K.plan[plan][0];
-        for (int p = 1; K.plan[plan][p]; ++p) {
-          const int R = K.plan[plan][p];
-          for (int q = 1; q < R; ++q)
-            for (long long jm = 0; jm < ns; ++jm) {
-              const long double ang = twopi * (long double)((jm * q) % (ns * R)) / (long double)(ns * R);
-              h.push_back(split_twiddle(make_longlong2(llroundl(cosl(ang) * one), llroundl(-sinl(ang) * one))));
-            }
-          ns *= R;
-        }
+    std::vector<int4> h;
+    for (int r = 0; r < kTwVar; ++r) {
+      long long ns = P.r[0];
+      for (int p = 1; p < P.S; ++p) {
+        const int R = P.r[p];
+        for (int q = 1; q < R; ++q)
+          for (long long jm = 0; jm < ns; ++jm) h.push_back(split_root(jm * q, ns * R, r));
+        ns *= R;
       }
-      if (plan == 0) second = h.size();
     }
     int4* d = nullptr;
     if (int rc = dev_alloc(d, h.size() + 1)) return rc;
@@ -318,11 +261,18 @@ int qsf::shared_line_twiddles(const KernelSet& K, const int4* out[2]) {
       cudaFree(d);
       return fail(QSF_ECUDA, std::string("line twiddles: ") + cudaGetErrorString(ce));
     }
-    it = cache.emplace(std::make_pair(dev, K.n), std::array<int4*, 2>{d, d + second}).first;
+    it = cache.emplace(std::array<int, 3>{dev, n, ppt}, d).first;
   }
-  out[0] = it->second[0];
-  out[1] = it->second[1];
+  *out = it->second;
   return QSF_OK;
+}
+
+// the twiddles of both line plans of a built length (none above 8192 points)
+int qsf::axis_twiddles(int n, const int4* out[2]) {
+  out[0] = out[1] = nullptr;
+  if (n > 8192) return QSF_OK;
+  if (int rc = shared_line_twiddles(n, 8, &out[0])) return rc;
+  return shared_line_twiddles(n, 16, &out[1]);
 }
 
 namespace {
@@ -477,7 +427,7 @@ int ensure_flux(qsf_grid* g, int nb, const int* types, int64_t box) {
   for (long long p : need) rp[(size_t)(p / nlast) + 1]++;
   for (long long r = 0; r < nrows; ++r) rp[(size_t)r + 1] += rp[(size_t)r];
   int rc;
-  if ((rc = dev_alloc(g->snap, std::max<size_t>(need.size(), 1)))) return rc;
+  if ((rc = dev_alloc(g->snap, std::max<size_t>(2 * need.size(), 1)))) return rc;  // 1D: two sets
   if ((rc = dev_alloc(g->snap_idx, std::max<size_t>(need.size(), 1)))) return rc;
   if ((rc = dev_alloc(g->row_ptr, rp.size()))) return rc;
   if ((rc = dev_alloc(g->fpts, std::max<size_t>(fps.size(), 1)))) return rc;
@@ -598,16 +548,16 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
   // (kind, axis) tables (X tables only in the length gauge), ~128 entries per block
   const int tb = std::max(1, std::min(64, q.nmax / 128));
   const dim3 gt(D * 4 * tb, count);
-  // a one-CTA line kernel also ends the step itself (its fluxes, row and counters); the
-  // tables stay a kernel of their own: their FP64 phases want many SMs
-  const bool full = D == 1 && K.line_full;
+  if (D == 1) {  // the line kernels end their steps themselves
+    const LineKernels& L = *line_kernels(q.n);
+    QSF_TIMED(QSF_K_TABLES, (rc = line_launch_tables(L, dG, dS, count, 1, q.gauge == QSF_GAUGE_LENGTH, st)));
+    if (rc) return rc;
+    QSF_TIMED(QSF_K_LINE_STEP, (rc = line_launch_steps(L, false, dG, dS, count, 1, st)));
+    return rc;
+  }
   QSF_TIMED(QSF_K_TABLES, (k_tables<<<gt, 256, 0, st>>>(dG, dS, tb)));
   const bool wait_fin = ov && ov->pending;
-  if (D == 1) {
-    if (wait_fin) QSF_CU(cudaStreamWaitEvent(st, ov->done, 0));
-    QSF_TIMED(QSF_K_LINE_STEP, (K.line_step<<<dim3(K.line_ctas, count), K.line_threads,
-                                               (size_t)(q.n / K.line_ctas) * sizeof(double2), st>>>(dG, dS)));
-  } else {
+  {
     const dim3 gr(q.nrowblk, count);
     if (with_open) QSF_TIMED(QSF_K_ROW_OPEN, (K.row_open<<<gr, K.row_threads, K.row_smem, st>>>(dG, dS)));
     if (D == 3)
@@ -625,14 +575,14 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
     }
   }
   if (ov) ov->pending = false;
-  if (!full && ov) {
+  if (ov) {
     QSF_CU(cudaEventRecord(ov->fork, st));
     QSF_CU(cudaStreamWaitEvent(ov->side, ov->fork, 0));
     k_finalize<<<dim3(nfblk, count), 256, 0, ov->side>>>(dG, dS);
     QSF_CU(cudaGetLastError());
     QSF_CU(cudaEventRecord(ov->done, ov->side));
     ov->pending = true;
-  } else if (!full) {
+  } else {
     QSF_TIMED(QSF_K_FINALIZE, (k_finalize<<<dim3(nfblk, count), 256, 0, st>>>(dG, dS)));
   }
 #undef QSF_TIMED
@@ -662,7 +612,7 @@ int ensure_fin_stream(qsf_grid* g, FinOverlap* ov) {
 // Validates a step program and stages everything a run of it needs on the device:
 // static tables for dt/2, flux point lists, coupling rows, observables rows, control
 // words; fills the step descriptor and uploads it to g->dS.
-int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_out) {
+int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_out, int64_t chunk = INT64_MAX) {
   if (d->mode != QSF_MODE_IM && d->mode != QSF_MODE_RE) return fail(QSF_EINVAL, "mode must be IM or RE");
   if (d->nsteps < 1) return fail(QSF_EINVAL, "nsteps < 1");
   if (d->nborders < 0 || d->nborders > QSF_MAX_BORDERS) return fail(QSF_EINVAL, "too many borders");
@@ -691,7 +641,7 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   }
   long long ctl_h[8] = {0, (long long)total, 0, 0, 0, 0, 0, 0};
   double en_h[2] = {d->last_energy, 0.0};
-  double sc_h[2] = {1.0, 1.0};
+  double sc_h[4] = {1.0, 1.0, 1.0, 1.0};
   QSF_CU(cudaMemcpyAsync(g->ctl, ctl_h, sizeof(ctl_h), cudaMemcpyHostToDevice, g->stream));
   QSF_CU(cudaMemcpyAsync(g->energy, en_h, sizeof(en_h), cudaMemcpyHostToDevice, g->stream));
   QSF_CU(cudaMemcpyAsync(g->scale, sc_h, sizeof(sc_h), cudaMemcpyHostToDevice, g->stream));
@@ -734,6 +684,7 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   S.nborders = nb;
   if (want_flux) {
     S.snap = g->snap;
+    S.nsnap = g->nsnap;
     S.row_ptr = g->row_ptr;
     S.snap_idx = g->snap_idx;
     S.fpts = g->fpts;
@@ -745,6 +696,7 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   S.energy_state = g->energy;
   S.rows = g->rows_dev;
   S.scale = g->scale;
+  if (G.dim == 1 && (rc = line_prepare(g, S, chunk))) return rc;
   QSF_CU(cudaMemcpyAsync(g->dS, &S, sizeof(StepDev), cudaMemcpyHostToDevice, g->stream));
   *out = S;
   *ncol_out = ncol;
@@ -960,7 +912,7 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   // lengths without fused kernels (not in the built list, or with a prime factor above
   // 5) take Bluestein transforms and the member-operation step
   const KernelSet* ks = kernels_for((int)d->n[0]);
-  if (!ks && !bs_size((int)d->n[0], d->dim))
+  if (!ks && !(d->dim == 1 ? line_conv_length((int)d->n[0]) : bs_size((int)d->n[0], d->dim)))
     return fail(QSF_EINVAL, "grid size " + std::to_string(d->n[0]) + " has no kernels and no Bluestein length in "
                             "this build (1D lines up to 8192 points, other grids up to 2048 points per axis)");
   qsf_grid* g = new qsf_grid();
@@ -986,8 +938,6 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
     G.ax[k].stride = s;
     s *= d->n[k];
   }
-  std::map<int64_t, double2*> tws;
-  std::map<int64_t, longlong2*> twxs, twfs;
   for (int k = 0; k < d->dim; ++k) {
     AxisDev& a = G.ax[k];
     a.n = (int)d->n[k];
@@ -999,38 +949,13 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
     a.xmin = -0.5 * L;
     a.inv_2dx = (1.0 / d->dx[k]) / 2.0;
     a.dp = 2.0 * M_PI / (double)d->n[k] / d->dx[k];
-    auto it = tws.find(a.n);
-    if (!ks) {
-      // Bluestein lengths run no n-point transform kernel: no n-point twiddles
-      a.tw = nullptr;
-      a.twx = nullptr;
-      a.twf = nullptr;
-    } else if (it == tws.end()) {
-      double2* dptr = nullptr;
-      longlong2 *xptr = nullptr, *fptr = nullptr;
-      if (int rc = shared_twiddles(a.n, &dptr, &xptr, &fptr)) {
-        qsf_grid_destroy(g);
-        return rc;
-      }
-      tws[a.n] = dptr;
-      twxs[a.n] = xptr;
-      twfs[a.n] = fptr;
-      a.tw = dptr;
-      a.twx = xptr;
-      a.twf = reinterpret_cast<decltype(a.twf)>(fptr);
-    } else {
-      a.tw = it->second;
-      a.twx = twxs[a.n];
-      a.twf = reinterpret_cast<decltype(a.twf)>(twfs[a.n]);
-    }
   }
   if (ks) {
-    const int4* twl[2];
-    if (int rc = shared_line_twiddles(*ks, twl)) {
+    if (int rc = axis_twiddles(G.ax[0].n, G.ax[0].twl)) {
       qsf_grid_destroy(g);
       return rc;
     }
-    for (int k = 0; k < d->dim; ++k) std::copy(twl, twl + 2, G.ax[k].twl);
+    for (int k = 1; k < d->dim; ++k) std::copy(G.ax[0].twl, G.ax[0].twl + 2, G.ax[k].twl);
   }
   G.inv_m = 1.0 / (double)G.m;
   G.dVm = G.dV * G.inv_m;
@@ -1072,7 +997,7 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
       }
     }
   } else {
-    g->nrowblk = ks ? ks->line_ctas : 1;  // partial sums per CTA of the line
+    g->nrowblk = 1;
   }
   g->nmax = 0;
   for (int k = 0; k < D; ++k) g->nmax = std::max(g->nmax, G.ax[k].n);
@@ -1083,13 +1008,14 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   while ((1LL << (g->l2m + 1)) <= G.m) ++g->l2m;
   g->m_mant = std::ldexp(1.0, g->l2m) / (double)G.m;
   if ((rc = dev_alloc(g->partials, (size_t)5 * g->pmax)) || (rc = dev_alloc(g->ctl, 8)) ||
-      (rc = dev_alloc(g->energy, 2)) || (rc = dev_alloc(g->scale, 2)) ||
+      (rc = dev_alloc(g->energy, 2)) || (rc = dev_alloc(g->scale, 4)) ||
       (rc = dev_alloc(g->fpartials, (size_t)kMaxFluxBlocks * kMaxFluxBorders))) {
     qsf_grid_destroy(g);
     return rc;
   }
   // the fused kernels' exponent slots, per-step tables and device descriptors
-  if (ks && ((rc = dev_alloc(g->ibuf, (size_t)kTexp + kGmin + 4 * (size_t)g->scmax)) ||
+  const bool fused = ks || D == 1;
+  if (fused && ((rc = dev_alloc(g->ibuf, (size_t)kTexp + kGmin + 4 * (size_t)g->scmax)) ||
              (rc = dev_alloc(g->ptab, (size_t)D * g->nmax)) ||
              (rc = dev_alloc(g->xdyn, (size_t)3 * D * g->nmax)) || (rc = dev_alloc(g->dG, 1)) ||
              (rc = dev_alloc(g->dS, 1)))) {
@@ -1097,11 +1023,11 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
     return rc;
   }
   g->fpmax = (size_t)kMaxFluxBlocks * kMaxFluxBorders;
-  if ((rc = ks ? make_tensor_maps(g) : bs_setup(g))) {
+  if ((rc = D == 1 ? line_setup(g) : ks ? make_tensor_maps(g) : bs_setup(g))) {
     qsf_grid_destroy(g);
     return rc;
   }
-  if (ks) cudaMemcpyAsync(g->dG, &g->G, sizeof(GridDev), cudaMemcpyHostToDevice, g->stream);
+  if (fused) cudaMemcpyAsync(g->dG, &g->G, sizeof(GridDev), cudaMemcpyHostToDevice, g->stream);
   cudaMemsetAsync(g->partials, 0, sizeof(double) * 5 * g->pmax, g->stream);
   if (cudaStreamSynchronize(g->stream) != cudaSuccess) {
     qsf_grid_destroy(g);
@@ -1148,6 +1074,7 @@ int qsf_grid_destroy(qsf_grid* g) {
   if (g->gen_exec) cudaGraphExecDestroy(g->gen_exec);
   fr(g->tmaps);
   bs_release(g);
+  line_release(g);
   if (g->mg_event) cudaEventDestroy(g->mg_event);
   if (g->fin_fork) cudaEventDestroy(g->fin_fork);
   if (g->fin_done) cudaEventDestroy(g->fin_done);
@@ -1224,7 +1151,9 @@ int qsf_fourier(qsf_grid* g, int to_rep) {
   for (int ax = D - 1; ax >= 0; --ax) {
     if ((G.free_mask >> ax) & 1) continue;
     const double post = ax == last && !fwd ? back : 1.0;
-    if (g->ks) {
+    if (D == 1 && (!g->ks || !g->ks->row_fft)) {
+      if (int rc = line_fourier(g, G, fwd, post)) return rc;
+    } else if (g->ks) {
       axis_fft(g, G, ax, fwd, post);
     } else if (int rc = bs_axis(g, g->G.psi, ax, fwd, post)) {
       return rc;
@@ -1263,7 +1192,9 @@ int qsf_region_transfer(qsf_grid* dst, const qsf_grid* src, int axis, int group)
                                                         dst->nmax);
   GridDev Gs = G;
   Gs.psi = dst->mg_slice;
-  if (dst->ks) axis_fft(dst, Gs, axis, true, 1.0);
+  if (G.dim == 1 && (!dst->ks || !dst->ks->row_fft)) {
+    if (int rc = line_fourier(dst, Gs, true, 1.0)) return rc;
+  } else if (dst->ks) axis_fft(dst, Gs, axis, true, 1.0);
   else if (int rc = bs_axis(dst, dst->mg_slice, axis, true, 1.0)) return rc;
   k_add_slice<<<grid_blocks(G.m), 256, 0, dst->stream>>>(G.psi, dst->mg_slice, G.m);
   QSF_CU(cudaGetLastError());
@@ -1434,14 +1365,43 @@ int qsf_add_gaussian(qsf_grid* g, double at, double delta) {
 
 static int generic_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_done);
 
+// `count` sub-steps of a 1D program, a launch pair per run of sub-steps that has tables;
+// with `ms` one sub-step per launch, each timed
+static int line_run(qsf_grid* g, const StepDev& S, int64_t count, float* ms, int64_t* launches) {
+  const LineKernels& L = *g->lk;
+  const bool lg = g->G.gauge == QSF_GAUGE_LENGTH;
+  Prof P;
+  int rc = QSF_OK;
+  if (ms) {
+    P.ms = ms;
+    P.count = launches;
+    rc = P.init(g->stream, (int)std::min<int64_t>(count * 2 + 2, 1 << 20));
+  }
+  for (int64_t k = 0; k < count && rc == QSF_OK;) {
+    const int now = ms ? 1 : (int)std::min<int64_t>(g->l_steps, count - k);
+    if ((rc = P.begin()) || (rc = line_launch_tables(L, g->dG, g->dS, 1, now, lg, g->stream)) ||
+        (rc = P.end(QSF_K_TABLES)) || (rc = P.begin()) ||
+        (rc = line_launch_steps(L, S.line.bs, g->dG, g->dS, 1, now, g->stream)) || (rc = P.end(QSF_K_LINE_STEP)))
+      break;
+    k += now;
+  }
+  if (rc == QSF_OK) rc = P.flush();
+  P.release();
+  return rc;
+}
+
 int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_done) {
   if (!g || !d) return fail(QSF_EINVAL, "null argument");
   if (steps_done) *steps_done = 0;
   if (d->nsteps == 0) return QSF_OK;
-  if (!g->ks) return generic_step(g, d, rows, steps_done);
+  if (!g->ks && g->G.dim > 1) return generic_step(g, d, rows, steps_done);
   StepDev S{};
   int ncol = 0, rc;
   if ((rc = prepare_step(g, d, &S, &ncol))) return rc;
+  if (g->G.dim == 1) {
+    if ((rc = line_run(g, S, S.nsteps, d->kernel_ms, d->kernel_launches))) return rc;
+    return finish_step(g, d->normalize, d->nsteps, ncol, rows, steps_done);
+  }
   if (d->kernel_ms) {
     // one event pair per launch of the whole call (at most 8 per step), read at the end,
     // so the profiled call has no host synchronisation between its steps
@@ -1550,7 +1510,7 @@ static int generic_ncol(const qsf_step_desc* d) {
 
 }  // extern "C"
 
-bool qsf::grid_fused(const qsf_grid* g) { return g->ks != nullptr; }
+bool qsf::grid_batched(const qsf_grid* g) { return g->ks && g->G.dim > 1; }
 
 // psi = 0, ordered on the grid's stream (a memset on another stream would not be
 // ordered before the grid's later work)
@@ -1572,6 +1532,14 @@ static std::vector<long long> generic_key(const qsf_grid* g, const qsf_step_desc
 
 int qsf::generic_begin(qsf_grid* g, const qsf_step_desc* d) {
   int rc;
+  if (g->G.dim == 1) {
+    int ncol = 0;
+    if ((rc = prepare_step(g, d, &g->l_S, &ncol))) return rc;
+    QSF_CU(cudaMemsetAsync(g->rows_dev, 0, (size_t)d->nsteps * ncol * sizeof(double), g->stream));
+    // the descriptors come from this frame's memory
+    QSF_CU(cudaStreamSynchronize(g->stream));
+    return QSF_OK;
+  }
   if ((rc = generic_check(g, d))) return rc;
   const int ncol = generic_ncol(d);
   const int K = std::max(1, d->substeps), cs = g->G.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
@@ -1670,6 +1638,7 @@ static int generic_prime(qsf_grid* g, const qsf_step_desc* d) {
 int qsf::generic_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count) {
   constexpr int kGenGraphSteps = QSF_GEN_GRAPH_STEPS;
   if (first < 0 || count < 0 || first + count > d->nsteps) return fail(QSF_EINVAL, "steps outside the program");
+  if (g->G.dim == 1) return line_run(g, g->l_S, count * std::max(1, d->substeps), nullptr, nullptr);
   int rc;
   int64_t s = first;
   const int64_t end = first + count;
@@ -1809,7 +1778,7 @@ int qsf::batch_add_nowait(qsf_batch* b, qsf_grid* g, const qsf_step_desc* d, int
   dd.kernel_ms = nullptr;
   dd.kernel_launches = nullptr;
   int rc;
-  if ((rc = prepare_step(g, &dd, &mb.S, &mb.ncol))) return rc;
+  if ((rc = prepare_step(g, &dd, &mb.S, &mb.ncol, 1))) return rc;  // 1D members: one sub-step per launch
   QSF_CU(cudaStreamSynchronize(g->stream));
   mb.nsteps = d->nsteps;
   mb.normalize = d->normalize;

@@ -53,6 +53,8 @@ int dev_reserve(T*& p, size_t& cap, size_t count) {
 using qsf::AxisDev;
 using qsf::GridDev;
 using qsf::KernelSet;
+using qsf::LineDev;
+using qsf::LineKernels;
 using qsf::StepDev;
 using qsf::FluxPoint;
 using qsf::FluxTerm;
@@ -148,42 +150,41 @@ struct qsf_grid {
   bool gen_primed = false;
   // TMA tensor maps of psi for the strided-axis passes (GridDev::tmap), 128 bytes each
   unsigned char* tmaps = nullptr;
-  // Bluestein transforms of a grid whose axis length has a prime factor above 5 (no
+  // Bluestein transforms of a 2D / 3D grid whose axis length has a prime factor above 5 (no
   // fused kernels, ks == nullptr): chirp c[j] = exp(-i pi j^2 / n), the transform of
   // the convolution kernel conj(c) padded to M (a length >= 2n - 1 with built
   // kernels), the M-point kernels and twiddles, and a scratch of (m / n) * M points.
-  // A 1D line longer than 8192 points takes M = M1 * M2 above 16384 as a four-step
-  // transform: M1-point transforms along the columns of the [M1][M2] view, the twiddles
-  // exp(-2 pi i k1 n2 / M), M2-point transforms along its rows (the output in the
-  // transposed order [k1][k2] = X[k1 + M1 k2], which the convolution does not mind).
   struct Bluestein {
     int n = 0, M = 0;
-    int M1 = 0, M2 = 0;  // four-step factors; 0: one M-point transform per line
-    const KernelSet* ks = nullptr;   // M-point kernels (or M2-point row kernels)
-    const KernelSet* ks1 = nullptr;  // M1-point column kernels (four-step)
+    const KernelSet* ks = nullptr;  // M-point kernels
     double2* chirp = nullptr;
     double2* bhat = nullptr;
     double2* scratch = nullptr;
-    // shared per-process tables (not owned by the grid)
-    double2* tw = nullptr;  // twiddles of M (or M2)
-    longlong2* twx = nullptr;
-    longlong2* twf = nullptr;
-    double2* tw1 = nullptr;  // twiddles of M1
-    longlong2* twx1 = nullptr;
-    longlong2* twf1 = nullptr;
-    double2* tw4 = nullptr;  // four-step twiddles [k1][n2]
-    const int4* twl[2] = {};   // line-plan twiddles of M (or M2)
-    const int4* twl1[2] = {};  // and of M1
+    const int4* twl[2] = {};  // line-plan twiddles of M (shared)
   } bs;
+  // 1D grids (qsf_line1d.cu): the step kernels, their geometry tables, the tables of a run of sub-steps and the current program
+  const LineKernels* lk = nullptr;
+  LineDev line{};
+  long long* l_sub0 = nullptr;
+  int4 *l_chirp = nullptr, *l_bhat = nullptr, *l_xab = nullptr;
+  int lx_mode = 0;
+  double lx_delta = 0.0;
+  int4 *l_ptab = nullptr, *l_ctab = nullptr;
+  int* l_texp = nullptr;
+  size_t l_ptab_cap = 0, l_ctab_cap = 0, l_texp_cap = 0;
+  int l_steps = 1;  // sub-steps the tables hold
+  StepDev l_S{};
 };
 
 namespace qsf {
 // whether n is a line length with fused step kernels in this build
 bool fused_length(int n);
-bool grid_fused(const qsf_grid* g);
+// whether the grid's solves run in batches (the others run on their own streams)
+bool grid_batched(const qsf_grid* g);
 // psi = 0 on the grid's stream
 int grid_clear(qsf_grid* g);
-// Member-operation steps of a grid without fused kernels (qsf_step's path for them),
+// Steps of a grid that is not batched: member operations of a 2D / 3D grid without fused
+// kernels (qsf_step's path for them), runs of the 1D kernels,
 // in parts for the server: begin checks the program and zeroes its device rows and
 // NaN flag; enqueue queues steps [first, first + count) on the grid's stream without
 // waiting (no convergence test); wait waits for the stream and reads the NaN flag;
@@ -200,13 +201,24 @@ int batch_add_nowait(qsf_batch* b, qsf_grid* g, const qsf_step_desc* d, int64_t*
 // steps' graph launches) and finish (wait, read every member's counters)
 int batch_launch(qsf_batch* b, int64_t steps);
 int batch_finish(qsf_batch* b, int64_t* active);
-// twiddle tables of an n-point transform shared by all grids of the process (not to
-// be freed by the caller)
-int shared_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf);
-// twiddle tables of an n-point transform (FP64, 2^62 fixed point, split form)
-int shared_line_twiddles(const KernelSet& K, const int4* out[2]);
+// exp(-2 pi i t / n) 2^-r in the split form of the kernels
+int4 split_root(long long t, long long n, int r);
+// device twiddles of the line plan (n, ppt), and of both plans of a built length; shared
+// by all grids of the process (not to be freed by the caller)
+int shared_line_twiddles(int n, int ppt, const int4** out);
+int axis_twiddles(int n, const int4* out[2]);
 void launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd, double sc, cudaStream_t st);
-int make_twiddles(int n, double2** tw, longlong2** twx, longlong2** twf);
+// 1D grids (qsf_line1d.cu)
+int init_line_table();
+int line_conv_length(int n);  // convolution length of an n-point line (0: none)
+int line_setup(qsf_grid* g);
+void line_release(qsf_grid* g);
+int line_prepare(qsf_grid* g, StepDev& S, int64_t chunk);
+int line_launch_tables(const LineKernels& L, const GridDev* dG, const StepDev* dS, int count, int steps, bool lg,
+                       cudaStream_t st);
+int line_launch_steps(const LineKernels& L, bool bs, const GridDev* dG, const StepDev* dS, int count, int steps,
+                      cudaStream_t st);
+int line_fourier(qsf_grid* g, const GridDev& G, bool fwd, double sc);
 // Bluestein plan of a grid without fused kernels (qsf_bluestein.cu)
 int bs_setup(qsf_grid* g);
 void bs_release(qsf_grid* g);

@@ -15,8 +15,8 @@
 //   k_finalize    deterministic reductions, border fluxes, Normalize scale,
 //                 imaginary-time convergence, step counter
 //
-// For dim == 1 the whole step is one kernel (k_line_step) over a line held in
-// shared memory.  A device step counter lets one captured CUDA graph replay any step.
+// For dim == 1 a run of whole steps is one kernel (k_line_run, qsf_line1d.cuh).  A
+// device step counter lets one captured CUDA graph replay any step.
 // Step kernels read their grid and step descriptors from device arrays indexed by
 // blockIdx.y, so one launch per stage advances every solve of a batch that shares
 // the line length (a single grid is a batch of one).
@@ -40,46 +40,12 @@
 namespace qsf {
 
 constexpr int kMaxDim = 3;
-constexpr int kLinePptDiv = 512;  // threads of the one-CTA line kernel (kLineThreads)
-// Points per thread of the one-CTA line kernel (512 threads, one line of n points): a
-// line shorter than 8192 points leaves threads idle in radix-16 passes, and with one
-// CTA per line the per-thread work sets the step's latency, so shorter lines take
-// smaller radices; the choice per length comes from the autotuner (tuned_line_ppt,
-// qsf_tuning.h).  At least n / 512 points per thread (the line must fit the threads);
-// the autotuner's candidate builds force one value with QSF_LINE_PPT.
-#ifdef QSF_LINE_PPT
-__host__ __device__ constexpr int line_ppt(int n) { return n / kLinePptDiv > QSF_LINE_PPT ? n / kLinePptDiv : QSF_LINE_PPT; }
-#else
-__host__ __device__ constexpr int line_ppt(int n) {
-  return n / kLinePptDiv > tuned_line_ppt(n) ? n / kLinePptDiv : tuned_line_ppt(n);
-}
-#endif
-constexpr int kLineThreads = 512;
 constexpr int kMaxFluxBorders = 16;
-// 1D lines of 1024 .. 8192 points (powers of two): one step spread over a cluster of
-// CTAs (k_line_step_mc) instead of one CTA.  Off by default: measured on GB300 it was
-// slower than the one-CTA line kernel (4096 points 0.095 vs 0.073 ms per step, 1024
-// 0.071 ms, 2048 0.080 ms, 8192 0.104 ms; every distributed-shared-memory access and
-// the two cluster barriers per pass cost more than the per-SM work they spread)
-#ifndef QSF_LINE_CLUSTER
-#define QSF_LINE_CLUSTER 0
-#endif
-// resident blocks per SM the FFT kernels are compiled for (caps registers per thread)
-#ifndef QSF_FFT_MIN_BLOCKS
-#define QSF_FFT_MIN_BLOCKS 2
-#endif
 struct AxisDev {
   int n, n2;
   int shift;  // log2(n) when n is a power of two, else -1
   long long stride;
   double dx, xmin, dp, inv_2dx;
-  const double2* tw;     // exp(-2 pi i t / n), t < n
-  const longlong2* twx;  // the same twiddles in 2^62 fixed point
-#if QSF_TWQ
-  const int4* twf;  // the 2^62 twiddles as signed 32-bit halves (fmul_tw), read by fft_fx
-#else
-  const longlong2* twf;
-#endif
   const int4* twl[2];  // per-pass twiddle tables of the 8- and the 16-point line plan (qsf_lines.cuh), kTwVar copies
 };
 
@@ -134,6 +100,25 @@ __device__ __forceinline__ void coup_load(const CoupDev& cd, double* cv) {
   cv[2] = p[2];
 }
 
+struct LineDev {
+  int n1, n2, ctas, nth, epp;  // factors (n2 == 0: one line), CTAs, worker threads per CTA, points per thread
+  int t1, t2;                  // threads per line of either layout
+  int bs;                      // Bluestein: M-point convolution
+  const int4 *tw1, *tw2;       // pass twiddles of the lines of either layout
+  const int4 *w1, *w2;         // exp(-2 pi i k1 n2 / N) as [n2][k1] and [k1][n2]
+  const int4 *xa, *xb;         // static factors of the closing / the opening X half, natural order (Bluestein: times
+                               // the chirp, conjugated in xa)
+  const int4* bhat;            // Bluestein: transformed chirp times 2^-*bexp / M, [k1][k2]
+  const int* bexp;
+  const int4* chirp;           // Bluestein: exp(-i pi j^2 / n)
+  const int4* ptab;            // [sub-step][slot order] P phases (pstride 0: the same for every sub-step)
+  long long pstride;
+  const int4* ctab;            // length gauge: [steps + 1] opening, then [steps] closing x.E factors, slot order
+  int csteps;                  // steps of ctab
+  const int* texp;             // [sub-step][3] exponents of the P, opening and closing tables
+  long long* sub0;             // first sub-step the tables hold
+};
+
 struct StepDev {
   int mode;  // 1 IM, 2 RE
   double dt;
@@ -174,7 +159,8 @@ struct StepDev {
   int energy_after_normalize;
   double state_accuracy;
   int nborders;
-  double2* snap;              // snapshot slots
+  double2* snap;              // snapshot slots (1D: two sets, by the parity of the step)
+  int nsnap;
   const int* row_ptr;         // CSR over rows: snapshot entries of row r are [row_ptr[r], row_ptr[r+1])
   const long long* snap_idx;  // flat index per snapshot entry (sorted)
   const FluxPoint* fpts;
@@ -192,7 +178,8 @@ struct StepDev {
   long long* ctl;
   double* energy_state;  // [0] last E
   double* rows;          // [nsteps][3 + nborders]
-  double* scale;         // pending Normalize factor (1 when none)
+  double* scale;         // pending Normalize factor (1 when none); [2] its square as the 1D kernels carry it
+  LineDev line;          // 1D grids (qsf_line1d.cuh)
 };
 
 __device__ __forceinline__ bool step_active(const StepDev& S) { return S.ctl[0] <= S.ctl[1] && S.ctl[0] < S.nsteps; }
@@ -399,55 +386,11 @@ constexpr int kTexp = 12;
 constexpr int kGmin = 5;
 __device__ __forceinline__ int gmin_slot(int pass, long long sub) { return pass ? pass : ((sub & 1) ? 4 : 0); }
 
-// sum |x|^2 and sum V |x|^2 of fixed-point values, exact in 128-bit integers
-struct Acc128 {
-  unsigned long long lo;
-  long long hi;
-};
-__device__ __forceinline__ void acc_add(Acc128& a, unsigned long long lo, long long hi) {
-  const unsigned long long l = a.lo + lo;
-  a.hi += hi + (l < lo ? 1 : 0);
-  a.lo = l;
-}
-__device__ __forceinline__ double acc_value(const Acc128& a) {
-  return (double)a.hi * 18446744073709551616.0 + (double)a.lo;
-}
-
-// Norm and E_pot partial sums of a block of psi_n in fixed point (components below
-// 2^56 after the block's common shift q): |x|^2 exactly, V|x|^2 with |x|^2 >> 50 and V
-// in 2^vshift fixed point (|V| < 2^50 there).
-__device__ __forceinline__ void acc_point_v(Acc128& an, Acc128& av, longlong2 x, int q, long long v, bool epot) {
-  const long long xr = q ? fshift(x.x, -q) : x.x, xi = q ? fshift(x.y, -q) : x.y;
-  const unsigned long long ar = (unsigned long long)(xr < 0 ? -xr : xr), ai = (unsigned long long)(xi < 0 ? -xi : xi);
-  const unsigned long long l1 = ar * ar, l2 = ai * ai;
-  const unsigned long long lo = l1 + l2;
-  const unsigned long long hi = __umul64hi(ar, ar) + __umul64hi(ai, ai) + (lo < l1 ? 1ull : 0ull);
-  acc_add(an, lo, (long long)hi);
-  if (epot) {
-    const long long n2 = (long long)((hi << 14) | (lo >> 50));
-    acc_add(av, (unsigned long long)n2 * (unsigned long long)v, __mul64hi(n2, v));
-  }
-}
-__device__ __forceinline__ void acc_point(Acc128& an, Acc128& av, longlong2 x, int q, const long long* Vx, long long p,
-                                          bool epot) {
-  const long long xr = q ? fshift(x.x, -q) : x.x, xi = q ? fshift(x.y, -q) : x.y;
-  const unsigned long long ar = (unsigned long long)(xr < 0 ? -xr : xr), ai = (unsigned long long)(xi < 0 ? -xi : xi);
-  const unsigned long long l1 = ar * ar, l2 = ai * ai;
-  const unsigned long long lo = l1 + l2;
-  const unsigned long long hi = __umul64hi(ar, ar) + __umul64hi(ai, ai) + (lo < l1 ? 1ull : 0ull);
-  acc_add(an, lo, (long long)hi);
-  if (epot) {
-    const long long n2 = (long long)((hi << 14) | (lo >> 50));
-    const long long v = Vx[p];
-    acc_add(av, (unsigned long long)n2 * (unsigned long long)v, __mul64hi(n2, v));
-  }
-}
-
 // Phase factors (|components| <= 1) are stored in 2^62 fixed point as the signed
 // 32-bit halves of each component (int4 {re lo, re hi, im lo, im hi}, as the FFT's
 // twiddles), with every low half kept away from -2^31 so that it can be negated.  A
-// product x * f (fapply) returns x * f / 4 from twelve 32 x 32 -> 64-bit multiply-adds
-// (fmul_tw) and needs |x| < 2^61.
+// product x * f returns x * f / 4 from twelve 32 x 32 -> 64-bit multiply-adds (fmul_tw)
+// and needs |x| < 2^61.
 __device__ __forceinline__ int4 split62(double2 f) {
   long long a = __double2ll_rn(f.x * 4611686018427387904.0), b = __double2ll_rn(f.y * 4611686018427387904.0);
   if ((a & 0xffffffffLL) == 0x80000000LL) ++a;
@@ -459,37 +402,6 @@ __device__ __forceinline__ int4 split_fx(longlong2 v) {
   if ((v.y & 0xffffffffLL) == 0x80000000LL) ++v.y;
   return make_int4((int)v.x, split_hi(v.x), (int)v.y, split_hi(v.y));
 }
-// a * w / 2^64 for a real w given as its signed halves (wl, wh)
-__device__ __forceinline__ i64 mul_re(i64 a, int wl, int wh) {
-  const int al = (int)a, ah = split_hi(a);
-  const i64 m = (i64)ah * wl + (i64)al * wh + (1LL << 31);
-  return (m >> 32) + (i64)ah * wh;
-}
-// x * f / 4 (real f: imaginary-time X factors, only f's real part is read)
-__device__ __forceinline__ longlong2 fapply(longlong2 x, int4 f, bool real_f) {
-  return real_f ? make_longlong2(mul_re(x.x, f.x, f.y), mul_re(x.y, f.x, f.y)) : fmul_tw(x, f);
-}
-// x * 4 (renormalises after two products: the data stay below 2^61)
-__device__ __forceinline__ longlong2 fshl2(longlong2 x) {
-  return make_longlong2((i64)((u64)x.x << 2), (i64)((u64)x.y << 2));
-}
-// k factors applied in a row (fapply each, fshl2 after every second one that is
-// followed by another): the exponent the value moves by and a bound on the change of
-// its bit length (each product adds at most one bit, for the complex modulus)
-__host__ __device__ constexpr int xshift(int k) { return 2 * k - 2 * ((k - 1) / 2); }
-__host__ __device__ constexpr int xbits(int k) { return 2 * ((k - 1) / 2) - k; }
-
-// Largest exponent shift that brings a block whose largest component has `bits`
-// bits below 2^(62 - guard of the first pass of an N-point transform)
-template <int N>
-__device__ __forceinline__ int first_pass_shift(int bits) {
-  return bits == 0 ? 0 : (62 - fguard(radix_at(N, 0))) - bits;
-}
-// shift that brings a block's largest component to 61 bits before phase products: the
-// split products need |x| < 2^61 and return x * f / 4, so starting at the top keeps
-// their rounding (1 unit of the output) at 2^-59 of the block maximum
-__device__ __forceinline__ int product_headroom(int bits) { return bits ? 61 - bits : 0; }
-
 // value of one per-step table entry: kind 0 P phase (hamiltonian.h:52-58: kinetic and,
 // in the velocity gauge, A.k), kind 1 / 2 length-gauge x.E factor of the open / close
 // X half (hamiltonian.h:60-66 via DipoleCoupling), kind 3 the close half times the open
@@ -756,232 +668,12 @@ __global__ void __launch_bounds__(256) k_tables(const GridDev* __restrict__ Gs, 
 
 #endif  // QSF_DEFINE_KERNELS
 
-// Factors of the X half `half` (0 opens the step, 1 closes it, 2 opens the next
-// sub-step): the static factor and, in the length gauge, one x.E factor per axis.
-__device__ __forceinline__ int xfactors(const GridDev& g) { return 1 + (g.gauge == 1 ? g.dim : 0); }
-// The X half applied to x at point p (row r of the last axis, position j on it): the
-// factors one after another (fapply; fshl2 after the second when more follow), x below
-// 2^61.  NA is the length of the axes before the last one when known at compile time
-// (0: read it).  The value moves by xhalf_exp (bits <= in + xbits(xfactors(g))).
-template <int NA = 0>
-__device__ __forceinline__ longlong2 xhalf(const GridDev& g, const StepDev& S, longlong2 x, long long p, long long r,
-                                           int j, int half, bool real_f) {
-  x = fapply(x, S.xs[p], real_f);
-  if (g.gauge == 1) {
-    const int D = g.dim;
-    const int4* t = S.xdyn + (size_t)half * D * S.nmax;
-    x = fapply(x, t[(D - 1) * S.nmax + j], false);
-    long long rr = r;
-    int k = 2;
-    for (int dd = D - 2; dd >= 0; --dd) {
-      const long long n = NA ? NA : g.ax[dd].n;
-      const int ii = (int)(rr % n);
-      rr /= n;
-      if (k % 2 == 0) x = fshl2(x);
-      x = fapply(x, t[dd * S.nmax + ii], false);
-      ++k;
-    }
-  }
-  return x;
-}
-// exponent taken out of the factors of one half (their table exponents) plus the
-// exponent the k products move the value by
-__device__ __forceinline__ int xfactor_exp(const GridDev& g, const StepDev& S, int half) {
-  int e = S.xs_exp;
-  if (g.gauge == 1)
-    for (int d = 0; d < g.dim; ++d) e += S.texp[(1 + half) * 3 + d];
-  return e;
-}
-__device__ __forceinline__ int xhalf_exp(const GridDev& g, const StepDev& S, int half) {
-  return xfactor_exp(g, S, half) + xshift(xfactors(g));
-}
-
-// psi (double) -> fixed point: the block exponent from the largest biased exponent
-// em of the block puts the largest component at 61 bits (below 2^61, as the phase
-// products need; the pending Normalize factor is at most 1)
-template <int N>
-__device__ __forceinline__ int scale_from_exponent(int em) {
-  return 61 - (em - 1022);
-}
-
 // pending Normalize factor s = F 2^-62 * 2^k with F in [2^61, 2^62)
 __device__ __forceinline__ void split_scale(double s, long long& F, int& k) {
   int e;
   const double f = frexp(s, &e);
   F = __double2ll_rn(f * 4611686018427387904.0);
   k = e;
-}
-
-// Loads psi (double) of `cnt` contiguous points at `base` into smx (one global read,
-// staged in smem as doubles, converted in place) as fixed point times the pending
-// Normalize factor and the opening X factor; returns the block exponent and (in bits)
-// the bit length of the largest component.
-template <int N>
-__device__ __forceinline__ int open_block(const GridDev& g, const StepDev& S, longlong2* smx, long long base, int cnt,
-                                          long long row0, int* red, int& bits) {
-  const bool real_f = S.mode == 1 && g.gauge != 1;
-  double2* sd = reinterpret_cast<double2*>(smx);
-  int em = 0;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const double2 v = g.psi[base + e];
-    sd[e] = v;
-    em = max(em, max(dexp(v.x), dexp(v.y)));
-  }
-  em = block_max_int(em, red);
-  // an Inf or NaN component (exponent field all ones) has no fixed-point image: flag
-  // the solve (QSF_ENUMERIC) instead of converting garbage
-  if (em >= 0x7ff && threadIdx.x == 0) S.ctl[4] = 1;
-  const int s_in = scale_from_exponent<N>(em);
-  int scale = s_in;
-  long long F = 0;
-  int k = 0;
-  const bool use_s = !S.fused && S.normalize && *S.scale != 1.0;
-  if (use_s) {
-    split_scale(*S.scale, F, k);
-    scale -= k;
-  }
-  u64 mag = 0;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const long long p = base + e;
-    const double2 v = sd[e];  // written by this thread
-    longlong2 x = make_longlong2(d2fx(v.x, s_in), d2fx(v.y, s_in));
-    if (use_s) x = make_longlong2(mulq62(x.x, F), mulq62(x.y, F));
-    x = xhalf<N>(g, S, x, p, row0 + e / N, e % N, 0, real_f);
-    smx[e] = x;
-    mag |= fmag(x);
-  }
-  bits = block_max_int(bitlen(mag), red);
-  return scale - xhalf_exp(g, S, 0);
-}
-
-// psi_n from the block after the last inverse transform (held conjugated in smx when
-// conj_in): closing X factor, 1/m's power of two, [store as double], norm / E_pot
-// partial sums (exact integers).  On return smx holds psi_n in fixed point with
-// exponent `scale` and bit length `bits`.
-template <int N>
-__device__ __forceinline__ void close_block(const GridDev& g, const StepDev& S, longlong2* smx, long long base, int cnt,
-                                            long long row0, int* red, int& scale, int& bits, double* dacc,
-                                            bool conj_in, bool store) {
-  const bool real_f = S.mode == 1 && g.gauge != 1;
-  const int pre = product_headroom(bits);
-  u64 mag = 0;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const long long p = base + e;
-    longlong2 x = smx[e];
-    if (conj_in) x = fconj(x);
-    if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-    x = xhalf<N>(g, S, x, p, row0 + e / N, e % N, 1, real_f);
-    smx[e] = x;
-    mag |= fmag(x);
-  }
-  scale += pre - xhalf_exp(g, S, 1) + S.l2m;
-  bits = block_max_int(bitlen(mag), red);
-  const int q = bits > 56 ? bits - 56 : 0;
-  Acc128 an{0ull, 0ll}, av{0ull, 0ll};
-  const bool epot = (S.obs & 2u) != 0;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const long long p = base + e;
-    const longlong2 x = smx[e];
-    if (store) g.psi[p] = make_double2(fx2d(x.x, scale), fx2d(x.y, scale));
-    acc_point(an, av, x, q, S.Vx, p, epot);
-  }
-  dacc[0] = acc_value(an);
-  dacc[1] = acc_value(av);
-  // block-uniform exponents of the two sums
-  dacc[3] = (double)(2 * q - 2 * scale);
-  dacc[4] = (double)(2 * q - 2 * scale + 50 - S.vshift);
-}
-
-// E_kin part of the last axis: forward transform of psi_n (in smx) and sum k^2 |.|^2
-template <int N, int PPT>
-__device__ __forceinline__ double ekin_rows(const AxisDev& a, longlong2* smx, const LineSet& ls, int cnt, int scale,
-                                            int bits, int* red) {
-  const int sh = first_pass_shift<N>(bits);
-  int sc = scale + sh, b = 0;
-  fft_fx<N, PPT>(smx, ls, a.twf, threadIdx.x, blockDim.x, sc, b, red, sh);
-  double ek = 0.0;
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const double kk = kpos(a, e % N);
-    const longlong2 x = smx[e];
-    const double xr = fx2d(x.x, sc), xi = fx2d(x.y, sc);
-    ek = fma(kk * kk, fma(xr, xr, xi * xi), ek);
-  }
-  return ek;
-}
-
-// P phase of a 1D line between the forward and the inverse transform, written conjugated
-// so that the inverse transform runs as a forward one; returns the exponent change and
-// the new bit length.
-__device__ __forceinline__ int p_phase(const StepDev& S, longlong2* smx, int n, int* red, int& bits) {
-  const bool real_f = S.mode == 1;
-  const int pre = product_headroom(bits);
-  u64 mag = 0;
-#pragma unroll 1
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    longlong2 x = smx[e];
-    if (pre) x = make_longlong2(fshift(x.x, pre), fshift(x.y, pre));
-    x = fconj(fapply(x, S.ptab[e], real_f));
-    smx[e] = x;
-    mag |= fmag(x);
-  }
-  bits = block_max_int(bitlen(mag), red);
-  return pre - xshift(1) - S.texp[0];
-}
-
-// ------------------------------------------------------------ 1D whole step
-// One block per line: X open . FFT . P . IFFT . X close . observables, line in smem.
-template <int N, bool FULL>
-__global__ void __launch_bounds__(kLineThreads, (QSF_FFT_MIN_BLOCKS + 1) / 2) k_line_step(const GridDev* __restrict__ Gs,
-                                                            const StepDev* __restrict__ Ss) {
-  const GridDev& g = Gs[blockIdx.y];
-  const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
-  if (threadIdx.x == 0) S.ctl[6] = S.ctl[5] + 1;  // the sub-step's only pass
-  extern __shared__ __align__(128) longlong2 smx[];
-  __shared__ int red[kRedInts];
-  __shared__ double dred[32 * kMaxFluxBorders];
-  const AxisDev& a = g.ax[0];
-  int bits = 0;
-  int scale = open_block<N>(g, S, smx, 0, N, 0, red, bits);
-  int sh = first_pass_shift<N>(bits);
-  scale += sh;
-  const LineSet ls{1, N, 1, false};
-  fft_fx<N, line_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  scale += p_phase(S, smx, N, red, bits);
-  sh = first_pass_shift<N>(bits);
-  scale += sh;
-  fft_fx<N, line_ppt(N)>(smx, ls, a.twf, threadIdx.x, blockDim.x, scale, bits, red, sh);
-  double dacc[5];
-  close_block<N>(g, S, smx, 0, N, 0, red, scale, bits, dacc, true, true);
-  __syncthreads();
-  if (S.row_ptr) {
-    const int e1 = S.row_ptr[1];
-    for (int e = threadIdx.x; e < e1; e += blockDim.x) S.snap[e] = g.psi[S.snap_idx[e]];
-  }
-  dacc[2] = ekin_at(S, S.ctl[5]) ? ekin_rows<N, line_ppt(N)>(a, smx, ls, N, scale, bits, red) : 0.0;
-  const double e_n = dacc[3], e_v = dacc[4];
-  block_sum<3>(dacc, dred);
-  if (threadIdx.x == 0) {
-    S.partials[0 * S.pmax] = ldexp(dacc[0], (int)e_n);
-    S.partials[1 * S.pmax] = ldexp(dacc[1], (int)e_v);
-    S.partials[2 * S.pmax] = dacc[2];
-  }
-  if constexpr (FULL) {  // the end of the step in this block: fluxes, row, counters
-    __syncthreads();
-    const long long sub = S.ctl[5];
-    const bool step_end = (sub + 1) % S.substeps == 0;
-    const long long step = sub / S.substeps;
-    const int nb = S.nborders;
-    if (S.nfterms > 0 && step_end) {
-      const double* A = (g.gauge == 0 && S.coupling && g.n_fields) ? S.coupling + sub * S.coup_stride : nullptr;
-      flux_block(g, S.fpts, S.fterms, 0, S.nfterms, S.snap, A, nb, dred, S.fpartials);
-    }
-    finalize_tail(g, S, sub, step_end, step, nb, 1, dred);
-  }
 }
 
 #ifdef QSF_DEFINE_KERNELS
@@ -1338,18 +1030,11 @@ struct KernelSet {
   void (*axis_one)(const GridDev*, const StepDev*, int, int);  // one transform: forward or inverse (last argument)
   void (*axis_fpi)(const GridDev*, const StepDev*, int, int);
   void (*axis_ekin)(const GridDev*, const StepDev*, int, int);
-  void (*line_step)(const GridDev*, const StepDev*);
   void (*row_fft)(GridDev, int, double);        // forward flag, scale on the way out
   void (*axis_fft)(GridDev, int, int, double);  // axis, forward flag, scale
-  int line_ctas;     // CTAs holding one 1D line in the step kernel (a cluster of 2 .. 8 CTAs for
-                     // power-of-two lines of 1024 or more points)
-  int line_threads;  // threads per CTA of the 1D line step kernel
-  int fft_ctas;      // CTAs of the plain row transform of one line (2: a cluster pair above 8192 points)
   int row_lines, row_threads, row_smem;  // last-axis passes: lines, threads, dynamic shared memory of a block
   int col_lines, col_threads, col_smem;  // strided-axis passes: columns, threads, dynamic shared memory
-  int fft_lines, fft_threads, fft_smem;  // row_fft
-  const int* plan[2];                    // radices of the 8- and the 16-point line plan, 0-terminated
-  bool line_full;   // line_step also ends the step (fluxes, row, counters: no k_finalize)
+  int fft_lines, fft_threads, fft_smem;  // row_fft (none above 8192 points: those lines are 1D, LineKernels::fft)
 };
 
 // kernel table of the supported sizes (qsf_sizes_*.cu); nullptr when n is not built
@@ -1357,31 +1042,18 @@ const KernelSet* kernels_for(int n);
 
 }  // namespace qsf
 #include "qsf_passes.cuh"
-#include "qsf_cluster.cuh"
+#include "qsf_line1d.cuh"
 namespace qsf {
 
-// sizes up to 4096 get the multi-dimensional passes; up to 8192 the 1D line kernel of
-// one CTA, up to 16384 the one of a cluster pair
+// sizes up to 4096 get the multi-dimensional passes, up to 8192 the plain row transform;
+// the 1D steps have kernels of their own (LineKernels)
 template <int N>
 KernelSet make_kernel_set() {
   static_assert(is_smooth(N), "grid sizes must be 2^a 3^b 5^c");
   static_assert(N <= 16384, "1D lines longer than 16384 points are not built");
   KernelSet k{};
   k.n = N;
-  k.line_ctas = 1;
-  k.line_threads = kLineThreads;
-  k.fft_ctas = 1;
-  k.line_full = false;
-  if constexpr (N > 8192) {
-    k.line_ctas = 2;
-    k.fft_ctas = 2;
-    k.line_step = k_line_step_cl<N>;
-    k.row_fft = k_row_fft_cl<N>;
-    k.fft_lines = 1;
-    k.fft_threads = kLineThreads;
-    k.fft_smem = N / 2 * (int)sizeof(double2);
-    return k;
-  } else {
+  if constexpr (N <= 8192) {
     using G = Ln<N, tuned_ppt(N)>;
     using A = Ln<N, axis_ppt(N)>;
     if constexpr (N <= 4096) {
@@ -1399,24 +1071,12 @@ KernelSet make_kernel_set() {
       k.col_threads = A::kColThreads;
       k.col_smem = A::kColSmem;
     }
-    k.line_step = k_line_step<N, true>;
-    k.line_full = true;
-#if QSF_LINE_CLUSTER
-    if constexpr (N >= 1024 && (N & (N - 1)) == 0) {  // the line spread over a cluster
-      constexpr int C = N / 512 < 8 ? N / 512 : 8;
-      k.line_ctas = C;
-      k.line_threads = mc_threads<N, C>();
-      k.line_step = k_line_step_mc<N, C>;
-    }
-#endif
     k.row_fft = k_row_fft<G>;
     k.fft_lines = G::L;
     k.fft_threads = G::kRowThreads;
     k.fft_smem = G::kRowSmem;
-    k.plan[0] = line_radices<N, 8>();
-    k.plan[1] = line_radices<N, 16>();
-    return k;
   }
+  return k;
 }
 
 }  // namespace qsf

@@ -58,7 +58,41 @@ __host__ __device__ constexpr int axis_ppt(int n) { return n == 128 || n == 256 
 struct LinePlan {
   int E, S, r[4];
 };
+constexpr int kEight = 1, kFour = 2;  // plan selectors: 8 or 4 points per thread at every length they list
 __host__ __device__ constexpr LinePlan line_plan(int n, int ppt) {
+  if (ppt == kFour) {
+    switch (n) {
+      case 16: return {4, 2, {4, 4, 1, 1}};
+      case 24: return {4, 3, {4, 3, 2, 1}};
+      case 32: return {4, 3, {4, 2, 4, 1}};
+      case 40: return {4, 3, {4, 5, 2, 1}};
+      case 48: return {4, 3, {4, 3, 4, 1}};
+      case 64: return {4, 3, {4, 4, 4, 1}};
+      case 80: return {4, 3, {4, 5, 4, 1}};
+      case 96: return {4, 4, {4, 3, 2, 4}};
+      case 128: return {4, 4, {4, 2, 4, 4}};
+      case 160: return {4, 4, {4, 5, 2, 4}};
+      case 192: return {4, 4, {4, 3, 4, 4}};
+      default: return {0, 0, {1, 1, 1, 1}};
+    }
+  }
+  if (ppt == kEight) {  // the factors of a 1D line spread over a cluster (qsf_line1d.cuh)
+    switch (n) {
+      case 16: return {8, 2, {8, 2, 1, 1}};
+      case 24: return {8, 3, {4, 3, 2, 1}};
+      case 32: return {8, 2, {8, 4, 1, 1}};
+      case 40: return {8, 3, {4, 5, 2, 1}};
+      case 48: return {8, 3, {8, 3, 2, 1}};
+      case 64: return {8, 2, {8, 8, 1, 1}};
+      case 80: return {8, 3, {8, 5, 2, 1}};
+      case 96: return {8, 3, {8, 3, 4, 1}};
+      case 128: return {8, 3, {8, 2, 8, 1}};
+      case 160: return {8, 3, {8, 5, 4, 1}};
+      case 192: return {8, 3, {8, 3, 8, 1}};
+      case 256: return {8, 3, {8, 4, 8, 1}};
+      default: return {0, 0, {1, 1, 1, 1}};
+    }
+  }
   const bool w = ppt >= 16;
   switch (n) {
     case 8: return {8, 1, {8, 1, 1, 1}};
@@ -124,14 +158,6 @@ __host__ __device__ constexpr int line_tw_off(int n, int ppt, int p) {
   return o;
 }
 __host__ __device__ constexpr int line_tw_len(int n, int ppt) { return line_tw_off(n, ppt, line_plan(n, ppt).S); }
-
-// the radices of a plan for the host (0-terminated)
-template <int N, int PPT>
-const int* line_radices() {
-  constexpr LinePlan p = line_plan(N, PPT);
-  static const int r[5] = {p.r[0], p.S > 1 ? p.r[1] : 0, p.S > 2 ? p.r[2] : 0, p.S > 3 ? p.r[3] : 0, 0};
-  return r;
-}
 
 // Compile-time layout of the line kernels of one length and plan.
 template <int N_, int PPT>
@@ -260,8 +286,10 @@ struct LineCtx {
   int l, t;
   longlong2* buf;
   unsigned (*slot)[32];
+  int nth;  // threads that take part in the block's barriers
+  bool on = true;  // false: a thread that only fills a warp (its values count for nothing)
   int par = 0;
-  __device__ __forceinline__ LineCtx(longlong2* smem, unsigned (*sl)[32]) : slot(sl) {
+  __device__ __forceinline__ LineCtx(longlong2* smem, unsigned (*sl)[32], int n = blockDim.x) : slot(sl), nth(n) {
     l = threadIdx.x / G::T;
     t = threadIdx.x % G::T;
     buf = smem + (size_t)l * G::LS;
@@ -272,12 +300,12 @@ struct LineCtx {
   __device__ __forceinline__ void sync() const {
     if constexpr (G::kSync == 0) __syncwarp();
     else if constexpr (G::kSync == 1) asm volatile("bar.sync %0, %1;" ::"r"(l + 1), "n"(G::T) : "memory");
-    else __syncthreads();
+    else asm volatile("bar.sync 15, %0;" ::"r"(nth) : "memory");
   }
   // the group's maximum in two halves around one of its barriers: put before, get after.
   // Slots alternate, so a slot is written again only after another barrier.
   __device__ __forceinline__ void put(unsigned& m) {
-    m = __reduce_max_sync(0xffffffffu, m);
+    m = __reduce_max_sync(0xffffffffu, on ? m : 0u);
     if constexpr (G::kSync != 0) {
       if ((threadIdx.x & 31) == 0) slot[par][threadIdx.x >> 5] = m;
     }
@@ -286,7 +314,7 @@ struct LineCtx {
     if constexpr (G::kSync != 0) {
       constexpr int nw = G::kSync == 1 ? G::T / 32 : 0;
       const int w0 = G::kSync == 1 ? l * nw : 0;
-      const int n = G::kSync == 1 ? nw : (int)(blockDim.x >> 5);
+      const int n = G::kSync == 1 ? nw : nth >> 5;
       m = slot[par][w0];
       for (int w = 1; w < n; ++w) m = max(m, slot[par][w0 + w]);
       par ^= 1;
@@ -424,15 +452,15 @@ __device__ __forceinline__ int line_bits(const longlong2* v, LineCtx<G>& c) {
   return LineCtx<G>::bits_of(c.group_max(h.mag()));
 }
 
-// the line outputs brought to 61 bits (products keep 2^-59 of the largest component);
-// returns the shift
-template <class G>
+// the line outputs brought to TOP bits (products keep 2^-(TOP - 2) of the largest
+// component); returns the shift
+template <class G, int TOP = 61>
 __device__ __forceinline__ int line_up(longlong2* v, LineCtx<G>& c) {
   const int bits = line_bits<G>(v, c);
-  const int sh = bits ? 61 - bits : 0;
+  const int sh = bits ? TOP - bits : 0;
 #pragma unroll
   for (int s = 0; s < G::E; ++s) {
-    if constexpr (G::S == 1) v[s] = Shift(sh)(v[s]);
+    if constexpr (G::S == 1 || TOP < 61) v[s] = Shift(sh)(v[s]);
     else v[s] = shl_by(v[s], sh);
   }
   return sh;

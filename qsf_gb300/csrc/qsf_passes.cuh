@@ -161,15 +161,18 @@ struct ObsSum {
     a3 += (i64)nl * vh;
     a4 += (i64)nl * vl;
   }
-  // the sums for points of exponent s (value = u 2^-s): rounded to one word in units of
-  // the largest point's 2^-59 (2^-58 for E_pot) and converted once
-  __device__ __forceinline__ double norm(int s) const {
-    const u64 n = (hh << 4) + (u64)((hl + (i64)(ll >> 29) + (1 << 22)) >> 23);
-    return pow2(60 - 2 * s) * (double)n;
+  // the sums as one word each, in units of the largest point's 2^-59 (2^-58 for E_pot):
+  // norm = norm_word 2^(60 - 2 s), E_pot = epot_word 2^(111 - vshift - 2 s) for points of
+  // exponent s (value = u 2^-s)
+  __device__ __forceinline__ u64 norm_word() const {
+    return (hh << 4) + (u64)((hl + (i64)(ll >> 29) + (1 << 22)) >> 23);
   }
+  __device__ __forceinline__ i64 epot_word() const {
+    return (a1 << 2) + ((a2 + (a3 >> 6) + (a4 >> 31) + (1 << 22)) >> 23);
+  }
+  __device__ __forceinline__ double norm(int s) const { return pow2(60 - 2 * s) * (double)norm_word(); }
   __device__ __forceinline__ double epot(int s, int vshift) const {
-    const i64 n = (a1 << 2) + ((a2 + (a3 >> 6) + (a4 >> 31) + (1 << 22)) >> 23);
-    return pow2(111 - vshift - 2 * s) * (double)n;
+    return pow2(111 - vshift - 2 * s) * (double)epot_word();
   }
 };
 

@@ -28,7 +28,7 @@ int batch_launch(qsf_batch* b, int64_t steps);
 int batch_finish(qsf_batch* b, int64_t* active);
 bool fused_length(int n);
 int bs_size(int n, int dim);
-bool grid_fused(const qsf_grid* g);
+bool grid_batched(const qsf_grid* g);
 int generic_begin(qsf_grid* g, const qsf_step_desc* d);
 int generic_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
 int generic_wait(qsf_grid* g, bool* bad);
@@ -269,7 +269,7 @@ int admit(qsf_server* s, Pending& p, Running& r, bool nowait) {
   for (int b = 0; b < QSF_MAX_BORDERS; ++b) d.border_types[b] = p.req.border_types[b];
   d.box_size = p.req.box_size;
   QSF_TRACE_T(t_add);
-  if (!qsf::grid_fused(g)) {
+  if (!qsf::grid_batched(g)) {
     r.generic = true;
     r.d = d;
     rc = qsf::generic_begin(g, &r.d);

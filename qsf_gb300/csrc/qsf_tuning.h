@@ -35,17 +35,17 @@ __host__ __device__ constexpr int tuned_tile(int n) {
   return 4096;
 }
 
-// Points per thread of the one-CTA 1D line kernel per line length (4: radix-4 plans,
-// 8: radix 8, 16: radix 16); a length between measured ones takes the plan of the next
-// longer measured length.  Measured (one call of graph-replayed steps, points per
+// Points per thread of 1D lines held by one CTA as one line (up to 640 points; 8: radix-8
+// plans, 16: radix 16); a length between measured ones takes the plan of the next longer
+// measured length.  Measured (one call of graph-replayed steps, points per
 // thread: ms per step):
-//   1d1024  ms/step  4: 0.0392  8: 0.0416  16: 0.0452
-//   1d1536  ms/step  4: 0.0479  8: 0.0472  16: 0.0568
-//   1d2048  ms/step  4: 0.0537  8: 0.0522  16: 0.0543
-//   1d3072  ms/step  8: 0.0663  16: 0.0683
-//   1d4096  ms/step  8: 0.0733  16: 0.0711
+//   1d64    ms/step  8: 0.0113  16: 0.0314
+//   1d128   ms/step  8: 0.0120  16: 0.0329
+//   1d256   ms/step  8: 0.0129  16: 0.0338
+//   1d384   ms/step  8: 0.0161  16: 0.0394
+//   1d640   ms/step  8: 0.0199  16: 0.0434
 __host__ __device__ constexpr int tuned_line_ppt(int n) {
-  return n <= 1024 ? 4 : n <= 3072 ? 8 : 16;
+  return n <= 640 ? 8 : 16;
 }
 
 }  // namespace qsf

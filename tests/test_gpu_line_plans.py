@@ -78,3 +78,85 @@ def test_imaginary_time_matches_oracle(dim, n, gauge, fields):
         if s % 2:
             assert out[s, 2] / out[s, 0] == pytest.approx(r["ekin"], rel=4 * tol)
     g.close()
+
+
+def _line_oracle(n, lg, mode, steps, dt, psi0, pulse, outs):
+    from oracle import oracle as O
+    oc = O.Coupling(O.GAUGE_LENGTH if lg else O.GAUGE_VELOCITY, [O.Field(1, [O.Pulse(**pulse)])] if pulse else [])
+    og = O.Grid(1, n, 0.2, nCAP=max(1, n // 10), pot=O.POT_EBERLY, Ncharge=1.0, coupling=oc)
+    og.psi[...] = psi0
+    prop = O.Propagator(O.MODE_RE if mode == "real" else O.MODE_IM, dt, steps, og, outs)
+    for _ in range(steps):
+        prop.make_step()
+        prop.compute_each()
+    return og.psi, prop.rows
+
+
+# one length per geometry of the 1D kernels: one line in a CTA (its lanes filling warps or
+# not), N1 x N2 over 1, 2, 4 and 8 CTAs with 4 and 8 points per thread, every radix family,
+# and convolution lengths for n at the edges of their ranges
+LINES = [8, 12, 20, 40, 96, 160, 256, 320, 384, 640, 512, 768, 1024, 1280, 1536, 2048, 2560, 3072, 4096, 5120, 6144, 8192,
+         10240, 12288, 16384, 7, 255, 257, 383, 1025, 4095, 5003, 8191, 10239, 12289, 16383]
+
+
+@pytest.mark.parametrize("n", LINES)
+@pytest.mark.parametrize("mode,gauge", [("real", "velocity"), ("real", "length"), ("imaginary", "velocity")])
+def test_line_steps_match_oracle(n, mode, gauge):
+    """Whole 1D steps: psi, norm, E_pot, E_kin (imaginary time, every second step, with
+    Normalize) and the BOX flux."""
+    import qsf_gb300 as Q
+    from oracle import oracle as O
+    from qsf_gb300.propagator import coupling_schedule
+    real, lg, steps = mode == "real", gauge == "length", 6
+    dt = 0.05 if real else 0.01
+    psi0 = _noise_state(1, n, 0.2, n)
+    pulse = dict(field=0.1, omega=1.1, ncycles=1.0) if real else None
+    box = n // 4
+    outs = ["norm", "epot", ("flux", ["BOX"], box)] if real else ["norm", "normalize", "epot", "ekin"]
+    O.set_border_nodes(25, 14, 10, 40)
+    opsi, orows = _line_oracle(n, lg, mode, steps, dt, psi0, pulse, outs)
+    g = Q.Grid(1, n, 0.2, nCAP=max(1, n // 10), Ncharge=1.0, gauge=Q.GAUGE_LENGTH if lg else Q.GAUGE_VELOCITY,
+               n_fields=1 if real else 0)
+    g.upload(psi0)
+    rows = None
+    if real:
+        c = Q.Coupling(Q.GAUGE_LENGTH if lg else Q.GAUGE_VELOCITY, [Q.Field(1, [Q.Pulse(**pulse)])])
+        rows = coupling_schedule(c, dt, steps)[0]
+        out, done = g.step(Q.MODE_RE, dt, steps, rows, obs=Q.OBS_NORM | Q.OBS_EPOT, borders=["BOX"], box_size=box)
+    else:
+        out, done = g.step(Q.MODE_IM, dt, steps, obs=Q.OBS_NORM | Q.OBS_EPOT | Q.OBS_EKIN, normalize=True, ekin_interval=2)
+    assert done == steps
+    # lengths with a large prime factor: the oracle's direct DFT passes add up to n terms
+    tol = _tol(1, n, steps) * (1 if n in LINES[:25] else math.sqrt(n))
+    assert C.rel_l2(g.download(), opsi) < tol
+    for s, r in enumerate(orows):
+        f = 1.0 if real else out[s, 0]
+        assert out[s, 0] == pytest.approx(r["norm"], rel=4 * tol)
+        assert out[s, 1] / f == pytest.approx(r["epot"], rel=4 * tol)
+        if real:
+            assert out[s, 3] == pytest.approx(r["flux"][0], abs=8 * tol * np.abs(psi0).max() ** 2 / 0.2)
+        elif s % 2:
+            assert out[s, 2] / f == pytest.approx(r["ekin"], rel=8 * tol)
+    g.close()
+
+
+@pytest.mark.parametrize("n", [96, 1536, 4096, 1021])
+def test_line_run_does_not_depend_on_its_launches(n):
+    """One call of 7 steps, seven calls of one step, and psi taken out and put back between
+    them give the same bits."""
+    import qsf_gb300 as Q
+    psi0 = _noise_state(1, n, 0.2, 3)
+    rng = np.random.default_rng(4)
+    rows = 0.1 * rng.standard_normal((7, 6))
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT | Q.OBS_EKIN, borders=["BOX"], box_size=n // 4)
+    g = Q.Grid(1, n, 0.2, nCAP=n // 10, gauge=Q.GAUGE_LENGTH, n_fields=1)
+    g.upload(psi0)
+    whole, _ = g.step(Q.MODE_RE, 0.05, 7, rows, **kw)
+    psi = g.download()
+    g.upload(psi0)
+    parts = []
+    for s in range(7):
+        parts.append(g.step(Q.MODE_RE, 0.05, 1, rows[s:s + 1], **kw)[0].copy())
+        g.upload(g.download())
+    assert np.array_equal(np.concatenate(parts), whole) and np.array_equal(g.download(), psi)
+    g.close()
