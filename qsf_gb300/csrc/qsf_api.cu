@@ -105,12 +105,15 @@ int init_kernel_table() {
     QSF_CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     return QSF_OK;
   };
+  // the plain transforms' tiles of kMaxAxis points and blocks of up to 16 points per thread
+  const int tile = kMaxAxis * (int)sizeof(double2), line = 16 * kPlainThreads * (int)sizeof(double2);
   for (const KernelSet& k : t) {
     int rc;
     if ((rc = lim((const void*)k.row_open, k.row_smem)) || (rc = lim((const void*)k.row_close, k.row_smem)) ||
         (rc = lim((const void*)k.row_ekin, k.row_smem)) || (rc = lim((const void*)k.axis_one, k.col_smem)) ||
         (rc = lim((const void*)k.axis_fpi, k.col_smem)) || (rc = lim((const void*)k.axis_ekin, k.col_smem)) ||
-        (rc = lim((const void*)k.axis_fft, k.col_smem)) || (rc = lim((const void*)k.row_fft, k.fft_smem)))
+        (rc = lim((const void*)k.axis_fft[0], tile)) || (rc = lim((const void*)k.axis_fft[1], tile)) ||
+        (rc = lim((const void*)k.row_fft[0], line)) || (rc = lim((const void*)k.row_fft[1], line)))
       return rc;
   }
   if (int rc = init_line_table()) return rc;
@@ -186,16 +189,16 @@ int make_tensor_maps(qsf_grid* g) {
 
 // One transform of axis ax of the array G.psi with the kernels K of that axis' length.
 void qsf::launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd, double sc, cudaStream_t st) {
-  GridDev V = G;
-  for (int k = 0; k < kMaxDim; ++k) V.tmap[k] = nullptr;  // G.psi need not be the mapped array
   const long long n = G.ax[ax].n, lines = G.m / n;
   if (ax == G.dim - 1) {
-    const int blocks = (int)((lines + K.fft_lines - 1) / K.fft_lines);
-    K.row_fft<<<blocks, K.fft_threads, K.fft_smem, st>>>(V, fwd, sc);
+    // rows of the last axis with up to 16 * kPlainThreads points per block
+    const int L = (int)std::max<long long>(1, std::min<long long>(lines, (16LL * kPlainThreads) / n));
+    K.row_fft[fwd]<<<(unsigned)((lines + L - 1) / L), kPlainThreads, (size_t)L * n * sizeof(double2), st>>>(G, L, sc);
   } else {
     const long long inner = G.ax[ax].stride, outer = lines / inner;
-    K.axis_fft<<<(unsigned)(outer * ((inner + K.col_lines - 1) / K.col_lines)), K.col_threads, K.col_smem, st>>>(V, ax, fwd,
-                                                                                                                sc);
+    const int C = (int)std::min<long long>(K.axis_cols, inner);
+    K.axis_fft[fwd]<<<(unsigned)(outer * ((inner + C - 1) / C)), K.axis_threads, (size_t)n * C * sizeof(double2), st>>>(
+        G, ax, C, sc);
   }
 }
 
@@ -232,18 +235,21 @@ int4 qsf::split_root(long long t, long long n, int r) {
 // Per-pass twiddles of a line plan (qsf_lines.cuh): kTwVar copies, copy r scaled by 2^-r;
 // pass p's entry [(q - 1) ns + jm] = exp(-2 pi i jm q / (ns R)).  Made once per length,
 // plan, process and device and shared by every grid (never freed: a few MB in all).
+// kPlain: exp(-2 pi i t / n), t < n, as the plain transforms read them.
 int qsf::shared_line_twiddles(int n, int ppt, const int4** out) {
   static std::mutex mu;
   static std::map<std::array<int, 3>, int4*> cache;
   *out = nullptr;
-  const LinePlan P = line_plan(n, ppt);
+  const LinePlan P = ppt == kPlain ? LinePlan{} : line_plan(n, ppt);
   int dev = 0;
   QSF_CU(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
   auto it = cache.find({dev, n, ppt});
   if (it == cache.end()) {
     std::vector<int4> h;
-    for (int r = 0; r < kTwVar; ++r) {
+    if (ppt == kPlain)
+      for (int t = 0; t < n; ++t) h.push_back(split_root(t, n, 0));
+    for (int r = 0; r < kTwVar && P.S; ++r) {
       long long ns = P.r[0];
       for (int p = 1; p < P.S; ++p) {
         const int R = P.r[p];
@@ -267,12 +273,14 @@ int qsf::shared_line_twiddles(int n, int ppt, const int4** out) {
   return QSF_OK;
 }
 
-// the twiddles of both line plans of a built length (none above 8192 points)
-int qsf::axis_twiddles(int n, const int4* out[2]) {
-  out[0] = out[1] = nullptr;
+// the twiddles of a built length (none above 8192 points): both line plans' and the plain
+// transforms'
+int qsf::axis_twiddles(int n, AxisDev* a) {
+  a->tw = a->twl[0] = a->twl[1] = nullptr;
   if (n > 8192) return QSF_OK;
-  if (int rc = shared_line_twiddles(n, 8, &out[0])) return rc;
-  return shared_line_twiddles(n, 16, &out[1]);
+  int rc;
+  if ((rc = shared_line_twiddles(n, 8, &a->twl[0])) || (rc = shared_line_twiddles(n, 16, &a->twl[1]))) return rc;
+  return shared_line_twiddles(n, kPlain, &a->tw);
 }
 
 namespace {
@@ -951,11 +959,11 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
     a.dp = 2.0 * M_PI / (double)d->n[k] / d->dx[k];
   }
   if (ks) {
-    if (int rc = axis_twiddles(G.ax[0].n, G.ax[0].twl)) {
-      qsf_grid_destroy(g);
-      return rc;
-    }
-    for (int k = 1; k < d->dim; ++k) std::copy(G.ax[0].twl, G.ax[0].twl + 2, G.ax[k].twl);
+    for (int k = 0; k < d->dim; ++k)
+      if (int rc = axis_twiddles(G.ax[k].n, &G.ax[k])) {
+        qsf_grid_destroy(g);
+        return rc;
+      }
   }
   G.inv_m = 1.0 / (double)G.m;
   G.dVm = G.dV * G.inv_m;
@@ -1151,7 +1159,7 @@ int qsf_fourier(qsf_grid* g, int to_rep) {
   for (int ax = D - 1; ax >= 0; --ax) {
     if ((G.free_mask >> ax) & 1) continue;
     const double post = ax == last && !fwd ? back : 1.0;
-    if (D == 1 && (!g->ks || !g->ks->row_fft)) {
+    if (D == 1 && (!g->ks || !g->ks->row_fft[0])) {
       if (int rc = line_fourier(g, G, fwd, post)) return rc;
     } else if (g->ks) {
       axis_fft(g, G, ax, fwd, post);
@@ -1192,7 +1200,7 @@ int qsf_region_transfer(qsf_grid* dst, const qsf_grid* src, int axis, int group)
                                                         dst->nmax);
   GridDev Gs = G;
   Gs.psi = dst->mg_slice;
-  if (G.dim == 1 && (!dst->ks || !dst->ks->row_fft)) {
+  if (G.dim == 1 && (!dst->ks || !dst->ks->row_fft[0])) {
     if (int rc = line_fourier(dst, Gs, true, 1.0)) return rc;
   } else if (dst->ks) axis_fft(dst, Gs, axis, true, 1.0);
   else if (int rc = bs_axis(dst, dst->mg_slice, axis, true, 1.0)) return rc;

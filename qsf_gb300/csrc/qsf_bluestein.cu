@@ -98,7 +98,7 @@ GridDev scratch_view(const qsf_grid* g, int ax) {
   S.ax[ax].n = g->bs.M;
   S.ax[ax].n2 = g->bs.M / 2;
   S.ax[ax].shift = (g->bs.M & (g->bs.M - 1)) == 0 ? __builtin_ctz((unsigned)g->bs.M) : -1;
-  std::copy(g->bs.twl, g->bs.twl + 2, S.ax[ax].twl);
+  S.ax[ax].tw = g->bs.ax.tw;
   long long st = 1;
   for (int k = S.dim - 1; k >= 0; --k) {
     S.ax[k].stride = st;
@@ -131,7 +131,7 @@ int bs_setup(qsf_grid* g) {
   b.M = M;
   b.ks = kernels_for(M);
   int rc;
-  if ((rc = axis_twiddles(M, b.twl))) return rc;
+  if ((rc = axis_twiddles(M, &b.ax))) return rc;
   const size_t scr = (size_t)(G.m / n) * (size_t)M;
   if ((rc = dev_alloc(b.chirp, (size_t)n)) || (rc = dev_alloc(b.bhat, (size_t)M)) ||
       (rc = dev_alloc(b.scratch, std::max(scr, (size_t)M))))
@@ -144,7 +144,7 @@ int bs_setup(qsf_grid* g) {
   L.psi = b.bhat;
   L.ax[0].n = M;
   L.ax[0].stride = 1;
-  std::copy(b.twl, b.twl + 2, L.ax[0].twl);
+  L.ax[0].tw = b.ax.tw;
   L.m = M;
   launch_axis_fft(*b.ks, L, 0, true, 1.0, g->stream);
   QSF_CU(cudaGetLastError());

@@ -160,7 +160,7 @@ struct qsf_grid {
     double2* chirp = nullptr;
     double2* bhat = nullptr;
     double2* scratch = nullptr;
-    const int4* twl[2] = {};  // line-plan twiddles of M (shared)
+    AxisDev ax{};  // twiddles of M (shared)
   } bs;
   // 1D grids (qsf_line1d.cu): the step kernels, their geometry tables, the tables of a run of sub-steps and the current program
   const LineKernels* lk = nullptr;
@@ -203,10 +203,11 @@ int batch_launch(qsf_batch* b, int64_t steps);
 int batch_finish(qsf_batch* b, int64_t* active);
 // exp(-2 pi i t / n) 2^-r in the split form of the kernels
 int4 split_root(long long t, long long n, int r);
-// device twiddles of the line plan (n, ppt), and of both plans of a built length; shared
+// device twiddles of the line plan (n, ppt), and all of a built length; shared
 // by all grids of the process (not to be freed by the caller)
 int shared_line_twiddles(int n, int ppt, const int4** out);
-int axis_twiddles(int n, const int4* out[2]);
+constexpr int kPlain = 0;  // selects the plain transforms' twiddles
+int axis_twiddles(int n, AxisDev* a);
 void launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd, double sc, cudaStream_t st);
 // 1D grids (qsf_line1d.cu)
 int init_line_table();

@@ -46,6 +46,7 @@ struct AxisDev {
   int shift;  // log2(n) when n is a power of two, else -1
   long long stride;
   double dx, xmin, dp, inv_2dx;
+  const int4* tw;      // exp(-2 pi i t / n), t < n, in split form, read by the plain transforms
   const int4* twl[2];  // per-pass twiddle tables of the 8- and the 16-point line plan (qsf_lines.cuh), kTwVar copies
 };
 
@@ -1030,11 +1031,12 @@ struct KernelSet {
   void (*axis_one)(const GridDev*, const StepDev*, int, int);  // one transform: forward or inverse (last argument)
   void (*axis_fpi)(const GridDev*, const StepDev*, int, int);
   void (*axis_ekin)(const GridDev*, const StepDev*, int, int);
-  void (*row_fft)(GridDev, int, double);        // forward flag, scale on the way out
-  void (*axis_fft)(GridDev, int, int, double);  // axis, forward flag, scale
+  // plain transforms, [0] inverse, [1] forward: lines (axis: ax, columns) of a block, scale on the way out
+  void (*row_fft[2])(GridDev, int, double);
+  void (*axis_fft[2])(GridDev, int, int, double);
+  int axis_cols, axis_threads;
   int row_lines, row_threads, row_smem;  // last-axis passes: lines, threads, dynamic shared memory of a block
   int col_lines, col_threads, col_smem;  // strided-axis passes: columns, threads, dynamic shared memory
-  int fft_lines, fft_threads, fft_smem;  // row_fft (none above 8192 points: those lines are 1D, LineKernels::fft)
 };
 
 // kernel table of the supported sizes (qsf_sizes_*.cu); nullptr when n is not built
@@ -1042,10 +1044,12 @@ const KernelSet* kernels_for(int n);
 
 }  // namespace qsf
 #include "qsf_passes.cuh"
+#include "qsf_plain.cuh"
 #include "qsf_line1d.cuh"
 namespace qsf {
 
-// sizes up to 4096 get the multi-dimensional passes, up to 8192 the plain row transform;
+// sizes up to 4096 get the multi-dimensional passes, up to 8192 the plain row transform
+// (longer lines are 1D: LineKernels::fft);
 // the 1D steps have kernels of their own (LineKernels)
 template <int N>
 KernelSet make_kernel_set() {
@@ -1063,7 +1067,10 @@ KernelSet make_kernel_set() {
       k.axis_one = k_axis<0, A>;
       k.axis_fpi = k_axis<2, A>;
       k.axis_ekin = k_axis<3, A>;
-      k.axis_fft = k_axis_fft<A>;
+      k.axis_fft[0] = k_axis_fft<N, false>;
+      k.axis_fft[1] = k_axis_fft<N, true>;
+      k.axis_threads = plain_threads(N);
+      k.axis_cols = plain_tile(N) / N < 64 ? plain_tile(N) / N : 64;
       k.row_lines = G::L;
       k.row_threads = G::kRowThreads;
       k.row_smem = G::kRowSmem;
@@ -1071,10 +1078,8 @@ KernelSet make_kernel_set() {
       k.col_threads = A::kColThreads;
       k.col_smem = A::kColSmem;
     }
-    k.row_fft = k_row_fft<G>;
-    k.fft_lines = G::L;
-    k.fft_threads = G::kRowThreads;
-    k.fft_smem = G::kRowSmem;
+    k.row_fft[0] = k_row_fft<N, false>;
+    k.row_fft[1] = k_row_fft<N, true>;
   }
   return k;
 }

@@ -1,5 +1,5 @@
 // qsf_passes.cuh -- the pass kernels of 2D and 3D grids over register-resident lines
-// (qsf_lines.cuh), and the plain transforms of one axis.
+// (qsf_lines.cuh).
 //
 // Passes leave psi in fixed point between them (int64 pairs in psi's buffer) with one
 // exponent per line of the producing pass:
@@ -536,10 +536,8 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
   }
 }
 
-// ------------------------------------------------------------ plain transforms
-// fourier<R>() without phases (qsf_fourier): each group takes its exponent from the
-// largest double it loads; an inverse is the forward transform between two conjugations
-// (the sign bit of the imaginary parts).
+// ------------------------------------------------------------ from and to doubles
+// conjugation of a double pair (the sign bit of the imaginary part)
 __device__ __forceinline__ longlong2 dconj(longlong2 x, bool on) {
   return on ? make_longlong2(x.x, x.y ^ (i64)0x8000000000000000ull) : x;
 }
@@ -552,43 +550,4 @@ __device__ __forceinline__ void line_to_double(longlong2* v, int scale, bool con
     v[s] = dconj(make_longlong2(__double_as_longlong(z.x), __double_as_longlong(z.y)), conj);
   }
 }
-template <class G>
-__global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
-    k_row_fft(GridDev g, int fwd, double post_scale) {
-  constexpr int N = G::N;
-  extern __shared__ __align__(1024) unsigned char sm[];
-  LineCtx<G> c(reinterpret_cast<longlong2*>(sm), reinterpret_cast<unsigned(*)[32]>(sm + G::buf_bytes(G::kRowThreads)));
-  const long long row = (long long)blockIdx.x * G::L + c.l;
-  const bool on = c.l < G::L && row < g.m / N;
-  longlong2* psi = reinterpret_cast<longlong2*>(g.psi) + (on ? row * N : 0) + c.t;
-  longlong2 v[G::K];
-#pragma unroll
-  for (int s = 0; s < G::E; ++s) v[s] = on ? dconj(psi[s * G::T], !fwd) : make_longlong2(0, 0);
-  unsigned em;
-  int scale = line_from_double<G>(v, c, em);
-  line_fft<G>(v, c, g.ax[g.dim - 1].twl[G::ppt >= 16], scale);
-  line_to_double<G>(v, scale, !fwd, post_scale);
-  if (!on) return;
-#pragma unroll
-  for (int s = 0; s < G::E; ++s) psi[s * G::T] = v[s];
-}
-template <class G>
-__global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
-    k_axis_fft(GridDev g, int ax, int fwd, double post_scale) {
-  extern __shared__ __align__(1024) unsigned char sm[];
-  const ColBlock<G> cb(g, ax, sm);
-  cb.load_begin();
-  LineCtx<G> c(cb.tile, cb.slots(sm));
-  longlong2 v[G::K];
-  cb.load_wait();
-  cb.read(v, c);
-#pragma unroll
-  for (int s = 0; s < G::E; ++s) v[s] = dconj(v[s], !fwd);
-  unsigned em;
-  int scale = line_from_double<G>(v, c, em);
-  line_fft<G>(v, c, g.ax[ax].twl[G::ppt >= 16], scale);
-  line_to_double<G>(v, scale, !fwd, post_scale);
-  cb.write(v, c);
-}
-
 }  // namespace qsf
