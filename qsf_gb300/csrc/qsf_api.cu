@@ -60,6 +60,7 @@ std::vector<KernelSet>& kernel_table();
 // kernel launch geometry
 constexpr int kMaxLine1D = 16384;       // 1D line in shared memory (one CTA up to 8192, a cluster pair above)
 constexpr int kMaxFluxBlocks = 512;  // blocks of the flux-term sums (256 terms each)
+constexpr int kTableSteps = 16;         // sub-steps whose tables are made at once, and steps per captured graph
 constexpr int kMaxAxis = 4096;          // points per axis in 2D and 3D
 
 }  // namespace
@@ -461,6 +462,12 @@ int ensure_flux(qsf_grid* g, int nb, const int* types, int64_t box) {
   return QSF_OK;
 }
 
+// blocks of k_finalize: one per 256 flux terms or 2048 row partials (a grid's own shape, so
+// that its sums do not depend on the batch it runs in)
+int fin_blocks(const qsf_grid* g, int nfterms) {
+  return std::max(nfterms > 0 ? g->nfblk : 1, std::min(kMaxFluxBlocks, (g->nrowblk + 2047) / 2048));
+}
+
 // Optional per-launch event timing (qsf_step_desc.kernel_ms): every launch of a step
 // is bracketed by a pair of events from a pool; the pairs are read after the step's
 // work is queued and synchronised once, so timing adds no host gaps between kernels.
@@ -538,8 +545,21 @@ struct FinOverlap {
   bool pending = false;
 };
 
-// One step's launches for `count` solves sharing kernels K and geometry q; every
-// kernel reads its solve's descriptors (blockIdx.y) and step counter from device memory.
+// The tables of the next `steps` sub-steps of `count` solves.
+int launch_tables(const Geom& q, const GridDev* dG, const StepDev* dS, int count, int steps, cudaStream_t st,
+                  Prof* P = nullptr) {
+  // (kind, axis) tables (X tables only in the length gauge), ~128 entries per block
+  const int tb = std::max(1, std::min(64, q.nmax / 128));
+  const int kinds = q.gauge == QSF_GAUGE_LENGTH ? 4 : 1;
+  int rc;
+  if (P && (rc = P->begin())) return rc;
+  k_tables<<<dim3(q.dim * kinds * tb, steps, count), 256, 0, st>>>(dG, dS, tb);
+  QSF_CU(cudaGetLastError());
+  return P ? P->end(QSF_K_TABLES) : QSF_OK;
+}
+
+// One step's passes for `count` solves sharing kernels K and geometry q; every kernel
+// reads its solve's descriptors (blockIdx.y) and step counter from device memory.
 int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const StepDev* dS, int count, bool ekin,
                  int nfblk, cudaStream_t st, Prof* P, bool with_open = true, FinOverlap* ov = nullptr) {
   Prof none;
@@ -553,17 +573,6 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
     if ((rc = pf.end(kind))) return rc;     \
   } while (0)
   const int D = q.dim;
-  // (kind, axis) tables (X tables only in the length gauge), ~128 entries per block
-  const int tb = std::max(1, std::min(64, q.nmax / 128));
-  const dim3 gt(D * 4 * tb, count);
-  if (D == 1) {  // the line kernels end their steps themselves
-    const LineKernels& L = *line_kernels(q.n);
-    QSF_TIMED(QSF_K_TABLES, (rc = line_launch_tables(L, dG, dS, count, 1, q.gauge == QSF_GAUGE_LENGTH, st)));
-    if (rc) return rc;
-    QSF_TIMED(QSF_K_LINE_STEP, (rc = line_launch_steps(L, false, dG, dS, count, 1, st)));
-    return rc;
-  }
-  QSF_TIMED(QSF_K_TABLES, (k_tables<<<gt, 256, 0, st>>>(dG, dS, tb)));
   const bool wait_fin = ov && ov->pending;
   {
     const dim3 gr(q.nrowblk, count);
@@ -598,8 +607,8 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
 }
 
 int launch_step(qsf_grid* g, const StepDev& S, Prof* P = nullptr, bool with_open = true, FinOverlap* ov = nullptr) {
-  return launch_group(*g->ks, geom_of(g), g->dG, g->dS, 1, (S.obs & QSF_OBS_EKIN) != 0,
-                      S.nfterms > 0 ? g->nfblk : 1, g->stream, P, with_open, ov);
+  return launch_group(*g->ks, geom_of(g), g->dG, g->dS, 1, (S.obs & QSF_OBS_EKIN) != 0, fin_blocks(g, S.nfterms),
+                      g->stream, P, with_open, ov);
 }
 
 // Whether k_finalize may run beside the next sub-step (FinOverlap), and its stream.
@@ -619,8 +628,10 @@ int ensure_fin_stream(qsf_grid* g, FinOverlap* ov) {
 
 // Validates a step program and stages everything a run of it needs on the device:
 // static tables for dt/2, flux point lists, coupling rows, observables rows, control
-// words; fills the step descriptor and uploads it to g->dS.
-int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_out, int64_t chunk = INT64_MAX) {
+// words; fills the step descriptor and uploads it to g->dS.  `direct`: one call of its own
+// (qsf_step), whose rows stay in the grid's call block when they are few.
+int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_out, int64_t chunk = INT64_MAX,
+                 bool direct = false) {
   if (d->mode != QSF_MODE_IM && d->mode != QSF_MODE_RE) return fail(QSF_EINVAL, "mode must be IM or RE");
   if (d->nsteps < 1) return fail(QSF_EINVAL, "nsteps < 1");
   if (d->nborders < 0 || d->nborders > QSF_MAX_BORDERS) return fail(QSF_EINVAL, "too many borders");
@@ -639,20 +650,26 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   const int nb = want_flux ? d->nborders : 0;
   const int ncol = 3 + nb;
   const int cstride = G.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
-  if ((rc = dev_reserve(g->rows_dev, g->rows_cap, (size_t)d->nsteps * ncol))) return rc;
+  const bool short_rows = direct && d->nsteps * ncol <= CallBlock::kRows;
+  if (!short_rows && (rc = dev_reserve(g->rows_dev, g->rows_cap, (size_t)d->nsteps * ncol))) return rc;
+  CallBlock h;
   const double* coup = nullptr;
-  if (d->coupling) {
-    if ((rc = dev_reserve(g->coup_dev, g->coup_cap, (size_t)total * cstride))) return rc;
-    QSF_CU(cudaMemcpyAsync(g->coup_dev, d->coupling, (size_t)total * cstride * sizeof(double),
-                           cudaMemcpyHostToDevice, g->stream));
+  const size_t nc = d->coupling ? (size_t)total * cstride : 0;
+  if (nc > CallBlock::kCoup) {
+    if ((rc = dev_reserve(g->coup_dev, g->coup_cap, nc))) return rc;
+    QSF_CU(cudaMemcpyAsync(g->coup_dev, d->coupling, nc * sizeof(double), cudaMemcpyHostToDevice, g->stream));
     coup = g->coup_dev;
+  } else if (nc) {
+    std::memcpy(h.coupling, d->coupling, nc * sizeof(double));
+    coup = g->blk->coupling;
   }
-  long long ctl_h[8] = {0, (long long)total, 0, 0, 0, 0, 0, 0};
-  double en_h[2] = {d->last_energy, 0.0};
-  double sc_h[4] = {1.0, 1.0, 1.0, 1.0};
-  QSF_CU(cudaMemcpyAsync(g->ctl, ctl_h, sizeof(ctl_h), cudaMemcpyHostToDevice, g->stream));
-  QSF_CU(cudaMemcpyAsync(g->energy, en_h, sizeof(en_h), cudaMemcpyHostToDevice, g->stream));
-  QSF_CU(cudaMemcpyAsync(g->scale, sc_h, sizeof(sc_h), cudaMemcpyHostToDevice, g->stream));
+  const long long ctl_h[8] = {0, (long long)total, 0, 0, 0, 0, 0, 0};
+  std::copy(ctl_h, ctl_h + 8, h.ctl);
+  h.energy[0] = d->last_energy;
+  h.energy[1] = 0.0;
+  std::fill(h.scale, h.scale + 3, 1.0);
+  h.scale[3] = 0.0;
+  std::fill(h.gmin, h.gmin + kGmin, 0x7fffffff);
   StepDev S{};
   S.mode = d->mode;
   S.dt = dt_sub;
@@ -662,6 +679,8 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   S.coup_stride = cstride;
   S.xs = reinterpret_cast<const int4*>(g->xs);
   S.Vx = g->Vx;
+  S.lg = G.dim >= 2 && G.gauge == QSF_GAUGE_LENGTH && G.n_fields && coup ? 1 : 0;
+  if (S.lg && (rc = dev_reserve(g->xdyn, g->xdyn_cap, (size_t)kTableSteps * 3 * G.dim * g->nmax))) return rc;
   S.ptab = reinterpret_cast<int4*>(g->ptab);
   S.xdyn = reinterpret_cast<int4*>(g->xdyn);
   S.xs_exp = g->xs_exp;
@@ -669,8 +688,9 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   S.l2m = g->l2m;
   S.m_mant = g->m_mant;
   S.texp = g->ibuf;
-  S.gmin = g->ibuf + kTexp;
-  S.sc = g->ibuf + kTexp + kGmin;
+  S.gmin = g->blk->gmin;
+  S.sc = g->ibuf + kTableSteps * kTexp;
+  S.tsteps = kTableSteps;
   S.scmax = g->scmax;
   S.nmax = g->nmax;
   S.partials = g->partials;
@@ -683,7 +703,6 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   // E_kin needs psi_n in memory (every ekin_interval-th step and the last one)
   // (an imaginary-time run with a length-gauge field changes |psi| by its x.E factors, so
   // its steps end and open one by one)
-  S.lg = G.dim >= 2 && G.gauge == QSF_GAUGE_LENGTH && G.n_fields && coup ? 1 : 0;
   S.fused = G.dim >= 2 && !(S.lg && d->mode == QSF_MODE_IM) ? 1 : 0;
   S.ekin_every = d->ekin_interval > 1 ? d->ekin_interval : 1;
   S.normalize = d->normalize;
@@ -699,33 +718,40 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
     S.fterms = g->fterms;
     S.nfterms = g->nfterms;
   }
+  S.nfin = fin_blocks(g, S.nfterms);
   S.fpartials = g->fpartials;
   S.ctl = g->ctl;
   S.energy_state = g->energy;
-  S.rows = g->rows_dev;
+  S.rows = short_rows ? g->blk->rows : g->rows_dev;
   S.scale = g->scale;
   if (G.dim == 1 && (rc = line_prepare(g, S, chunk))) return rc;
-  QSF_CU(cudaMemcpyAsync(g->dS, &S, sizeof(StepDev), cudaMemcpyHostToDevice, g->stream));
+  h.S = S;
+  const size_t bytes = offsetof(CallBlock, coupling) + (nc <= CallBlock::kCoup ? nc * sizeof(double) : 0);
+  QSF_CU(cudaMemcpyAsync(g->blk, &h, bytes, cudaMemcpyHostToDevice, g->stream));
   *out = S;
   *ncol_out = ncol;
   return QSF_OK;
 }
 
 // After a run: pending Normalize factor, observables rows and progress back to host.
-int finish_step(qsf_grid* g, int normalize, int64_t nsteps, int ncol, double* rows, int64_t* steps_done) {
+int finish_step(qsf_grid* g, const StepDev& S, int normalize, int64_t nsteps, int ncol, double* rows,
+                int64_t* steps_done) {
   if (normalize) {
     k_scale<<<grid_blocks(g->G.m), 256, 0, g->stream>>>(g->G.psi, g->G.m, g->scale);
     QSF_CU(cudaGetLastError());
   }
-  long long ctl_h[8];
-  QSF_CU(cudaMemcpyAsync(ctl_h, g->ctl, sizeof(ctl_h), cudaMemcpyDeviceToHost, g->stream));
-  if (rows)
-    QSF_CU(cudaMemcpyAsync(rows, g->rows_dev, (size_t)nsteps * ncol * sizeof(double), cudaMemcpyDeviceToHost,
-                           g->stream));
+  CallBlock h;
+  const size_t nr = rows ? (size_t)nsteps * ncol : 0;
+  const bool short_rows = S.rows == g->blk->rows;
+  const size_t bytes = short_rows ? offsetof(CallBlock, rows) + nr * sizeof(double) : sizeof(h.ctl);
+  if (nr && !short_rows)
+    QSF_CU(cudaMemcpyAsync(rows, g->rows_dev, nr * sizeof(double), cudaMemcpyDeviceToHost, g->stream));
+  QSF_CU(cudaMemcpyAsync(h.ctl, g->blk, bytes, cudaMemcpyDeviceToHost, g->stream));
   QSF_CU(cudaStreamSynchronize(g->stream));
-  if (steps_done) *steps_done = ctl_h[2];
-  if (ctl_h[4] == 2) return fail(QSF_ETIMEDOUT, "a bulk copy into shared memory did not complete in time");
-  if (ctl_h[4]) return fail(QSF_ENUMERIC, "non-positive norm or NaN in a step's reductions");
+  if (nr && short_rows) std::memcpy(rows, h.rows, nr * sizeof(double));
+  if (steps_done) *steps_done = h.ctl[2];
+  if (h.ctl[4] == 2) return fail(QSF_ETIMEDOUT, "a bulk copy into shared memory did not complete in time");
+  if (h.ctl[4]) return fail(QSF_ENUMERIC, "non-positive norm or NaN in a step's reductions");
   return QSF_OK;
 }
 
@@ -813,7 +839,7 @@ int rebuild_batch(qsf_batch* b) {
     gr.q.gauge = std::max(gr.q.gauge, g->G.gauge);
     gr.slots.push_back(kv.first);
     gr.ekin = gr.ekin || (kv.second.S.obs & QSF_OBS_EKIN);
-    if (kv.second.S.nfterms > 0) gr.nfblk = std::max(gr.nfblk, g->nfblk);
+    gr.nfblk = std::max(gr.nfblk, fin_blocks(g, kv.second.S.nfterms));
   }
   const size_t total = b->members.size();
   int rc;
@@ -855,6 +881,7 @@ int rebuild_batch(qsf_batch* b) {
           QSF_CU(cudaEventRecord(b->gfork, b->stream));
           for (size_t i = 0; i < b->groups.size(); ++i) {
             const BatchGroup& gr = b->groups[i];
+            if (gr.q.dim == 1) continue;  // whole runs of steps per launch (batch_launch)
             QSF_CU(cudaStreamWaitEvent(b->gstreams[i], b->gfork, 0));
             const int r = launch_group(*gr.ks, gr.q, gr.dG, gr.dS, (int)gr.slots.size(), gr.ekin, gr.nfblk,
                                        b->gstreams[i], nullptr);
@@ -1015,22 +1042,23 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   g->l2m = 0;
   while ((1LL << (g->l2m + 1)) <= G.m) ++g->l2m;
   g->m_mant = std::ldexp(1.0, g->l2m) / (double)G.m;
-  if ((rc = dev_alloc(g->partials, (size_t)5 * g->pmax)) || (rc = dev_alloc(g->ctl, 8)) ||
-      (rc = dev_alloc(g->energy, 2)) || (rc = dev_alloc(g->scale, 4)) ||
-      (rc = dev_alloc(g->fpartials, (size_t)kMaxFluxBlocks * kMaxFluxBorders))) {
+  if ((rc = dev_alloc(g->partials, (size_t)5 * g->pmax)) || (rc = dev_alloc(g->blk, 1)) ||
+      (rc = dev_alloc(g->fpartials, (size_t)kMaxFluxBlocks * kFinCols))) {
     qsf_grid_destroy(g);
     return rc;
   }
+  g->ctl = g->blk->ctl;  // device addresses inside the block
+  g->energy = g->blk->energy;
+  g->scale = g->blk->scale;
+  g->dS = &g->blk->S;
   // the fused kernels' exponent slots, per-step tables and device descriptors
   const bool fused = ks || D == 1;
-  if (fused && ((rc = dev_alloc(g->ibuf, (size_t)kTexp + kGmin + 4 * (size_t)g->scmax)) ||
-             (rc = dev_alloc(g->ptab, (size_t)D * g->nmax)) ||
-             (rc = dev_alloc(g->xdyn, (size_t)3 * D * g->nmax)) || (rc = dev_alloc(g->dG, 1)) ||
-             (rc = dev_alloc(g->dS, 1)))) {
+  if (fused && ((rc = dev_alloc(g->ibuf, (size_t)kTableSteps * kTexp + 4 * (size_t)g->scmax)) ||
+             (D > 1 && (rc = dev_alloc(g->ptab, (size_t)kTableSteps * D * g->nmax))) || (rc = dev_alloc(g->dG, 1)))) {
     qsf_grid_destroy(g);
     return rc;
   }
-  g->fpmax = (size_t)kMaxFluxBlocks * kMaxFluxBorders;
+  g->fpmax = (size_t)kMaxFluxBlocks * kFinCols;
   if ((rc = D == 1 ? line_setup(g) : ks ? make_tensor_maps(g) : bs_setup(g))) {
     qsf_grid_destroy(g);
     return rc;
@@ -1060,9 +1088,7 @@ int qsf_grid_destroy(qsf_grid* g) {
   fr(g->xdyn);
   fr(g->partials);
   fr(g->fpartials);
-  fr(g->ctl);
-  fr(g->energy);
-  fr(g->scale);
+  fr(g->blk);
   fr(g->rows_dev);
   fr(g->coup_dev);
   fr(g->snap);
@@ -1071,7 +1097,6 @@ int qsf_grid_destroy(qsf_grid* g) {
   fr(g->fpts);
   fr(g->fterms);
   fr(g->dG);
-  fr(g->dS);
   fr(g->mg_slice);
   fr(g->etab);
   fr(g->eptab);
@@ -1343,12 +1368,12 @@ int qsf_flux(qsf_grid* g, const double* A3, int nb, const int* types, int64_t bo
                                             A3 ? A3[1] : 0.0, A3 ? A3[2] : 0.0, A3 ? 1 : 0, nb, g->fpartials,
                                             CoupDev{nullptr, nullptr, 0, 0});
     QSF_CU(cudaGetLastError());
-    std::vector<double> part((size_t)g->nfblk * kMaxFluxBorders);
+    std::vector<double> part((size_t)g->nfblk * kFinCols);
     QSF_CU(cudaMemcpyAsync(part.data(), g->fpartials, part.size() * sizeof(double), cudaMemcpyDeviceToHost,
                            g->stream));
     QSF_CU(cudaStreamSynchronize(g->stream));
     for (int k = 0; k < g->nfblk; ++k)
-      for (int b = 0; b < nb; ++b) res[(size_t)b] += part[(size_t)k * kMaxFluxBorders + b];
+      for (int b = 0; b < nb; ++b) res[(size_t)b] += part[(size_t)k * kFinCols + b];
   }
   for (int b = 0; b < nb; ++b) out[b] = res[(size_t)b] * g->G.dV / g->G.ax[0].dx;
   return QSF_OK;
@@ -1405,10 +1430,10 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
   if (!g->ks && g->G.dim > 1) return generic_step(g, d, rows, steps_done);
   StepDev S{};
   int ncol = 0, rc;
-  if ((rc = prepare_step(g, d, &S, &ncol))) return rc;
+  if ((rc = prepare_step(g, d, &S, &ncol, INT64_MAX, true))) return rc;
   if (g->G.dim == 1) {
     if ((rc = line_run(g, S, S.nsteps, d->kernel_ms, d->kernel_launches))) return rc;
-    return finish_step(g, d->normalize, d->nsteps, ncol, rows, steps_done);
+    return finish_step(g, S, d->normalize, d->nsteps, ncol, rows, steps_done);
   }
   if (d->kernel_ms) {
     // one event pair per launch of the whole call (at most 8 per step), read at the end,
@@ -1417,11 +1442,13 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
     P.ms = d->kernel_ms;
     P.count = d->kernel_launches;
     rc = P.init(g->stream, (int)std::min<int64_t>(S.nsteps * 8 + 8, 1 << 20));
-    for (int64_t k = 0; k < S.nsteps && rc == QSF_OK; ++k) rc = launch_step(g, S, &P);
+    for (int64_t k = 0; k < S.nsteps && rc == QSF_OK; ++k)
+      if (!(rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream, &P))) rc = launch_step(g, S, &P);
     if (rc == QSF_OK) rc = P.flush();
     P.release();
     if (rc) return rc;
   } else if (S.nsteps < 4) {
+    if ((rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)S.nsteps, g->stream))) return rc;
     for (int64_t k = 0; k < S.nsteps; ++k)
       if ((rc = launch_step(g, S))) return rc;
   } else {
@@ -1433,18 +1460,18 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
     const bool skip_open = S.fused != 0 && !(S.obs & QSF_OBS_EKIN);
     int64_t first = 0;
     if (skip_open) {
-      if ((rc = launch_step(g, S))) return rc;
+      if ((rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream)) || (rc = launch_step(g, S))) return rc;
       first = 1;
     }
     const int64_t rest = S.nsteps - first;
-    constexpr int64_t kGraphSteps = 16;
+    constexpr int64_t kGraphSteps = kTableSteps;
     const int64_t per = std::max<int64_t>(1, std::min<int64_t>(kGraphSteps, rest));
     if (rest > 0) {
       cudaGraphExec_t exec = nullptr;
       FinOverlap ov;
       const bool overlap = fin_overlap_ok(S);
       if (overlap && (rc = ensure_fin_stream(g, &ov))) return rc;
-      const int ekin = (S.obs & QSF_OBS_EKIN) ? 1 : 0, nfblk = S.nfterms > 0 ? g->nfblk : 1;
+      const int ekin = (S.obs & QSF_OBS_EKIN) ? 1 : 0, nfblk = fin_blocks(g, S.nfterms);
       for (const qsf_grid::StepGraph& sg : g->step_graphs)
         if (sg.per == per && sg.skip_open == (int)skip_open && sg.overlap == (int)overlap && sg.ekin == ekin &&
             sg.nfblk == nfblk)
@@ -1453,6 +1480,7 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
         if ((rc = capture_graph(
                  g->stream,
                  [&]() {
+                   if (int r = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)per, g->stream)) return r;
                    for (int64_t k = 0; k < per; ++k)
                      if (int r = launch_step(g, S, nullptr, !skip_open, overlap ? &ov : nullptr)) return r;
                    if (ov.pending) QSF_CU(cudaStreamWaitEvent(g->stream, ov.done, 0));  // join
@@ -1466,11 +1494,12 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
         const cudaError_t ce = cudaGraphLaunch(exec, g->stream);
         if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
       }
+      if (rest % per && (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)(rest % per), g->stream))) return rc;
       for (int64_t k = rest - rest % per; k < rest; ++k)
         if ((rc = launch_step(g, S, nullptr, !skip_open))) return rc;
     }
   }
-  return finish_step(g, d->normalize, d->nsteps, ncol, rows, steps_done);
+  return finish_step(g, S, d->normalize, d->nsteps, ncol, rows, steps_done);
 }
 
 // End of one member-operation step: the flux partials summed per border in block order
@@ -1483,7 +1512,7 @@ __global__ void k_generic_row(const double* __restrict__ fpart, int nfblk, int n
   double* row = rows + (*step) * ncol;
   if ((int)threadIdx.x < nb) {
     double v = 0.0;
-    for (int k = 0; k < nfblk; ++k) v += fpart[k * kMaxFluxBorders + threadIdx.x];
+    for (int k = 0; k < nfblk; ++k) v += fpart[k * kFinCols + threadIdx.x];
     row[3 + threadIdx.x] = v * dV / dx;
   }
   __syncthreads();
@@ -1786,7 +1815,7 @@ int qsf::batch_add_nowait(qsf_batch* b, qsf_grid* g, const qsf_step_desc* d, int
   dd.kernel_ms = nullptr;
   dd.kernel_launches = nullptr;
   int rc;
-  if ((rc = prepare_step(g, &dd, &mb.S, &mb.ncol, 1))) return rc;  // 1D members: one sub-step per launch
+  if ((rc = prepare_step(g, &dd, &mb.S, &mb.ncol, kTableSteps))) return rc;
   QSF_CU(cudaStreamSynchronize(g->stream));
   mb.nsteps = d->nsteps;
   mb.normalize = d->normalize;
@@ -1829,11 +1858,36 @@ int qsf::batch_launch(qsf_batch* b, int64_t steps) {
   if (!b || steps < 0) return fail(QSF_EINVAL, "bad argument");
   int rc;
   if (b->dirty && (rc = rebuild_batch(b))) return rc;
-  if (b->exec)
-    for (int64_t k = 0; k < steps; ++k) {
-      const cudaError_t ce = cudaGraphLaunch(b->exec, b->stream);
-      if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
+  bool planes = false, lines = false;
+  for (const BatchGroup& gr : b->groups) (gr.q.dim == 1 ? lines : planes) = true;
+  for (int64_t k = 0; k < steps; k += kTableSteps) {
+    const int now = (int)std::min<int64_t>(kTableSteps, steps - k);
+    if (lines) {  // the 1D groups beside the others, each on its stream
+      QSF_CU(cudaEventRecord(b->gfork, b->stream));
+      for (size_t i = 0; i < b->groups.size(); ++i) {
+        const BatchGroup& gr = b->groups[i];
+        if (gr.q.dim != 1) continue;
+        const LineKernels& L = *line_kernels(gr.q.n);
+        const int count = (int)gr.slots.size();
+        QSF_CU(cudaStreamWaitEvent(b->gstreams[i], b->gfork, 0));
+        if ((rc = line_launch_tables(L, gr.dG, gr.dS, count, now, gr.q.gauge == QSF_GAUGE_LENGTH, b->gstreams[i])) ||
+            (rc = line_launch_steps(L, false, gr.dG, gr.dS, count, now, b->gstreams[i])))
+          return rc;
+        QSF_CU(cudaEventRecord(b->gjoin[i], b->gstreams[i]));
+      }
     }
+    if (planes) {
+      for (const BatchGroup& gr : b->groups)
+        if (gr.q.dim != 1 && (rc = launch_tables(gr.q, gr.dG, gr.dS, (int)gr.slots.size(), now, b->stream))) return rc;
+      for (int s = 0; s < now; ++s) {
+        const cudaError_t ce = cudaGraphLaunch(b->exec, b->stream);
+        if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
+      }
+    }
+    if (lines)
+      for (size_t i = 0; i < b->groups.size(); ++i)
+        if (b->groups[i].q.dim == 1) QSF_CU(cudaStreamWaitEvent(b->stream, b->gjoin[i], 0));
+  }
   return QSF_OK;
 }
 

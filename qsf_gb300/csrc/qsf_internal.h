@@ -60,6 +60,22 @@ using qsf::FluxPoint;
 using qsf::FluxTerm;
 using qsf::BorderNodes;
 
+// What a call sends to the device and brings back, in one copy each way: control words,
+// convergence and Normalize state, the observables rows and the coupling rows of a short
+// call, the step descriptor.  (Five copies down and two back took half of a one-step
+// call on a 1024-point line.)
+struct CallBlock {
+  static constexpr int kRows = 256, kCoup = 256;  // doubles of rows and of coupling kept here
+  long long ctl[8];
+  double energy[2], scale[4];
+  double rows[kRows];
+  // the pass minima change by atomics while every block reads the words around them: lines
+  // of their own
+  alignas(128) int gmin[32];
+  alignas(128) StepDev S;
+  double coupling[kCoup];
+};
+
 struct qsf_grid {
   qsf_grid_desc desc{};
   GridDev G{};
@@ -68,6 +84,7 @@ struct qsf_grid {
   BorderNodes bn;
   const KernelSet* ks = nullptr;  // kernels for this grid's line length
   GridDev* dG = nullptr;          // device copy of G (step kernels read descriptors from device arrays)
+  CallBlock* blk = nullptr;       // device memory of the words below and of short calls' rows
   StepDev* dS = nullptr;          // device copy of the current step descriptor
   // the batch this grid is a member of (qsf_batch_add) and its slot there: destroying
   // the grid removes it from that batch first (the batch's graph reads its memory)
@@ -88,7 +105,8 @@ struct qsf_grid {
   int nmax = 0;
   int l2m = 0;
   double m_mant = 1.0;
-  // fixed-point pass bookkeeping: [kTexp] table exponents, [4] pass minima, [4][scmax] block exponents
+  size_t xdyn_cap = 0;
+  // fixed-point pass bookkeeping: [kTableSteps][kTexp] table exponents, [4][scmax] line exponents
   int* ibuf = nullptr;
   int scmax = 1;
   // reductions

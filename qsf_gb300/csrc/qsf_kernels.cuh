@@ -41,6 +41,7 @@ namespace qsf {
 
 constexpr int kMaxDim = 3;
 constexpr int kMaxFluxBorders = 16;
+constexpr int kFinCols = kMaxFluxBorders + 5;  // sums of a k_finalize block: borders, norm, E_pot, E_kin per axis
 struct AxisDev {
   int n, n2;
   int shift;  // log2(n) when n is a power of two, else -1
@@ -129,20 +130,21 @@ struct StepDev {
   // phase tables in the split form (split62: 2^62 fixed point as signed 32-bit halves)
   const int4* xs;          // static X half-step factor per point (dt/2, incl. absorber), * 2^-xs_exp
   const long long* Vx;     // potential per point in 2^vshift fixed point
-  int4* ptab;              // [dim][nmax] P-phase tables of the current step (|.| <= 1)
-  int4* xdyn;              // [3][dim][nmax] length-gauge factors: open half, close half, close . next open half
+  // tables of the sub-steps ctl[7] .. ctl[7] + tsteps - 1 (k_tables), one after another
+  int4* ptab;              // [tsteps][dim][nmax] P-phase tables (|.| <= 1)
+  int4* xdyn;              // [tsteps][3][dim][nmax] length-gauge factors: open half, close half, close . next open half
+  int tsteps;
   int lg;                  // 2D / 3D: the X halves carry length-gauge factors (a field couples x.E)
   int xs_exp;              // exponent taken out of xs (imaginary time: factors above 1)
   int vshift;              // Vx = round(V * 2^vshift)
   int l2m;                 // 1/m = m_mant * 2^-l2m, m_mant in (0.5, 1] (folded into axis 0's P table)
   double m_mant;
-  int* texp;               // [3][3] exponents taken out of the per-step tables (set by k_tables)
-  int* gmin;               // [kGmin] minimum block exponent of each fixed-point pass (gmin_slot)
+  int* texp;               // [tsteps][kTexp] exponents taken out of the per-step tables (set by k_tables)
+  int* gmin;               // [kGmin] minimum line exponent of each fixed-point pass (gmin_slot)
   int* sc;                 // [4][scmax] line exponents of each fixed-point pass (qsf_passes.cuh)
   int scmax;
   // fused: a sub-step's closing row pass also applies the next sub-step's opening X half
-  // and forward transform (ψ stays in fixed point between the steps of a call); the
-  // pending Normalize factor then folds into the next sub-step's axis-0 P table
+  // and forward transform (ψ stays in fixed point between the steps of a call)
   int fused;
   // E_kin (QSF_OBS_EKIN) at the end of every ekin_every-th step of the call and of its
   // last step; such a step ends with psi_n stored as complex128 (its other transforms
@@ -167,23 +169,27 @@ struct StepDev {
   const FluxPoint* fpts;
   const FluxTerm* fterms;
   int nfterms;
-  double* fpartials;  // [nblk][kMaxFluxBorders]
+  int nfin;           // blocks of k_finalize
+  double* fpartials;  // [blocks][kFinCols] sums of k_finalize's blocks
   // control (device): ctl[0] sub-step within call (k_finalize's), ctl[1] stop after
   // this sub-step (or nsteps), ctl[2] steps done, ctl[3] finalize block counter,
-  // ctl[4] NaN flag, ctl[5] sub-step of the pass kernels (k_tables copies it from
-  // ctl[6]), ctl[6] next sub-step of the pass kernels (advanced by the sub-step's last
-  // pass).  The two counters let k_finalize of one sub-step run beside the next
-  // sub-step's tables and first passes.
+  // ctl[4] NaN flag, ctl[6] sub-step of the pass kernels up to axis 0's, which copies it to
+  // ctl[5] for those after it (the closing pass advances ctl[6]: no kernel reads the word
+  // that it or a kernel beside it writes), ctl[7] first sub-step the tables hold.  The
+  // pass kernels' own counter lets k_finalize of one sub-step run beside the next one's
+  // first passes.
   // nsteps counts sub-steps: steps * substeps (MultiProductSplit order).
   int substeps;
   long long* ctl;
   double* energy_state;  // [0] last E
   double* rows;          // [nsteps][3 + nborders]
-  double* scale;         // pending Normalize factor (1 when none); [2] its square as the 1D kernels carry it
+  // Normalize only scales psi: psi stays unscaled in a call and the sums are scaled.
+  // [0] the pending factor of psi in memory, [2] its square for psi as the passes hold it,
+  // [3] the power of two that the next sub-step takes out of it (exact)
+  double* scale;
   LineDev line;          // 1D grids (qsf_line1d.cuh)
 };
 
-__device__ __forceinline__ bool step_active(const StepDev& S) { return S.ctl[0] <= S.ctl[1] && S.ctl[0] < S.nsteps; }
 // whether sub-step `sub` ends a step whose observables include E_kin
 __device__ __forceinline__ bool ekin_at(const StepDev& S, long long sub) {
   if (!(S.obs & 4u) || (sub + 1) % S.substeps) return false;
@@ -192,7 +198,7 @@ __device__ __forceinline__ bool ekin_at(const StepDev& S, long long sub) {
 }
 // hint: move the 128-byte line holding p from DRAM into L2 (p must be in an allocation)
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-__device__ __forceinline__ bool pass_active(const StepDev& S) { return S.ctl[5] <= S.ctl[1] && S.ctl[5] < S.nsteps; }
+__device__ __forceinline__ bool pass_active(const StepDev& S, long long sub) { return sub <= S.ctl[1] && sub < S.nsteps; }
 
 // ------------------------------------------------------------ reductions
 __device__ __forceinline__ double warp_sum(double v) {
@@ -381,11 +387,11 @@ __host__ __device__ constexpr int tma_box_rows(int n) {
 //   axis d (open / close half), texp[3][d]: opening half of the next sub-step (fused).
 //   The static X table's exponent is StepDev::xs_exp.
 constexpr int kTexp = 12;
-// Pass minima: [1..3] passes 1-3 of the sub-step; pass 0 alternates between [0] and
-// [4] with the parity of the sub-step, because in fused mode the closing pass of
-// sub-step k produces pass 0 of sub-step k + 1 while pass 0 of k may still be read.
-constexpr int kGmin = 5;
-__device__ __forceinline__ int gmin_slot(int pass, long long sub) { return pass ? pass : ((sub & 1) ? 4 : 0); }
+// Pass minima alternate with the parity of the sub-step: the closing pass of sub-step k
+// produces pass 0 of k + 1 while pass 0 of k may still be read.  Axis 0's pass resets the
+// next sub-step's slot of pass 0, the closing pass those of passes 1 - 3.
+constexpr int kGmin = 8;
+__device__ __forceinline__ int gmin_slot(int pass, long long sub) { return pass * 2 + (int)(sub & 1); }
 
 // Phase factors (|components| <= 1) are stored in 2^62 fixed point as the signed
 // 32-bit halves of each component (int4 {re lo, re hi, im lo, im hi}, as the FFT's
@@ -428,48 +434,6 @@ __device__ __forceinline__ double2 table_entry(const GridDev& g, const StepDev& 
   return expop(S.mode, (S.dt * 0.5) * (xpos(a, i) * E));
 }
 
-// One (kind, axis) table of a step's per-step tables, or its slice `part` of `tb` (all
-// threads of the block call it; red: 32 doubles of shared memory, e_sh: one shared int)
-__device__ __forceinline__ void tables_one(const GridDev& g, const StepDev& S, long long sub, int kind, int d, int part,
-                                           int tb, double* red, int* e_sh) {
-  const int D = g.dim;
-  if (kind > 0 && g.gauge != 1) return;
-  if (kind == 3 && (!S.fused || sub + 1 >= S.nsteps)) return;
-  const double* cp = S.coupling ? S.coupling + sub * S.coup_stride : nullptr;
-  const double* cn = (S.coupling && sub + 1 < S.nsteps) ? S.coupling + (sub + 1) * S.coup_stride : nullptr;
-  const int n = g.ax[d].n;
-  double mant = 1.0;
-  if (kind == 0 && d == 0) {
-    mant = S.m_mant;
-    if (S.fused && S.normalize) mant *= *S.scale;
-  }
-  double mx = mant;  // real time: phases of modulus 1 times the mantissa
-  if (S.mode == 1) {  // imaginary time: real factors, maximum over the table
-    mx = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, table_entry(g, S, cp, cn, kind, d, i).x * mant);
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = fmax(mx, red[w]);
-  }
-  if (threadIdx.x == 0) {
-    int e = 0;
-    if (mx > 1.0) frexp(mx, &e);  // mx < 2^e
-    *e_sh = e;
-    if (part == 0) S.texp[kind * 3 + d] = e;
-  }
-  __syncthreads();
-  const double sc = ldexp(mant, -*e_sh);
-  int4* out = kind == 0 ? S.ptab + (size_t)d * S.nmax : S.xdyn + ((size_t)(kind - 1) * D + d) * S.nmax;
-  const int chunk = (n + tb - 1) / tb;
-  const int i1 = min(n, (part + 1) * chunk);
-  for (int i = part * chunk + threadIdx.x; i < i1; i += blockDim.x) {
-    const double2 f = table_entry(g, S, cp, cn, kind, d, i);
-    out[i] = split62(make_double2(fmin(fmax(f.x * sc, -1.0), 1.0), fmin(fmax(f.y * sc, -1.0), 1.0)));
-  }
-}
-
 __device__ __forceinline__ void flux_block(const GridDev& g, const FluxPoint* __restrict__ fpts, const FluxTerm* __restrict__ fterms,
                            int t0, int t1, const double2* __restrict__ snap, const double* A, int nb, double* red,
                            double* out) {
@@ -510,72 +474,6 @@ __device__ __forceinline__ void flux_block(const GridDev& g, const FluxPoint* __
     out[threadIdx.x] = v;
   }
   __syncthreads();
-}
-
-// End of a (sub-)step, run by one block once every block's partials and flux partials
-// (nfb blocks of them) are in memory: fixed-order sums, the observables row, the
-// Normalize factor, the convergence test and the step counters.  red: 32 *
-// kMaxFluxBorders doubles of shared memory.
-__device__ __forceinline__ void finalize_tail(const GridDev& g, const StepDev& S, long long sub, bool step_end,
-                                              long long step, int nb, int nfb, double* red) {
-  if (!step_end) {
-    if (threadIdx.x == 0) {
-      if (S.normalize) *S.scale = 1.0;  // no Normalize between sub-steps
-      S.ctl[3] = 0;
-      S.ctl[0] = sub + 1;
-    }
-    return;
-  }
-  // last block: deterministic sums in a fixed order
-  const bool ek = ekin_at(S, sub);
-  double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < S.nrowblk; i += blockDim.x) {
-    acc[0] += S.partials[0 * S.pmax + i];
-    acc[1] += S.partials[1 * S.pmax + i];
-  }
-  if (ek) {
-    for (int d = 0; d < g.dim; ++d)
-      for (int i = threadIdx.x; i < (d == g.dim - 1 ? S.nrowblk : S.naxblk[d]); i += blockDim.x)
-        acc[2 + d] += S.partials[(2 + d) * S.pmax + i];
-  }
-  __shared__ double fsum[kMaxFluxBorders];
-  if (threadIdx.x < nb) {  // per border, the blocks' partials in block order
-    double v = 0.0;  // 0 where no point of the grid lies on a border (no block wrote partials)
-    for (int k = 0; k < nfb && S.nfterms > 0; ++k) v += S.fpartials[k * kMaxFluxBorders + threadIdx.x];
-    fsum[threadIdx.x] = v;
-  }
-  block_sum<5>(acc, red);  // its barriers also publish fsum
-  if (threadIdx.x == 0) {
-    const double norm = acc[0] * g.dV;
-    const double epot = acc[1] * g.dV;
-    double ekin = 0.0;
-    if (ek) {
-      for (int d = 0; d < g.dim; ++d) ekin += (double)(g.m / g.ax[d].n) * acc[2 + d];
-      ekin = 0.5 * g.dVm * ekin;
-    }
-    const int ncol = 3 + nb;
-    double* row = S.rows + step * ncol;
-    row[0] = norm;
-    row[1] = epot;
-    row[2] = ekin;
-    for (int b = 0; b < nb; ++b) row[3 + b] = fsum[b] * g.dV / g.ax[0].dx;
-    if (!(norm > 0.0) || isnan(epot) || isnan(ekin)) S.ctl[4] = 1;
-    if (S.normalize && norm > 0.0) *S.scale = sqrt(1.0 / norm);
-    // the convergence test needs E = E_pot + E_kin: with E_kin on every k-th step only,
-    // it runs on those steps (comparing with the previous one that had it)
-    if (S.mode == 1 && S.state_accuracy > 0.0 && (ek || !(S.obs & 4u))) {
-      const double se = (S.energy_after_normalize & 1) ? 1.0 / norm : 1.0;
-      const double sk = (S.energy_after_normalize & 2) ? 1.0 / norm : 1.0;
-      const double E = epot * se + ekin * sk;
-      const double dE = E - S.energy_state[0];
-      S.energy_state[0] = E;
-      // converged: one more step runs (its last sub-step is sub + substeps)
-      if (S.ctl[1] >= S.nsteps && fabs(dE) <= S.state_accuracy) S.ctl[1] = sub + S.substeps;
-    }
-    S.ctl[2] = step + 1;
-    S.ctl[3] = 0;
-    S.ctl[0] = sub + 1;
-  }
 }
 
 #ifdef QSF_DEFINE_KERNELS
@@ -638,44 +536,59 @@ __global__ void k_build_static(GridDev g, int mode, double delta, int xs_exp, in
   }
 }
 
-// Per-step tables: `tb` blocks per (kind, axis) table, each storing a contiguous slice.
-// A table whose values exceed 1 in magnitude (imaginary time, or a Normalize factor
-// folded in) is stored times 2^-e, e from its maximum (every block of the table
-// evaluates that maximum, so the slices agree), and e is recorded in texp.  Axis 0's P
-// table carries the mantissa of 1/m (its power of two goes into the exponent) and, in
-// fused mode, the pending Normalize factor.  Block 0 resets the pass minima this
-// sub-step's passes will produce.
+// The tables of the next `steps` sub-steps, so that no step waits for its own: `tb` blocks
+// per (kind, axis) table, each storing a contiguous slice; gridDim.y sub-steps, z solves.  A
+// table whose values exceed 1 in magnitude (imaginary time) is stored times 2^-e, e from
+// its maximum (every block of the table evaluates that maximum, so the slices agree), and
+// e is recorded in texp.  Axis 0's P table carries the mantissa of 1/m (its power of two
+// goes into the exponent).
 __global__ void __launch_bounds__(256) k_tables(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss,
                                                 int tb) {
-  const GridDev& g = Gs[blockIdx.y];
-  const StepDev& S = Ss[blockIdx.y];
-  // the sub-step of this step's passes; every block stores the same value, also when
-  // the step is inactive (its passes then read an inactive sub-step too)
-  const long long sub = S.ctl[6];
-  if (threadIdx.x == 0) S.ctl[5] = sub;
-  if (!(sub <= S.ctl[1] && sub < S.nsteps)) return;
+  const GridDev& g = Gs[blockIdx.z];
+  const StepDev& S = Ss[blockIdx.z];
+  const long long first = S.ctl[6], sub = first + blockIdx.y;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) S.ctl[7] = first;
+  if (!pass_active(S, sub)) return;
   __shared__ double red[32];
   __shared__ int e_sh;
   const int D = g.dim;
   const int table = blockIdx.x / tb, part = blockIdx.x % tb;
   const int kind = table / D, d = table % D;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    S.gmin[1] = S.gmin[2] = S.gmin[3] = 0x7fffffff;
-    S.gmin[gmin_slot(0, sub + 1)] = 0x7fffffff;               // produced by this sub-step's closing pass
-    if (!S.fused || sub == 0) S.gmin[gmin_slot(0, sub)] = 0x7fffffff;  // produced by this sub-step's opening pass
+  if (kind > 0 && !S.lg) return;
+  if (kind == 3 && (!S.fused || sub + 1 >= S.nsteps)) return;
+  const double* cp = S.coupling ? S.coupling + sub * S.coup_stride : nullptr;
+  const double* cn = (S.coupling && sub + 1 < S.nsteps) ? S.coupling + (sub + 1) * S.coup_stride : nullptr;
+  const int n = g.ax[d].n;
+  const double mant = kind == 0 && d == 0 ? S.m_mant : 1.0;
+  double mx = mant;  // real time: phases of modulus 1 times the mantissa
+  if (S.mode == 1) {  // imaginary time: real factors, maximum over the table
+    mx = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, table_entry(g, S, cp, cn, kind, d, i).x * mant);
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = fmax(mx, red[w]);
   }
-  tables_one(g, S, sub, kind, d, part, tb, red, &e_sh);
+  if (threadIdx.x == 0) {
+    int e = 0;
+    if (mx > 1.0) frexp(mx, &e);  // mx < 2^e
+    e_sh = e;
+    if (part == 0) S.texp[blockIdx.y * kTexp + kind * 3 + d] = e;
+  }
+  __syncthreads();
+  const double sc = ldexp(mant, -e_sh);
+  int4* out = kind == 0 ? S.ptab + ((size_t)blockIdx.y * D + d) * S.nmax
+                        : S.xdyn + (((size_t)blockIdx.y * 3 + kind - 1) * D + d) * S.nmax;
+  const int chunk = (n + tb - 1) / tb;
+  const int i1 = min(n, (part + 1) * chunk);
+  for (int i = part * chunk + threadIdx.x; i < i1; i += blockDim.x) {
+    const double2 f = table_entry(g, S, cp, cn, kind, d, i);
+    out[i] = split62(make_double2(fmin(fmax(f.x * sc, -1.0), 1.0), fmin(fmax(f.y * sc, -1.0), 1.0)));
+  }
 }
 
 #endif  // QSF_DEFINE_KERNELS
-
-// pending Normalize factor s = F 2^-62 * 2^k with F in [2^61, 2^62)
-__device__ __forceinline__ void split_scale(double s, long long& F, int& k) {
-  int e;
-  const double f = frexp(s, &e);
-  F = __double2ll_rn(f * 4611686018427387904.0);
-  k = e;
-}
 
 #ifdef QSF_DEFINE_KERNELS
 // ------------------------------------------------------------ flux + finalize
@@ -691,40 +604,123 @@ __global__ void __launch_bounds__(256) k_flux(GridDev g, const FluxPoint* fpts, 
   coup_load(cd, Av);
   const int chunk = (nfterms + gridDim.x - 1) / gridDim.x;
   const int t0 = blockIdx.x * chunk, t1 = min(nfterms, t0 + chunk);
-  flux_block(g, fpts, fterms, t0, t1, snap, useA ? Av : nullptr, nb, red, out_partials + blockIdx.x * kMaxFluxBorders);
+  flux_block(g, fpts, fterms, t0, t1, snap, useA ? Av : nullptr, nb, red, out_partials + blockIdx.x * kFinCols);
 }
 
-// Border fluxes (grid.h:519-573, propagator.h:249-265) from the psi_n snapshot,
-// deterministic reductions of all partials, Normalize scale and IM convergence.
-// Grid: nblk blocks; block b sums flux terms [b*chunk, (b+1)*chunk); the last block
-// to finish reduces everything in a fixed order and writes the observables row.
+// End of a sub-step: border fluxes (grid.h:519-573, propagator.h:249-265) from the psi_n
+// snapshot, the sums of all partials in a fixed order, the observables row, the Normalize
+// factor, the imaginary-time convergence test and the counters.  Block b sums its share of
+// the flux terms and of the row and E_kin partials; the last block to finish adds the
+// blocks' sums and writes the row.  What bounds it: chains of dependent loads, so the words
+// of the last part are loaded before the sums they wait for.
 __global__ void __launch_bounds__(256) k_finalize(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss) {
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
-  if (!step_active(S)) return;
+  const long long sub = S.ctl[0], stop = S.ctl[1], nsteps = S.nsteps;
+  const int nblk = S.nfin;  // its own count, whatever the launch's: the sums do not depend on the batch
+  if (!(sub <= stop && sub < nsteps) || (int)blockIdx.x >= nblk) return;
   __shared__ double red[32 * kMaxFluxBorders];
   __shared__ int is_last;
-  const long long sub = S.ctl[0];
+  const int K = S.substeps, nb = S.nborders, tid = threadIdx.x;
   // observables, Normalize and the convergence test once per step (its last sub-step)
-  const bool step_end = (sub + 1) % S.substeps == 0;
-  const long long step = sub / S.substeps;
-  const int nb = S.nborders;
-  if (S.nfterms > 0 && step_end) {
+  const bool step_end = K == 1 || (sub + 1) % K == 0;
+  const long long step = K == 1 ? sub : sub / K;
+  if (!step_end) {
+    if (blockIdx.x == 0 && tid == 0) {
+      S.scale[3] = 0.0;
+      S.ctl[0] = sub + 1;
+    }
+    return;
+  }
+  const bool ek = ekin_at(S, sub);
+  const double cf0 = S.scale[2], e0 = S.energy_state[0];
+  const int nrow = S.nrowblk, nft = S.nfterms, D = g.dim;
+  double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  double* mine = S.fpartials + (size_t)blockIdx.x * kFinCols;
+  {
+    const int chunk = (nrow + nblk - 1) / nblk, i1 = min(nrow, ((int)blockIdx.x + 1) * chunk);
+    for (int i = blockIdx.x * chunk + tid; i < i1; i += blockDim.x) {
+      acc[0] += S.partials[i];
+      acc[1] += S.partials[S.pmax + i];
+    }
+    if (ek)
+      for (int d = 0; d < D; ++d) {
+        const int n = d == D - 1 ? nrow : S.naxblk[d], c = (n + nblk - 1) / nblk, j1 = min(n, ((int)blockIdx.x + 1) * c);
+        for (int i = blockIdx.x * c + tid; i < j1; i += blockDim.x) acc[2 + d] += S.partials[(size_t)(2 + d) * S.pmax + i];
+      }
+  }
+  if (nft > 0) {
     const double* A = (g.gauge == 0 && S.coupling && g.n_fields) ? S.coupling + sub * S.coup_stride : nullptr;
-    const int chunk = (S.nfterms + gridDim.x - 1) / gridDim.x;
-    const int t0 = blockIdx.x * chunk, t1 = min(S.nfterms, t0 + chunk);
-    flux_block(g, S.fpts, S.fterms, t0, t1, S.snap, A, nb, red, S.fpartials + blockIdx.x * kMaxFluxBorders);
+    const int chunk = (nft + nblk - 1) / nblk;
+    const int t0 = blockIdx.x * chunk, t1 = min(nft, t0 + chunk);
+    flux_block(g, S.fpts, S.fterms, t0, t1, S.snap, A, nb, red, mine);
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned long long done = atomicAdd((unsigned long long*)&S.ctl[3], 1ull);
-    is_last = (done == (unsigned long long)gridDim.x - 1);
+  if (ek) block_sum<5>(acc, red);
+  else block_sum<2>(acc, red);
+  if (nblk > 1) {
+    if (tid == 0) {
+      for (int k = 0; k < 5; ++k) mine[kMaxFluxBorders + k] = acc[k];
+      __threadfence();
+      const unsigned long long done = atomicAdd((unsigned long long*)&S.ctl[3], 1ull);
+      is_last = done == (unsigned long long)nblk - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+  } else {
+    __syncthreads();  // this block's fluxes
+  }
+  // the blocks' sums: one warp per column, blocks in order of lanes and strides
+  __shared__ double tot[kFinCols];
+  const int lane = tid & 31;
+  for (int c = tid >> 5; c < kFinCols; c += (int)(blockDim.x >> 5)) {
+    if (c < kMaxFluxBorders ? c >= nb || nft == 0 : nblk == 1) continue;
+    double v = 0.0;
+    for (int k = lane; k < nblk; k += 32) v += S.fpartials[(size_t)k * kFinCols + c];
+    v = warp_sum(v);
+    if (lane == 0) tot[c] = v;
   }
   __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  finalize_tail(g, S, sub, step_end, step, nb, (int)gridDim.x, red);
+  double* row = S.rows + step * (3 + nb);
+  if (tid < nb) row[3 + tid] = nft > 0 ? tot[tid] * cf0 * g.dV / g.ax[0].dx : 0.0;
+  if (tid == 0) {
+    if (nblk > 1)
+      for (int k = 0; k < 5; ++k) acc[k] = tot[kMaxFluxBorders + k];
+    double cfac = cf0;
+    const double norm = acc[0] * g.dV * cfac;
+    const double epot = acc[1] * g.dV * cfac;
+    double ekin = 0.0;
+    if (ek) {
+      for (int d = 0; d < D; ++d) ekin += (double)(g.m / g.ax[d].n) * acc[2 + d];
+      ekin = 0.5 * g.dVm * ekin * cfac;
+    }
+    row[0] = norm;
+    row[1] = epot;
+    row[2] = ekin;
+    if (!(norm > 0.0) || isnan(epot) || isnan(ekin)) S.ctl[4] = 1;
+    if (S.normalize && norm > 0.0) {
+      cfac = cfac / norm;
+      *S.scale = sqrt(cfac);
+      int e;
+      frexp(cfac, &e);
+      e >>= 1;
+      S.scale[3] = (double)e;
+      S.scale[2] = ldexp(cfac, -2 * e);
+    }
+    // the convergence test needs E = E_pot + E_kin: with E_kin on every k-th step only,
+    // it runs on those steps (comparing with the previous one that had it)
+    if (S.mode == 1 && S.state_accuracy > 0.0 && (ek || !(S.obs & 4u))) {
+      const double se = (S.energy_after_normalize & 1) ? 1.0 / norm : 1.0;
+      const double sk = (S.energy_after_normalize & 2) ? 1.0 / norm : 1.0;
+      const double E = epot * se + ekin * sk;
+      S.energy_state[0] = E;
+      // converged: one more step runs (its last sub-step is sub + substeps)
+      if (stop >= nsteps && fabs(E - e0) <= S.state_accuracy) S.ctl[1] = sub + K;
+    }
+    S.ctl[2] = step + 1;
+    S.ctl[3] = 0;
+    S.ctl[0] = sub + 1;
+  }
 }
 
 // apply a pending Normalize factor (end of a qsf_step call / qsf_normalize)

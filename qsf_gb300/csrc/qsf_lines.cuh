@@ -195,9 +195,12 @@ struct Ln {
   static constexpr int kRowSmem = buf_bytes(kRowThreads) + 256;
   static constexpr int kColSmem = (kColBytes + 127) / 128 * 128 + 256 + 128;
   // resident blocks per SM the kernels are compiled for: 128 registers a thread for 12
-  // and more points, 80 for 8
+  // and more points, 112 for 8 (rows of 256^3: 597, 568, 550, 545 us with 64, 80, 96, 112
+  // registers, the wider ones without spills; 144 and more with 16 points lose a quarter of
+  // the warps and 29 % at 2048^2)
   __host__ __device__ static constexpr int blocks(int nth) {
-    return 65536 / ((E > 8 ? 128 : 80) * nth) > 16 ? 16 : 65536 / ((E > 8 ? 128 : 80) * nth) < 1 ? 1 : 65536 / ((E > 8 ? 128 : 80) * nth);
+    constexpr int regs = E > 8 ? 128 : 112;
+    return 65536 / (regs * nth) > 32 ? 32 : 65536 / (regs * nth) < 1 ? 1 : 65536 / (regs * nth);
   }
   // slots of register arrays: a middle radix that does not divide E takes whole rounds
   __host__ __device__ static constexpr int rounds(int p) { return E % R(p) == 0 ? E / R(p) : (N / R(p) + T - 1) / T; }

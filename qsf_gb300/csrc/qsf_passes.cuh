@@ -177,19 +177,20 @@ struct ObsSum {
 };
 
 // Length-gauge factors of half `kind` (0 open, 1 close, 2 close of this sub-step times
-// open of the next): the last axis' table and the factor of the other axes at `row`.
+// open of the next): the last axis' table and the
+// factor of the other axes at `row`.
 template <int N>
-__device__ __forceinline__ int4 lg_row(const GridDev& g, const StepDev& S, int kind, long long row) {
-  const int4* t = S.xdyn + (size_t)kind * g.dim * S.nmax;
+__device__ __forceinline__ int4 lg_row(const GridDev& g, const StepDev& S, long long sub, int kind, long long row) {
+  const int4* t = S.xdyn + ((size_t)(sub - S.ctl[7]) * 3 + kind) * g.dim * S.nmax;
   if (g.dim == 2) return t[(int)row];
   return split_fx(fmul62(tw_join(t[(int)(row / N)]), tw_join(t[S.nmax + (int)(row % N)])));
 }
-__device__ __forceinline__ const int4* lg_col(const GridDev& g, const StepDev& S, int kind) {
-  return S.xdyn + ((size_t)kind * g.dim + g.dim - 1) * S.nmax;
+__device__ __forceinline__ const int4* lg_col(const GridDev& g, const StepDev& S, long long sub, int kind) {
+  return S.xdyn + (((size_t)(sub - S.ctl[7]) * 3 + kind) * g.dim + g.dim - 1) * S.nmax;
 }
-__device__ __forceinline__ int lg_exp(const GridDev& g, const StepDev& S, int kind) {
+__device__ __forceinline__ int lg_exp(const GridDev& g, const StepDev& S, long long sub, int kind) {
   int e = 0;
-  for (int d = 0; d < g.dim; ++d) e += S.texp[(1 + kind) * 3 + d];
+  for (int d = 0; d < g.dim; ++d) e += S.texp[(int)(sub - S.ctl[7]) * kTexp + (1 + kind) * 3 + d];
   return e;
 }
 
@@ -199,7 +200,7 @@ __device__ __forceinline__ int lg_exp(const GridDev& g, const StepDev& S, int ki
 // used)
 template <class G>
 __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S, const longlong2* v, LineCtx<G>& c,
-                                             longlong2* smx, long long row0, long long nrows, int s) {
+                                             longlong2* smx, long long row0, long long nrows, int s, long long sub) {
   constexpr int N = G::N;
   constexpr int gl = G::kSync == 1 ? 1 : G::kSync == 0 ? 32 / G::T : G::L;  // lines of a group
   const int l0 = c.l / gl * gl;
@@ -209,7 +210,7 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
   const int e0 = S.row_ptr[r0], e1 = S.row_ptr[r1];
   if (e0 == e1) return false;
   const bool lg = S.lg != 0;
-  const int sy = s - 2 - S.xs_exp + S.l2m - (lg ? 2 + lg_exp(g, S, 1) : 0);
+  const int sy = s - 2 - S.xs_exp + S.l2m - (lg ? 2 + lg_exp(g, S, sub, 1) : 0);
   constexpr int gt = G::kSync == 1 ? G::T : G::kSync == 0 ? 32 : G::kRowThreads;
   const int ti = G::kSync == 1 ? c.t : G::kSync == 0 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
   if constexpr (G::S == 1) {  // lines of one thread each: an entry is found by its owner
@@ -222,7 +223,7 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
         for (int k = 0; k < G::E; ++k)
           if (k == j) x = v[k];
         x = fmul_tw(fconj(x), S.xs[r * N + j]);
-        if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, 1)[j]), 2), lg_row<N>(g, S, 1, r));
+        if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, sub, 1)[j]), 2), lg_row<N>(g, S, sub, 1, r));
         S.snap[e] = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
       }
     return true;
@@ -237,7 +238,7 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
     const int j = (int)(p % N);
     longlong2 x = fconj(smx[(r - row0) * G::LS + G::pad(j)]);
     x = fmul_tw(x, S.xs[p]);
-    if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, 1)[j]), 2), lg_row<N>(g, S, 1, r));
+    if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, sub, 1)[j]), 2), lg_row<N>(g, S, sub, 1, r));
     S.snap[e] = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
   }
   c.sync();
@@ -253,8 +254,8 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
-  const long long sub = S.ctl[5];
+  const long long sub = S.ctl[6];
+  if (!pass_active(S, sub)) return;
   // the previous sub-step's closing pass produced pass 0, unless it ended with psi_n in
   // memory for E_kin
   if (S.fused && sub > 0 && !ekin_at(S, sub - 1)) return;
@@ -271,25 +272,17 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   // an Inf or NaN component (exponent field all ones) has no fixed-point image: flag
   // the solve (QSF_ENUMERIC) instead of converting garbage
   if (em >= 0x7ff) S.ctl[4] = 1;
-  if (!S.fused && S.normalize && *S.scale != 1.0) {
-    long long F;
-    int k;
-    split_scale(*S.scale, F, k);
-#pragma unroll
-    for (int s = 0; s < G::E; ++s) v[s] = make_longlong2(mulq62(v[s].x, F), mulq62(v[s].y, F));
-    scale -= k;
-  }
   const int4* xs = S.xs + (on ? row * N : 0) + c.t;
 #pragma unroll
   for (int s = 0; s < G::E; ++s) v[s] = fmul_tw(v[s], xs[s * G::T]);
   scale -= 2 + S.xs_exp;
   if (S.lg) {
-    const int4* cf = lg_col(g, S, 0) + c.t;
-    const int4 rf = lg_row<N>(g, S, 0, on ? row : 0);
+    const int4* cf = lg_col(g, S, sub, 0) + c.t;
+    const int4 rf = lg_row<N>(g, S, sub, 0, on ? row : 0);
 #pragma unroll
     for (int s = 0; s < G::E; ++s)
       v[s] = fmul_tw(shl_by(fmul_tw(shl_by(v[s], 2), cf[s * G::T]), 2), rf);
-    scale -= lg_exp(g, S, 0);
+    scale -= lg_exp(g, S, sub, 0);
   }
   line_fft<G>(v, c, g.ax[g.dim - 1].twl[G::ppt >= 16], scale);
   if (!on) return;
@@ -314,12 +307,12 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
+  const long long sub = S.ctl[5];
+  if (!pass_active(S, sub)) return;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ double dred[32 * 2];
   longlong2* smx = reinterpret_cast<longlong2*>(sm);
   LineCtx<G> c(smx, reinterpret_cast<unsigned(*)[32]>(sm + G::buf_bytes(G::kRowThreads)));
-  const long long sub = S.ctl[5];
   const long long row0 = (long long)blockIdx.x * G::L, nrows = g.m / N, row = row0 + c.l;
   const bool on = c.l < G::L && row < nrows;
   const long long base = on ? row * N : 0;
@@ -333,13 +326,16 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     int d[G::E];
 #pragma unroll
     for (int s = 0; s < G::E; ++s) v[s] = on ? psi[s * G::T] : make_longlong2(0, 0);
-    const int gm = S.gmin[in_pass];
+    const int gm = S.gmin[gmin_slot(in_pass, sub)];
     const int* sc = S.sc + (size_t)in_pass * S.scmax + (g.dim == 3 && on ? row / N * N : 0) + c.t;
 #pragma unroll
     for (int s = 0; s < G::E; ++s) d[s] = gm - sc[s * G::T];
     scale = line_align<G>(v, d, gm, c);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) S.ctl[6] = sub + 1;  // the sub-step's last pass
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    S.ctl[6] = sub + 1;  // the sub-step's last pass
+    for (int p = 1; p < 4; ++p) S.gmin[gmin_slot(p, sub + 1)] = 0x7fffffff;
+  }
   const bool last = !S.fused || sub >= S.ctl[1] || sub + 1 >= S.nsteps || ekin_at(S, sub);
   const int4* tw = g.ax[g.dim - 1].twl[G::ppt >= 16];
   const int4* xs = S.xs + base + c.t;
@@ -355,7 +351,7 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     line_fft<G>(v, c, tw, scale, fetch);
     if (h) break;
     scale += line_up<G>(v, c);
-    if (S.row_ptr && row_snapshot<G>(g, S, v, c, smx, row0, nrows, scale) && G::S > 1) {
+    if (S.row_ptr && row_snapshot<G>(g, S, v, c, smx, row0, nrows, scale, sub) && G::S > 1) {
 #pragma unroll
       for (int s = 0; s < G::E; ++s) fetch(s);  // the snapshot took the slots
     }
@@ -380,12 +376,12 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     }
     if (S.lg) {
       const int kind = last ? 1 : 2, pre = last ? 0 : 2;
-      const int4* cf = lg_col(g, S, kind) + c.t;
-      const int4 rf = lg_row<N>(g, S, kind, on ? row : 0);
+      const int4* cf = lg_col(g, S, sub, kind) + c.t;
+      const int4 rf = lg_row<N>(g, S, sub, kind, on ? row : 0);
 #pragma unroll
       for (int s = 0; s < G::E; ++s)
         v[s] = fmul_tw(shl_by(fmul_tw(shl_by(v[s], pre), cf[s * G::T]), 2), rf);
-      scale += pre - 2 - lg_exp(g, S, kind);
+      scale += pre - 2 - lg_exp(g, S, sub, kind);
     }
     if (__builtin_expect(last, 0)) {
       su = scale;  // (in imaginary time the x.E factors are real and count)
@@ -438,7 +434,7 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S) || !ekin_at(S, S.ctl[5])) return;
+  if (!pass_active(S, S.ctl[5]) || !ekin_at(S, S.ctl[5])) return;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ double dred[32];
   LineCtx<G> c(reinterpret_cast<longlong2*>(sm), reinterpret_cast<unsigned(*)[32]>(sm + G::buf_bytes(G::kRowThreads)));
@@ -468,8 +464,9 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
   constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
-  if (!pass_active(S)) return;
-  const long long sub = S.ctl[5];
+  const long long sub = MODE == 3 ? S.ctl[5] : S.ctl[6];
+  if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) S.ctl[5] = sub;  // also when there is nothing left to do
+  if (!pass_active(S, sub)) return;
   if (MODE == 3 && !ekin_at(S, sub)) return;
   extern __shared__ __align__(1024) unsigned char sm[];
   const ColBlock<G> cb(g, ax, sm);
@@ -509,17 +506,22 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
       scale = line_align<G>(v, d, gm, c);
     }
     if constexpr (MODE == 2) {
+      const int at = (int)(sub - S.ctl[7]);
+      if (blockIdx.x == 0 && threadIdx.x == 0) S.gmin[gmin_slot(0, sub + 1)] = 0x7fffffff;
       // per-column factor: product of the P tables of the other axes
-      longlong2 f = tw_join(S.ptab[(size_t)(g.dim - 1) * S.nmax + (g.dim == 3 ? i2 : col)]);
-      if (g.dim == 3) f = fmul62(f, tw_join(S.ptab[S.nmax + col / N]));
+      const int4* tab = S.ptab + (size_t)at * g.dim * S.nmax;
+      longlong2 f = tw_join(tab[(size_t)(g.dim - 1) * S.nmax + (g.dim == 3 ? i2 : col)]);
+      if (g.dim == 3) f = fmul62(f, tw_join(tab[S.nmax + col / N]));
       const int4 pc = split_fx(f);
-      const int4* pt = S.ptab + (size_t)ax * S.nmax + c.t;
+      const int4* pt = tab + c.t;
+      // the exponents of the P phase's two products and tables, and of the pending Normalize factor
+      scale -= 4 + (S.normalize ? (int)S.scale[3] : 0);
+      for (int d = 0; d < g.dim; ++d) scale -= S.texp[at * kTexp + d];
 #pragma unroll 1  // one code body for both transforms
       for (int h = 0;; ++h) {
         line_fft<G>(v, c, a.twl[G::ppt >= 16], scale);
         if (h) break;
-        scale += line_up<G>(v, c) - 4;
-        for (int d = 0; d < g.dim; ++d) scale -= S.texp[d];
+        scale += line_up<G>(v, c);
         // (the table is the same for every line: it stays in L1, where a copy through
         // the exchange slots as in k_row_close came from L2, 315 -> 364 us at 256^3)
 #pragma unroll
@@ -531,7 +533,7 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
     cb.write(v, c);
     if (on && c.t == 0) {
       S.sc[(size_t)out_pass * S.scmax + out_at] = scale;
-      atomicMin(&S.gmin[out_pass], scale);
+      atomicMin(&S.gmin[gmin_slot(out_pass, sub)], scale);
     }
   }
 }

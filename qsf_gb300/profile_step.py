@@ -36,6 +36,7 @@ WORKLOADS = {
     "2d768": (2, 768, 0.3, 77, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
     "2d4096": (2, 4096, 0.3, 410, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
     "3d128": (3, 128, 0.4, 13, 3.0, 1, 1e15, 800.0, 2.0, "ZOA_FLUX_3D", 0),
+    "3d64": (3, 64, 0.4, 6, 3.0, 1, 1e15, 800.0, 2.0, "ZOA_FLUX_3D", 0),
     "1d64": (1, 64, 0.2, 6, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 24),
     "1d128": (1, 128, 0.2, 13, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 48),
     "1d256": (1, 256, 0.2, 26, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 100),
