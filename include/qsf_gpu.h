@@ -131,10 +131,9 @@ typedef struct qsf_grid qsf_grid;
  * to 16384 on a 1D line and 4096 on the axes of a 2D / 3D grid.  The lengths of the
  * built kernel list (2^a, 3*2^a and 5*2^a from 8 to 16384: 33 lengths) take the fused
  * kernels; the others (up to 16384 in 1D, 2048 in 2D / 3D) transform each axis by
- * Bluestein's chirp-z convolution over a built length M >= 2n - 1 (a four-step
- * M1 x M2 transform for 1D lines above 8192 points), and qsf_step runs their steps as
- * the member operations evolve / fourier / average; batches take built lengths only
- * (QSF_EINVAL), the server runs the others beside its batch.  Other lengths:
+ * Bluestein's chirp-z convolution over a built length M >= 2n - 1 in fused kernels of
+ * their own; batches of 2D / 3D grids take built lengths only (QSF_EINVAL), the server
+ * runs the others beside its batch.  Other lengths:
  * QSF_EINVAL. */
 int qsf_grid_create(const qsf_grid_desc* desc, void* stream, qsf_grid** out);
 /* Frees the grid's device state; a member of a batch leaves the batch first. */
@@ -298,8 +297,8 @@ int qsf_batch_result(qsf_batch* b, int64_t slot, double* rows, int64_t* steps_do
  * between rounds of steps (their wavefunctions stay resident on the device for the
  * whole solve), and leave it when their last step is done, returning yields, flux
  * integrals and latencies.  Admissions are prepared while a round runs.  Solves of
- * axis lengths outside the built kernel list run beside the batch, each on its own
- * stream, as graph-replayed member-operation programs.  No counterpart in the
+ * 1D lines and of axis lengths outside the built kernel list run beside the batch, each
+ * on its own stream.  No counterpart in the
  * reference. */
 typedef struct qsf_request {
   qsf_grid_desc grid;

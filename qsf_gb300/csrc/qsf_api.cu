@@ -113,6 +113,9 @@ int init_kernel_table() {
     if ((rc = lim((const void*)k.row_open, k.row_smem)) || (rc = lim((const void*)k.row_close, k.row_smem)) ||
         (rc = lim((const void*)k.row_ekin, k.row_smem)) || (rc = lim((const void*)k.axis_one, k.col_smem)) ||
         (rc = lim((const void*)k.axis_fpi, k.col_smem)) || (rc = lim((const void*)k.axis_ekin, k.col_smem)) ||
+        (rc = lim((const void*)k.conv_open, k.row_smem)) || (rc = lim((const void*)k.conv_close, k.row_smem)) ||
+        (rc = lim((const void*)k.conv_rekin, k.row_smem)) || (rc = lim((const void*)k.conv_one, k.col_smem)) ||
+        (rc = lim((const void*)k.conv_fpi, k.col_smem)) || (rc = lim((const void*)k.conv_aekin, k.col_smem)) ||
         (rc = lim((const void*)k.axis_fft[0], tile)) || (rc = lim((const void*)k.axis_fft[1], tile)) ||
         (rc = lim((const void*)k.row_fft[0], line)) || (rc = lim((const void*)k.row_fft[1], line)))
       return rc;
@@ -151,7 +154,7 @@ EncodeTiledFn encode_tiled() {
 }
 
 // Tensor maps of psi for the strided-axis passes of axes 0 .. dim-2: psi as 64-bit
-// words, dims {2 * stride, n, outer}, box {2 * block columns, tma_box_rows(n), 1}, each
+// words, dims {2 * stride, n, outer}, box {2 * block columns, rows, 1}, each
 // box row swizzled over its own length (column_swz); left null (plain copies) without an
 // encoder.
 int make_tensor_maps(qsf_grid* g) {
@@ -160,29 +163,33 @@ int make_tensor_maps(qsf_grid* g) {
   EncodeTiledFn fn = encode_tiled();
   if (G.dim < 2 || !fn) return QSF_OK;
   if (int rc = dev_alloc(g->tmaps, (size_t)kMaxDim * 128)) return rc;
+  alignas(64) unsigned char maps[kMaxDim * 128] = {};
   for (int ax = 0; ax + 1 < G.dim; ++ax) {
     const AxisDev& a = G.ax[ax];
     const long long inner = a.stride, outer = G.m / ((long long)a.n * inner);
     const cuuint64_t dims[3] = {(cuuint64_t)(2 * inner), (cuuint64_t)a.n, (cuuint64_t)outer};
     const cuuint64_t strides[2] = {(cuuint64_t)(16 * inner), (cuuint64_t)(16 * inner * a.n)};
-    const int C = g->ks->col_lines;
+    const int C = g->pass.col_lines;
+    const int rows = g->ks ? tma_box_rows(a.n) : kConvBoxRows;
+    if (a.n < 64 && !g->ks) continue;
     const CUtensorMapSwizzle swz = C == 8   ? CU_TENSOR_MAP_SWIZZLE_128B
                                    : C == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
                                    : C == 2 ? CU_TENSOR_MAP_SWIZZLE_32B
                                             : CU_TENSOR_MAP_SWIZZLE_NONE;
-    const cuuint32_t box[3] = {(cuuint32_t)(2 * C), (cuuint32_t)tma_box_rows(a.n), 1};
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * C), (cuuint32_t)rows, 1};
     const cuuint32_t elem[3] = {1, 1, 1};
     alignas(64) CUtensorMap map;
     if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, G.psi, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
            swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
         CUDA_SUCCESS)
       continue;  // this axis keeps plain copies
-    // on the grid's stream and waited for: a pageable copy on another stream may still
-    // be in flight when it returns, unordered with the grid's later work
-    QSF_CU(cudaMemcpyAsync(g->tmaps + 128 * ax, &map, sizeof(map), cudaMemcpyHostToDevice, g->stream));
-    QSF_CU(cudaStreamSynchronize(g->stream));
+    std::memcpy(maps + 128 * ax, &map, sizeof(map));
     G.tmap[ax] = g->tmaps + 128 * ax;
   }
+  // on the grid's stream and waited for: a pageable copy on another stream may still be in
+  // flight when it returns, unordered with the grid's later work
+  QSF_CU(cudaMemcpyAsync(g->tmaps, maps, sizeof(maps), cudaMemcpyHostToDevice, g->stream));
+  QSF_CU(cudaStreamSynchronize(g->stream));
   return QSF_OK;
 }
 
@@ -607,7 +614,7 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
 }
 
 int launch_step(qsf_grid* g, const StepDev& S, Prof* P = nullptr, bool with_open = true, FinOverlap* ov = nullptr) {
-  return launch_group(*g->ks, geom_of(g), g->dG, g->dS, 1, (S.obs & QSF_OBS_EKIN) != 0, fin_blocks(g, S.nfterms),
+  return launch_group(g->pass, geom_of(g), g->dG, g->dS, 1, (S.obs & QSF_OBS_EKIN) != 0, fin_blocks(g, S.nfterms),
                       g->stream, P, with_open, ov);
 }
 
@@ -770,6 +777,61 @@ int capture_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec) {
   ce = cudaGraphInstantiate(exec, graph, 0);
   cudaGraphDestroy(graph);
   if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
+  return QSF_OK;
+}
+
+// The next `count` sub-steps of a program of the 2D and 3D passes, queued on the grid's
+// stream (start: its first ones).  One graph holds kTableSteps steps (the kernels read the
+// step index from the device, so every copy is the same), the remainder runs as single
+// steps.  In a fused program only the first step's opening row pass works, so it runs once,
+// before the graphs, which leave it out.  The executable graph stays with the grid and is
+// replayed by later calls of the same launch shape (no capture per call).
+int run_passes(qsf_grid* g, const StepDev& S, int64_t count, bool start) {
+  int rc;
+  if (count < 4) {
+    if (count > 0 && (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)count, g->stream))) return rc;
+    for (int64_t k = 0; k < count; ++k)
+      if ((rc = launch_step(g, S))) return rc;
+    return QSF_OK;
+  }
+  const bool skip_open = S.fused != 0 && !(S.obs & QSF_OBS_EKIN);
+  int64_t first = 0;
+  if (skip_open && start) {
+    if ((rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream)) || (rc = launch_step(g, S))) return rc;
+    first = 1;
+  }
+  const int64_t rest = count - first;
+  const int64_t per = std::min<int64_t>(kTableSteps, rest);
+  cudaGraphExec_t exec = nullptr;
+  FinOverlap ov;
+  const bool overlap = fin_overlap_ok(S);
+  if (overlap && (rc = ensure_fin_stream(g, &ov))) return rc;
+  const int ekin = (S.obs & QSF_OBS_EKIN) ? 1 : 0, nfblk = fin_blocks(g, S.nfterms);
+  for (const qsf_grid::StepGraph& sg : g->step_graphs)
+    if (sg.per == per && sg.skip_open == (int)skip_open && sg.overlap == (int)overlap && sg.ekin == ekin &&
+        sg.nfblk == nfblk)
+      exec = sg.exec;
+  if (!exec) {
+    if ((rc = capture_graph(
+             g->stream,
+             [&]() {
+               if (int r = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)per, g->stream)) return r;
+               for (int64_t k = 0; k < per; ++k)
+                 if (int r = launch_step(g, S, nullptr, !skip_open, overlap ? &ov : nullptr)) return r;
+               if (ov.pending) QSF_CU(cudaStreamWaitEvent(g->stream, ov.done, 0));  // join
+               return QSF_OK;
+             },
+             &exec)))
+      return rc;
+    g->step_graphs.push_back({per, (int)skip_open, (int)overlap, ekin, nfblk, exec});
+  }
+  for (int64_t k = 0; k + per <= rest; k += per) {
+    const cudaError_t ce = cudaGraphLaunch(exec, g->stream);
+    if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
+  }
+  if (rest % per && (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)(rest % per), g->stream))) return rc;
+  for (int64_t k = rest - rest % per; k < rest; ++k)
+    if ((rc = launch_step(g, S, nullptr, !skip_open))) return rc;
   return QSF_OK;
 }
 
@@ -944,8 +1006,8 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
       return fail(QSF_EINVAL, "multi-region grids need a reduced-dimensionality interaction (no partial Coulomb)");
   }
   if (int rc = init_kernel_table()) return rc;
-  // lengths without fused kernels (not in the built list, or with a prime factor above
-  // 5) take Bluestein transforms and the member-operation step
+  // lengths outside the built list (or with a prime factor above 5) run as Bluestein
+  // convolutions
   const KernelSet* ks = kernels_for((int)d->n[0]);
   if (!ks && !(d->dim == 1 ? line_conv_length((int)d->n[0]) : bs_size((int)d->n[0], d->dim)))
     return fail(QSF_EINVAL, "grid size " + std::to_string(d->n[0]) + " has no kernels and no Bluestein length in "
@@ -1020,16 +1082,15 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   cudaMemsetAsync(G.psi, 0, (size_t)G.m * sizeof(double2), g->stream);
   // launch geometry
   const int D = d->dim;
+  if (D > 1) g->pass = ks ? *ks : conv_kernels(*kernels_for(bs_size((int)d->n[0], D)));
   const int nlast = G.ax[D - 1].n;
   const long long nrows = G.m / nlast;
   if (D >= 2) {
-    if (ks) {
-      g->nrowblk = (int)((nrows + ks->row_lines - 1) / ks->row_lines);
-      for (int ax = 0; ax < D - 1; ++ax) {
-        const AxisDev& a = G.ax[ax];
-        const long long inner = a.stride, outer = G.m / ((long long)a.n * inner);
-        g->ax_blocks[ax] = (int)(outer * ((inner + ks->col_lines - 1) / ks->col_lines));
-      }
+    g->nrowblk = (int)((nrows + g->pass.row_lines - 1) / g->pass.row_lines);
+    for (int ax = 0; ax < D - 1; ++ax) {
+      const AxisDev& a = G.ax[ax];
+      const long long inner = a.stride, outer = G.m / ((long long)a.n * inner);
+      g->ax_blocks[ax] = (int)(outer * ((inner + g->pass.col_lines - 1) / g->pass.col_lines));
     }
   } else {
     g->nrowblk = 1;
@@ -1052,18 +1113,17 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   g->scale = g->blk->scale;
   g->dS = &g->blk->S;
   // the fused kernels' exponent slots, per-step tables and device descriptors
-  const bool fused = ks || D == 1;
-  if (fused && ((rc = dev_alloc(g->ibuf, (size_t)kTableSteps * kTexp + 4 * (size_t)g->scmax)) ||
-             (D > 1 && (rc = dev_alloc(g->ptab, (size_t)kTableSteps * D * g->nmax))) || (rc = dev_alloc(g->dG, 1)))) {
+  if ((rc = dev_alloc(g->ibuf, (size_t)kTableSteps * kTexp + 4 * (size_t)g->scmax)) ||
+      (D > 1 && (rc = dev_alloc(g->ptab, (size_t)kTableSteps * D * g->nmax))) || (rc = dev_alloc(g->dG, 1))) {
     qsf_grid_destroy(g);
     return rc;
   }
   g->fpmax = (size_t)kMaxFluxBlocks * kFinCols;
-  if ((rc = D == 1 ? line_setup(g) : ks ? make_tensor_maps(g) : bs_setup(g))) {
+  if ((rc = D == 1 ? line_setup(g) : make_tensor_maps(g)) || (D > 1 && !ks && (rc = bs_setup(g)))) {
     qsf_grid_destroy(g);
     return rc;
   }
-  if (fused) cudaMemcpyAsync(g->dG, &g->G, sizeof(GridDev), cudaMemcpyHostToDevice, g->stream);
+  cudaMemcpyAsync(g->dG, &g->G, sizeof(GridDev), cudaMemcpyHostToDevice, g->stream);
   cudaMemsetAsync(g->partials, 0, sizeof(double) * 5 * g->pmax, g->stream);
   if (cudaStreamSynchronize(g->stream) != cudaSuccess) {
     qsf_grid_destroy(g);
@@ -1104,7 +1164,6 @@ int qsf_grid_destroy(qsf_grid* g) {
   fr(g->vtab);
   fr(g->mtab);
   for (const qsf_grid::StepGraph& sg : g->step_graphs) cudaGraphExecDestroy(sg.exec);
-  if (g->gen_exec) cudaGraphExecDestroy(g->gen_exec);
   fr(g->tmaps);
   bs_release(g);
   line_release(g);
@@ -1236,15 +1295,6 @@ int qsf_region_transfer(qsf_grid* dst, const qsf_grid* src, int axis, int group)
   return QSF_OK;
 }
 
-static int evolve_impl(qsf_grid* g, int mode, int rep, double delta, const double* c3, CoupDev cd);
-
-int qsf_evolve(qsf_grid* g, int mode, int rep, double delta, const double* c3) {
-  if (!g || (mode != 1 && mode != 2) || (rep != 1 && rep != 2)) return fail(QSF_EINVAL, "bad argument");
-  return evolve_impl(g, mode, rep, delta, c3, CoupDev{nullptr, nullptr, 0, 0});
-}
-
-// evolve<mode, rep>(delta) with the coupling values from c3 (host) or, when cd.c is
-// set, from the device rows of a step program
 // the X factor table of evolve<mode, X>(delta) without X-space coupling, per point:
 // evaluated once and reused while (mode, delta) stay the same
 static int ensure_xtab(qsf_grid* g, int mode, double delta) {
@@ -1267,7 +1317,8 @@ static int ensure_vtab(qsf_grid* g) {
   return QSF_OK;
 }
 
-static int evolve_impl(qsf_grid* g, int mode, int rep, double delta, const double* c3, CoupDev cd) {
+int qsf_evolve(qsf_grid* g, int mode, int rep, double delta, const double* c3) {
+  if (!g || (mode != 1 && mode != 2) || (rep != 1 && rep != 2)) return fail(QSF_EINVAL, "bad argument");
   const double c0 = c3 ? c3[0] : 0.0, c1 = c3 ? c3[1] : 0.0, c2 = c3 ? c3[2] : 0.0;
   const GridDev& G = g->G;
   if (rep == QSF_REP_X && !(G.gauge == QSF_GAUGE_LENGTH && G.n_fields)) {
@@ -1277,10 +1328,10 @@ static int evolve_impl(qsf_grid* g, int mode, int rep, double delta, const doubl
     if (!g->eptab)
       if (int rc = dev_alloc(g->eptab, (size_t)3 * g->nmax)) return rc;
     k_evolve_ptab<<<(G.dim * g->nmax + 255) / 256, 256, 0, g->stream>>>(G, mode, delta, c0, c1, c2, g->nmax,
-                                                                        g->eptab, cd);
+                                                                        g->eptab);
     k_apply_ptab<<<grid_blocks(G.m), 256, 0, g->stream>>>(G, g->eptab, g->nmax);
   } else {
-    k_evolve<<<grid_blocks(G.m), 256, 0, g->stream>>>(G, mode, rep, delta, c0, c1, c2, cd);
+    k_evolve<<<grid_blocks(G.m), 256, 0, g->stream>>>(G, mode, rep, delta, c0, c1, c2);
   }
   QSF_CU(cudaGetLastError());
   return QSF_OK;
@@ -1365,8 +1416,7 @@ int qsf_flux(qsf_grid* g, const double* A3, int nb, const int* types, int64_t bo
     k_gather<<<std::max(1, std::min(1024, (g->nsnap + 255) / 256)), 256, 0, g->stream>>>(g->G.psi, g->snap_idx,
                                                                                          g->nsnap, g->snap);
     k_flux<<<g->nfblk, 256, 0, g->stream>>>(g->G, g->fpts, g->fterms, g->nfterms, g->snap, A3 ? A3[0] : 0.0,
-                                            A3 ? A3[1] : 0.0, A3 ? A3[2] : 0.0, A3 ? 1 : 0, nb, g->fpartials,
-                                            CoupDev{nullptr, nullptr, 0, 0});
+                                            A3 ? A3[1] : 0.0, A3 ? A3[2] : 0.0, A3 ? 1 : 0, nb, g->fpartials);
     QSF_CU(cudaGetLastError());
     std::vector<double> part((size_t)g->nfblk * kFinCols);
     QSF_CU(cudaMemcpyAsync(part.data(), g->fpartials, part.size() * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1396,7 +1446,6 @@ int qsf_add_gaussian(qsf_grid* g, double at, double delta) {
   return QSF_OK;
 }
 
-static int generic_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_done);
 
 // `count` sub-steps of a 1D program, a launch pair per run of sub-steps that has tables;
 // with `ms` one sub-step per launch, each timed
@@ -1427,7 +1476,6 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
   if (!g || !d) return fail(QSF_EINVAL, "null argument");
   if (steps_done) *steps_done = 0;
   if (d->nsteps == 0) return QSF_OK;
-  if (!g->ks && g->G.dim > 1) return generic_step(g, d, rows, steps_done);
   StepDev S{};
   int ncol = 0, rc;
   if ((rc = prepare_step(g, d, &S, &ncol, INT64_MAX, true))) return rc;
@@ -1447,102 +1495,10 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
     if (rc == QSF_OK) rc = P.flush();
     P.release();
     if (rc) return rc;
-  } else if (S.nsteps < 4) {
-    if ((rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)S.nsteps, g->stream))) return rc;
-    for (int64_t k = 0; k < S.nsteps; ++k)
-      if ((rc = launch_step(g, S))) return rc;
-  } else {
-    // one graph holds kGraphSteps steps (the kernels read the step index from the
-    // device, so every copy is the same), the remainder runs as single steps.  In a
-    // fused call only the first step's opening row pass works, so it runs once, before
-    // the graphs, which leave it out.  The executable graph stays with the grid and
-    // is replayed by later calls of the same launch shape (no capture per call).
-    const bool skip_open = S.fused != 0 && !(S.obs & QSF_OBS_EKIN);
-    int64_t first = 0;
-    if (skip_open) {
-      if ((rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream)) || (rc = launch_step(g, S))) return rc;
-      first = 1;
-    }
-    const int64_t rest = S.nsteps - first;
-    constexpr int64_t kGraphSteps = kTableSteps;
-    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(kGraphSteps, rest));
-    if (rest > 0) {
-      cudaGraphExec_t exec = nullptr;
-      FinOverlap ov;
-      const bool overlap = fin_overlap_ok(S);
-      if (overlap && (rc = ensure_fin_stream(g, &ov))) return rc;
-      const int ekin = (S.obs & QSF_OBS_EKIN) ? 1 : 0, nfblk = fin_blocks(g, S.nfterms);
-      for (const qsf_grid::StepGraph& sg : g->step_graphs)
-        if (sg.per == per && sg.skip_open == (int)skip_open && sg.overlap == (int)overlap && sg.ekin == ekin &&
-            sg.nfblk == nfblk)
-          exec = sg.exec;
-      if (!exec) {
-        if ((rc = capture_graph(
-                 g->stream,
-                 [&]() {
-                   if (int r = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)per, g->stream)) return r;
-                   for (int64_t k = 0; k < per; ++k)
-                     if (int r = launch_step(g, S, nullptr, !skip_open, overlap ? &ov : nullptr)) return r;
-                   if (ov.pending) QSF_CU(cudaStreamWaitEvent(g->stream, ov.done, 0));  // join
-                   return QSF_OK;
-                 },
-                 &exec)))
-          return rc;
-        g->step_graphs.push_back({per, (int)skip_open, (int)overlap, ekin, nfblk, exec});
-      }
-      for (int64_t k = 0; k + per <= rest; k += per) {
-        const cudaError_t ce = cudaGraphLaunch(exec, g->stream);
-        if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
-      }
-      if (rest % per && (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)(rest % per), g->stream))) return rc;
-      for (int64_t k = rest - rest % per; k < rest; ++k)
-        if ((rc = launch_step(g, S, nullptr, !skip_open))) return rc;
-    }
+  } else if ((rc = run_passes(g, S, S.nsteps, true))) {
+    return rc;
   }
   return finish_step(g, S, d->normalize, d->nsteps, ncol, rows, steps_done);
-}
-
-// End of one member-operation step: the flux partials summed per border in block order
-// (the order qsf_flux sums them in) into row *step, the NaN / non-positive norm flag,
-// the Normalize factor, and the step counter advanced, all on the device so that the
-// steps of a program need no host synchronisation and replay from a graph.
-__global__ void k_generic_row(const double* __restrict__ fpart, int nfblk, int nb, double dV, double dx,
-                              double* __restrict__ rows, long long* __restrict__ step, int ncol,
-                              long long* __restrict__ flag, double* __restrict__ scale, int normalize) {
-  double* row = rows + (*step) * ncol;
-  if ((int)threadIdx.x < nb) {
-    double v = 0.0;
-    for (int k = 0; k < nfblk; ++k) v += fpart[k * kFinCols + threadIdx.x];
-    row[3 + threadIdx.x] = v * dV / dx;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double norm = row[0];
-    if (!(norm > 0.0) || isnan(row[1]) || isnan(row[2])) *flag = 1;
-    *scale = normalize && norm > 0.0 ? sqrt(1.0 / norm) : 1.0;
-    *step += 1;
-  }
-}
-
-// The Strang steps of a grid without fused kernels, through the member operations
-// (the reference's own sequence: evolve<X>(dt/2), fourier<P>, evolve<P>(dt),
-// fourier<X>, evolve<X>(dt/2), propagator.h:311-346), with the same descriptor, rows,
-// Normalize, E_kin interval and convergence rule as the fused path.  Observables
-// reduce into device rows; the host waits once per call (and once per step that runs
-// the imaginary-time convergence test).
-static int generic_check(const qsf_grid* g, const qsf_step_desc* d) {
-  if (d->mode != QSF_MODE_IM && d->mode != QSF_MODE_RE) return fail(QSF_EINVAL, "mode must be IM or RE");
-  if (d->nsteps < 1) return fail(QSF_EINVAL, "nsteps < 1");
-  if (d->nborders < 0 || d->nborders > QSF_MAX_BORDERS) return fail(QSF_EINVAL, "too many borders");
-  if (d->substeps < 0 || d->substeps > 64) return fail(QSF_EINVAL, "substeps must be in [0, 64]");
-  if (d->ekin_interval < 0) return fail(QSF_EINVAL, "ekin_interval must be >= 0");
-  if (g->G.free_mask)
-    return fail(QSF_EINVAL, "a region with free axes keeps them in momentum space: step it with the member operations");
-  return QSF_OK;
-}
-
-static int generic_ncol(const qsf_step_desc* d) {
-  return 3 + ((d->obs & QSF_OBS_FLUX) && d->nborders > 0 ? d->nborders : 0);
 }
 
 }  // extern "C"
@@ -1556,159 +1512,25 @@ int qsf::grid_clear(qsf_grid* g) {
   return QSF_OK;
 }
 
-// the launch-shape key of a step program: what its captured kernels bake in
-static std::vector<long long> generic_key(const qsf_grid* g, const qsf_step_desc* d) {
-  long long dtb;
-  std::memcpy(&dtb, &d->dt, sizeof(dtb));
-  return {d->mode, dtb, std::max(1, d->substeps), (long long)d->obs, generic_ncol(d), d->normalize,
-          d->coupling != nullptr, (long long)(uintptr_t)g->rows_dev, (long long)(uintptr_t)g->coup_dev,
-          (long long)(uintptr_t)g->snap, (long long)(uintptr_t)g->fpts, (long long)(uintptr_t)g->fterms, g->nfterms,
-          g->nsnap, g->nfblk, (long long)(uintptr_t)g->etab, (long long)(uintptr_t)g->eptab,
-          (long long)(uintptr_t)g->vtab};
-}
-
-int qsf::generic_begin(qsf_grid* g, const qsf_step_desc* d) {
-  int rc;
-  if (g->G.dim == 1) {
-    int ncol = 0;
-    if ((rc = prepare_step(g, d, &g->l_S, &ncol))) return rc;
-    QSF_CU(cudaMemsetAsync(g->rows_dev, 0, (size_t)d->nsteps * ncol * sizeof(double), g->stream));
-    // the descriptors come from this frame's memory
-    QSF_CU(cudaStreamSynchronize(g->stream));
-    return QSF_OK;
-  }
-  if ((rc = generic_check(g, d))) return rc;
-  const int ncol = generic_ncol(d);
-  const int K = std::max(1, d->substeps), cs = g->G.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
-  if (ncol > 3 && (rc = ensure_flux(g, d->nborders, d->border_types, d->box_size))) return rc;
-  if ((rc = dev_reserve(g->rows_dev, g->rows_cap, (size_t)d->nsteps * ncol))) return rc;
-  if (d->coupling) {
-    const size_t nc = (size_t)d->nsteps * K * cs;
-    if ((rc = dev_reserve(g->coup_dev, g->coup_cap, nc))) return rc;
-    QSF_CU(cudaMemcpyAsync(g->coup_dev, d->coupling, nc * sizeof(double), cudaMemcpyHostToDevice, g->stream));
-  }
+// A solve that runs on its own stream beside a batch (1D lines, and grids whose lines are
+// convolutions): everything a program needs, staged.
+int qsf::solo_begin(qsf_grid* g, const qsf_step_desc* d) {
+  int ncol = 0, rc;
+  if ((rc = prepare_step(g, d, &g->solo, &ncol))) return rc;
   QSF_CU(cudaMemsetAsync(g->rows_dev, 0, (size_t)d->nsteps * ncol * sizeof(double), g->stream));
-  QSF_CU(cudaMemsetAsync(g->ctl, 0, 8 * sizeof(long long), g->stream));  // [0] step, [4] NaN flag
-  g->gen_primed = false;
+  // the descriptors come from this frame's memory
+  QSF_CU(cudaStreamSynchronize(g->stream));
   return QSF_OK;
 }
 
-// one step of the program d at the device step index ctl[0] (its sub-steps, then the
-// observables row, then ctl[0] + 1), queued on the grid's stream; E_kin when ek.  The
-// launches do not depend on the step index, so a run of them replays from a graph.
-static int generic_one(qsf_grid* g, const qsf_step_desc* d, bool ek) {
-  const GridDev& G = g->G;
-  const bool lg = G.gauge == QSF_GAUGE_LENGTH;
-  const int K = std::max(1, d->substeps), cs = lg ? 6 : 3;
-  const double dts = d->dt / K;
-  const int ncol = generic_ncol(d), nb = ncol - 3;
-  const CoupDev none{nullptr, nullptr, 0, 0};
-  const bool has_c = d->coupling != nullptr;
-  const long long sstride = (long long)K * cs;
-  int rc;
-  for (int k = 0; k < K; ++k) {
-    // sub-step k of the step: E at its opening / closing X half (length gauge), A at
-    // its P sub-step (velocity gauge)
-    const CoupDev c1 = has_c ? CoupDev{g->coup_dev, g->ctl, sstride, k * cs} : none;
-    const CoupDev c2 = has_c && lg ? CoupDev{g->coup_dev, g->ctl, sstride, k * cs + 3} : none;
-    if ((rc = evolve_impl(g, d->mode, QSF_REP_X, 0.5 * dts, nullptr, lg ? c1 : none)) ||
-        (rc = qsf_fourier(g, QSF_REP_P)) || (rc = evolve_impl(g, d->mode, QSF_REP_P, dts, nullptr, lg ? none : c1)) ||
-        (rc = qsf_fourier(g, QSF_REP_X)) || (rc = evolve_impl(g, d->mode, QSF_REP_X, 0.5 * dts, nullptr, c2)))
-      return rc;
-  }
-  int nbk = 0;
-  if ((rc = launch_average(g, QSF_REP_X, QSF_OP_IDENTITY, &nbk))) return rc;
-  k_reduce_row<<<1, 256, 0, g->stream>>>(g->partials, nbk, G.dV, g->rows_dev, g->ctl, ncol, 0);
-  if (d->obs & QSF_OBS_EPOT) {
-    if ((rc = launch_average(g, QSF_REP_X, QSF_OP_POTENTIAL, &nbk))) return rc;
-    k_reduce_row<<<1, 256, 0, g->stream>>>(g->partials, nbk, G.dV, g->rows_dev, g->ctl, ncol, 1);
-  }
-  if (ek) {
-    if ((rc = qsf_fourier(g, QSF_REP_P)) || (rc = launch_average(g, QSF_REP_P, QSF_OP_KINETIC, &nbk))) return rc;
-    k_reduce_row<<<1, 256, 0, g->stream>>>(g->partials, nbk, G.dVm, g->rows_dev, g->ctl, ncol, 2);
-    if ((rc = qsf_fourier(g, QSF_REP_X))) return rc;
-  }
-  if (nb && g->nfterms > 0) {
-    // fluxes of psi_n with the A of the step's last P sub-step (velocity gauge)
-    const bool useA = !lg && has_c && G.n_fields;
-    const CoupDev ca = useA ? CoupDev{g->coup_dev, g->ctl, sstride, (K - 1) * cs} : none;
-    k_gather<<<std::max(1, std::min(1024, (g->nsnap + 255) / 256)), 256, 0, g->stream>>>(G.psi, g->snap_idx,
-                                                                                         g->nsnap, g->snap);
-    k_flux<<<g->nfblk, 256, 0, g->stream>>>(G, g->fpts, g->fterms, g->nfterms, g->snap, 0.0, 0.0, 0.0, useA ? 1 : 0,
-                                            nb, g->fpartials, ca);
-  }
-  k_generic_row<<<1, 32, 0, g->stream>>>(g->fpartials, g->nfterms > 0 ? g->nfblk : 0, nb, G.dV, G.ax[0].dx,
-                                         g->rows_dev, g->ctl, ncol, g->ctl + 4, g->scale + 1, d->normalize);
-  if (d->normalize) k_scale<<<grid_blocks(G.m), 256, 0, g->stream>>>(G.psi, G.m, g->scale + 1);
-  QSF_CU(cudaGetLastError());
-  return QSF_OK;
-}
-
-static bool generic_ekin_at(const qsf_step_desc* d, int64_t s, int64_t stop_after) {
-  const int every = d->ekin_interval > 1 ? d->ekin_interval : 1;
-  return (d->obs & QSF_OBS_EKIN) && ((s + 1) % every == 0 || s + 1 == d->nsteps || s == stop_after);
-}
-
-// steps per captured graph of a member-operation step program
-#ifndef QSF_GEN_GRAPH_STEPS
-#define QSF_GEN_GRAPH_STEPS 16
-#endif
-
-// The member operations' tables a step program uses, made before any capture (a
-// capture may not allocate): the X factor for (mode, dt/2K) where no coupling acts in X,
-// the P factor table, the potential table for E_pot.
-static int generic_prime(qsf_grid* g, const qsf_step_desc* d) {
-  const GridDev& G = g->G;
-  const int K = std::max(1, d->substeps);
-  int rc;
-  if (!(G.gauge == QSF_GAUGE_LENGTH && G.n_fields) && (rc = ensure_xtab(g, d->mode, 0.5 * (d->dt / K)))) return rc;
-  if (!g->eptab && (rc = dev_alloc(g->eptab, (size_t)3 * g->nmax))) return rc;
-  if ((d->obs & QSF_OBS_EPOT) && (rc = ensure_vtab(g))) return rc;
-  g->gen_primed = true;
-  return QSF_OK;
-}
-
-// Steps [first, first + count) of the program (the device step index must be `first`):
-// without E_kin, runs of kGenGraphSteps steps replay one captured graph per grid (its
-// launches bake in the program's shape, so it is recaptured when that changes); the
-// remainder runs as plain launches.
-int qsf::generic_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count) {
-  constexpr int kGenGraphSteps = QSF_GEN_GRAPH_STEPS;
+// Steps [first, first + count) of the program, the ones that come next.
+int qsf::solo_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count) {
   if (first < 0 || count < 0 || first + count > d->nsteps) return fail(QSF_EINVAL, "steps outside the program");
-  if (g->G.dim == 1) return line_run(g, g->l_S, count * std::max(1, d->substeps), nullptr, nullptr);
-  int rc;
-  int64_t s = first;
-  const int64_t end = first + count;
-  const bool graphs = !(d->obs & QSF_OBS_EKIN);
-  if (!g->gen_primed && (rc = generic_prime(g, d))) return rc;
-  if (graphs && end - s >= kGenGraphSteps) {
-    const std::vector<long long> key = generic_key(g, d);
-    if (!g->gen_exec || g->gen_key != key) {
-      if (g->gen_exec) cudaGraphExecDestroy(g->gen_exec);
-      g->gen_exec = nullptr;
-      if ((rc = capture_graph(
-               g->stream,
-               [&]() {
-                 for (int k = 0; k < kGenGraphSteps; ++k)
-                   if (int r = generic_one(g, d, false)) return r;
-                 return QSF_OK;
-               },
-               &g->gen_exec)))
-        return rc;
-      g->gen_key = key;
-      g->gen_steps = kGenGraphSteps;
-    }
-    for (; end - s >= g->gen_steps; s += g->gen_steps) {
-      const cudaError_t ce = cudaGraphLaunch(g->gen_exec, g->stream);
-      if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
-    }
-  }
-  for (; s < end; ++s)
-    if ((rc = generic_one(g, d, generic_ekin_at(d, s, d->nsteps)))) return rc;
-  return QSF_OK;
+  const int64_t subs = count * std::max(1, d->substeps);
+  return g->G.dim == 1 ? line_run(g, g->solo, subs, nullptr, nullptr) : run_passes(g, g->solo, subs, first == 0);
 }
 
-int qsf::generic_wait(qsf_grid* g, bool* bad) {
+int qsf::solo_wait(qsf_grid* g, bool* bad) {
   long long flag = 0;
   QSF_CU(cudaMemcpyAsync(&flag, g->ctl + 4, sizeof(flag), cudaMemcpyDeviceToHost, g->stream));
   QSF_CU(cudaStreamSynchronize(g->stream));
@@ -1716,49 +1538,16 @@ int qsf::generic_wait(qsf_grid* g, bool* bad) {
   return QSF_OK;
 }
 
-int qsf::generic_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps) {
+int qsf::solo_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps) {
   if (nsteps > d->nsteps) return fail(QSF_EINVAL, "more rows than steps");
   if (rows && nsteps > 0)
-    QSF_CU(cudaMemcpyAsync(rows, g->rows_dev, (size_t)nsteps * generic_ncol(d) * sizeof(double),
+    QSF_CU(cudaMemcpyAsync(rows, g->rows_dev, (size_t)nsteps * (3 + g->solo.nborders) * sizeof(double),
                            cudaMemcpyDeviceToHost, g->stream));
   QSF_CU(cudaStreamSynchronize(g->stream));
   return QSF_OK;
 }
 
 extern "C" {
-
-static int generic_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_done) {
-  int rc;
-  if ((rc = qsf::generic_begin(g, d))) return rc;
-  const bool conv = d->mode == QSF_MODE_IM && d->state_accuracy > 0.0;
-  const int ncol = generic_ncol(d);
-  double last_e = d->last_energy;
-  int64_t stop_after = d->nsteps;  // set by the convergence rule
-  int64_t s = 0;
-  if (!conv) {
-    if ((rc = qsf::generic_enqueue(g, d, 0, d->nsteps))) return rc;
-    s = d->nsteps;
-  }
-  for (; conv && s < d->nsteps && s <= stop_after; ++s) {
-    const bool ek = generic_ekin_at(d, s, stop_after);
-    if ((rc = generic_one(g, d, ek))) return rc;
-    if (ek || !(d->obs & QSF_OBS_EKIN)) {
-      double r[3];
-      QSF_CU(cudaMemcpyAsync(r, g->rows_dev + (size_t)s * ncol, sizeof(r), cudaMemcpyDeviceToHost, g->stream));
-      QSF_CU(cudaStreamSynchronize(g->stream));
-      const double se = (d->energy_after_normalize & 1) ? 1.0 / r[0] : 1.0;
-      const double sk = (d->energy_after_normalize & 2) ? 1.0 / r[0] : 1.0;
-      const double e = r[1] * se + r[2] * sk;
-      if (stop_after == d->nsteps && std::fabs(e - last_e) <= d->state_accuracy) stop_after = s + 1;
-      last_e = e;
-    }
-  }
-  bool bad = false;
-  if ((rc = qsf::generic_wait(g, &bad)) || (rc = qsf::generic_rows(g, d, rows, d->nsteps))) return rc;
-  if (steps_done) *steps_done = s;
-  if (bad) return fail(QSF_ENUMERIC, "non-positive norm or NaN in a step's reductions");
-  return QSF_OK;
-}
 
 int qsf_batch_create(void* stream, qsf_batch** out) {
   if (!out) return fail(QSF_EINVAL, "null argument");

@@ -1,5 +1,5 @@
 // qsf_bluestein.cu -- fourier<R>() of 2D and 3D grids whose axis length is outside the
-// built kernel list.
+// built kernel list, and what their step kernels need.
 //
 // The reference's FFTW plans take any n (wf/grid.h:251-274); the fused step kernels of
 // this library are compiled for a list of lengths 2^a, 3*2^a and 5*2^a (8 ... 16384,
@@ -12,10 +12,10 @@
 //     X[k] = c[k] a[k], k < n.
 // The inverse transform is the forward one between two conjugations.  The chirp comes
 // from exact integer angle reduction (j^2 mod 2n) and sincospi on the device; B is
-// transformed once per grid.  Grids of such lengths step through the member operations
-// (qsf_step's step programs, replayed from graphs); batches take built lengths only,
-// the server runs such solves beside its batch.  1D lines of such lengths have step
-// kernels of their own (qsf_line1d.cuh).
+// transformed once per grid.  The steps of such grids are the convolution form of the pass
+// kernels (qsf_passes.cuh), which take the same chirp and B; what is here serves the member
+// operations.  Batches take built lengths only, the server runs such solves beside its
+// batch.  1D lines of such lengths have step kernels of their own (qsf_line1d.cuh).
 #include <algorithm>
 #include <string>
 #include <vector>
@@ -86,6 +86,25 @@ __global__ void k_bs_chirp(double2* __restrict__ chirp, double2* __restrict__ w,
   }
 }
 
+// bhat / M times 2^-e, e such that its largest modulus lies in [1/2, 1), in split form; one
+// block
+__global__ void __launch_bounds__(1024) k_bs_split(const double2* __restrict__ b, int4* __restrict__ out, int* bexp, int M) {
+  __shared__ double red[32];
+  double mx = 0.0;
+  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, hypot(b[j].x, b[j].y));
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = 0.0;
+  for (int w = 0; w < 32; ++w) mx = fmax(mx, red[w]);
+  const double one = 1.0 / (double)M;
+  int e;
+  frexp(mx * one, &e);
+  if (threadIdx.x == 0) *bexp = e;
+  const double sc = ldexp(one, -e);
+  for (int j = threadIdx.x; j < M; j += blockDim.x) out[j] = split62(make_double2(b[j].x * sc, b[j].y * sc));
+}
+
 int blocks_for(long long count) {
   const long long b = (count + 255) / 256;
   return (int)std::min<long long>(std::max<long long>(b, 1), (long long)device_sm_count() * 16);
@@ -121,7 +140,7 @@ int bs_plan(int n) {
 int bs_size(int n, int dim) { return dim == 1 ? line_conv_length(n) : bs_plan(n); }
 
 int bs_setup(qsf_grid* g) {
-  const GridDev& G = g->G;
+  GridDev& G = g->G;
   const int n = G.ax[0].n, M = bs_plan(n);
   if (!M)
     return fail(QSF_EINVAL, "grid size " + std::to_string(n) + " has no kernels and no Bluestein length in this build " +
@@ -147,13 +166,21 @@ int bs_setup(qsf_grid* g) {
   L.ax[0].tw = b.ax.tw;
   L.m = M;
   launch_axis_fft(*b.ks, L, 0, true, 1.0, g->stream);
+  if ((rc = dev_alloc(b.bsplit, (size_t)M + 1))) return rc;
+  int* bexp = reinterpret_cast<int*>(b.bsplit + M);
+  k_bs_split<<<1, 1024, 0, g->stream>>>(b.bhat, b.bsplit, bexp, M);
   QSF_CU(cudaGetLastError());
+  G.chirp = b.chirp;
+  G.bhat = b.bsplit;
+  G.bexp = bexp;
+  for (int k = 0; k < G.dim; ++k)
+    for (int p = 0; p < 2; ++p) G.ax[k].twl[p] = b.ax.twl[p];
   return QSF_OK;
 }
 
 void bs_release(qsf_grid* g) {
   qsf_grid::Bluestein& b = g->bs;
-  for (void* p : {(void*)b.chirp, (void*)b.bhat, (void*)b.scratch})  // the twiddles are shared
+  for (void* p : {(void*)b.chirp, (void*)b.bhat, (void*)b.bsplit, (void*)b.scratch})  // the twiddles are shared
     if (p) cudaFree(p);
   b = qsf_grid::Bluestein();
 }

@@ -82,7 +82,8 @@ struct qsf_grid {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   BorderNodes bn;
-  const KernelSet* ks = nullptr;  // kernels for this grid's line length
+  const KernelSet* ks = nullptr;  // kernels for this grid's line length (nullptr: none are built)
+  qsf::KernelSet pass{};          // 2D and 3D: the kernels of its steps
   GridDev* dG = nullptr;          // device copy of G (step kernels read descriptors from device arrays)
   CallBlock* blk = nullptr;       // device memory of the words below and of short calls' rows
   StepDev* dS = nullptr;          // device copy of the current step descriptor
@@ -159,13 +160,7 @@ struct qsf_grid {
     cudaGraphExec_t exec;
   };
   std::vector<StepGraph> step_graphs;
-  // member-operation step programs (grids without fused kernels): the executable graph
-  // of gen_steps steps, the program it was captured for, and whether the member
-  // operations' tables of the current program are made (before any capture)
-  cudaGraphExec_t gen_exec = nullptr;
-  int gen_steps = 0;
-  std::vector<long long> gen_key;
-  bool gen_primed = false;
+  StepDev solo{};  // the program of a solve that runs beside a batch (solo_begin)
   // TMA tensor maps of psi for the strided-axis passes (GridDev::tmap), 128 bytes each
   unsigned char* tmaps = nullptr;
   // Bluestein transforms of a 2D / 3D grid whose axis length has a prime factor above 5 (no
@@ -178,6 +173,7 @@ struct qsf_grid {
     double2* chirp = nullptr;
     double2* bhat = nullptr;
     double2* scratch = nullptr;
+    int4* bsplit = nullptr;  // bhat as the step kernels read it
     AxisDev ax{};  // twiddles of M (shared)
   } bs;
   // 1D grids (qsf_line1d.cu): the step kernels, their geometry tables, the tables of a run of sub-steps and the current program
@@ -191,7 +187,6 @@ struct qsf_grid {
   int* l_texp = nullptr;
   size_t l_ptab_cap = 0, l_ctab_cap = 0, l_texp_cap = 0;
   int l_steps = 1;  // sub-steps the tables hold
-  StepDev l_S{};
 };
 
 namespace qsf {
@@ -201,16 +196,15 @@ bool fused_length(int n);
 bool grid_batched(const qsf_grid* g);
 // psi = 0 on the grid's stream
 int grid_clear(qsf_grid* g);
-// Steps of a grid that is not batched: member operations of a 2D / 3D grid without fused
-// kernels (qsf_step's path for them), runs of the 1D kernels,
-// in parts for the server: begin checks the program and zeroes its device rows and
+// Steps of a grid that is not batched (2D and 3D lines run as convolutions, 1D lines), in
+// parts for the server: begin checks the program and zeroes its device rows and
 // NaN flag; enqueue queues steps [first, first + count) on the grid's stream without
 // waiting (no convergence test); wait waits for the stream and reads the NaN flag;
 // rows copies the first nsteps rows to the host.
-int generic_begin(qsf_grid* g, const qsf_step_desc* d);
-int generic_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
-int generic_wait(qsf_grid* g, bool* bad);
-int generic_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps);
+int solo_begin(qsf_grid* g, const qsf_step_desc* d);
+int solo_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
+int solo_wait(qsf_grid* g, bool* bad);
+int solo_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps);
 // qsf_batch_add without waiting for the batch's stream, for a grid that no queued work
 // of the batch touches (a solve the server prepares while a round runs); it joins at
 // the next batch_launch
@@ -238,7 +232,7 @@ int line_launch_tables(const LineKernels& L, const GridDev* dG, const StepDev* d
 int line_launch_steps(const LineKernels& L, bool bs, const GridDev* dG, const StepDev* dS, int count, int steps,
                       cudaStream_t st);
 int line_fourier(qsf_grid* g, const GridDev& G, bool fwd, double sc);
-// Bluestein plan of a grid without fused kernels (qsf_bluestein.cu)
+// Bluestein plan of a grid whose length has no kernels (qsf_bluestein.cu)
 int bs_setup(qsf_grid* g);
 void bs_release(qsf_grid* g);
 // one axis of fourier<R>() by Bluestein's chirp-z convolution, in place on the array

@@ -70,6 +70,11 @@ struct GridDev {
   // {2 * stride_d, n_d, outer}, box {2 * tile columns, tma_box_rows(n_d), 1}, swizzled
   // over the row of a box; null when the driver offers no encoder (plain copies then)
   const void* tmap[kMaxDim];
+  // lines run as convolutions (qsf_bluestein.cu): exp(-i pi j^2 / n), and the transformed
+  // kernel over the plan's M points divided by M, times 2^-bexp[0]
+  const double2* chirp;
+  const int4* bhat;
+  const int* bexp;
 };
 
 // flux evaluation point: slots into the snapshot of psi_n
@@ -84,23 +89,6 @@ struct FluxTerm {
   int border;
   double w[kMaxDim];
 };
-
-// Where a member-operation kernel finds its coupling values when they live on the
-// device (a step program replayed from a graph): the row at c + (*step) * stride + off
-// for the current step index *step; c == nullptr: the kernel's by-value arguments.
-struct CoupDev {
-  const double* c;
-  const long long* step;
-  long long stride;
-  int off;
-};
-__device__ __forceinline__ void coup_load(const CoupDev& cd, double* cv) {
-  if (!cd.c) return;
-  const double* p = cd.c + (*cd.step) * cd.stride + cd.off;
-  cv[0] = p[0];
-  cv[1] = p[1];
-  cv[2] = p[2];
-}
 
 struct LineDev {
   int n1, n2, ctas, nth, epp;  // factors (n2 == 0: one line), CTAs, worker threads per CTA, points per thread
@@ -376,6 +364,9 @@ __host__ __device__ constexpr int tma_box_rows(int n) {
   while (n % b) --b;
   return b;
 }
+// rows of a box when a line of n >= 64 points runs on a tile of M >= 2n - 1 rows: rounded up
+// to whole boxes the n rows still fit into the tile
+constexpr int kConvBoxRows = 64;
 // Passes that leave the wavefunction in fixed point inside a step; each line of a pass
 // records its exponent in sc[pass] and the pass minimum in gmin[pass]: 0 last-axis rows
 // (open), 1 axis-1 lines forward (3D), 2 axis-0 lines, 3 axis-1 lines inverse (3D).  The
@@ -598,10 +589,9 @@ __global__ void __launch_bounds__(256) k_tables(const GridDev* __restrict__ Gs, 
 // gauge), dotted with the normalised border vector.  out[b] written by thread b.
 __global__ void __launch_bounds__(256) k_flux(GridDev g, const FluxPoint* fpts, const FluxTerm* fterms, int nfterms,
                                               const double2* snap, double A0, double A1, double A2, int useA, int nb,
-                                              double* out_partials, CoupDev cd) {
+                                              double* out_partials) {
   __shared__ double red[32 * kMaxFluxBorders];
   double Av[3] = {A0, A1, A2};
-  coup_load(cd, Av);
   const int chunk = (nfterms + gridDim.x - 1) / gridDim.x;
   const int t0 = blockIdx.x * chunk, t1 = min(nfterms, t0 + chunk);
   flux_block(g, fpts, fterms, t0, t1, snap, useA ? Av : nullptr, nb, red, out_partials + blockIdx.x * kFinCols);
@@ -749,9 +739,8 @@ __global__ void k_evolve_xtab(GridDev g, int mode, double delta, double2* __rest
 // per-axis factors of evolve<M, P>(delta): expOp(delta (k^2 / 2 + A_d k)) for axis d
 // (the P Hamiltonian is a sum over axes, so its exponential is their product)
 __global__ void k_evolve_ptab(GridDev g, int mode, double delta, double c0, double c1, double c2, int nmax,
-                              double2* __restrict__ tab, CoupDev cd) {
+                              double2* __restrict__ tab) {
   double cv[3] = {c0, c1, c2};
-  coup_load(cd, cv);
   if (g.p_swap && g.dim >= 2) {
     const double t = cv[0];
     cv[0] = cv[1];
@@ -788,9 +777,8 @@ __global__ void k_apply_ptab(GridDev g, const double2* __restrict__ tab, int nma
   }
 }
 
-__global__ void k_evolve(GridDev g, int mode, int rep, double delta, double c0, double c1, double c2, CoupDev cd) {
+__global__ void k_evolve(GridDev g, int mode, int rep, double delta, double c0, double c1, double c2) {
   double cv[3] = {c0, c1, c2};
-  coup_load(cd, cv);
   if (rep == 2 && g.p_swap && g.dim >= 2) {
     const double t = cv[0];
     cv[0] = cv[1];
@@ -890,16 +878,6 @@ __global__ void k_reduce_partials(const double* part, int n, double scale, doubl
   for (int i = threadIdx.x; i < n; i += blockDim.x) acc += part[i];
   block_sum<1>(&acc, red);
   if (threadIdx.x == 0) *out = acc * scale;
-}
-
-// the same into column col of row *step of rows (ncol columns): a step program's row
-__global__ void k_reduce_row(const double* part, int n, double scale, double* rows, const long long* step, int ncol,
-                             int col) {
-  __shared__ double red[32];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += part[i];
-  block_sum<1>(&acc, red);
-  if (threadIdx.x == 0) rows[(*step) * ncol + col] = acc * scale;
 }
 
 // gather psi at the snapshot indices (granular flux)
@@ -1027,6 +1005,13 @@ struct KernelSet {
   void (*axis_one)(const GridDev*, const StepDev*, int, int);  // one transform: forward or inverse (last argument)
   void (*axis_fpi)(const GridDev*, const StepDev*, int, int);
   void (*axis_ekin)(const GridDev*, const StepDev*, int, int);
+  // the same six for shorter lines as convolutions over the n points
+  void (*conv_open)(const GridDev*, const StepDev*);
+  void (*conv_close)(const GridDev*, const StepDev*);
+  void (*conv_rekin)(const GridDev*, const StepDev*);
+  void (*conv_one)(const GridDev*, const StepDev*, int, int);
+  void (*conv_fpi)(const GridDev*, const StepDev*, int, int);
+  void (*conv_aekin)(const GridDev*, const StepDev*, int, int);
   // plain transforms, [0] inverse, [1] forward: lines (axis: ax, columns) of a block, scale on the way out
   void (*row_fft[2])(GridDev, int, double);
   void (*axis_fft[2])(GridDev, int, int, double);
@@ -1034,6 +1019,18 @@ struct KernelSet {
   int row_lines, row_threads, row_smem;  // last-axis passes: lines, threads, dynamic shared memory of a block
   int col_lines, col_threads, col_smem;  // strided-axis passes: columns, threads, dynamic shared memory
 };
+
+// the passes of grids whose lines are convolutions over k.n points
+inline KernelSet conv_kernels(const KernelSet& k) {
+  KernelSet c = k;
+  c.row_open = k.conv_open;
+  c.row_close = k.conv_close;
+  c.row_ekin = k.conv_rekin;
+  c.axis_one = k.conv_one;
+  c.axis_fpi = k.conv_fpi;
+  c.axis_ekin = k.conv_aekin;
+  return c;
+}
 
 // kernel table of the supported sizes (qsf_sizes_*.cu); nullptr when n is not built
 const KernelSet* kernels_for(int n);
@@ -1063,6 +1060,12 @@ KernelSet make_kernel_set() {
       k.axis_one = k_axis<0, A>;
       k.axis_fpi = k_axis<2, A>;
       k.axis_ekin = k_axis<3, A>;
+      k.conv_open = k_row_open<G, true>;
+      k.conv_close = k_row_close<G, true>;
+      k.conv_rekin = k_row_ekin<G, true>;
+      k.conv_one = k_axis<0, A, true>;
+      k.conv_fpi = k_axis<2, A, true>;
+      k.conv_aekin = k_axis<3, A, true>;
       k.axis_fft[0] = k_axis_fft<N, false>;
       k.axis_fft[1] = k_axis_fft<N, true>;
       k.axis_threads = plain_threads(N);

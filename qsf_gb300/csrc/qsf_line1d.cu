@@ -109,13 +109,13 @@ __global__ void k_line_chirp(int4* __restrict__ chirp, double2* __restrict__ w, 
     w[j] = v;
   }
 }
-// transformed kernel / M, scaled by 2^-e so that its largest component lies in [1/2, 1),
+// transformed kernel / M, scaled by 2^-e so that its largest modulus lies in [1/2, 1),
 // as [k1][k2]; one block
 __global__ void __launch_bounds__(1024) k_line_bhat(const double2* __restrict__ b, int4* __restrict__ out, int* bexp, int M,
                                                     int n1, int n2) {
   __shared__ double red[32];
   double mx = 0.0;
-  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, fmax(fabs(b[j].x), fabs(b[j].y)));
+  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, hypot(b[j].x, b[j].y));
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();

@@ -32,10 +32,16 @@ __device__ __forceinline__ void tma_store3(const void* tmap, int x, int y, int z
                : "memory");
 }
 
+// Points of a line of axis d: the plan's, or in a convolution plan (BS) the axis' own.
+template <class G, bool BS>
+__device__ __forceinline__ int line_len(const AxisDev& a) {
+  return BS ? a.n : G::N;
+}
+
 // Geometry of a strided-axis block and its shared memory.
-template <class G>
+template <class G, bool BS>
 struct ColBlock {
-  static constexpr int N = G::N;
+  const int N;  // rows of the tile that psi has
   longlong2* tile;
   unsigned long long* bar;
   const void* tmap;
@@ -43,7 +49,7 @@ struct ColBlock {
   long long inner, o, c0, obase;
   int Ch;
   bool boxes;
-  __device__ __forceinline__ ColBlock(const GridDev& g, int ax, unsigned char* sm) {
+  __device__ __forceinline__ ColBlock(const GridDev& g, int ax, unsigned char* sm) : N(line_len<G, BS>(g.ax[ax])) {
     tile = reinterpret_cast<longlong2*>(sm);
     bar = reinterpret_cast<unsigned long long*>(sm + (G::kColBytes + 127) / 128 * 128 + 256);
     psi = reinterpret_cast<longlong2*>(g.psi);
@@ -63,8 +69,9 @@ struct ColBlock {
       if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        mbar_expect_tx(bar, (unsigned)(N * G::C * 16));
-        constexpr int br = tma_box_rows(N);
+        // (a convolution plan's last box ends beyond psi: its rows there arrive as zeros)
+        constexpr int br = BS ? kConvBoxRows : tma_box_rows(G::N);
+        mbar_expect_tx(bar, (unsigned)((N + br - 1) / br * br * G::C * 16));
         for (int r0 = 0; r0 < N; r0 += br) tma_load3(tile + (size_t)r0 * G::C, tmap, (int)(2 * c0), r0, (int)o, bar);
       }
     } else {
@@ -90,7 +97,7 @@ struct ColBlock {
     for (int s = 0; s < G::E; ++s) {
       const int i = c.t + s * G::T;
       const int sw = column_swz<G::C>(G::T % 8 == 0 ? c.t : i);
-      v[s] = tile[i * G::C + (l ^ sw)];
+      v[s] = !BS || i < N ? tile[i * G::C + (l ^ sw)] : make_longlong2(0, 0);
     }
     __syncthreads();  // the tile becomes the lines' exchange buffer
   }
@@ -109,7 +116,7 @@ struct ColBlock {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
       if (threadIdx.x == 0) {
-        constexpr int br = tma_box_rows(N);
+        constexpr int br = BS ? kConvBoxRows : tma_box_rows(G::N);
         for (int r0 = 0; r0 < N; r0 += br) tma_store3(tmap, (int)(2 * c0), r0, (int)o, tile + (size_t)r0 * G::C);
         asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group 0;" ::: "memory");
       }
@@ -177,10 +184,9 @@ struct ObsSum {
 };
 
 // Length-gauge factors of half `kind` (0 open, 1 close, 2 close of this sub-step times
-// open of the next): the last axis' table and the
-// factor of the other axes at `row`.
-template <int N>
-__device__ __forceinline__ int4 lg_row(const GridDev& g, const StepDev& S, long long sub, int kind, long long row) {
+// open of the next): the last axis' table and the factor of the other axes at `row` of
+// lines of N points.
+__device__ __forceinline__ int4 lg_row(const GridDev& g, const StepDev& S, long long sub, int kind, long long row, int N) {
   const int4* t = S.xdyn + ((size_t)(sub - S.ctl[7]) * 3 + kind) * g.dim * S.nmax;
   if (g.dim == 2) return t[(int)row];
   return split_fx(fmul62(tw_join(t[(int)(row / N)]), tw_join(t[S.nmax + (int)(row % N)])));
@@ -194,14 +200,62 @@ __device__ __forceinline__ int lg_exp(const GridDev& g, const StepDev& S, long l
   return e;
 }
 
+// ------------------------------------------------------------ convolution plans
+// Lines of n points without a plan of their own (BS below) run Bluestein's convolution on
+// a plan of M >= 2n - 1 points (qsf_bluestein.cu).  With c[j] = exp(-i pi j^2 / n), B the
+// transform of the wrapped conj(c) over M, and
+//     D(w) = FFT_M(conj(FFT_M(w) B)),
+// a transform is X = c conj(D(c x)) and an inverse one x = conj(c) D(c conj(X)) / n, and
+// D(a w) = conj(a) D(w) for a factor a constant along the line.  So every pass is a
+// conjugation of what it loads and a D, with zeros beyond n: the chirps of the transforms
+// cancel against those of the inverses at the P phase, and what is left is the factor
+// C = prod_d c[j_d] of psi, which the opening half puts on (conv_row, g.chirp), which the
+// middle of a run (X half . X half) carries along, and which the last step's psi and the
+// flux snapshot lose again.  Bound by integer issue as the plain plans are, with four
+// M-point transforms in place of two n-point ones per pass.  1000^2 points: 262 us a step,
+// 780 through the member operations (pre, transform, product, transform and post kernels
+// per axis, in doubles).
+
+// C without the last axis' part
+__device__ __forceinline__ double2 conv_row(const GridDev& g, long long row) {
+  if (g.dim == 2) return g.chirp[row];
+  const int n = g.ax[2].n;
+  return cmul(g.chirp[row / n], g.chirp[row % n]);
+}
+// psi (double, in v) times `c`
+__device__ __forceinline__ longlong2 conv_chirp(longlong2 v, double2 c) {
+  const double2 z = cmul(make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y)), c);
+  return make_longlong2(__double_as_longlong(z.x), __double_as_longlong(z.y));
+}
+// the line's transform, or D of it.  taken: see line_fft, of the last transform
+template <class G, bool BS, class F = NoHook>
+__device__ __forceinline__ void line_pass(longlong2* v, LineCtx<G>& c, const GridDev& g, const int4* tw, int& scale,
+                                          const F& taken = F()) {
+  if constexpr (!BS) {
+    line_fft<G>(v, c, tw, scale, taken);
+  } else {
+#pragma unroll 1
+    for (int q = 0;; ++q) {
+      line_fft<G>(v, c, tw, scale, [&](int s) {
+        if (q) taken(s);
+      });
+      if (q) break;
+      scale += line_up<G, 59>(v, c) - 2 - __ldg(g.bexp);
+      const int4* b = g.bhat + c.t;
+#pragma unroll
+      for (int s = 0; s < G::E; ++s) v[s] = fconj(fmul_tw(v[s], __ldg(b + s * G::T)));
+    }
+  }
+}
+
 // the flux snapshot of psi_n for the rows of this thread's group: v holds the conjugated
 // points of exponent s before the closing half; the group's lines pass through the
 // exchange buffer because an entry's point lies in any of its threads (true when it was
 // used)
-template <class G>
+template <class G, bool BS>
 __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S, const longlong2* v, LineCtx<G>& c,
                                              longlong2* smx, long long row0, long long nrows, int s, long long sub) {
-  constexpr int N = G::N;
+  const int N = line_len<G, BS>(g.ax[g.dim - 1]);
   constexpr int gl = G::kSync == 1 ? 1 : G::kSync == 0 ? 32 / G::T : G::L;  // lines of a group
   const int l0 = c.l / gl * gl;
   const long long r0 = row0 + l0;
@@ -222,9 +276,10 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
 #pragma unroll
         for (int k = 0; k < G::E; ++k)
           if (k == j) x = v[k];
-        x = fmul_tw(fconj(x), S.xs[r * N + j]);
-        if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, sub, 1)[j]), 2), lg_row<N>(g, S, sub, 1, r));
-        S.snap[e] = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
+        x = fmul_tw(BS ? x : fconj(x), S.xs[r * N + j]);
+        if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, sub, 1)[j]), 2), lg_row(g, S, sub, 1, r, N));
+        const double2 z = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
+        S.snap[e] = BS ? cmulc(z, cmul(conv_row(g, r), g.chirp[j])) : z;
       }
     return true;
   }
@@ -236,10 +291,11 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
   for (int e = e0 + ti; e < e1; e += gt) {
     const long long p = S.snap_idx[e], r = p / N;
     const int j = (int)(p % N);
-    longlong2 x = fconj(smx[(r - row0) * G::LS + G::pad(j)]);
-    x = fmul_tw(x, S.xs[p]);
-    if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, sub, 1)[j]), 2), lg_row<N>(g, S, sub, 1, r));
-    S.snap[e] = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
+    longlong2 x = smx[(r - row0) * G::LS + G::pad(j)];
+    x = fmul_tw(BS ? x : fconj(x), S.xs[p]);
+    if (lg) x = fmul_tw(shl_by(fmul_tw(x, lg_col(g, S, sub, 1)[j]), 2), lg_row(g, S, sub, 1, r, N));
+    const double2 z = make_double2(fx2d(x.x, sy), fx2d(x.y, sy));
+    S.snap[e] = BS ? cmulc(z, cmul(conv_row(g, r), g.chirp[j])) : z;
   }
   c.sync();
   return true;
@@ -248,12 +304,12 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
 // ------------------------------------------------------------ row passes
 // Open: psi (double) . [Normalize] . X half . forward transform of the last axis ->
 // fixed point (pass 0).
-template <class G>
+template <class G, bool BS = false>
 __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     k_row_open(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss) {
-  constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
+  const int N = line_len<G, BS>(g.ax[g.dim - 1]);
   const long long sub = S.ctl[6];
   if (!pass_active(S, sub)) return;
   // the previous sub-step's closing pass produced pass 0, unless it ended with psi_n in
@@ -264,9 +320,16 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   const long long nrows = g.m / N, row = (long long)blockIdx.x * G::L + c.l;
   const bool on = c.l < G::L && row < nrows;
   longlong2* psi = reinterpret_cast<longlong2*>(g.psi) + (on ? row * N : 0) + c.t;
+  auto has = [&](int s) { return !BS || c.t + s * G::T < N; };  // points beyond a convolution's line are zero
   longlong2 v[G::K];
 #pragma unroll
-  for (int s = 0; s < G::E; ++s) v[s] = on ? psi[s * G::T] : make_longlong2(0, 0);
+  for (int s = 0; s < G::E; ++s) v[s] = on && has(s) ? psi[s * G::T] : make_longlong2(0, 0);
+  if constexpr (BS) {
+    const double2 cr = conv_row(g, on ? row : 0);
+#pragma unroll
+    for (int s = 0; s < G::E; ++s)
+      if (has(s)) v[s] = conv_chirp(v[s], cmul(cr, g.chirp[c.t + s * G::T]));
+  }
   unsigned em;
   int scale = line_from_double<G>(v, c, em, kLineIn + 2);
   // an Inf or NaN component (exponent field all ones) has no fixed-point image: flag
@@ -274,20 +337,22 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   if (em >= 0x7ff) S.ctl[4] = 1;
   const int4* xs = S.xs + (on ? row * N : 0) + c.t;
 #pragma unroll
-  for (int s = 0; s < G::E; ++s) v[s] = fmul_tw(v[s], xs[s * G::T]);
+  for (int s = 0; s < G::E; ++s)
+    if (has(s)) v[s] = fmul_tw(v[s], xs[s * G::T]);
   scale -= 2 + S.xs_exp;
   if (S.lg) {
     const int4* cf = lg_col(g, S, sub, 0) + c.t;
-    const int4 rf = lg_row<N>(g, S, sub, 0, on ? row : 0);
+    const int4 rf = lg_row(g, S, sub, 0, on ? row : 0, N);
 #pragma unroll
     for (int s = 0; s < G::E; ++s)
-      v[s] = fmul_tw(shl_by(fmul_tw(shl_by(v[s], 2), cf[s * G::T]), 2), rf);
+      if (has(s)) v[s] = fmul_tw(shl_by(fmul_tw(shl_by(v[s], 2), cf[s * G::T]), 2), rf);
     scale -= lg_exp(g, S, sub, 0);
   }
-  line_fft<G>(v, c, g.ax[g.dim - 1].twl[G::ppt >= 16], scale);
+  line_pass<G, BS>(v, c, g, g.ax[g.dim - 1].twl[G::ppt >= 16], scale);
   if (!on) return;
 #pragma unroll
-  for (int s = 0; s < G::E; ++s) psi[s * G::T] = v[s];
+  for (int s = 0; s < G::E; ++s)
+    if (has(s)) psi[s * G::T] = v[s];
   if (c.t == 0) {
     S.sc[row] = scale;
     atomicMin(&S.gmin[gmin_slot(0, sub)], scale);
@@ -301,12 +366,12 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
 // opening X half and forward transform, leaving pass 0 of that sub-step.  In the length
 // gauge the closing half's x.E phases do not change |psi_n|, so going on they merge with
 // the next opening half's into one factor per axis (kind 2).
-template <class G>
+template <class G, bool BS = false>
 __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     k_row_close(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss) {
-  constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
+  const int N = line_len<G, BS>(g.ax[g.dim - 1]);
   const long long sub = S.ctl[5];
   if (!pass_active(S, sub)) return;
   extern __shared__ __align__(1024) unsigned char sm[];
@@ -320,17 +385,22 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   const int in_pass = g.dim == 3 ? 3 : 2;
   // the potential is read in the middle of the pass: start moving it into L2 now
   for (int i = c.t * 16; i < N; i += G::T * 16) prefetch_l2(S.Vx + base + i);
+  auto has = [&](int s) { return !BS || c.t + s * G::T < N; };  // points beyond a convolution's line are zero
   longlong2 v[G::K];
   int scale;
   {
     int d[G::E];
 #pragma unroll
-    for (int s = 0; s < G::E; ++s) v[s] = on ? psi[s * G::T] : make_longlong2(0, 0);
+    for (int s = 0; s < G::E; ++s) v[s] = on && has(s) ? psi[s * G::T] : make_longlong2(0, 0);
     const int gm = S.gmin[gmin_slot(in_pass, sub)];
     const int* sc = S.sc + (size_t)in_pass * S.scmax + (g.dim == 3 && on ? row / N * N : 0) + c.t;
 #pragma unroll
-    for (int s = 0; s < G::E; ++s) d[s] = gm - sc[s * G::T];
+    for (int s = 0; s < G::E; ++s) d[s] = has(s) ? gm - sc[s * G::T] : 0;
     scale = line_align<G>(v, d, gm, c);
+    if constexpr (BS) {
+#pragma unroll
+      for (int s = 0; s < G::E; ++s) v[s] = fconj(v[s]);
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     S.ctl[6] = sub + 1;  // the sub-step's last pass
@@ -344,14 +414,14 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   // the last pass of the inverse transform works on what it read from them
   int h = 0;
   auto fetch = [&](int s) {
-    if (h == 0) own_copy(c.own(s), xs + s * G::T);
+    if (h == 0 && has(s)) own_copy(c.own(s), xs + s * G::T);
   };
 #pragma unroll 1  // one code body for both transforms
   for (;; ++h) {
-    line_fft<G>(v, c, tw, scale, fetch);
+    line_pass<G, BS>(v, c, g, tw, scale, fetch);
     if (h) break;
     scale += line_up<G>(v, c);
-    if (S.row_ptr && row_snapshot<G>(g, S, v, c, smx, row0, nrows, scale, sub) && G::S > 1) {
+    if (S.row_ptr && row_snapshot<G, BS>(g, S, v, c, smx, row0, nrows, scale, sub) && G::S > 1) {
 #pragma unroll
       for (int s = 0; s < G::E; ++s) fetch(s);  // the snapshot took the slots
     }
@@ -362,31 +432,37 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     if (__builtin_expect(!last, 1)) {
 #pragma unroll
       for (int s = 0; s < G::E; ++s) {
+        if (!has(s)) {
+          v[s] = make_longlong2(0, 0);
+          continue;
+        }
         int4 f;
         if constexpr (G::S > 1) f = *reinterpret_cast<const int4*>(c.own(s));
         else f = xs[s * G::T];
-        const longlong2 u = fmul_tw(fconj(v[s]), f);
+        const longlong2 u = fmul_tw(BS ? v[s] : fconj(v[s]), f);
         ob.add(u, __ldg(Vx + s * G::T));
         v[s] = fmul_tw(u, f);
       }
       scale -= 2 + S.xs_exp;
     } else {
 #pragma unroll
-      for (int s = 0; s < G::E; ++s) v[s] = fmul_tw(fconj(v[s]), xs[s * G::T]);
+      for (int s = 0; s < G::E; ++s)
+        v[s] = has(s) ? fmul_tw(BS ? v[s] : fconj(v[s]), xs[s * G::T]) : make_longlong2(0, 0);
     }
     if (S.lg) {
       const int kind = last ? 1 : 2, pre = last ? 0 : 2;
       const int4* cf = lg_col(g, S, sub, kind) + c.t;
-      const int4 rf = lg_row<N>(g, S, sub, kind, on ? row : 0);
+      const int4 rf = lg_row(g, S, sub, kind, on ? row : 0, N);
 #pragma unroll
       for (int s = 0; s < G::E; ++s)
-        v[s] = fmul_tw(shl_by(fmul_tw(shl_by(v[s], pre), cf[s * G::T]), 2), rf);
+        if (has(s)) v[s] = fmul_tw(shl_by(fmul_tw(shl_by(v[s], pre), cf[s * G::T]), 2), rf);
       scale += pre - 2 - lg_exp(g, S, sub, kind);
     }
     if (__builtin_expect(last, 0)) {
       su = scale;  // (in imaginary time the x.E factors are real and count)
 #pragma unroll
-      for (int s = 0; s < G::E; ++s) ob.add(v[s], Vx[s * G::T]);
+      for (int s = 0; s < G::E; ++s)
+        if (has(s)) ob.add(v[s], Vx[s * G::T]);
     }
     double acc[2] = {ob.norm(su), S.obs & 2u ? ob.epot(su, S.vshift) : 0.0};
     block_sum<2>(acc, dred);
@@ -396,9 +472,12 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     }
     if (__builtin_expect(last, 0)) {
       if (on) {
+        const double2 cr = BS ? conv_row(g, row) : make_double2(1.0, 0.0);
 #pragma unroll
         for (int s = 0; s < G::E; ++s) {
-          const double2 z = make_double2(fx2d(v[s].x, scale), fx2d(v[s].y, scale));
+          if (!has(s)) continue;
+          double2 z = make_double2(fx2d(v[s].x, scale), fx2d(v[s].y, scale));
+          if constexpr (BS) z = cmulc(z, cmul(cr, g.chirp[c.t + s * G::T]));
           psi[s * G::T] = make_longlong2(__double_as_longlong(z.x), __double_as_longlong(z.y));
         }
       }
@@ -407,7 +486,8 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   }
   if (!on) return;
 #pragma unroll
-  for (int s = 0; s < G::E; ++s) psi[s * G::T] = v[s];
+  for (int s = 0; s < G::E; ++s)
+    if (has(s)) psi[s * G::T] = v[s];
   if (c.t == 0) {
     S.sc[row] = scale;
     atomicMin(&S.gmin[gmin_slot(0, sub + 1)], scale);
@@ -415,11 +495,12 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
 }
 
 // sum k^2 |X|^2 over this thread's points of a transformed line
-template <class G>
+template <class G, bool BS>
 __device__ __forceinline__ double line_ekin(const AxisDev& a, const longlong2* v, int t, int scale) {
   double ek = 0.0;
 #pragma unroll
   for (int s = 0; s < G::E; ++s) {
+    if (BS && t + s * G::T >= a.n) continue;
     const double k = kpos(a, t + s * G::T);
     const double xr = fx2d(v[s].x, scale), xi = fx2d(v[s].y, scale);
     ek = fma(k * k, fma(xr, xr, xi * xi), ek);
@@ -428,12 +509,12 @@ __device__ __forceinline__ double line_ekin(const AxisDev& a, const longlong2* v
 }
 
 // E_kin part of the last axis: forward transform of psi_n (double, left as it is)
-template <class G>
+template <class G, bool BS = false>
 __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     k_row_ekin(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss) {
-  constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
+  const int N = line_len<G, BS>(g.ax[g.dim - 1]);
   if (!pass_active(S, S.ctl[5]) || !ekin_at(S, S.ctl[5])) return;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ double dred[32];
@@ -442,13 +523,19 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
   const bool on = c.l < G::L && row < g.m / N;
   const AxisDev& a = g.ax[g.dim - 1];
   const longlong2* psi = reinterpret_cast<const longlong2*>(g.psi) + (on ? row * N : 0) + c.t;
+  auto has = [&](int s) { return !BS || c.t + s * G::T < N; };  // points beyond a convolution's line are zero
   longlong2 v[G::K];
 #pragma unroll
-  for (int s = 0; s < G::E; ++s) v[s] = on ? psi[s * G::T] : make_longlong2(0, 0);
+  for (int s = 0; s < G::E; ++s) v[s] = on && has(s) ? psi[s * G::T] : make_longlong2(0, 0);
+  if constexpr (BS) {
+#pragma unroll
+    for (int s = 0; s < G::E; ++s)
+      if (has(s)) v[s] = conv_chirp(v[s], g.chirp[c.t + s * G::T]);
+  }
   unsigned em;
   int scale = line_from_double<G>(v, c, em);
-  line_fft<G>(v, c, a.twl[G::ppt >= 16], scale);
-  double ek = on ? line_ekin<G>(a, v, c.t, scale) : 0.0;
+  line_pass<G, BS>(v, c, g, a.twl[G::ppt >= 16], scale);
+  double ek = on ? line_ekin<G, BS>(a, v, c.t, scale) : 0.0;
   block_sum<1>(&ek, dred);
   if (threadIdx.x == 0) S.partials[(size_t)(2 + g.dim - 1) * S.pmax + blockIdx.x] = ek;
 }
@@ -458,32 +545,38 @@ __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
 //   0 forward (3D axis 1: pass 0 -> 1) or, with inv, inverse (pass 2 -> 3)
 //   2 forward . P phase . inverse (axis 0: pass 0 (2D) or 1 (3D) -> 2)
 //   3 forward of psi_n (double) + E_kin partial
-template <int MODE, class G>
+template <int MODE, class G, bool BS = false>
 __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
     k_axis(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss, int ax, int inv) {
-  constexpr int N = G::N;
   const GridDev& g = Gs[blockIdx.y];
   const StepDev& S = Ss[blockIdx.y];
+  const int N = line_len<G, BS>(g.ax[g.dim - 1]);
   const long long sub = MODE == 3 ? S.ctl[5] : S.ctl[6];
   if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) S.ctl[5] = sub;  // also when there is nothing left to do
   if (!pass_active(S, sub)) return;
   if (MODE == 3 && !ekin_at(S, sub)) return;
   extern __shared__ __align__(1024) unsigned char sm[];
-  const ColBlock<G> cb(g, ax, sm);
+  const ColBlock<G, BS> cb(g, ax, sm);
   cb.load_begin();
   LineCtx<G> c(cb.tile, cb.slots(sm));
   const bool on = c.l < cb.Ch;
   const long long col = cb.c0 + (on ? c.l : 0);
   const AxisDev& a = g.ax[ax];
+  auto has = [&](int s) { return !BS || c.t + s * G::T < N; };  // points beyond a convolution's line are zero
   longlong2 v[G::K];
   if constexpr (MODE == 3) {
     __shared__ double dred[32];
     if (!cb.load_wait()) S.ctl[4] = 2;
     cb.read(v, c);
+    if constexpr (BS) {
+#pragma unroll
+      for (int s = 0; s < G::E; ++s)
+        if (has(s)) v[s] = conv_chirp(v[s], g.chirp[c.t + s * G::T]);
+    }
     unsigned em;
     int scale = line_from_double<G>(v, c, em);
-    line_fft<G>(v, c, a.twl[G::ppt >= 16], scale);
-    double ek = on ? line_ekin<G>(a, v, c.t, scale) : 0.0;
+    line_pass<G, BS>(v, c, g, a.twl[G::ppt >= 16], scale);
+    double ek = on ? line_ekin<G, BS>(a, v, c.t, scale) : 0.0;
     block_sum<1>(&ek, dred);
     if (threadIdx.x == 0) S.partials[(size_t)(2 + ax) * S.pmax + blockIdx.x] = ek;
     return;
@@ -500,10 +593,14 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
       const int gm = S.gmin[gmin_slot(in_pass, sub)];
       const int* sc = S.sc + (size_t)in_pass * S.scmax + in_at + c.t;
 #pragma unroll
-      for (int s = 0; s < G::E; ++s) d[s] = gm - sc[s * G::T];
+      for (int s = 0; s < G::E; ++s) d[s] = has(s) ? gm - sc[s * G::T] : 0;
       if (!cb.load_wait()) S.ctl[4] = 2;  // the copy did not complete in time: QSF_ETIMEDOUT
       cb.read(v, c);
       scale = line_align<G>(v, d, gm, c);
+      if constexpr (BS) {
+#pragma unroll
+        for (int s = 0; s < G::E; ++s) v[s] = fconj(v[s]);
+      }
     }
     if constexpr (MODE == 2) {
       const int at = (int)(sub - S.ctl[7]);
@@ -519,16 +616,17 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
       for (int d = 0; d < g.dim; ++d) scale -= S.texp[at * kTexp + d];
 #pragma unroll 1  // one code body for both transforms
       for (int h = 0;; ++h) {
-        line_fft<G>(v, c, a.twl[G::ppt >= 16], scale);
+        line_pass<G, BS>(v, c, g, a.twl[G::ppt >= 16], scale);
         if (h) break;
         scale += line_up<G>(v, c);
         // (the table is the same for every line: it stays in L1, where a copy through
         // the exchange slots as in k_row_close came from L2, 315 -> 364 us at 256^3)
 #pragma unroll
-        for (int s = 0; s < G::E; ++s) v[s] = fconj(fmul_tw(fmul_tw(v[s], __ldg(pt + s * G::T)), pc));
+        for (int s = 0; s < G::E; ++s)
+          v[s] = has(s) ? fconj(fmul_tw(fmul_tw(BS ? fconj(v[s]) : v[s], __ldg(pt + s * G::T)), pc)) : make_longlong2(0, 0);
       }
     } else {
-      line_fft<G>(v, c, a.twl[G::ppt >= 16], scale);
+      line_pass<G, BS>(v, c, g, a.twl[G::ppt >= 16], scale);
     }
     cb.write(v, c);
     if (on && c.t == 0) {

@@ -29,10 +29,10 @@ int batch_finish(qsf_batch* b, int64_t* active);
 bool fused_length(int n);
 int bs_size(int n, int dim);
 bool grid_batched(const qsf_grid* g);
-int generic_begin(qsf_grid* g, const qsf_step_desc* d);
-int generic_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
-int generic_wait(qsf_grid* g, bool* bad);
-int generic_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps);
+int solo_begin(qsf_grid* g, const qsf_step_desc* d);
+int solo_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
+int solo_wait(qsf_grid* g, bool* bad);
+int solo_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps);
 }
 
 namespace {
@@ -60,9 +60,9 @@ struct Running {
   std::vector<double> coupling;  // kept alive while in the batch
   clk::time_point submitted, admitted;
   bool cancel = false;           // qsf_server_cancel: leave after this round
-  // a grid without fused kernels (Bluestein lengths): its steps run as member
-  // operations on the grid's own stream, beside the batch, with this step program
-  bool generic = false;
+  // a 1D line or a grid of a Bluestein length: its steps run on the grid's own stream,
+  // beside the batch, with this step program
+  bool solo = false;
   qsf_step_desc d{};
   bool bad = false;  // NaN / non-positive norm seen
   int rc = 0;        // error of a queued round
@@ -81,8 +81,7 @@ size_t solve_bytes(const qsf_request& r) {
   const int64_t m = grid_points(r.grid);
   const int stride = r.grid.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
   size_t b = (size_t)m * (16 + 16 + 8) + (size_t)r.nsteps * (size_t)(3 + r.nborders + stride) * 8 + (1u << 20);
-  // Bluestein lengths: the convolution scratch (up to 4 m points) and the member
-  // operations' X / P phase tables
+  // Bluestein lengths: the convolution scratch (up to 4 m points)
   if (!qsf::fused_length((int)r.grid.n[0])) b += (size_t)m * 16 * 6;
   return b;
 }
@@ -105,7 +104,7 @@ struct qsf_server {
   int device = 0;  // the caller's current device at qsf_server_start; the worker thread selects it
 #ifdef QSF_SERVER_TRACE
   // decide, admit, enqueue, batch, wait, retire, rounds, admits, batch launch (rebuilds)
-  // admits of member-operation / batched solves (incl. their first queued steps)
+  // admits of solves beside the batch / batched ones (incl. their first queued steps)
   // admission parts: grid (pool or new), psi upload, batch add / member program begin,
   // grids created new
   double trace[15] = {0};
@@ -189,8 +188,8 @@ void release_grid(qsf_server* s, const qsf_grid_desc& d, qsf_grid* g) {
 void finish(qsf_server* s, Running& r, int status, const double* rows, int64_t steps) {
 #ifdef QSF_SERVER_TRACE
   if (status && status != QSF_ECANCELED)
-    std::fprintf(stderr, "qsf_server trace: ticket %lld status %d generic %d in_round %d remaining %lld n %lld: %s\n",
-                 (long long)r.ticket, status, (int)r.generic, (int)r.in_round, (long long)r.remaining,
+    std::fprintf(stderr, "qsf_server trace: ticket %lld status %d solo %d in_round %d remaining %lld n %lld: %s\n",
+                 (long long)r.ticket, status, (int)r.solo, (int)r.in_round, (long long)r.remaining,
                  (long long)r.desc.n[0], qsf_last_error());
 #endif
   qsf_result res{};
@@ -270,9 +269,9 @@ int admit(qsf_server* s, Pending& p, Running& r, bool nowait) {
   d.box_size = p.req.box_size;
   QSF_TRACE_T(t_add);
   if (!qsf::grid_batched(g)) {
-    r.generic = true;
+    r.solo = true;
     r.d = d;
-    rc = qsf::generic_begin(g, &r.d);
+    rc = qsf::solo_begin(g, &r.d);
   } else {
     rc = nowait ? qsf::batch_add_nowait(s->batch, g, &d, &r.slot) : qsf_batch_add(s->batch, g, &d, &r.slot);
   }
@@ -344,7 +343,7 @@ void worker_loop(qsf_server* s) {
     QSF_TRACE_ADD(s, 0, t_decide);
     // Admissions cost host time (grid creation or reuse, psi upload, tables).  While
     // solves are resident, the new ones are prepared after this round's work is queued,
-    // so that this host work overlaps the GPU's round: a member-operation solve starts
+    // so that this host work overlaps the GPU's round: a solve beside the batch starts
     // its first steps at once on its own stream, a batched one joins the next round.
     const bool overlap = !s->running.empty();
     auto admit_all = [&]() {
@@ -360,16 +359,16 @@ void worker_loop(qsf_server* s) {
           finish(s, r, rc, nullptr, 0);
           continue;
         }
-        if (r.generic && overlap) {
+        if (r.solo && overlap) {
           const int64_t count = std::min<int64_t>(s->cfg.steps_per_round, r.remaining);
           r.d.coupling = r.coupling.empty() ? nullptr : r.coupling.data();
-          r.rc = qsf::generic_enqueue(r.grid, &r.d, 0, count);
+          r.rc = qsf::solo_enqueue(r.grid, &r.d, 0, count);
           r.in_round = true;
         } else {
           r.in_round = !overlap;
         }
 #ifdef QSF_SERVER_TRACE
-        QSF_TRACE_ADD(s, r.generic ? 9 : 10, t_one);
+        QSF_TRACE_ADD(s, r.solo ? 9 : 10, t_one);
 #endif
         s->running.emplace(r.ticket, std::move(r));
       }
@@ -381,21 +380,21 @@ void worker_loop(qsf_server* s) {
     if (!overlap) admit_all();
     if (s->running.empty()) continue;
     QSF_TRACE_T(t_enqueue);
-    // one round of steps for every resident solve: the member-operation solves' steps
+    // one round of steps for every resident solve: the solves beside the batch
     // queued on their own streams (they overlap with one another and with the batch),
     // then the batch's round; then the admissions; then the waits
     bool any_fused = false;
     for (auto& kv : s->running) {
       Running& r = kv.second;
       r.in_round = true;
-      if (!r.generic) {
+      if (!r.solo) {
         any_fused = true;
         continue;
       }
       const int64_t first = r.nsteps - r.remaining;
       const int64_t count = std::min<int64_t>(s->cfg.steps_per_round, r.remaining);
       r.d.coupling = r.coupling.empty() ? nullptr : r.coupling.data();
-      if (!r.cancel && !r.rc && count > 0) r.rc = qsf::generic_enqueue(r.grid, &r.d, first, count);
+      if (!r.cancel && !r.rc && count > 0) r.rc = qsf::solo_enqueue(r.grid, &r.d, first, count);
     }
     QSF_TRACE_ADD(s, 2, t_enqueue);
     QSF_TRACE_T(t_batch);
@@ -409,8 +408,8 @@ void worker_loop(qsf_server* s) {
     QSF_TRACE_T(t_wait);
     for (auto& kv : s->running) {
       Running& r = kv.second;
-      if (!r.generic || !r.in_round) continue;
-      const int rw = qsf::generic_wait(r.grid, &r.bad);
+      if (!r.solo || !r.in_round) continue;
+      const int rw = qsf::solo_wait(r.grid, &r.bad);
       if (rw && !r.rc) r.rc = rw;
     }
     QSF_TRACE_ADD(s, 4, t_wait);
@@ -426,10 +425,10 @@ void worker_loop(qsf_server* s) {
     for (auto& kv : s->running) {
       Running& r = kv.second;
       if (!r.in_round && !fatal) continue;  // joined the batch during this round: runs from the next
-      const int64_t ran = r.cancel && r.generic ? 0 : std::min<int64_t>(s->cfg.steps_per_round, r.remaining);
-      if (r.in_round) r.remaining -= r.generic ? ran : s->cfg.steps_per_round;
-      bool bad = r.generic && (r.bad || r.rc);
-      if (!r.generic && r.in_round && rc_run == QSF_ENUMERIC) {
+      const int64_t ran = r.cancel && r.solo ? 0 : std::min<int64_t>(s->cfg.steps_per_round, r.remaining);
+      if (r.in_round) r.remaining -= r.solo ? ran : s->cfg.steps_per_round;
+      bool bad = r.solo && (r.bad || r.rc);
+      if (!r.solo && r.in_round && rc_run == QSF_ENUMERIC) {
         int64_t st = 0;
         bad = qsf_batch_result(s->batch, r.slot, nullptr, &st) != QSF_OK;
       }
@@ -442,15 +441,15 @@ void worker_loop(qsf_server* s) {
       int rc;
       if (fatal) {
         rc = rc_run;
-      } else if (r.generic) {
+      } else if (r.solo) {
         steps = r.nsteps - std::max<int64_t>(r.remaining, 0);
-        rc = r.rc ? r.rc : qsf::generic_rows(r.grid, &r.d, rows.data(), steps);
+        rc = r.rc ? r.rc : qsf::solo_rows(r.grid, &r.d, rows.data(), steps);
         if (rc == QSF_OK && r.bad) rc = QSF_ENUMERIC;
       } else {
         rc = qsf_batch_result(s->batch, r.slot, rows.data(), &steps);
       }
       if (rc == QSF_OK && r.cancel && r.remaining > 0) rc = QSF_ECANCELED;
-      if (!r.generic) qsf_batch_remove(s->batch, r.slot);
+      if (!r.solo) qsf_batch_remove(s->batch, r.slot);
       if (rc && rc != QSF_ECANCELED) qsf_grid_destroy(r.grid);
       else release_grid(s, r.desc, r.grid);
       finish(s, r, rc, rows.data(), steps);

@@ -80,6 +80,47 @@ def test_imaginary_time_matches_oracle(dim, n, gauge, fields):
     g.close()
 
 
+# lines run as convolutions: shorter and longer than a box of the strided copies, ragged last
+# column blocks and boxes, plans of exactly 2 n - 1 + 1 points and with spare ones
+@pytest.mark.parametrize("dim,n", [(2, n) for n in (3, 7, 33, 63, 65, 100, 127, 129, 250, 513)] + [(3, n) for n in (5, 21, 50, 66)])
+@pytest.mark.parametrize("gauge,mode", [("velocity", "real"), ("length", "real"), ("velocity", "imaginary")])
+def test_convolution_steps_match_oracle(dim, n, gauge, mode):
+    """sqrt(n): the oracle's direct DFT passes of a large prime factor add up to n terms."""
+    import qsf_gb300 as Q
+    from oracle import oracle as O
+    from qsf_gb300.propagator import coupling_schedule
+    real, lg, steps = mode == "real", gauge == "length", 4
+    dt, axis = (0.05 if real else 0.01), {2: 3, 3: 7}[dim]
+    psi0 = _noise_state(dim, n, 0.3, n)
+    pulse = dict(field=0.1, omega=1.1, ncycles=1.0)
+    og_g, qg = (O.GAUGE_LENGTH, Q.GAUGE_LENGTH) if lg else (O.GAUGE_VELOCITY, Q.GAUGE_VELOCITY)
+    oc = O.Coupling(og_g, [O.Field(axis, [O.Pulse(**pulse)])] if real else [])
+    og = O.Grid(dim, n, 0.3, nCAP=max(1, n // 10), pot=O.POT_EBERLY, Ncharge=float(dim), coupling=oc)
+    og.psi[...] = psi0
+    outs = ["norm", "epot"] if real else ["norm", "normalize", "epot", "ekin"]
+    prop = O.Propagator(O.MODE_RE if real else O.MODE_IM, dt, steps, og, outs)
+    for _ in range(steps):
+        prop.make_step()
+        prop.compute_each()
+    g = Q.Grid(dim, n, 0.3, nCAP=max(1, n // 10), Ncharge=float(dim), gauge=qg, n_fields=1 if real else 0)
+    g.upload(psi0)
+    if real:
+        rows = coupling_schedule(Q.Coupling(qg, [Q.Field(axis, [Q.Pulse(**pulse)])]), dt, steps)[0]
+        out, done = g.step(Q.MODE_RE, dt, steps, rows, obs=Q.OBS_NORM | Q.OBS_EPOT)
+    else:
+        out, done = g.step(Q.MODE_IM, dt, steps, obs=Q.OBS_NORM | Q.OBS_EPOT | Q.OBS_EKIN, normalize=True, ekin_interval=2)
+    assert done == steps
+    tol = _tol(dim, n, steps) * math.sqrt(n)
+    assert C.rel_l2(g.download(), og.psi) < tol
+    for s, r in enumerate(prop.rows):
+        f = 1.0 if real else out[s, 0]
+        assert out[s, 0] == pytest.approx(r["norm"], rel=4 * tol)
+        assert out[s, 1] / f == pytest.approx(r["epot"], rel=4 * tol)
+        if not real and s % 2:
+            assert out[s, 2] / f == pytest.approx(r["ekin"], rel=8 * tol)
+    g.close()
+
+
 def _line_oracle(n, lg, mode, steps, dt, psi0, pulse, outs):
     from oracle import oracle as O
     oc = O.Coupling(O.GAUGE_LENGTH if lg else O.GAUGE_VELOCITY, [O.Field(1, [O.Pulse(**pulse)])] if pulse else [])
