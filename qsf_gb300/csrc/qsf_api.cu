@@ -545,7 +545,8 @@ Geom geom_of(const qsf_grid* g) {
 // k_finalize on a second stream (`side`): it forks from `st` after the sub-step's last
 // pass, and the next sub-step waits for it (`done`) only before its pass that rewrites
 // the partials and the flux snapshot.  Valid when k_finalize writes nothing the next
-// sub-step's earlier kernels read: no pending Normalize factor, no convergence stop.
+// sub-step's earlier kernels read: no convergence stop (Normalize reaches psi one sub-step
+// later still, StepDev::scale).
 struct FinOverlap {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, done = nullptr;
@@ -619,7 +620,7 @@ int launch_step(qsf_grid* g, const StepDev& S, Prof* P = nullptr, bool with_open
 }
 
 // Whether k_finalize may run beside the next sub-step (FinOverlap), and its stream.
-bool fin_overlap_ok(const StepDev& S) { return !S.normalize && !(S.mode == 1 && S.state_accuracy > 0.0); }
+bool fin_overlap_ok(const StepDev& S) { return !(S.mode == 1 && S.state_accuracy > 0.0); }
 int ensure_fin_stream(qsf_grid* g, FinOverlap* ov) {
   if (!g->fin_stream) {
     QSF_CU(cudaStreamCreateWithFlags(&g->fin_stream, cudaStreamNonBlocking));
@@ -674,8 +675,8 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   std::copy(ctl_h, ctl_h + 8, h.ctl);
   h.energy[0] = d->last_energy;
   h.energy[1] = 0.0;
-  std::fill(h.scale, h.scale + 3, 1.0);
-  h.scale[3] = 0.0;
+  h.scale[0] = h.scale[2] = 1.0;
+  h.scale[1] = h.scale[3] = 0.0;
   std::fill(h.gmin, h.gmin + kGmin, 0x7fffffff);
   StepDev S{};
   S.mode = d->mode;
@@ -1399,8 +1400,8 @@ int qsf_normalize(qsf_grid* g, double* norm_out) {
   if (int rc = qsf_average(g, QSF_REP_X, QSF_OP_IDENTITY, &nrm)) return rc;
   if (!(nrm > 0.0)) return fail(QSF_ENUMERIC, "norm is not positive");
   const double s = std::sqrt(1.0 / nrm);
-  QSF_CU(cudaMemcpyAsync(g->scale + 1, &s, sizeof(double), cudaMemcpyHostToDevice, g->stream));
-  k_scale<<<grid_blocks(g->G.m), 256, 0, g->stream>>>(g->G.psi, g->G.m, g->scale + 1);
+  QSF_CU(cudaMemcpyAsync(g->energy + 1, &s, sizeof(double), cudaMemcpyHostToDevice, g->stream));
+  k_scale<<<grid_blocks(g->G.m), 256, 0, g->stream>>>(g->G.psi, g->G.m, g->energy + 1);
   QSF_CU(cudaGetLastError());
   QSF_CU(cudaStreamSynchronize(g->stream));
   if (norm_out) *norm_out = nrm;

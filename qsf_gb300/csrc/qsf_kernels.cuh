@@ -173,11 +173,14 @@ struct StepDev {
   double* rows;          // [nsteps][3 + nborders]
   // Normalize only scales psi: psi stays unscaled in a call and the sums are scaled.
   // [0] the pending factor of psi in memory, [2] its square for psi as the passes hold it,
-  // [3] the power of two that the next sub-step takes out of it (exact)
+  // [scale_slot(s)] the power of two (exact) that sub-step s + 2 takes out of it: the step
+  // end of s may still run beside the passes of s + 1 (1024^2: 101 us a step when those
+  // waited for it)
   double* scale;
   LineDev line;          // 1D grids (qsf_line1d.cuh)
 };
 
+__device__ __forceinline__ int scale_slot(long long sub) { return 1 + 2 * (int)(sub & 1); }
 // whether sub-step `sub` ends a step whose observables include E_kin
 __device__ __forceinline__ bool ekin_at(const StepDev& S, long long sub) {
   if (!(S.obs & 4u) || (sub + 1) % S.substeps) return false;
@@ -617,13 +620,13 @@ __global__ void __launch_bounds__(256) k_finalize(const GridDev* __restrict__ Gs
   const long long step = K == 1 ? sub : sub / K;
   if (!step_end) {
     if (blockIdx.x == 0 && tid == 0) {
-      S.scale[3] = 0.0;
+      S.scale[scale_slot(sub)] = 0.0;
       S.ctl[0] = sub + 1;
     }
     return;
   }
   const bool ek = ekin_at(S, sub);
-  const double cf0 = S.scale[2], e0 = S.energy_state[0];
+  const double cf0 = S.scale[2], e0 = S.energy_state[0], e1 = S.scale[scale_slot(sub + 1)];
   const int nrow = S.nrowblk, nft = S.nfterms, D = g.dim;
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   double* mine = S.fpartials + (size_t)blockIdx.x * kFinCols;
@@ -691,11 +694,13 @@ __global__ void __launch_bounds__(256) k_finalize(const GridDev* __restrict__ Gs
     if (S.normalize && norm > 0.0) {
       cfac = cfac / norm;
       *S.scale = sqrt(cfac);
+      // the next sub-step takes e1, the one after it the power chosen here
+      if (K == 1) cfac = ldexp(cfac, -2 * (int)e1);
       int e;
       frexp(cfac, &e);
       e >>= 1;
-      S.scale[3] = (double)e;
-      S.scale[2] = ldexp(cfac, -2 * e);
+      S.scale[scale_slot(sub)] = (double)e;
+      S.scale[2] = K == 1 ? cfac : ldexp(cfac, -2 * e);
     }
     // the convergence test needs E = E_pot + E_kin: with E_kin on every k-th step only,
     // it runs on those steps (comparing with the previous one that had it)

@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(G::kColThreads, G::blocks(G::kColThreads))
       const int4 pc = split_fx(f);
       const int4* pt = tab + c.t;
       // the exponents of the P phase's two products and tables, and of the pending Normalize factor
-      scale -= 4 + (S.normalize ? (int)S.scale[3] : 0);
+      scale -= 4 + (S.normalize ? (int)S.scale[scale_slot(sub)] : 0);
       for (int d = 0; d < g.dim; ++d) scale -= S.texp[at * kTexp + d];
 #pragma unroll 1  // one code body for both transforms
       for (int h = 0;; ++h) {

@@ -80,6 +80,27 @@ def test_imaginary_time_matches_oracle(dim, n, gauge, fields):
     g.close()
 
 
+@pytest.mark.parametrize("substeps,n", [(1, 64), (2, 64), (3, 64), (1, 100)])
+def test_normalize_in_one_call_matches_one_step_per_call(substeps, n):
+    """The powers of two that Normalize takes out reach psi two sub-steps later: a long
+    call against calls of one step, where none is pending.  The noise state loses most of
+    its norm in each of the first steps."""
+    import qsf_gb300 as Q
+    steps, dt = 40, 0.05
+    psi0 = _noise_state(2, n, 0.3, n)
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT, normalize=True, substeps=substeps)
+    g = Q.Grid(2, n, 0.3, nCAP=n // 10, Ncharge=2.0)
+    g.upload(psi0)
+    one, _ = g.step(Q.MODE_IM, dt, steps, **kw)
+    psi = g.download()
+    g.upload(psi0)
+    each = np.concatenate([g.step(Q.MODE_IM, dt, 1, **kw)[0] for _ in range(steps)])
+    tol = _tol(2, n, steps * substeps)
+    assert C.rel_l2(psi, g.download()) < tol
+    np.testing.assert_allclose(one[:, :2], each[:, :2], rtol=4 * tol, atol=0)
+    g.close()
+
+
 # lines run as convolutions: shorter and longer than a box of the strided copies, ragged last
 # column blocks and boxes, plans of exactly 2 n - 1 + 1 points and with spare ones
 @pytest.mark.parametrize("dim,n", [(2, n) for n in (3, 7, 33, 63, 65, 100, 127, 129, 250, 513)] + [(3, n) for n in (5, 21, 50, 66)])
