@@ -2,7 +2,7 @@
 and the radix plan (points per thread) of the one-CTA 1D line kernel per length.
 
 A row shape is written as points x threads (4096 x 256: 16 points per thread, radix-16
-plans, 128 registers; 4096 x 512: 8 points per thread, radix-8 plans, 80 registers and
+plans, 128 registers; 4096 x 512: 8 points per thread, radix-8 plans, 112 registers and
 half the code per pass, twice the warps); the ratio selects the line plan
 (qsf_lines.cuh).  For each candidate the library is built with every line length forced
 to it (`QSF_TILE`, `QSF_ROW_THREADS`, in qsf_gb300/_build/tune_<points>_<threads>/);
@@ -11,7 +11,7 @@ one call of K graph-replayed steps after a warm-up call) in a subprocess that lo
 build; per line length the shape with the least summed step time over the workloads of
 that edge wins (the 2D grid and the 3D cube of one edge share their kernels).  With
 --write the choice goes to qsf_gb300/csrc/qsf_tuning.h, which the default build
-compiles in.  The plan of 1D lines held by one CTA as one line (up to 640 points) is
+compiles in.  The plan of 1D lines held by one CTA as one line (up to 320 points) is
 tuned the same way: candidate builds force 8 or 16 points per thread (`QSF_LINE_PPT`),
 the 1D workloads are timed, and each measured length keeps its fastest plan; a length
 between measured ones takes the plan of the next longer measured length.  Needs a GPU.
@@ -35,7 +35,7 @@ CANDIDATES = ((4096, 256), (4096, 512))
 ALL_CANDIDATES = CANDIDATES
 DEFAULT_SHAPE = (4096, 256)
 LINE_CANDIDATES = (8, 16)
-LINE_WORKLOADS = [("1d64", 400), ("1d128", 400), ("1d256", 400), ("1d384", 400), ("1d640", 400)]
+LINE_WORKLOADS = [("1d64", 400), ("1d128", 400), ("1d320", 400)]
 # (workload of profile_step, steps per timed call)
 TUNE_WORKLOADS = [("2d64", 400), ("2d128", 400), ("2d192", 400), ("2d256", 400), ("2d320", 400), ("2d384", 400), ("2d512", 400), ("2d640", 300), ("2d768", 300),
                   ("2d1024", 300), ("2d1280", 200),
@@ -102,7 +102,7 @@ def shape_function(choice: dict, k: int, default: int) -> str:
 
 
 def header_text(choice: dict, times: dict, lchoice: dict = None, ltimes: dict = None) -> str:
-    lchoice = lchoice if lchoice is not None else {640: 8}
+    lchoice = lchoice if lchoice is not None else {320: 8}
     rows = []
     for w, _ in TUNE_WORKLOADS:
         cells = "  ".join(f"{c[0]}x{c[1]}: {times[(w, c)]:.4f}" for c in ALL_CANDIDATES if (w, c) in times)
@@ -135,7 +135,7 @@ __host__ __device__ constexpr int tuned_tile(int n) {{
   return {shape_function(choice, 0, DEFAULT_SHAPE[0])};
 }}
 
-// Points per thread of 1D lines held by one CTA as one line (up to 640 points; 8: radix-8
+// Points per thread of 1D lines held by one CTA as one line (up to 320 points; 8: radix-8
 // plans, 16: radix 16); a length between measured ones takes the plan of the next longer
 // measured length.  Measured (one call of graph-replayed steps, points per
 // thread: ms per step):

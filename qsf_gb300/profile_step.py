@@ -41,12 +41,13 @@ WORKLOADS = {
     "1d128": (1, 128, 0.2, 13, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 48),
     "1d256": (1, 256, 0.2, 26, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 100),
     "1d384": (1, 384, 0.2, 38, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 150),
+    "1d320": (1, 320, 0.2, 32, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 125),
     "1d640": (1, 640, 0.2, 64, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 250),
     "1d1024": (1, 1024, 0.2, 102, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 400),
     "1d2048": (1, 2048, 0.2, 205, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 800),
     "1d8192": (1, 8192, 0.2, 819, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 1638),
     "1d1536": (1, 1536, 0.2, 153, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 600),
-    # lengths outside the built list: Bluestein transforms, member-operation programs
+    # lengths outside the built list: Bluestein convolutions
     "1d4099": (1, 4099, 0.2, 410, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 1638),
     "2d1000": (2, 1000, 0.3, 100, 2.0, 0, 5e14, 800.0, 3.0, "ZOA_FLUX_2D", 0),
     "1d3072": (1, 3072, 0.2, 307, 1.0, 1, 1e14, 800.0, 2.0, ["BOX"], 1200),
