@@ -614,8 +614,8 @@ int launch_group(const KernelSet& K, const Geom& q, const GridDev* dG, const Ste
   return QSF_OK;
 }
 
-int launch_step(qsf_grid* g, const StepDev& S, Prof* P = nullptr, bool with_open = true, FinOverlap* ov = nullptr) {
-  return launch_group(g->pass, geom_of(g), g->dG, g->dS, 1, (S.obs & QSF_OBS_EKIN) != 0, fin_blocks(g, S.nfterms),
+int launch_step(qsf_grid* g, const StepDev& S, Prof* P, bool with_open, FinOverlap* ov, bool ekin) {
+  return launch_group(g->pass, geom_of(g), g->dG, g->dS, 1, ekin, fin_blocks(g, S.nfterms),
                       g->stream, P, with_open, ov);
 }
 
@@ -781,58 +781,78 @@ int capture_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec) {
   return QSF_OK;
 }
 
-// The next `count` sub-steps of a program of the 2D and 3D passes, queued on the grid's
-// stream (start: its first ones).  One graph holds kTableSteps steps (the kernels read the
-// step index from the device, so every copy is the same), the remainder runs as single
-// steps.  In a fused program only the first step's opening row pass works, so it runs once,
-// before the graphs, which leave it out.  The executable graph stays with the grid and is
-// replayed by later calls of the same launch shape (no capture per call).
-int run_passes(qsf_grid* g, const StepDev& S, int64_t count, bool start) {
+// The next `count` sub-steps, from sub-step `at` on, of a program of the 2D and 3D passes,
+// queued on the grid's stream.  One graph holds up to kTableSteps steps (the kernels read
+// the step index from the device, so every copy is the same), the remainder runs as single
+// steps.  The executable graph stays with the grid and is replayed by later calls of the
+// same launch shape (no capture per call).
+//
+// A fused program's opening row pass works only in its first sub-step and after an E_kin
+// step, the E_kin passes only in E_kin steps: what is idle is not launched.  Runs with
+// E_kin every few steps replay whole periods (up to kGraphMax sub-steps) of passes; with a
+// convergence stop, whose last step only the device knows, every step launches everything.
+// (1024^2 with E_kin every tenth step: 96 us a step with the idle launches.)
+int run_passes(qsf_grid* g, const StepDev& S, int64_t at, int64_t count) {
+  constexpr int64_t kGraphMax = 4 * kTableSteps;
+  const bool ekin = (S.obs & QSF_OBS_EKIN) != 0;
+  const int64_t period = ekin ? (int64_t)S.ekin_every * S.substeps : 1;
+  const bool known = S.fused && !(S.mode == 1 && S.state_accuracy > 0.0) && period <= kGraphMax;
+  auto has_ekin = [&](int64_t s) { return ekin && (!known || (s + 1) % period == 0 || s + 1 >= S.nsteps); };
+  auto opens = [&](int64_t s) { return !known || s == 0 || has_ekin(s - 1); };
   int rc;
-  if (count < 4) {
-    if (count > 0 && (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)count, g->stream))) return rc;
-    for (int64_t k = 0; k < count; ++k)
-      if ((rc = launch_step(g, S))) return rc;
-    return QSF_OK;
+  const int64_t end = at + count;
+  auto single = [&](int64_t s) {
+    if (int r = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream)) return r;
+    return launch_step(g, S, nullptr, opens(s), nullptr, has_ekin(s));
+  };
+  int64_t s = at;
+  if (count >= 4) {
+    // up to where a graph may start: after the first opening pass, or at a period's start
+    for (; s < end && (known && !ekin ? s == 0 : known && s % period != 0); ++s)
+      if ((rc = single(s))) return rc;
+    const int64_t rest = end - s;
+    const int64_t per = known && ekin ? period * std::max<int64_t>(1, kTableSteps / period) : std::min<int64_t>(kTableSteps, rest);
+    if (rest >= per && rest > 0) {
+      cudaGraphExec_t exec = nullptr;
+      FinOverlap ov;
+      const bool overlap = fin_overlap_ok(S);
+      if (overlap && (rc = ensure_fin_stream(g, &ov))) return rc;
+      const int nfblk = fin_blocks(g, S.nfterms);
+      const int64_t shape = !known ? (ekin ? -2 : -1) : ekin ? period : 0;
+      for (const qsf_grid::StepGraph& sg : g->step_graphs)
+        if (sg.per == per && sg.shape == shape && sg.overlap == (int)overlap && sg.nfblk == nfblk) exec = sg.exec;
+      if (!exec) {
+        if ((rc = capture_graph(
+                 g->stream,
+                 [&]() {
+                   for (int64_t k = 0; k < per; ++k) {
+                     if (k % kTableSteps == 0)
+                       if (int r = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)std::min<int64_t>(kTableSteps, per - k),
+                                                 g->stream))
+                         return r;
+                     const bool first = known && ekin && k % period == 0, last = known && ekin && (k + 1) % period == 0;
+                     if (int r = launch_step(g, S, nullptr, first || !known, overlap ? &ov : nullptr, last || (ekin && !known)))
+                       return r;
+                   }
+                   if (ov.pending) QSF_CU(cudaStreamWaitEvent(g->stream, ov.done, 0));  // join
+                   return QSF_OK;
+                 },
+                 &exec)))
+          return rc;
+        g->step_graphs.push_back({per, shape, (int)overlap, nfblk, exec});
+      }
+      for (; end - s >= per; s += per) {
+        const cudaError_t ce = cudaGraphLaunch(exec, g->stream);
+        if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
+      }
+    }
   }
-  const bool skip_open = S.fused != 0 && !(S.obs & QSF_OBS_EKIN);
-  int64_t first = 0;
-  if (skip_open && start) {
-    if ((rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream)) || (rc = launch_step(g, S))) return rc;
-    first = 1;
-  }
-  const int64_t rest = count - first;
-  const int64_t per = std::min<int64_t>(kTableSteps, rest);
-  cudaGraphExec_t exec = nullptr;
-  FinOverlap ov;
-  const bool overlap = fin_overlap_ok(S);
-  if (overlap && (rc = ensure_fin_stream(g, &ov))) return rc;
-  const int ekin = (S.obs & QSF_OBS_EKIN) ? 1 : 0, nfblk = fin_blocks(g, S.nfterms);
-  for (const qsf_grid::StepGraph& sg : g->step_graphs)
-    if (sg.per == per && sg.skip_open == (int)skip_open && sg.overlap == (int)overlap && sg.ekin == ekin &&
-        sg.nfblk == nfblk)
-      exec = sg.exec;
-  if (!exec) {
-    if ((rc = capture_graph(
-             g->stream,
-             [&]() {
-               if (int r = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)per, g->stream)) return r;
-               for (int64_t k = 0; k < per; ++k)
-                 if (int r = launch_step(g, S, nullptr, !skip_open, overlap ? &ov : nullptr)) return r;
-               if (ov.pending) QSF_CU(cudaStreamWaitEvent(g->stream, ov.done, 0));  // join
-               return QSF_OK;
-             },
-             &exec)))
+  for (int64_t k = s; k < end; ++k) {
+    if ((k - s) % kTableSteps == 0 &&
+        (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)std::min<int64_t>(kTableSteps, end - k), g->stream)))
       return rc;
-    g->step_graphs.push_back({per, (int)skip_open, (int)overlap, ekin, nfblk, exec});
+    if ((rc = launch_step(g, S, nullptr, opens(k), nullptr, has_ekin(k)))) return rc;
   }
-  for (int64_t k = 0; k + per <= rest; k += per) {
-    const cudaError_t ce = cudaGraphLaunch(exec, g->stream);
-    if (ce != cudaSuccess) return fail(QSF_ECUDA, std::string("graph launch: ") + cudaGetErrorString(ce));
-  }
-  if (rest % per && (rc = launch_tables(geom_of(g), g->dG, g->dS, 1, (int)(rest % per), g->stream))) return rc;
-  for (int64_t k = rest - rest % per; k < rest; ++k)
-    if ((rc = launch_step(g, S, nullptr, !skip_open))) return rc;
   return QSF_OK;
 }
 
@@ -1492,11 +1512,11 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
     P.count = d->kernel_launches;
     rc = P.init(g->stream, (int)std::min<int64_t>(S.nsteps * 8 + 8, 1 << 20));
     for (int64_t k = 0; k < S.nsteps && rc == QSF_OK; ++k)
-      if (!(rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream, &P))) rc = launch_step(g, S, &P);
+      if (!(rc = launch_tables(geom_of(g), g->dG, g->dS, 1, 1, g->stream, &P))) rc = launch_step(g, S, &P, true, nullptr, (S.obs & QSF_OBS_EKIN) != 0);
     if (rc == QSF_OK) rc = P.flush();
     P.release();
     if (rc) return rc;
-  } else if ((rc = run_passes(g, S, S.nsteps, true))) {
+  } else if ((rc = run_passes(g, S, 0, S.nsteps))) {
     return rc;
   }
   return finish_step(g, S, d->normalize, d->nsteps, ncol, rows, steps_done);
@@ -1528,7 +1548,7 @@ int qsf::solo_begin(qsf_grid* g, const qsf_step_desc* d) {
 int qsf::solo_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count) {
   if (first < 0 || count < 0 || first + count > d->nsteps) return fail(QSF_EINVAL, "steps outside the program");
   const int64_t subs = count * std::max(1, d->substeps);
-  return g->G.dim == 1 ? line_run(g, g->solo, subs, nullptr, nullptr) : run_passes(g, g->solo, subs, first == 0);
+  return g->G.dim == 1 ? line_run(g, g->solo, subs, nullptr, nullptr) : run_passes(g, g->solo, first * std::max(1, d->substeps), subs);
 }
 
 int qsf::solo_wait(qsf_grid* g, bool* bad) {

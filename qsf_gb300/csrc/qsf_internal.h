@@ -155,8 +155,8 @@ struct qsf_grid {
   // executable step graphs of qsf_step, kept per launch shape and replayed by later
   // calls (the kernels read every per-call value from the device descriptors)
   struct StepGraph {
-    int64_t per;
-    int skip_open, overlap, ekin, nfblk;
+    int64_t per, shape;  // sub-steps, and which passes they launch (run_passes)
+    int overlap, nfblk;
     cudaGraphExec_t exec;
   };
   std::vector<StepGraph> step_graphs;

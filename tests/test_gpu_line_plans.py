@@ -101,6 +101,29 @@ def test_normalize_in_one_call_matches_one_step_per_call(substeps, n):
     g.close()
 
 
+@pytest.mark.parametrize("every,substeps", [(1, 1), (3, 1), (20, 1), (5, 2), (70, 1)])
+def test_ekin_interval_in_one_call_matches_one_step_per_call(every, substeps):
+    """Whole periods of passes in a graph (shorter and longer than the tables of one
+    launch, and too long for a graph), with steps left over."""
+    import qsf_gb300 as Q
+    n, steps, dt = 64, 73, 0.01
+    psi0 = _noise_state(2, n, 0.3, n)
+    obs = Q.OBS_NORM | Q.OBS_EPOT | Q.OBS_EKIN
+    g = Q.Grid(2, n, 0.3, nCAP=n // 10, Ncharge=2.0)
+    g.upload(psi0)
+    one, _ = g.step(Q.MODE_IM, dt, steps, obs=obs, normalize=True, substeps=substeps, ekin_interval=every)
+    psi = g.download()
+    g.upload(psi0)
+    each = np.concatenate([g.step(Q.MODE_IM, dt, 1, obs=obs, normalize=True, substeps=substeps)[0] for _ in range(steps)])
+    tol = _tol(2, n, steps * substeps)
+    assert C.rel_l2(psi, g.download()) < tol
+    np.testing.assert_allclose(one[:, :2], each[:, :2], rtol=4 * tol, atol=0)
+    at = [s for s in range(steps) if (s + 1) % every == 0 or s + 1 == steps]
+    np.testing.assert_allclose(one[at, 2], each[at, 2], rtol=8 * tol, atol=0)
+    assert not np.delete(one[:, 2], at).any()
+    g.close()
+
+
 # lines run as convolutions: shorter and longer than a box of the strided copies, ragged last
 # column blocks and boxes, plans of exactly 2 n - 1 + 1 points and with spare ones
 @pytest.mark.parametrize("dim,n", [(2, n) for n in (3, 7, 33, 63, 65, 100, 127, 129, 250, 513)] + [(3, n) for n in (5, 21, 50, 66)])
