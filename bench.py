@@ -443,8 +443,8 @@ def run_served(rate, duration_s, steps_per_solve=256, seed=0, max_slots=128, ste
             "value": pts / wall, "unit": UNIT,
             "p50_s": pct(0.50), "p99_s": pct(0.99), "wall_s": wall,
             "workload": f"served: Poisson {rate}/s for {duration_s}s, 50/50 1D N uniform over the integers "
-                        f"1024..16384 (lengths outside the fused-kernel list through Bluestein transforms and "
-                        f"member operations) / 2D edge in {SERVE_2D}, I log-U[1e14,1e15], lambda U[400,1600] nm, "
+                        f"1024..16384 (lengths outside the fused-kernel list as Bluestein "
+                        f"convolutions) / 2D edge in {SERVE_2D}, I log-U[1e14,1e15], lambda U[400,1600] nm, "
                         f"{steps_per_solve} steps per solve, seed {seed}"}
 
 

@@ -132,8 +132,8 @@ typedef struct qsf_grid qsf_grid;
  * built kernel list (2^a, 3*2^a and 5*2^a from 8 to 16384: 33 lengths) take the fused
  * kernels; the others (up to 16384 in 1D, 2048 in 2D / 3D) transform each axis by
  * Bluestein's chirp-z convolution over a built length M >= 2n - 1 in fused kernels of
- * their own; batches of 2D / 3D grids take built lengths only (QSF_EINVAL), the server
- * runs the others beside its batch.  Other lengths:
+ * their own; batches take built lengths only (QSF_EINVAL), the server runs the others
+ * beside its batch.  Other lengths:
  * QSF_EINVAL. */
 int qsf_grid_create(const qsf_grid_desc* desc, void* stream, qsf_grid** out);
 /* Frees the grid's device state; a member of a batch leaves the batch first. */
