@@ -1,0 +1,55 @@
+"""The ends of steps: the counters, sums and factors that a step leaves for the next one."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_at_size import _noise_state
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dim,n,nodes", [(2, 128, (25, 14, 10, 40)), (2, 100, (17, 10, 8, 25)), (3, 32, (6, 4, 3, 12))])
+@pytest.mark.parametrize("substeps", [2, 3])
+def test_substeps_of_a_step_match_steps_of_their_own(dim, n, nodes, substeps):
+    """A step of K sub-steps is K steps of dt / K whose rows between are left out: the same
+    launches, so the same bits.  Border sets of several hundred terms, which several blocks
+    sum up, and many steps, because what is tested is the order of those blocks."""
+    import qsf_gb300 as Q
+    steps, dt = 48, 0.06
+    psi0 = _noise_state(dim, n, 0.3, n)
+    rows = np.zeros((steps * substeps, 3))
+    rows[:, :dim] = 0.2 * np.random.default_rng(1).standard_normal((steps * substeps, 1))
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT, borders=Q.ZOA_FLUX_2D if dim == 2 else Q.ZOA_FLUX_3D)
+    g = Q.Grid(dim, n, 0.3, nCAP=n // 10, Ncharge=float(dim), n_fields=1, border_nodes=nodes)
+    g.upload(psi0)
+    each, _ = g.step(Q.MODE_RE, dt / substeps, steps * substeps, rows, **kw)
+    psi = g.download()
+    assert np.abs(each[:, 3:]).max() > 0
+    for _ in range(8):
+        g.upload(psi0)
+        got, done = g.step(Q.MODE_RE, dt, steps, rows, substeps=substeps, **kw)
+        assert done == steps
+        assert np.array_equal(got, each[substeps - 1::substeps])
+        assert np.array_equal(g.download(), psi)
+    g.close()
+
+
+@pytest.mark.parametrize("dim,n", [(2, 128), (3, 32)])
+def test_substeps_under_normalize_match_one_step_per_call(dim, n):
+    """Normalize takes its factor from those sums: 2e-13 is the rounding of 64 steps at the
+    (2 dim log2(n) + 10) eps a step of a correct run."""
+    import qsf_gb300 as Q
+    steps, dt = 32, 0.02
+    psi0 = _noise_state(dim, n, 0.3, n)
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT, normalize=True, substeps=2,
+              borders=Q.ZOA_FLUX_2D if dim == 2 else Q.ZOA_FLUX_3D)
+    g = Q.Grid(dim, n, 0.3, nCAP=n // 10, Ncharge=float(dim), border_nodes=(25, 14, 10, 40) if dim == 2 else (6, 4, 3, 12))
+    g.upload(psi0)
+    each = np.concatenate([g.step(Q.MODE_IM, dt, 1, **kw)[0] for _ in range(steps)])
+    ref = g.download()
+    for _ in range(8):
+        g.upload(psi0)
+        got, done = g.step(Q.MODE_IM, dt, steps, **kw)
+        assert done == steps
+        np.testing.assert_allclose(got[:, :2], each[:, :2], rtol=4 * 2e-13, atol=0)
+        assert np.linalg.norm(g.download() - ref) < 2e-13 * np.linalg.norm(ref)
+    g.close()
