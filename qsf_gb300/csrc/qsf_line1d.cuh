@@ -23,9 +23,9 @@
 //
 // One extra warp of CTA 0 ends the steps (sums, fluxes, the observables row, the
 // Normalize factor, the convergence test) while the others work on the next one.  The
-// Normalize factor only scales psi, so psi stays unscaled within a launch and the sums of
-// later steps are scaled instead; a launch starts by taking the factor's power of two,
-// which is exact.
+// Normalize factor only scales psi: psi takes its power of two, which is exact, at the
+// start of a launch and one step after it is known (psi left unscaled over the 256
+// sub-steps of a launch would leave the range of a double), and the sums take the rest.
 #pragma once
 #include "qsf_lines.cuh"
 
@@ -274,14 +274,15 @@ __device__ __forceinline__ void limb_sum(i64 n, int* out) {
   out[2] = __reduce_add_sync(0xffffffffu, (int)(n >> 44));
 }
 
-// the power of two a launch takes out of the pending Normalize factor: psi starts as
-// psi 2^two, the factor's square as cfac 2^(-2 two)
-__device__ __forceinline__ int line_two(const StepDev& S) {
-  if (!S.normalize) return 0;
+// the power of two psi takes out of a pending Normalize factor of square cfac: psi goes on
+// as psi 2^two, the square as cfac 2^(-2 two)
+__device__ __forceinline__ int line_two(double cfac) {
+  if (!(cfac > 0.0) || isinf(cfac)) return 0;
   int e;
-  frexp(S.scale[2], &e);
+  frexp(cfac, &e);
   return e >> 1;
 }
+__device__ __forceinline__ int line_two(const StepDev& S) { return S.normalize ? line_two(S.scale[2]) : 0; }
 // whether sub-step `sub` ends a step with E_kin when the run stops after sub-step `stop`
 // (ekin_at with a stop that every thread of the cluster agrees on)
 __device__ __forceinline__ bool line_ekin_at(const StepDev& S, long long sub, long long stop) {
@@ -310,7 +311,9 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
   int* sc = reinterpret_cast<int*>(part + 2 * F::C * M::W);
   short* own = reinterpret_cast<short*>(sc + F::N1 + F::N2);       // first snapshot entry of a thread, -1: none
   short* next = own + F::nth;                                     // next entry of the same thread
-  int* flags = reinterpret_cast<int*>(next + kLineSnap + 16);      // [1] last sub-step of a converged run, counted from the launch's first
+  // [1] last sub-step of a converged run, counted from the launch's first; [2] the power of
+  // two psi takes at the end of the first sub-step after a step
+  int* flags = reinterpret_cast<int*>(next + kLineSnap + 16);
   int4* xat = reinterpret_cast<int4*>((reinterpret_cast<unsigned long long>(flags + 4) + 15) & ~15ull);
   int4* xbt = xat + (BS ? F::nth * E : 0);
   long long* vt = reinterpret_cast<long long*>(xbt + F::nth * E);
@@ -328,7 +331,7 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
     const int two = line_two(S);
     double cfac = S.scale[2] * pow2(-2 * two), energy = S.energy_state[0];
     long long step = sub0 / K;
-    int k = (int)(sub0 % K), par = 0;
+    int k = (int)(sub0 % K), par = 0, due = 0;  // due: the power of two psi takes in this sub-step
     bool pending = false, pek = false, stopped = false;
     long long psub = 0;
     cl_sync<F::C>();
@@ -343,6 +346,10 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
           __syncwarp();
           if (lane == 0) S.ctl[1] = psub + K;
         }
+        if (S.normalize) {
+          due = line_two(cfac);
+          for (int r = lane; r < F::C; r += 32) put4<F::C>(flags + 2, r, due);
+        }
       }
       ++step;
       pending = false;
@@ -352,6 +359,8 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
       cl_sync<F::C>();
       if (pending) finish();
       for (int i = 1; i < kb; ++i) cl_sync<F::C>();
+      cfac *= pow2(-2 * due);
+      due = 0;
       const long long stop = min(stop_at, sub0 + (long long)*(volatile int*)(flags + 1));
       const bool end = ++k == K;
       const bool ek = end && line_ekin_at(S, sub, stop);
@@ -452,7 +461,7 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
   };
   int scale = open(sub0 - t0, line_two(S));
   const int l2m = S.l2m, vexp = 111 - S.vshift;
-  const bool any_ek = S.obs & 4u;
+  const bool any_ek = S.obs & 4u, normalize = S.normalize;
   double2* const snap = S.snap;
   const int* const texp = D.texp;
   const int4* const ptab = D.ptab;
@@ -489,8 +498,9 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
       for (int s = 0; s < E; ++s) v[s] = shl_by(fmul_tw(v[s], __ldg(c + s * sstr)), 2);
       scale -= ce;
     }
+    // the step-ending warp has set this and the stop, if any, before the sub-step's last barrier
+    if (normalize && k == 0 && sub > sub0) scale -= *(volatile int*)(flags + 2);
     const bool end = ++k == K;
-    // the step-ending warp has set the stop, if any, before the sub-step's last barrier
     const long long stop = min(stop_at, sub0 + (long long)*(volatile int*)(flags + 1));
     const bool ek = any_ek && end && line_ekin_at(S, sub, stop);
     const bool last = sub + 1 >= sub1 || sub >= stop;

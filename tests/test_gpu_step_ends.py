@@ -53,3 +53,29 @@ def test_substeps_under_normalize_match_one_step_per_call(dim, n):
         np.testing.assert_allclose(got[:, :2], each[:, :2], rtol=4 * 2e-13, atol=0)
         assert np.linalg.norm(g.download() - ref) < 2e-13 * np.linalg.norm(ref)
     g.close()
+
+
+@pytest.mark.parametrize("n", [96, 1536, 1021])
+@pytest.mark.parametrize("substeps", [1, 3])
+def test_line_normalize_keeps_psi_in_range(n, substeps):
+    """300 large imaginary-time steps in one call: the raw norm grows by exp(2 |E| dt), about
+    18, a step, past the range of a double within the 256 sub-steps of a launch.  Against
+    calls of one step; the bound is that of the oracle comparison of these lines."""
+    import math
+
+    import qsf_gb300 as Q
+    steps, dt = 300, 1.0
+    psi0 = _noise_state(1, n, 0.2, n)
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT, normalize=True, substeps=substeps)
+    g = Q.Grid(1, n, 0.2, nCAP=n // 10, Ncharge=2.0)
+    g.upload(psi0)
+    got, done = g.step(Q.MODE_IM, dt, steps, **kw)
+    psi = g.download()
+    assert done == steps
+    g.upload(psi0)
+    each = np.concatenate([g.step(Q.MODE_IM, dt, 1, **kw)[0] for _ in range(steps)])
+    assert np.prod(each[-256:, 0], dtype=np.longdouble) > np.finfo(np.float64).max
+    tol = steps * substeps * (2 * math.log2(n) + 10) * 2.2e-16
+    np.testing.assert_allclose(got[:, :2], each[:, :2], rtol=4 * tol, atol=0)
+    assert np.linalg.norm(psi - g.download()) < tol * np.linalg.norm(psi)
+    g.close()
