@@ -130,11 +130,6 @@ int grid_blocks(long long m) {
   return (int)std::min<long long>(std::max<long long>(b, 1), (long long)device_sm_count() * 16);
 }
 
-// blocks of the elementwise member kernels: a point per thread (grid_blocks gives 1024^2
-// points two each to some threads and one to the rest; 4 regions of 1024^2, 44 steps, with
-// the tables of k_evolve_ptab on more SMs: 24.56 -> 24.47 ms)
-unsigned point_blocks(long long m) { return (unsigned)std::min<long long>(std::max<long long>((m + 255) / 256, 1), 1LL << 30); }
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against the
 // driver library); null when the driver does not offer it
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1306,7 +1301,7 @@ int qsf_region_transfer(qsf_grid* dst, const qsf_grid* src, int axis, int group)
   // boxes of nCAP planes along the sliding axis (multigrid.h:184, 296-317): n / nCAP of them
   const long long slide_lim = G.dim == 3 ? (G.ax[0].n / G.nCAP) * G.nCAP : 0;
   if (int rc = ensure_mtab(dst)) return rc;
-  k_mg_slice<<<point_blocks(G.m), 256, 0, dst->stream>>>(G, H.psi, dst->mg_slice, axis, group, slide_lim, dst->mtab,
+  k_mg_slice<<<grid_blocks(G.m), 256, 0, dst->stream>>>(G, H.psi, dst->mg_slice, axis, group, slide_lim, dst->mtab,
                                                         dst->nmax);
   GridDev Gs = G;
   Gs.psi = dst->mg_slice;
@@ -1314,7 +1309,7 @@ int qsf_region_transfer(qsf_grid* dst, const qsf_grid* src, int axis, int group)
     if (int rc = line_fourier(dst, Gs, true, 1.0)) return rc;
   } else if (dst->ks) axis_fft(dst, Gs, axis, true, 1.0);
   else if (int rc = bs_axis(dst, dst->mg_slice, axis, true, 1.0)) return rc;
-  k_add_slice<<<point_blocks(G.m), 256, 0, dst->stream>>>(G.psi, dst->mg_slice, G.m);
+  k_add_slice<<<grid_blocks(G.m), 256, 0, dst->stream>>>(G.psi, dst->mg_slice, G.m);
   QSF_CU(cudaGetLastError());
   QSF_CU(cudaEventRecord(dst->mg_event, dst->stream));
   QSF_CU(cudaStreamWaitEvent(s->stream, dst->mg_event, 0));
@@ -1349,14 +1344,13 @@ int qsf_evolve(qsf_grid* g, int mode, int rep, double delta, const double* c3) {
   const GridDev& G = g->G;
   if (rep == QSF_REP_X && !(G.gauge == QSF_GAUGE_LENGTH && G.n_fields)) {
     if (int rc = ensure_xtab(g, mode, delta)) return rc;
-    k_apply_xtab<<<point_blocks(G.m), 256, 0, g->stream>>>(G.psi, g->etab, G.m);
+    k_apply_xtab<<<grid_blocks(G.m), 256, 0, g->stream>>>(G.psi, g->etab, G.m);
   } else if (rep == QSF_REP_P) {
     if (!g->eptab)
       if (int rc = dev_alloc(g->eptab, (size_t)3 * g->nmax)) return rc;
-    // one warp per block: an SM issues an FP64 instruction of a warp every 16 clocks
-    k_evolve_ptab<<<(G.dim * g->nmax + 31) / 32, 32, 0, g->stream>>>(G, mode, delta, c0, c1, c2, g->nmax,
+    k_evolve_ptab<<<(G.dim * g->nmax + 255) / 256, 256, 0, g->stream>>>(G, mode, delta, c0, c1, c2, g->nmax,
                                                                         g->eptab);
-    k_apply_ptab<<<point_blocks(G.m), 256, 0, g->stream>>>(G, g->eptab, g->nmax);
+    k_apply_ptab<<<grid_blocks(G.m), 256, 0, g->stream>>>(G, g->eptab, g->nmax);
   } else {
     k_evolve<<<grid_blocks(G.m), 256, 0, g->stream>>>(G, mode, rep, delta, c0, c1, c2);
   }
@@ -1460,7 +1454,7 @@ int qsf_mask_region(qsf_grid* g, const int* b3) {
   if (!g || !b3) return fail(QSF_EINVAL, "null argument");
   if (g->G.nCAP <= 0) return QSF_OK;  // no absorber: the mask is 1 everywhere
   if (int rc = ensure_mtab(g)) return rc;
-  k_mask<<<point_blocks(g->G.m), 256, 0, g->stream>>>(g->G, b3[0], g->G.dim > 1 ? b3[1] : 1, g->G.dim > 2 ? b3[2] : 1,
+  k_mask<<<grid_blocks(g->G.m), 256, 0, g->stream>>>(g->G, b3[0], g->G.dim > 1 ? b3[1] : 1, g->G.dim > 2 ? b3[2] : 1,
                                                      g->mtab, g->nmax);
   QSF_CU(cudaGetLastError());
   return QSF_OK;
