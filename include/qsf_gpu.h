@@ -208,7 +208,8 @@ int qsf_add_gaussian(qsf_grid* g, double at, double delta);
  * With normalize != 0 the step ends with OPERATION<Normalize> (grid.h:601-606).
  * In imaginary time with state_accuracy > 0 the run follows shouldContinue()
  * (propagator.h:304-309): after the first step whose |E_n - E_{n-1}| <= accuracy
- * exactly one more step runs and the call returns; *steps_done says how many ran.
+ * exactly one more step runs and the call returns; *steps_done says how many ran, and
+ * the rows after those are 0.
  * E_n = epot + ekin; bit 0 of energy_after_normalize divides epot, bit 1 divides ekin
  * by the step's norm (the observables declared after OPERATION<Normalize>).
  *

@@ -660,7 +660,7 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   const int cstride = G.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
   const bool short_rows = direct && d->nsteps * ncol <= CallBlock::kRows;
   if (!short_rows && (rc = dev_reserve(g->rows_dev, g->rows_cap, (size_t)d->nsteps * ncol))) return rc;
-  CallBlock h;
+  CallBlock h{};
   const double* coup = nullptr;
   const size_t nc = d->coupling ? (size_t)total * cstride : 0;
   if (nc > CallBlock::kCoup) {
@@ -757,6 +757,8 @@ int finish_step(qsf_grid* g, const StepDev& S, int normalize, int64_t nsteps, in
   QSF_CU(cudaMemcpyAsync(h.ctl, g->blk, bytes, cudaMemcpyDeviceToHost, g->stream));
   QSF_CU(cudaStreamSynchronize(g->stream));
   if (nr && short_rows) std::memcpy(rows, h.rows, nr * sizeof(double));
+  // a converged run's rows after its last step are 0, not what the memory held
+  if (nr) std::fill(rows + (size_t)h.ctl[2] * ncol, rows + nr, 0.0);
   if (steps_done) *steps_done = h.ctl[2];
   if (h.ctl[4] == 2) return fail(QSF_ETIMEDOUT, "a bulk copy into shared memory did not complete in time");
   if (h.ctl[4]) return fail(QSF_ENUMERIC, "non-positive norm or NaN in a step's reductions");

@@ -79,3 +79,23 @@ def test_line_normalize_keeps_psi_in_range(n, substeps):
     np.testing.assert_allclose(got[:, :2], each[:, :2], rtol=4 * tol, atol=0)
     assert np.linalg.norm(psi - g.download()) < tol * np.linalg.norm(psi)
     g.close()
+
+
+@pytest.mark.parametrize("dim,n", [(1, 96), (1, 1021), (2, 64), (2, 100)])
+@pytest.mark.parametrize("steps", [60, 200])
+def test_rows_after_a_converged_step_are_zero(dim, n, steps):
+    """Calls whose rows travel with the control words (up to 256 values) and longer ones.  A
+    full run goes before, so that the memory of the rows has held something."""
+    import qsf_gb300 as Q
+    psi0 = _noise_state(dim, n, 0.3, n)
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT | Q.OBS_EKIN, normalize=True, energy_after_normalize=3)
+    g = Q.Grid(dim, n, 0.3, nCAP=n // 10, Ncharge=float(dim))
+    g.upload(psi0)
+    full, done = g.step(Q.MODE_IM, 0.05, steps, **kw)
+    assert done == steps and full.all()
+    g.upload(psi0)
+    rows, done = g.step(Q.MODE_IM, 0.05, steps, state_accuracy=0.05, **kw)
+    assert 1 < done < steps
+    assert np.array_equal(rows[:done, :2], full[:done, :2])
+    assert not rows[done:].any()
+    g.close()
