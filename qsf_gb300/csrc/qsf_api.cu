@@ -637,8 +637,9 @@ int ensure_fin_stream(qsf_grid* g, FinOverlap* ov) {
 // Validates a step program and stages everything a run of it needs on the device:
 // static tables for dt/2, flux point lists, coupling rows, observables rows, control
 // words; fills the step descriptor and uploads it to g->dS.  `direct`: one call of its own
-// (qsf_step), whose rows stay in the grid's call block when they are few.
-int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_out, int64_t chunk = INT64_MAX,
+// (qsf_step), whose rows stay in the grid's call block when they are few.  `chunk`: sub-steps
+// whose tables 1D grids hold at a time (0: the program's).
+int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_out, int64_t chunk = 0,
                  bool direct = false) {
   if (d->mode != QSF_MODE_IM && d->mode != QSF_MODE_RE) return fail(QSF_EINVAL, "mode must be IM or RE");
   if (d->nsteps < 1) return fail(QSF_EINVAL, "nsteps < 1");
@@ -732,7 +733,7 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   S.energy_state = g->energy;
   S.rows = short_rows ? g->blk->rows : g->rows_dev;
   S.scale = g->scale;
-  if (G.dim == 1 && (rc = line_prepare(g, S, chunk))) return rc;
+  if (G.dim == 1 && (rc = line_prepare(g, S, chunk > 0 ? chunk : S.nsteps))) return rc;
   h.S = S;
   const size_t bytes = offsetof(CallBlock, coupling) + (nc <= CallBlock::kCoup ? nc * sizeof(double) : 0);
   QSF_CU(cudaMemcpyAsync(g->blk, &h, bytes, cudaMemcpyHostToDevice, g->stream));
@@ -1501,7 +1502,7 @@ int qsf_step(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t* steps_d
   if (d->nsteps == 0) return QSF_OK;
   StepDev S{};
   int ncol = 0, rc;
-  if ((rc = prepare_step(g, d, &S, &ncol, INT64_MAX, true))) return rc;
+  if ((rc = prepare_step(g, d, &S, &ncol, 0, true))) return rc;
   if (g->G.dim == 1) {
     if ((rc = line_run(g, S, S.nsteps, d->kernel_ms, d->kernel_launches))) return rc;
     return finish_step(g, S, d->normalize, d->nsteps, ncol, rows, steps_done);
@@ -1537,9 +1538,9 @@ int qsf::grid_clear(qsf_grid* g) {
 
 // A solve that runs on its own stream beside a batch (1D lines, and grids whose lines are
 // convolutions): everything a program needs, staged.
-int qsf::solo_begin(qsf_grid* g, const qsf_step_desc* d) {
+int qsf::solo_begin(qsf_grid* g, const qsf_step_desc* d, int64_t round) {
   int ncol = 0, rc;
-  if ((rc = prepare_step(g, d, &g->solo, &ncol))) return rc;
+  if ((rc = prepare_step(g, d, &g->solo, &ncol, round * std::max(1, d->substeps)))) return rc;
   QSF_CU(cudaMemsetAsync(g->rows_dev, 0, (size_t)d->nsteps * ncol * sizeof(double), g->stream));
   // the descriptors come from this frame's memory
   QSF_CU(cudaStreamSynchronize(g->stream));

@@ -200,8 +200,8 @@ int grid_clear(qsf_grid* g);
 // parts for the server: begin checks the program and zeroes its device rows and
 // NaN flag; enqueue queues steps [first, first + count) on the grid's stream without
 // waiting (no convergence test); wait waits for the stream and reads the NaN flag;
-// rows copies the first nsteps rows to the host.
-int solo_begin(qsf_grid* g, const qsf_step_desc* d);
+// rows copies the first nsteps rows to the host.  round: steps queued at a time at most.
+int solo_begin(qsf_grid* g, const qsf_step_desc* d, int64_t round);
 int solo_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
 int solo_wait(qsf_grid* g, bool* bad);
 int solo_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps);
@@ -227,6 +227,7 @@ int line_conv_length(int n);  // convolution length of an n-point line (0: none)
 int line_setup(qsf_grid* g);
 void line_release(qsf_grid* g);
 int line_prepare(qsf_grid* g, StepDev& S, int64_t chunk);
+size_t line_table_bytes(int n, bool field, bool lg, int64_t chunk);
 int line_launch_tables(const LineKernels& L, const GridDev* dG, const StepDev* dS, int count, int steps, bool lg,
                        cudaStream_t st);
 int line_launch_steps(const LineKernels& L, bool bs, const GridDev* dG, const StepDev* dS, int count, int steps,

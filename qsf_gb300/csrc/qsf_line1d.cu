@@ -174,6 +174,19 @@ int shared_turns(const LineKernels& L, const int4** w1, const int4** w2) {
 constexpr int kLineSteps = 256;              // sub-steps of one launch at most
 constexpr size_t kLineTableBytes = 48 << 20;  // bytes of their tables at most (at least 16 sub-steps)
 
+// the tables of a run made `chunk` sub-steps at a time: sub-steps they hold, entries (vg, lg:
+// a velocity- or a length-gauge field couples)
+struct LineTables {
+  int64_t steps;
+  size_t ptab, ctab, texp;
+};
+LineTables line_tables(const LineKernels& L, bool vg, bool lg, int64_t chunk) {
+  const size_t slots = (size_t)L.ctas * L.nth * L.epp, per = slots * sizeof(int4) * (lg ? 2 : 1);
+  const int64_t fit = std::min<int64_t>(std::max<int64_t>(16, (int64_t)(kLineTableBytes / per)), kLineSteps);
+  const int64_t steps = std::max<int64_t>(1, std::min(fit, chunk));
+  return {steps, slots * (vg ? (size_t)steps : 1), lg ? slots * (size_t)(2 * steps + 1) : 0, (size_t)(steps + 1) * 3};
+}
+
 }  // namespace
 
 const LineKernels* line_kernels(int n) {
@@ -260,22 +273,27 @@ void line_release(qsf_grid* g) {
     if (p) cudaFree(p);
 }
 
-// the tables a program of `total` sub-steps runs on, `chunk` sub-steps at a time, into S.line
+// device bytes of the tables of n-point lines whose runs are made `chunk` sub-steps at a time
+size_t line_table_bytes(int n, bool field, bool lg, int64_t chunk) {
+  const LineKernels* L = fused_length(n) ? line_kernels(n) : line_kernels(line_conv_length(n));
+  if (!L) return 0;
+  const LineTables t = line_tables(*L, field && !lg, field && lg, chunk);
+  return (t.ptab + t.ctab) * sizeof(int4) + t.texp * sizeof(int);
+}
+
+// the tables a program runs on, `chunk` sub-steps at a time, into S.line
 int line_prepare(qsf_grid* g, StepDev& S, int64_t chunk) {
   const LineKernels& L = *g->lk;
   LineDev D = g->line;
   const size_t slots = (size_t)L.ctas * L.nth * L.epp;
-  const bool lg = g->G.gauge == QSF_GAUGE_LENGTH && g->G.n_fields && S.coupling;
-  const bool vg = g->G.gauge != QSF_GAUGE_LENGTH && g->G.n_fields && S.coupling;
-  const size_t per = slots * sizeof(int4) * (lg ? 2 : 1);
-  int64_t steps = std::min<int64_t>(std::max<int64_t>(16, (int64_t)(kLineTableBytes / per)), kLineSteps);
-  steps = std::max<int64_t>(1, std::min({steps, chunk, (int64_t)S.nsteps}));
+  const bool field = g->G.n_fields && S.coupling, lg = field && g->G.gauge == QSF_GAUGE_LENGTH, vg = field && !lg;
+  const LineTables t = line_tables(L, vg, lg, chunk);
+  const int64_t steps = t.steps;
   g->l_steps = (int)steps;
   int rc;
-  if ((rc = dev_reserve(g->l_ptab, g->l_ptab_cap, slots * (vg ? (size_t)steps : 1))) ||
-      (rc = dev_reserve(g->l_texp, g->l_texp_cap, (size_t)(steps + 1) * 3)))
+  if ((rc = dev_reserve(g->l_ptab, g->l_ptab_cap, t.ptab)) || (rc = dev_reserve(g->l_texp, g->l_texp_cap, t.texp)))
     return rc;
-  if (lg && (rc = dev_reserve(g->l_ctab, g->l_ctab_cap, slots * (size_t)(2 * steps + 1)))) return rc;
+  if (lg && (rc = dev_reserve(g->l_ctab, g->l_ctab_cap, t.ctab))) return rc;
   D.ptab = g->l_ptab;
   D.pstride = vg ? (long long)slots : 0;
   D.ctab = g->l_ctab;

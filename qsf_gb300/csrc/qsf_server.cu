@@ -28,8 +28,9 @@ int batch_launch(qsf_batch* b, int64_t steps);
 int batch_finish(qsf_batch* b, int64_t* active);
 bool fused_length(int n);
 int bs_size(int n, int dim);
+size_t line_table_bytes(int n, bool field, bool lg, int64_t chunk);
 bool grid_batched(const qsf_grid* g);
-int solo_begin(qsf_grid* g, const qsf_step_desc* d);
+int solo_begin(qsf_grid* g, const qsf_step_desc* d, int64_t round);
 int solo_enqueue(qsf_grid* g, const qsf_step_desc* d, int64_t first, int64_t count);
 int solo_wait(qsf_grid* g, bool* bad);
 int solo_rows(qsf_grid* g, const qsf_step_desc* d, double* rows, int64_t nsteps);
@@ -75,15 +76,22 @@ int64_t grid_points(const qsf_grid_desc& d) {
   return m;
 }
 
-// device bytes a solve holds: psi, static X factor and potential, observables rows,
-// coupling rows, plus small tables
-size_t solve_bytes(const qsf_request& r) {
-  const int64_t m = grid_points(r.grid);
-  const int stride = r.grid.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
-  size_t b = (size_t)m * (16 + 16 + 8) + (size_t)r.nsteps * (size_t)(3 + r.nborders + stride) * 8 + (1u << 20);
+// device bytes a grid keeps from one solve to the next: psi, static X factor and potential,
+// the tables of a round's steps (1D; 2D and 3D: 16 steps at a time, line exponents and sums)
+size_t grid_bytes(const qsf_grid_desc& d, int64_t round) {
+  const int64_t m = grid_points(d), n = d.n[0];
+  const bool lg = d.gauge == QSF_GAUGE_LENGTH;
+  const size_t tables = d.dim == 1 ? qsf::line_table_bytes((int)n, d.n_fields > 0, lg, round)
+                                   : (size_t)16 * d.dim * n * 16 * (lg ? 4 : 1) + (size_t)(m / n) * (4 * 4 + 5 * 8);
   // Bluestein lengths: the convolution scratch (up to 4 m points)
-  if (!qsf::fused_length((int)r.grid.n[0])) b += (size_t)m * 16 * 6;
-  return b;
+  const size_t conv = qsf::fused_length((int)n) ? 0 : (size_t)m * 16 * 6;
+  return (size_t)m * (16 + 16 + 8) + tables + conv;
+}
+
+// device bytes a solve holds: its grid, observables rows, coupling rows, plus small tables
+size_t solve_bytes(const qsf_request& r, int64_t round) {
+  const int stride = r.grid.gauge == QSF_GAUGE_LENGTH ? 6 : 3;
+  return grid_bytes(r.grid, round) + (size_t)r.nsteps * (size_t)(3 + r.nborders + stride) * 8 + (1u << 20);
 }
 
 }  // namespace
@@ -144,11 +152,7 @@ bool same_grid(const qsf_grid_desc& a, const qsf_grid_desc& b) {
 
 size_t pooled_bytes(const qsf_server* s) {
   size_t b = 0;
-  for (const auto& e : s->pool) {
-    int64_t m = 1;
-    for (int k = 0; k < e.first.dim; ++k) m *= e.first.n[k];
-    b += (size_t)m * (16 + 16 + 8);
-  }
+  for (const auto& e : s->pool) b += grid_bytes(e.first, s->cfg.steps_per_round);
   return b;
 }
 
@@ -271,7 +275,7 @@ int admit(qsf_server* s, Pending& p, Running& r, bool nowait) {
   if (!qsf::grid_batched(g)) {
     r.solo = true;
     r.d = d;
-    rc = qsf::solo_begin(g, &r.d);
+    rc = qsf::solo_begin(g, &r.d, s->cfg.steps_per_round);
   } else {
     rc = nowait ? qsf::batch_add_nowait(s->batch, g, &d, &r.slot) : qsf_batch_add(s->batch, g, &d, &r.slot);
   }
@@ -305,7 +309,7 @@ void worker_loop(qsf_server* s) {
       double budget = (double)free_b - reserve + (double)pooled_bytes(s);  // pooled grids can be freed
       const double capacity = (double)total_b - reserve;  // what an otherwise empty device could give
       while (!s->queue.empty() && (int)(s->running.size() + take.size()) < s->cfg.max_slots) {
-        const double need = (double)solve_bytes(s->queue.front().req);
+        const double need = (double)solve_bytes(s->queue.front().req, s->cfg.steps_per_round);
         if (need > capacity) {  // can never be admitted: finish it now, do not block the queue
           Pending p = std::move(s->queue.front());
           s->queue.pop_front();
