@@ -212,32 +212,28 @@ void qsf::launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd
 
 bool qsf::fused_length(int n) { return init_kernel_table() == QSF_OK && kernels_for(n) != nullptr; }
 
-// exp(-2 pi i t / n) 2^-r in the split form of the kernels (2^62 fixed point, the signed
-// 32-bit halves of each component; a component whose low half would be -2^31 moves one
-// unit, 2^-62, so that the kernels can negate the halves).  The angle is reduced to the
-// first octant.
-int4 qsf::split_root(long long t, long long n, int r) {
-  t %= n;
-  long double c, s;
-  const long long o = 8 * t / n;  // octant
-  const long double a = 6.283185307179586476925286766559005768L;
-  // distance to the octant's axis, as a fraction of n / 8 turns
-  auto base = [&](long long num) { return a * (long double)num / (8.0L * (long double)n); };
-  switch (o) {
-    case 0: c = cosl(base(8 * t)); s = sinl(base(8 * t)); break;
-    case 1: c = sinl(base(2 * n - 8 * t)); s = cosl(base(2 * n - 8 * t)); break;
-    case 2: c = -sinl(base(8 * t - 2 * n)); s = cosl(base(8 * t - 2 * n)); break;
-    case 3: c = -cosl(base(4 * n - 8 * t)); s = sinl(base(4 * n - 8 * t)); break;
-    case 4: c = -cosl(base(8 * t - 4 * n)); s = -sinl(base(8 * t - 4 * n)); break;
-    case 5: c = -sinl(base(6 * n - 8 * t)); s = -cosl(base(6 * n - 8 * t)); break;
-    case 6: c = sinl(base(8 * t - 6 * n)); s = -cosl(base(8 * t - 6 * n)); break;
-    default: c = cosl(base(8 * n - 8 * t)); s = -sinl(base(8 * n - 8 * t)); break;
+qsf::Roots::Roots(long long len) : n(len) {
+  // a microsecond each where long double is software
+  for (long long t = 0; 8 * t <= n; ++t) {
+    const long double a = 6.283185307179586476925286766559005768L * (long double)t / (long double)n;
+    cs.push_back({cosl(a), sinl(a)});
   }
+}
+int4 qsf::Roots::split(long long t, int r) const {
+  t %= n;
+  const long long q = n / 4;
+  // the octant, and the angle's distance to its axis
+  const long long o = 8 * t / n, d = o == 0 ? t : o < 3 ? std::llabs(q - t) : o < 5 ? std::llabs(2 * q - t)
+                                   : o < 7 ? std::llabs(3 * q - t) : n - t;
+  long double c = cs[(size_t)d].first, s = cs[(size_t)d].second;
+  if ((o + 1) / 2 % 2) std::swap(c, s);  // next to the imaginary axis
+  if (o > 1 && o < 6) c = -c;
+  if (o > 3) s = -s;
   const long double one = ldexpl(1.0L, 62 - r);
-  long long q[2] = {llroundl(c * one), llroundl(-s * one)};
-  for (long long& v : q)
+  long long w[2] = {llroundl(c * one), llroundl(-s * one)};
+  for (long long& v : w)
     if ((v & 0xffffffffLL) == 0x80000000LL) v += 1;
-  return make_int4(k_lo(q[0]), k_hi(q[0]), k_lo(q[1]), k_hi(q[1]));
+  return make_int4(k_lo(w[0]), k_hi(w[0]), k_lo(w[1]), k_hi(w[1]));
 }
 
 // Per-pass twiddles of a line plan (qsf_lines.cuh): kTwVar copies, copy r scaled by 2^-r;
@@ -255,14 +251,15 @@ int qsf::shared_line_twiddles(int n, int ppt, const int4** out) {
   auto it = cache.find({dev, n, ppt});
   if (it == cache.end()) {
     std::vector<int4> h;
+    const Roots root(n);
     if (ppt == kPlain)
-      for (int t = 0; t < n; ++t) h.push_back(split_root(t, n, 0));
+      for (int t = 0; t < n; ++t) h.push_back(root.split(t));
     for (int r = 0; r < kTwVar && P.S; ++r) {
       long long ns = P.r[0];
       for (int p = 1; p < P.S; ++p) {
         const int R = P.r[p];
         for (int q = 1; q < R; ++q)
-          for (long long jm = 0; jm < ns; ++jm) h.push_back(split_root(jm * q, ns * R, r));
+          for (long long jm = 0; jm < ns; ++jm) h.push_back(root.split(jm * q * (n / (ns * R)), r));
         ns *= R;
       }
     }
@@ -281,13 +278,14 @@ int qsf::shared_line_twiddles(int n, int ppt, const int4** out) {
   return QSF_OK;
 }
 
-// the twiddles of a built length (none above 8192 points): both line plans' and the plain
-// transforms'
-int qsf::axis_twiddles(int n, AxisDev* a) {
+// the twiddles of a built length (none above 8192 points): the plain transforms' and, for the
+// passes of 2D and 3D grids, both line plans'
+int qsf::axis_twiddles(int n, bool passes, AxisDev* a) {
   a->tw = a->twl[0] = a->twl[1] = nullptr;
   if (n > 8192) return QSF_OK;
   int rc;
-  if ((rc = shared_line_twiddles(n, 8, &a->twl[0])) || (rc = shared_line_twiddles(n, 16, &a->twl[1]))) return rc;
+  if (passes && ((rc = shared_line_twiddles(n, 8, &a->twl[0])) || (rc = shared_line_twiddles(n, 16, &a->twl[1]))))
+    return rc;
   return shared_line_twiddles(n, kPlain, &a->tw);
 }
 
@@ -1073,7 +1071,7 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   }
   if (ks) {
     for (int k = 0; k < d->dim; ++k)
-      if (int rc = axis_twiddles(G.ax[k].n, &G.ax[k])) {
+      if (int rc = axis_twiddles(G.ax[k].n, d->dim > 1, &G.ax[k])) {
         qsf_grid_destroy(g);
         return rc;
       }

@@ -150,7 +150,7 @@ int bs_setup(qsf_grid* g) {
   b.M = M;
   b.ks = kernels_for(M);
   int rc;
-  if ((rc = axis_twiddles(M, &b.ax))) return rc;
+  if ((rc = axis_twiddles(M, true, &b.ax))) return rc;
   const size_t scr = (size_t)(G.m / n) * (size_t)M;
   if ((rc = dev_alloc(b.chirp, (size_t)n)) || (rc = dev_alloc(b.bhat, (size_t)M)) ||
       (rc = dev_alloc(b.scratch, std::max(scr, (size_t)M))))

@@ -4,6 +4,7 @@
 #pragma once
 #include <algorithm>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -213,13 +214,23 @@ int batch_add_nowait(qsf_batch* b, qsf_grid* g, const qsf_step_desc* d, int64_t*
 // steps' graph launches) and finish (wait, read every member's counters)
 int batch_launch(qsf_batch* b, int64_t steps);
 int batch_finish(qsf_batch* b, int64_t* active);
-// exp(-2 pi i t / n) 2^-r in the split form of the kernels
-int4 split_root(long long t, long long n, int r);
+// exp(-2 pi i t / n), n a multiple of 4, from the angles of one octant, evaluated once
+class Roots {
+  long long n;
+  std::vector<std::pair<long double, long double>> cs;
+
+ public:
+  explicit Roots(long long n);
+  // times 2^-r, in the split form of the kernels: 2^62 fixed point, the signed 32-bit halves
+  // of each component; a component whose low half would be -2^31 moves one unit, 2^-62, so
+  // that the kernels can negate the halves
+  int4 split(long long t, int r = 0) const;
+};
 // device twiddles of the line plan (n, ppt), and all of a built length; shared
 // by all grids of the process (not to be freed by the caller)
 int shared_line_twiddles(int n, int ppt, const int4** out);
 constexpr int kPlain = 0;  // selects the plain transforms' twiddles
-int axis_twiddles(int n, AxisDev* a);
+int axis_twiddles(int n, bool passes, AxisDev* a);
 void launch_axis_fft(const KernelSet& K, const GridDev& G, int ax, bool fwd, double sc, cudaStream_t st);
 // 1D grids (qsf_line1d.cu)
 int init_line_table();

@@ -148,11 +148,12 @@ int shared_turns(const LineKernels& L, const int4** w1, const int4** w2) {
   auto it = cache.find({dev, L.n});
   if (it == cache.end()) {
     const int N = L.n;
-    std::vector<int4> h((size_t)2 * N), root((size_t)N);
-    for (int t = 0; t < N; ++t) root[(size_t)t] = split_root(t, N, 0);
+    std::vector<int4> h((size_t)2 * N), turn((size_t)N);
+    const Roots root(N);
+    for (int t = 0; t < N; ++t) turn[(size_t)t] = root.split(t);
     for (int a = 0; a < L.n1; ++a)
       for (int b = 0; b < L.n2; ++b) {
-        const int4 w = root[(size_t)((long long)a * b % N)];
+        const int4 w = turn[(size_t)((long long)a * b % N)];
         h[(size_t)b * L.n1 + a] = w;
         h[(size_t)N + (size_t)a * L.n2 + b] = w;
       }
