@@ -99,3 +99,65 @@ def test_rows_after_a_converged_step_are_zero(dim, n, steps):
     assert np.array_equal(rows[:done, :2], full[:done, :2])
     assert not rows[done:].any()
     g.close()
+
+
+@pytest.mark.parametrize("dim,n", [(1, 96), (1, 1536), (1, 1021), (2, 64), (2, 100)])
+@pytest.mark.parametrize("substeps,every,accuracy", [(1, 1, 0.05), (1, 1, 1e-4), (3, 1, 0.05), (1, 7, 0.05), (2, 4, 1e-3),
+                                                     (1, 0, 0.02)])
+def test_convergence_stop(dim, n, substeps, every, accuracy):
+    """The stop comes after the first step whose energy (with E_kin every so often: among the
+    steps that have it) is within the accuracy of the one before, one step later; that last
+    step has E_kin, and psi is that of a call of as many steps.  every = 0: no E_kin."""
+    import qsf_gb300 as Q
+    steps, dt = 400, 0.05
+    psi0 = _noise_state(dim, n, 0.3, n)
+    kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT | (Q.OBS_EKIN if every else 0), normalize=True, energy_after_normalize=3,
+              substeps=substeps, ekin_interval=max(every, 1))
+    g = Q.Grid(dim, n, 0.3, nCAP=n // 10, Ncharge=float(dim))
+    g.upload(psi0)
+    full, _ = g.step(Q.MODE_IM, dt, steps, **kw)
+    energy = (full[:, 1] + full[:, 2]) / full[:, 0]
+    at = [s for s in range(steps) if every == 0 or (s + 1) % every == 0]
+    last = next(s for before, s in zip([None] + at, at)
+                if abs(energy[s] - (energy[before] if before is not None else 0.0)) <= accuracy) + 1
+    assert 1 < last < steps - 1
+    g.upload(psi0)
+    rows, done = g.step(Q.MODE_IM, dt, steps, state_accuracy=accuracy, **kw)
+    psi = g.download()
+    assert done == last + 1
+    assert np.array_equal(rows[:last], full[:last])
+    g.upload(psi0)
+    ref, _ = g.step(Q.MODE_IM, dt, done, **kw)
+    assert np.array_equal(rows[:done], ref) and np.array_equal(psi, g.download())
+    assert every == 0 or rows[last, 2] > 0
+    g.close()
+
+
+def test_batch_with_normalize_and_ekin_matches_alone():
+    """Imaginary-time members, E_kin every step or every few, several groups, and a batch that
+    advances in runs that end inside a member's period: the bits of each solve run alone."""
+    import qsf_gb300 as Q
+    specs = [(2, 48, 1, 60), (2, 64, 3, 50), (2, 64, 1, 40), (2, 128, 0, 45), (1, 256, 4, 60), (1, 1536, 1, 33),
+             (3, 16, 5, 50), (3, 32, 0, 20)]
+    made, alone = [], []
+    for dim, n, every, steps in specs:
+        nodes = (25, 14, 10, 40) if dim == 1 or n == 128 else (6, 4, 3, 12)
+        psi0 = _noise_state(dim, n, 0.3, n + steps)
+        g = Q.Grid(dim, n, 0.3, nCAP=n // 10, Ncharge=float(dim), border_nodes=nodes)
+        kw = dict(obs=Q.OBS_NORM | Q.OBS_EPOT | (Q.OBS_EKIN if every else 0), normalize=True, ekin_interval=max(every, 1),
+                  borders=[] if dim == 1 else Q.ZOA_FLUX_2D if dim == 2 else Q.ZOA_FLUX_3D)
+        g.upload(psi0)
+        rows, _ = g.step(Q.MODE_IM, 0.05, steps, **kw)
+        alone.append((rows, g.download()))
+        g.upload(psi0)
+        made.append((g, steps, kw))
+    b = Q.Batch()
+    slots = [b.add(g, Q.MODE_IM, 0.05, steps, **kw) for g, steps, kw in made]
+    while b.run(11):
+        pass
+    for (g, steps, _), slot, (rows, psi) in zip(made, slots, alone):
+        got, done = b.result(slot)
+        assert done == steps and np.array_equal(got, rows)
+        b.remove(slot)
+        assert np.array_equal(g.download(), psi)
+    b.close()
