@@ -288,6 +288,8 @@ int line_prepare(qsf_grid* g, StepDev& S, int64_t chunk) {
   LineDev D = g->line;
   const size_t slots = (size_t)L.ctas * L.nth * L.epp;
   const bool field = g->G.n_fields && S.coupling, lg = field && g->G.gauge == QSF_GAUGE_LENGTH, vg = field && !lg;
+  // (BOX, the one border of a line, needs six)
+  if (S.row_ptr && S.nsnap > kLineSnap) return fail(QSF_EINVAL, "too many border points on a 1D line");
   const LineTables t = line_tables(L, vg, lg, chunk);
   const int64_t steps = t.steps;
   g->l_steps = (int)steps;

@@ -3,8 +3,9 @@
 // A 1D line is one small transform after another, so what bounds a step is latency: the
 // chain of passes, exchanges and launches, not any pipe.  k_line_run therefore keeps psi
 // in registers over all the sub-steps of a launch and spreads a line over the CTAs of a
-// cluster, one warp per scheduler or so.  Short lines (below 256 points, and 320) sit in one CTA as
-// one line of qsf_lines.cuh.  Longer ones are N = N1 x N2 with 8 points per thread:
+// cluster, one warp per scheduler or so.  Short lines (below 256 points, and 320) sit in one
+// CTA as one line of qsf_lines.cuh.  Longer ones are N = N1 x N2 with 4 points per thread,
+// 8 above 12288:
 //   X layout  thread (column n2, t1) holds x[N2 (t1 + s T1) + n2]
 //   K layout  thread (row k1, t2) holds X[k1 + N1 (t2 + s T2)]
 // The transform is N1-point lines along the columns, twiddles exp(-2 pi i k1 n2 / N), one
@@ -19,7 +20,8 @@
 // part of the static factors.
 //
 // psi is rounded to complex128 at the end of every step, in registers, as it would be in
-// memory: a run does not depend on how it is cut into launches, calls or backups.
+// memory: a run does not depend on how it is cut into launches, and without Normalize not
+// on how it is cut into calls or by backups either (each call's end applies its factor).
 //
 // One extra warp of CTA 0 ends the steps (sums, fluxes, the observables row, the
 // Normalize factor, the convergence test) while the others work on the next one.  The
@@ -290,7 +292,7 @@ __device__ __forceinline__ bool line_ekin_at(const StepDev& S, long long sub, lo
   return (sub / S.substeps + 1) % S.ekin_every == 0 || sub + 1 >= S.nsteps || sub >= stop;
 }
 
-constexpr int kLineSnap = 256;  // snapshot entries with a place in shared memory
+constexpr int kLineSnap = 256;  // snapshot entries a 1D program may have (their lists are in shared memory)
 
 template <class F, bool BS>
 __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
@@ -309,8 +311,7 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
   unsigned(*slot)[32] = reinterpret_cast<unsigned(*)[32]>(rest);
   WarpSum* part = reinterpret_cast<WarpSum*>(rest + 256);  // [2][C W], CTA 0's are written
   int* sc = reinterpret_cast<int*>(part + 2 * F::C * M::W);
-  short* own = reinterpret_cast<short*>(sc + F::N1 + F::N2);       // first snapshot entry of a thread, -1: none
-  short* next = own + F::nth;                                     // next entry of the same thread
+  short* next = reinterpret_cast<short*>(sc + F::N1 + F::N2);      // next snapshot entry of the same thread
   // [1] last sub-step of a converged run, counted from the launch's first; [2] the power of
   // two psi takes at the end of the first sub-step after a step
   int* flags = reinterpret_cast<int*>(next + kLineSnap + 16);
@@ -430,11 +431,10 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
 #pragma unroll
     for (int s = 0; s < E; ++s)
       if ((valid >> s & 1) && en.xi(s) == i) {
-        if (e < kLineSnap) next[e] = (short)mine;
+        next[e] = (short)mine;
         mine = e;
       }
   }
-  own[tid] = (short)mine;
   cl_sync<F::C>();  // every CTA of the cluster runs and has its flags set
   longlong2 v[F::K];
 #pragma unroll
@@ -521,7 +521,7 @@ __global__ void __cluster_dims__(F::C, 1, 1) __launch_bounds__(F::nth + 32, 1)
                     make_longlong2((i64)((u64)(unsigned)lv[0] | (u64)(unsigned)lv[1] << 32),
                                    (i64)((u64)(unsigned)lv[2] | (u64)(unsigned)(vexp - 2 * scale) << 32)));
       }
-      for (int e = mine; e >= 0; e = e < kLineSnap ? next[e] : -1) {
+      for (int e = mine; e >= 0; e = next[e]) {
         const int i = (int)S.snap_idx[e];
         longlong2 x = make_longlong2(0, 0);
 #pragma unroll
