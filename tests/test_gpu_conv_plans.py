@@ -30,3 +30,37 @@ def test_long_convolution_steps_match_oracle(n, gauge):
     rho = np.abs(opsi) ** 2 * 0.3 ** 2
     np.testing.assert_allclose(got[-1, :2], [rho.sum(), (V * rho).sum()], rtol=2 * tol, atol=0)
     np.testing.assert_allclose(got[:, 2:], ref[:, 2:], rtol=0, atol=1e-12 * np.abs(ref[:, 2:]).max())
+
+
+@pytest.mark.parametrize("dim,n", [(1, 3), (1, 96), (1, 1021), (1, 1536), (2, 65), (2, 100), (2, 320), (3, 21), (3, 24)])
+def test_imaginary_time_with_a_length_gauge_field(dim, n):
+    """The x.E factors are real there and change |psi|: the halves do not merge.  Lines and
+    passes of built and other lengths, Normalize, E_kin every third step."""
+    import qsf_gb300 as Q
+    from oracle import oracle as O
+    from qsf_gb300.propagator import coupling_schedule
+    from tests.test_gpu_at_size import _noise_state
+    steps, dt, axis = 7, 0.01, {1: 1, 2: 3, 3: 7}[dim]
+    psi0 = _noise_state(dim, n, 0.3, n)
+    pulse = dict(field=0.3, omega=1.1, ncycles=1.0)
+    og = O.Grid(dim, n, 0.3, nCAP=max(1, n // 10), pot=O.POT_EBERLY, Ncharge=float(dim),
+                coupling=O.Coupling(O.GAUGE_LENGTH, [O.Field(axis, [O.Pulse(**pulse)])]))
+    og.psi[...] = psi0
+    prop = O.Propagator(O.MODE_IM, dt, steps, og, ["norm", "normalize", "epot", "ekin"])
+    for _ in range(steps):
+        prop.make_step()
+        prop.compute_each()
+    g = Q.Grid(dim, n, 0.3, nCAP=max(1, n // 10), Ncharge=float(dim), gauge=Q.GAUGE_LENGTH, n_fields=1)
+    g.upload(psi0)
+    rows = coupling_schedule(Q.Coupling(Q.GAUGE_LENGTH, [Q.Field(axis, [Q.Pulse(**pulse)])]), dt, steps)[0]
+    out, done = g.step(Q.MODE_IM, dt, steps, rows, obs=Q.OBS_NORM | Q.OBS_EPOT | Q.OBS_EKIN, normalize=True, ekin_interval=3)
+    assert done == steps
+    # sqrt(n): the oracle's direct DFT passes of a large prime factor add up to n terms
+    tol = steps * (2 * dim * math.log2(n) + 10) * 2.2e-16 * math.sqrt(n)
+    assert C.rel_l2(g.download(), og.psi) < tol
+    for s, r in enumerate(prop.rows):
+        assert out[s, 0] == pytest.approx(r["norm"], rel=4 * tol)
+        assert out[s, 1] / out[s, 0] == pytest.approx(r["epot"], rel=4 * tol)
+        if (s + 1) % 3 == 0 or s + 1 == steps:
+            assert out[s, 2] / out[s, 0] == pytest.approx(r["ekin"], rel=8 * tol)
+    g.close()
