@@ -47,7 +47,7 @@ int device_sm_count() {
 
 namespace {
 
-// the compile-time radix plan of qsf_fft.cuh, for reporting
+// the compile-time radix plan of qsf_fft.cuh (the plain row transforms'), for reporting
 bool plan_radices(int64_t n, std::vector<int>& r) {
   r.clear();
   if (n < 2 || n > (1 << 24) || !is_smooth((int)n)) return false;
@@ -58,7 +58,7 @@ bool plan_radices(int64_t n, std::vector<int>& r) {
 std::vector<KernelSet>& kernel_table();
 
 // kernel launch geometry
-constexpr int kMaxLine1D = 16384;       // 1D line in shared memory (one CTA up to 8192, a cluster pair above)
+constexpr int kMaxLine1D = 16384;       // points of a 1D line (a cluster of up to 8 CTAs holds it)
 constexpr int kMaxFluxBlocks = 512;  // blocks of the flux-term sums (256 terms each)
 constexpr int kTableSteps = 16;         // sub-steps whose tables are made at once, and steps per captured graph
 constexpr int kMaxAxis = 4096;          // points per axis in 2D and 3D
@@ -697,7 +697,6 @@ int prepare_step(qsf_grid* g, const qsf_step_desc* d, StepDev* out, int* ncol_ou
   S.texp = g->ibuf;
   S.gmin = g->blk->gmin;
   S.sc = g->ibuf + kTableSteps * kTexp;
-  S.tsteps = kTableSteps;
   S.scmax = g->scmax;
   S.nmax = g->nmax;
   S.partials = g->partials;
@@ -1033,7 +1032,7 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
   const KernelSet* ks = kernels_for((int)d->n[0]);
   if (!ks && !(d->dim == 1 ? line_conv_length((int)d->n[0]) : bs_size((int)d->n[0], d->dim)))
     return fail(QSF_EINVAL, "grid size " + std::to_string(d->n[0]) + " has no kernels and no Bluestein length in "
-                            "this build (1D lines up to 8192 points, other grids up to 2048 points per axis)");
+                            "this build (1D lines up to 16384 points, other grids up to 2048 points per axis)");
   qsf_grid* g = new qsf_grid();
   g->desc = *d;
   g->ks = ks;
@@ -1140,7 +1139,6 @@ int qsf_grid_create(const qsf_grid_desc* d, void* stream, qsf_grid** out) {
     qsf_grid_destroy(g);
     return rc;
   }
-  g->fpmax = (size_t)kMaxFluxBlocks * kFinCols;
   if ((rc = D == 1 ? line_setup(g) : make_tensor_maps(g)) || (D > 1 && !ks && (rc = bs_setup(g)))) {
     qsf_grid_destroy(g);
     return rc;

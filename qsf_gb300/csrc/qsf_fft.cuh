@@ -1,5 +1,5 @@
 // qsf_fft.cuh -- FP64 complex helpers and the radix factorisation of a built length, as
-// qsf_fft_plan_radices reports it.
+// the plain row transforms take it and qsf_fft_plan_radices reports it.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

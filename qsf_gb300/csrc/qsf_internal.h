@@ -115,7 +115,6 @@ struct qsf_grid {
   double* partials = nullptr;
   int pmax = 0;
   double* fpartials = nullptr;
-  size_t fpmax = 0;
   long long* ctl = nullptr;
   double* energy = nullptr;
   double* scale = nullptr;

@@ -5,9 +5,10 @@
 // over the wavefunction, ending with psi back in X space:
 //
 //   k_tables      per-step per-axis phase tables (A(t) / E(t) change every step)
-//   k_row_open    [pending Normalize scale] . X half-phase . forward FFT (last axis)
+//   k_row_open    X half-phase . forward FFT (last axis)
 //   k_axis  (3D)  forward FFT axis 1
-//   k_axis        forward FFT axis 0 . P phase . inverse FFT axis 0 (1/m folded in)
+//   k_axis        forward FFT axis 0 . P phase (with 1/m and Normalize's power of two) .
+//                 inverse FFT axis 0
 //   k_axis  (3D)  inverse FFT axis 1
 //   k_row_close   inverse FFT (last axis) . X half-phase . norm / E_pot partials,
 //                 flux snapshot . [next step's X half-phase . forward FFT (last axis)]
@@ -118,16 +119,15 @@ struct StepDev {
   // phase tables in the split form (split62: 2^62 fixed point as signed 32-bit halves)
   const int4* xs;          // static X half-step factor per point (dt/2, incl. absorber), * 2^-xs_exp
   const long long* Vx;     // potential per point in 2^vshift fixed point
-  // tables of the sub-steps ctl[7] .. ctl[7] + tsteps - 1 (k_tables), one after another
-  int4* ptab;              // [tsteps][dim][nmax] P-phase tables (|.| <= 1)
-  int4* xdyn;              // [tsteps][3][dim][nmax] length-gauge factors: open half, close half, close . next open half
-  int tsteps;
+  // tables of the sub-steps from ctl[7] on (k_tables), one after another
+  int4* ptab;              // [sub-step][dim][nmax] P-phase tables (|.| <= 1)
+  int4* xdyn;              // [sub-step][3][dim][nmax] length-gauge factors: open half, close half, close . next open half
   int lg;                  // 2D / 3D: the X halves carry length-gauge factors (a field couples x.E)
   int xs_exp;              // exponent taken out of xs (imaginary time: factors above 1)
   int vshift;              // Vx = round(V * 2^vshift)
   int l2m;                 // 1/m = m_mant * 2^-l2m, m_mant in (0.5, 1] (folded into axis 0's P table)
   double m_mant;
-  int* texp;               // [tsteps][kTexp] exponents taken out of the per-step tables (set by k_tables)
+  int* texp;               // [sub-step][kTexp] exponents taken out of the per-step tables (set by k_tables)
   int* gmin;               // [kGmin] minimum line exponent of each fixed-point pass (gmin_slot)
   int* sc;                 // [4][scmax] line exponents of each fixed-point pass (qsf_passes.cuh)
   int scmax;
@@ -1053,9 +1053,9 @@ const KernelSet* kernels_for(int n);
 #include "qsf_line1d.cuh"
 namespace qsf {
 
-// sizes up to 4096 get the multi-dimensional passes, up to 8192 the plain row transform
-// (longer lines are 1D: LineKernels::fft);
-// the 1D steps have kernels of their own (LineKernels)
+// sizes up to 4096 get the multi-dimensional passes, up to 8192 the plain row transform;
+// longer lines are 1D and only have their place in the list of built lengths here: the 1D
+// steps, and the transforms of the longer lines, have kernels of their own (LineKernels)
 template <int N>
 KernelSet make_kernel_set() {
   static_assert(is_smooth(N), "grid sizes must be 2^a 3^b 5^c");

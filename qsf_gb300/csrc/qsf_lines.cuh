@@ -43,7 +43,12 @@ __host__ __device__ constexpr int tile_size(int) { return QSF_TILE; }
 __host__ __device__ constexpr int tile_size(int n) { return tuned_tile(n); }
 #endif
 __host__ __device__ constexpr int tuned_ppt(int n) { return tile_size(n) / row_threads(n); }
-// points per thread of the strided-axis passes
+// Points per thread of the strided-axis passes (candidate builds force one with QSF_COL_PPT):
+// 16 from 1024 points on, where the lines fill the SMs, and at 256, where cubes gain what
+// planes run alone lose; 128 goes with 256.  ms a step with 8 / 16 points, 2D: 64 0.0275 /
+// 0.0300, 128 0.0289 / 0.0333, 256 0.0282 / 0.0336, 512 0.0312 / 0.0411, 768 0.0570 / 0.0634,
+// 1024 0.0810 / 0.0742, 1280 0.173 / 0.164, 2048 0.329 / 0.294, 4096 1.333 / 1.164; 3D: 64
+// 0.0489 / 0.0579, 128 0.206 / 0.210, 256 1.386 / 1.189.
 #ifdef QSF_COL_PPT
 __host__ __device__ constexpr int axis_ppt(int) { return QSF_COL_PPT; }
 #else
@@ -58,7 +63,7 @@ __host__ __device__ constexpr int axis_ppt(int n) { return n == 128 || n == 256 
 struct LinePlan {
   int E, S, r[4];
 };
-constexpr int kEight = 1, kFour = 2;  // plan selectors: 8 or 4 points per thread at every length they list
+constexpr int kEight = 1, kFour = 2;  // plan selectors: the factors of 1D lines (qsf_line1d.cuh), 8 or 4 points per thread
 __host__ __device__ constexpr LinePlan line_plan(int n, int ppt) {
   if (ppt == kFour) {
     switch (n) {
@@ -76,16 +81,8 @@ __host__ __device__ constexpr LinePlan line_plan(int n, int ppt) {
       default: return {0, 0, {1, 1, 1, 1}};
     }
   }
-  if (ppt == kEight) {  // the factors of a 1D line spread over a cluster (qsf_line1d.cuh)
+  if (ppt == kEight) {
     switch (n) {
-      case 16: return {8, 2, {8, 2, 1, 1}};
-      case 24: return {8, 3, {4, 3, 2, 1}};
-      case 32: return {8, 2, {8, 4, 1, 1}};
-      case 40: return {8, 3, {4, 5, 2, 1}};
-      case 48: return {8, 3, {8, 3, 2, 1}};
-      case 64: return {8, 2, {8, 8, 1, 1}};
-      case 80: return {8, 3, {8, 5, 2, 1}};
-      case 96: return {8, 3, {8, 3, 4, 1}};
       case 128: return {8, 3, {8, 2, 8, 1}};
       case 160: return {8, 3, {8, 5, 4, 1}};
       case 192: return {8, 3, {8, 3, 8, 1}};
@@ -122,10 +119,6 @@ __host__ __device__ constexpr LinePlan line_plan(int n, int ppt) {
     case 2560: return w ? LinePlan{16, 3, {16, 10, 16, 1}} : LinePlan{8, 4, {8, 5, 8, 8}};
     case 3072: return w ? LinePlan{16, 4, {16, 3, 4, 16}} : LinePlan{8, 4, {8, 6, 8, 8}};
     case 4096: return w ? LinePlan{16, 3, {16, 16, 16, 1}} : LinePlan{8, 4, {8, 8, 8, 8}};
-    // one row of a 1D line
-    case 5120: return {16, 4, {16, 5, 4, 16}};
-    case 6144: return {16, 4, {16, 6, 4, 16}};
-    case 8192: return {16, 4, {16, 16, 2, 16}};
     default: return {0, 0, {1, 1, 1, 1}};
   }
 }
@@ -194,10 +187,10 @@ struct Ln {
   static constexpr int kColBytes = C * N * 16 > buf_bytes(kColThreads) ? C * N * 16 : buf_bytes(kColThreads);
   static constexpr int kRowSmem = buf_bytes(kRowThreads) + 256;
   static constexpr int kColSmem = (kColBytes + 127) / 128 * 128 + 256 + 128;
-  // resident blocks per SM the kernels are compiled for: 128 registers a thread for 12
-  // and more points, 112 for 8 (rows of 256^3: 597, 568, 550, 545 us with 64, 80, 96, 112
-  // registers, the wider ones without spills; 144 and more with 16 points lose a quarter of
-  // the warps and 29 % at 2048^2)
+  // resident blocks per SM the kernels are compiled for: those of 128 registers a thread for
+  // 12 and more points, of 112 for 8 (rows of 256^3: 597, 568, 550, 545 us with bounds of 64,
+  // 80, 96, 112 registers, the wider ones without spills; the compiler needs 96 of the 112.
+  // 144 and more with 16 points lose a quarter of the warps and 29 % at 2048^2)
   __host__ __device__ static constexpr int blocks(int nth) {
     constexpr int regs = E > 8 ? 128 : 112;
     return 65536 / (regs * nth) > 32 ? 32 : 65536 / (regs * nth) < 1 ? 1 : 65536 / (regs * nth);

@@ -302,8 +302,7 @@ __device__ __forceinline__ bool row_snapshot(const GridDev& g, const StepDev& S,
 }
 
 // ------------------------------------------------------------ row passes
-// Open: psi (double) . [Normalize] . X half . forward transform of the last axis ->
-// fixed point (pass 0).
+// Open: psi (double) . X half . forward transform of the last axis -> fixed point (pass 0).
 template <class G, bool BS = false>
 __global__ void __launch_bounds__(G::kRowThreads, G::blocks(G::kRowThreads))
     k_row_open(const GridDev* __restrict__ Gs, const StepDev* __restrict__ Ss) {

@@ -1,4 +1,4 @@
-// Kernel instantiations for 1D lines above 8192 points, held by a cluster pair of CTAs.
+// Built lengths above 8192 points: 1D lines, whose kernels are those of qsf_lines_*.cu.
 #include <vector>
 #include "qsf_kernels.cuh"
 namespace qsf {
