@@ -586,9 +586,12 @@ def run_c1(steps, warmup, flush):
                             box, flush)
     value = n * 1000.0 / ms
     return {"value": value, "unit": UNIT, "ms_per_step": ms, "steps": steps,
-            "roofline": _roofline(32, n, steps, prof, "1D: the line is held on chip for the whole step (one "
-                                  "pass, 32 B per point-step); latency-bound on one SM, not HBM-bound"),
+            "roofline": _roofline(32, n, steps, {max(prof, key=lambda k: prof[k][0]): (ms * steps, steps)},
+                                  "1D: the line is held on chip over the steps of a launch (32 B per point-step "
+                                  "counted); latency-bound on a cluster of 8 SMs, not HBM-bound; a step's time in the "
+                                  "timed call, which makes up to 256 steps a launch"),
             "kernels_ms_per_step": {k: v[0] / steps for k, v in prof.items()},
+            "kernels_note": "from the profiled call, which makes one step a launch",
             "job_s": job_s, "job_steps": 2000 + len(rows) - 1,
             "yield_1_minus_norm": 1.0 - rows[-1]["norm"],
             "workload": "1D plain: 4096 points, dx 0.2, soft-core H (e-n charge 1, eps 1), IM ground state "
