@@ -101,8 +101,12 @@ __global__ void __launch_bounds__(1024) k_bs_split(const double2* __restrict__ b
   int e;
   frexp(mx * one, &e);
   if (threadIdx.x == 0) *bexp = e;
-  const double sc = ldexp(one, -e);
-  for (int j = threadIdx.x; j < M; j += blockDim.x) out[j] = split62(make_double2(b[j].x * sc, b[j].y * sc));
+  // 1 / M in two parts: the rounding of one would be the same at every step
+  const double hi = ldexp(one, -e), lo = ldexp(fma(-one, (double)M, 1.0) / (double)M, -e);
+  for (int j = threadIdx.x; j < M; j += blockDim.x) {
+    const double2 v = b[j];
+    out[j] = split62(make_double2(fma(v.x, hi, v.x * lo), fma(v.y, hi, v.y * lo)));
+  }
 }
 
 int blocks_for(long long count) {

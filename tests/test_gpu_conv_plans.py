@@ -64,3 +64,24 @@ def test_imaginary_time_with_a_length_gauge_field(dim, n):
         if (s + 1) % 3 == 0 or s + 1 == steps:
             assert out[s, 2] / out[s, 0] == pytest.approx(r["ekin"], rel=8 * tol)
     g.close()
+
+
+@pytest.mark.parametrize("dim,n,steps", [(1, 700, 2000), (1, 5003, 2000), (1, 9001, 1500), (2, 260, 300), (2, 371, 200)])
+def test_norm_of_a_long_run(dim, n, steps):
+    """Convolution plans of 3 2^k and 5 2^k points, whose 1 / M no double holds: its rounding
+    must not add up over the steps.  Without an absorber the norm changes by what the tables
+    hold: 1 / m rounded to a double, known exactly, and the moduli of the phase factors, whose
+    roundings average over the points: together within 2^-53 of that a step."""
+    from fractions import Fraction
+
+    import qsf_gb300 as Q
+    from tests.test_gpu_at_size import _noise_state
+    g = Q.Grid(dim, n, 0.2, nCAP=0, Ncharge=float(dim))
+    g.upload(_noise_state(dim, n, 0.2, n, width=0.1))
+    g.normalize()
+    rows, _ = g.step(Q.MODE_RE, 0.05, steps, obs=Q.OBS_NORM)
+    g.close()
+    m = n ** dim
+    one = 1 << (m.bit_length() - 1)
+    known = 2.0 * float(Fraction(one / m) * m / one - 1)
+    assert abs((rows[-1, 0] - rows[0, 0]) / (steps - 1) - known) < 2.0 ** -53
