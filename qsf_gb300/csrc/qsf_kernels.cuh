@@ -621,10 +621,8 @@ __global__ void __launch_bounds__(256) k_finalize(const GridDev* __restrict__ Gs
   if (!step_end) {
     // only the counters move, and only when every block has read them: a block that starts
     // late would take the next sub-step for its own
-    if (nblk > 1) {
-      __syncthreads();  // this block's threads have
-      __threadfence();
-    }
+    __syncthreads();  // this block's threads have
+    if (nblk > 1) __threadfence();
     if (tid == 0 && (nblk == 1 || atomicAdd((unsigned long long*)&S.ctl[3], 1ull) == (unsigned long long)nblk - 1)) {
       S.scale[scale_slot(sub)] = 0.0;
       S.ctl[3] = 0;
