@@ -91,7 +91,7 @@ __global__ void k_bs_chirp(double2* __restrict__ chirp, double2* __restrict__ w,
 __global__ void __launch_bounds__(1024) k_bs_split(const double2* __restrict__ b, int4* __restrict__ out, int* bexp, int M) {
   __shared__ double red[32];
   double mx = 0.0;
-  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, hypot(b[j].x, b[j].y));
+  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, fma(b[j].x, b[j].x, b[j].y * b[j].y));
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(1024) k_bs_split(const double2* __restrict__ b
   for (int w = 0; w < 32; ++w) mx = fmax(mx, red[w]);
   const double one = 1.0 / (double)M;
   int e;
-  frexp(mx * one, &e);
+  frexp(sqrt(mx) * one, &e);
   if (threadIdx.x == 0) *bexp = e;
   // 1 / M in two parts: the rounding of one would be the same at every step
   const double hi = ldexp(one, -e), lo = ldexp(fma(-one, (double)M, 1.0) / (double)M, -e);

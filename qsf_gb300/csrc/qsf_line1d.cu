@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(1024) k_line_bhat(const double2* __restrict__ 
                                                     int n1, int n2) {
   __shared__ double red[32];
   double mx = 0.0;
-  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, hypot(b[j].x, b[j].y));
+  for (int j = threadIdx.x; j < M; j += blockDim.x) mx = fmax(mx, fma(b[j].x, b[j].x, b[j].y * b[j].y));
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(1024) k_line_bhat(const double2* __restrict__ 
   for (int w = 0; w < 32; ++w) mx = fmax(mx, red[w]);
   const double one = 1.0 / (double)M;
   int e;
-  frexp(mx * one, &e);
+  frexp(sqrt(mx) * one, &e);
   if (threadIdx.x == 0) *bexp = e;
   // 1 / M in two parts: the rounding of one would be the same at every step (5003 points, M =
   // 10240: the norm grew by 1.9e-16 a step)
