@@ -337,9 +337,18 @@ int ensure_static(qsf_grid* g, int mode, double delta) {
     g->vshift = 50 - e;
   }
   g->xs_exp = 0;
-  if (mode == QSF_MODE_IM && g->vneg > 0.0) {
-    const double fmax = std::exp(delta * g->vneg);
-    if (!std::isfinite(fmax)) return fail(QSF_EINVAL, "imaginary-time X factor overflows (dt * |V| too large)");
+  // the largest factor: exp(-delta V) in imaginary time, times the absorber's, which is above
+  // 1 when time runs backwards (all of it at the corner nodes)
+  double lmax = mode != QSF_MODE_IM ? 0.0 : delta > 0.0 ? delta * g->vneg : -delta * g->vmax;
+  const GridDev& G = g->G;
+  if (delta < 0.0 && G.nCAP > 0 && !G.multi) {
+    const double c = (double)G.nCAP;
+    lmax += G.dim * (G.abs_kind == QSF_ABS_COS8 ? delta * G.abs_rate * 0.125 * std::log(std::cos(1.5707963267948966))
+                                                : -delta * (c * c) * (c * c) * G.eta);
+  }
+  if (lmax > 0.0) {
+    const double fmax = std::exp(lmax);
+    if (!std::isfinite(fmax)) return fail(QSF_EINVAL, "X factor overflows (|dt| times the potential or absorber too large)");
     if (fmax > 1.0) std::frexp(fmax, &g->xs_exp);
   }
   k_build_static<<<grid_blocks(m), 256, 0, g->stream>>>(g->G, mode, delta, g->xs_exp, reinterpret_cast<int4*>(g->xs),

@@ -123,7 +123,7 @@ struct StepDev {
   int4* ptab;              // [sub-step][dim][nmax] P-phase tables (|.| <= 1)
   int4* xdyn;              // [sub-step][3][dim][nmax] length-gauge factors: open half, close half, close . next open half
   int lg;                  // 2D / 3D: the X halves carry length-gauge factors (a field couples x.E)
-  int xs_exp;              // exponent taken out of xs (imaginary time: factors above 1)
+  int xs_exp;              // exponent taken out of xs (factors above 1: imaginary time, absorbers backwards in time)
   int vshift;              // Vx = round(V * 2^vshift)
   int l2m;                 // 1/m = m_mant * 2^-l2m, m_mant in (0.5, 1] (folded into axis 0's P table)
   double m_mant;
