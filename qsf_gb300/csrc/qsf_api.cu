@@ -346,7 +346,7 @@ int ensure_static(qsf_grid* g, int mode, double delta) {
     lmax += G.dim * (G.abs_kind == QSF_ABS_COS8 ? delta * G.abs_rate * 0.125 * std::log(std::cos(1.5707963267948966))
                                                 : -delta * (c * c) * (c * c) * G.eta);
   }
-  if (lmax > 0.0) {
+  if (!(lmax <= 0.0)) {
     const double fmax = std::exp(lmax);
     if (!std::isfinite(fmax)) return fail(QSF_EINVAL, "X factor overflows (|dt| times the potential or absorber too large)");
     if (fmax > 1.0) std::frexp(fmax, &g->xs_exp);

@@ -39,3 +39,20 @@ def test_backwards_steps_match_oracle(dim, n, absorber):
     for s, r in enumerate(prop.rows):
         np.testing.assert_allclose(out[s, :2], [r["norm"], r["epot"]], rtol=4 * tol, atol=0)
     g.close()
+
+
+@pytest.mark.parametrize("dim,n", [(1, 96), (1, 777), (2, 64), (2, 100), (3, 20)])
+def test_time_steps_without_a_finite_factor_are_refused(dim, n):
+    """A dt that is not a number, or whose imaginary-time factors no double holds, is an invalid
+    argument, and the grid can be used afterwards."""
+    import qsf_gb300 as Q
+    g = Q.Grid(dim, n, 0.3, nCAP=2)
+    for dt in (float("nan"), 1e6, -1e9):
+        g.add_gaussian()
+        with pytest.raises(Q.QsfError) as e:
+            g.step(Q.MODE_IM, dt, 2)
+        assert e.value.code == 1
+    g.normalize()
+    rows, done = g.step(Q.MODE_IM, 0.01, 2, normalize=True)
+    assert done == 2 and np.isfinite(rows).all()
+    g.close()
